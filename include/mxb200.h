@@ -99,6 +99,14 @@ MXB200_API int mxb200_quantize_mx_relu_square_bwd(const void* g, const void* h, 
 MXB200_API int mxb200_softcap_ce_loss(const void* logits, int64_t rows, int64_t ld, const int64_t* targets, int vocab,
                                       int padded, float softcap, float* loss, float* lse, void* stream);
 
+/* The reductions around the chunked loss, one launch each (the reference uses torch ops there, ops/softcap_ce.cpp:139-160).
+ * count_valid: *out = how many of targets[0, n) are >= 0. reduce_losses: *out = sum of losses[0, n), in a fixed order,
+ * divided by *num_valid when that is not null. scale_bf16: y = bf16(x * bf16(*scale)) over n values (n % 8 == 0; the
+ * saved gradient times the incoming one); y may alias x. All pointers are on the device. */
+MXB200_API int mxb200_count_valid(const int64_t* targets, int64_t n, int64_t* out, void* stream);
+MXB200_API int mxb200_reduce_losses(const float* losses, int64_t n, const int64_t* num_valid, float* out, void* stream);
+MXB200_API int mxb200_scale_bf16(const void* x, const float* scale, void* y, int64_t n, void* stream);
+
 /* Replaces nanochat::kernels::softcap_ce_grad_mx (softcap_ce_kernel.h:24-29; kernel nanochat_softcap_ce_grad_mx,
  * softcap_ce_kernel.cu:118-176): the loss's gradient with respect to the logits, as the bf16 the reference's grad
  * kernel would write, g = bf16((softmax(capped) - onehot(target)) * (1 - tanh^2) * scale), MX-quantized in both

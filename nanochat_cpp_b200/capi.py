@@ -23,6 +23,7 @@ SYMBOLS = (
     "mxb200_quantize_mx", "mxb200_quantize_mx_batch", "mxb200_quantize_mx_relu_square_bwd", "mxb200_gemm_bf16", "mxb200_gemm_f32",
     "mxb200_gemm_relu_square", "mxb200_gemm_relu_square_bwd", "mxb200_residual_norm_mx_fwd",
     "mxb200_softcap_ce_loss", "mxb200_softcap_ce_grad_mx",
+    "mxb200_count_valid", "mxb200_reduce_losses", "mxb200_scale_bf16",
     "mxb200_gemm_splits", "mxb200_gemm_workspace_bytes", "mxb200_gemm_splitk", "mxb200_gemm_splitk_static",
     "mxb200_strerror",
     "mxb200_device_status", "mxb200_selftest_bounded_wait", "mxb200_set_gemm_config", "mxb200_launch_count", "mxb200_version",
@@ -72,6 +73,9 @@ def _load() -> ctypes.CDLL:
     f32 = ctypes.c_float
     lib.mxb200_softcap_ce_loss.argtypes = [vp, i64, i64, vp, i32, i32, f32, vp, vp, vp]
     lib.mxb200_softcap_ce_grad_mx.argtypes = [vp, i64, i64, vp, vp, i32, i32, f32, vp, i64, vp, MxOut, MxOut, i32, vp]
+    lib.mxb200_count_valid.argtypes = [vp, i64, vp, vp]
+    lib.mxb200_reduce_losses.argtypes = [vp, i64, vp, vp, vp]
+    lib.mxb200_scale_bf16.argtypes = [vp, vp, vp, i64, vp]
     lib.mxb200_gemm_splits.argtypes = [i64, i64, i64]
     lib.mxb200_gemm_workspace_bytes.argtypes = [i64, i64, i64, i32]
     lib.mxb200_gemm_workspace_bytes.restype = ctypes.c_size_t

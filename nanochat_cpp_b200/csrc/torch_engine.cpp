@@ -1,0 +1,992 @@
+// Native host path of the engine's public entry points: argument checks, buffers, launch order and the autograd nodes of
+// the MX Linears, as a Python extension over libmxb200's C ABI. Mirrors the reference's C++ host code
+// (src/nanochat/model/fp8/fp8.cpp:113-171, 240-338, 424-571; ops/softcap_ce.cpp:27-205; ops/residual_norm.cpp:33-96).
+//
+// Why native: every launch of a small Linear takes 3 to 15 us on the device, while a Python autograd function with a
+// ctypes call and a handful of tensor objects per launch cost the host 30 to 50 us each, so every shape up to a few
+// thousand tokens was bound by the host (fp8_matmul of 2048 x 768 -> 3072, forward and backward: 59 us of kernels in a
+// 250 us pass). Here a call costs a few allocations from torch's caching allocator and the launches. Tensors that
+// nobody outside sees (quantized operands) are one byte buffer per lifetime, data then scales.
+#include <mutex>
+#include <optional>
+#include <stdexcept>
+#include <unordered_map>
+#include <utility>
+#include <vector>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include "mxb200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+constexpr auto kE4M3 = at::kFloat8_e4m3fn;
+constexpr auto kE8M0 = at::kFloat8_e8m0fnu;
+
+// ---------------------------------------------------------------------------------------------------- plumbing
+
+struct StatusError : std::runtime_error {
+  int status;
+  std::string what_failed;
+  StatusError(int s, const char* w)
+      : std::runtime_error(std::string(w) + ": " + mxb200_strerror(s) + " (status " + std::to_string(s) + ")"),
+        status(s),
+        what_failed(w) {}
+};
+
+inline void check(int status, const char* what) {
+  if (status != MXB200_OK)
+    throw StatusError(status, what);
+}
+
+[[noreturn]] void fail(const char* message) {
+  throw std::runtime_error(message);
+}
+
+inline void require(bool ok, const char* message) {
+  if (!ok)
+    fail(message);
+}
+
+inline void require_cuda(const Tensor& t, const char* what) {
+  if (!t.is_cuda())
+    throw std::runtime_error(std::string(what) + ": expected a CUDA tensor; this engine has no CPU path");
+}
+
+inline void* stream() {
+  return c10::cuda::getCurrentCUDAStream().stream();
+}
+
+inline Tensor empty(at::IntArrayRef size, at::ScalarType dtype, at::Device device) {
+  return at::detail::empty_cuda(size, dtype, device, std::nullopt);
+}
+
+inline bool fits(int64_t rows, int64_t cols) {
+  return rows % 128 == 0 && cols % 128 == 0;
+}
+
+// One layout of a quantized (R, C) tensor by address: data row-major, then its scales.
+struct Layout {
+  void* data = nullptr;
+  void* scale = nullptr;
+};
+
+constexpr int64_t mx_bytes(int64_t R, int64_t C) {
+  return R * C + R * C / 32;
+}
+
+// An (R, C) layout in one byte buffer; R * C is a multiple of 16384, so the scales start aligned.
+inline Tensor layout_buffer(int64_t R, int64_t C, at::Device device) {
+  return empty({mx_bytes(R, C)}, at::kByte, device);
+}
+
+inline Layout layout_of(const Tensor& buffer, int64_t R, int64_t C) {
+  auto* p = static_cast<unsigned char*>(buffer.data_ptr());
+  return {p, p + R * C};
+}
+
+inline Layout layout_of(const Tensor& data, const Tensor& scale) {
+  return {data.data_ptr(), scale.data_ptr()};
+}
+
+// The kernels' view of a layout whose rows have `ld` values, from (row, col) on; both multiples of 128.
+inline mxb200_mx_out view(const Layout& l, int64_t ld, int64_t row = 0, int64_t col = 0) {
+  const int64_t tiles = ld / 128;
+  return {static_cast<unsigned char*>(l.data) + row * ld + col, ld,
+          static_cast<unsigned char*>(l.scale) + (row / 128 * tiles + col / 128) * 512, tiles};
+}
+
+constexpr mxb200_mx_out kNoLayout{nullptr, 0, nullptr, 0};
+
+// The four tensors of a quantized matrix as Python sees them.
+struct Mx {
+  Tensor data, data_t, scale, scale_t;
+  Layout rows() const { return layout_of(data, scale); }
+  Layout cols() const { return layout_of(data_t, scale_t); }
+};
+
+Mx empty_mx(int64_t R, int64_t C, at::Device device, bool rows = true, bool cols = true) {
+  Mx q;
+  if (rows)
+    q.data = empty({R, C}, kE4M3, device), q.scale = empty({R * C / 32}, kE8M0, device);
+  if (cols)
+    q.data_t = empty({C, R}, kE4M3, device), q.scale_t = empty({R * C / 32}, kE8M0, device);
+  return q;
+}
+
+void check_quantizable(const Tensor& x) {
+  require_cuda(x, "quantize_mx");
+  require(x.dim() == 2 && x.is_contiguous() && fits(x.size(0), x.size(1)) &&
+                (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kFloat),
+          "MX: expected an aligned, contiguous 2D tensor with dims % 128");
+}
+
+void quantize(const Tensor& x, const mxb200_mx_out& out, const mxb200_mx_out& out_t) {
+  check_quantizable(x);
+  check(mxb200_quantize_mx(x.data_ptr(), x.scalar_type() == at::kBFloat16, x.size(0), x.size(1), out, out_t,
+                           MXB200_PROLOGUE_NONE, MXB200_SCALE_REFERENCE, stream()),
+        "quantize_mx");
+}
+
+// Split-K scratch, grown on demand and kept per (device, stream): GEMMs on different streams may overlap and must not
+// share partial tiles; launches on one stream are ordered and reuse theirs (the reference borrows torch's per-stream
+// cuBLAS workspace, mx_gemm.cpp:236-237). A replaced buffer goes back to the caching allocator, which keeps it for the
+// stream it was allocated on until that stream's queued work has run.
+Tensor workspace(at::Device device, size_t bytes) {
+  static std::mutex mu;
+  static auto* buffers = new std::unordered_map<uint64_t, Tensor>();  // never destroyed: outlives the CUDA context
+  const auto s = c10::cuda::getCurrentCUDAStream(device.index());
+  const uint64_t key = (static_cast<uint64_t>(device.index()) << 48) ^ reinterpret_cast<uint64_t>(s.stream());
+  std::lock_guard<std::mutex> lock(mu);
+  Tensor& t = (*buffers)[key];
+  if (!t.defined() || static_cast<size_t>(t.numel()) < bytes)
+    t = empty({static_cast<int64_t>(std::max<size_t>(bytes, size_t(1) << 20))}, at::kByte, device);
+  return t;
+}
+
+// d (M, N) = a (M, K) . b (N, K)^T, bf16 or fp32 (alpha, +=), split along K where the library says so.
+void gemm(void* d, bool f32, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device,
+          const float* alpha = nullptr, bool accumulate = false) {
+  const int splits = mxb200_gemm_splits(M, N, K);
+  if (splits > 1) {
+    const Tensor ws = workspace(device, mxb200_gemm_workspace_bytes(M, N, K, splits));
+    check(mxb200_gemm_splitk(a.data, a.scale, b.data, b.scale, d, f32 ? MXB200_OUT_F32 : MXB200_OUT_BF16, nullptr, M, N,
+                             K, alpha, accumulate, splits, ws.data_ptr(), ws.numel(), stream()),
+          f32 ? "mx_gemm_f32" : "mx_gemm");
+  } else if (f32) {
+    check(mxb200_gemm_f32(a.data, a.scale, b.data, b.scale, static_cast<float*>(d), M, N, K, alpha, accumulate, stream()),
+          "mx_gemm_f32");
+  } else {
+    check(mxb200_gemm_bf16(a.data, a.scale, b.data, b.scale, d, nullptr, M, N, K, stream()), "mx_gemm");
+  }
+}
+
+Tensor gemm_bf16(const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device) {
+  Tensor d = empty({M, N}, at::kBFloat16, device);
+  gemm(d.data_ptr(), false, a, b, M, N, K, device);
+  return d;
+}
+
+bool grad_direct(const Tensor& w) {  // fp8.h:114-116
+  return w.is_leaf() && w.requires_grad() && w.scalar_type() == at::kFloat && w.is_contiguous();
+}
+
+// dW = alpha * go_t (n, K) . in_t (C, K)^T into the .grad of ws, whose rows concatenate to n: allocated (=) when
+// undefined, else accumulated (+=); several ws whose gradients share one buffer take one GEMM (fp8.cpp:470-514).
+void grad_weights(const Layout& go_t, const Layout& in_t, int64_t n, int64_t C, int64_t K, const std::vector<Tensor>& ws,
+                  const float* alpha, at::Device device) {
+  int64_t total = 0;
+  bool shapes = true, all = true;
+  for (const Tensor& w : ws)
+    total += w.size(0), shapes &= w.size(1) == C, all &= w.grad().defined();
+  require(shapes && total == n, "mx_grad_weights: weight rows must concatenate to the gradient's");
+  if (all) {
+    const Tensor& g0 = ws[0].grad();
+    const char* base = static_cast<const char*>(g0.data_ptr());
+    bool contiguous = true;
+    int64_t row = 0;
+    for (const Tensor& w : ws) {
+      const Tensor& g = w.grad();
+      contiguous &= g.is_contiguous() && g.scalar_type() == at::kFloat && g.data_ptr() == base + row * C * 4;
+      row += w.size(0);
+    }
+    if (contiguous && (ws.size() == 1 || (g0.is_view() && g0._base().numel() == n * C))) {
+      gemm(const_cast<char*>(base), true, go_t, in_t, n, C, K, device, alpha, true);
+      return;
+    }
+  }
+  Tensor buf = empty({n, C}, at::kFloat, device);
+  gemm(buf.data_ptr(), true, go_t, in_t, n, C, K, device, alpha, false);
+  int64_t row = 0;
+  for (const Tensor& w : ws) {
+    // row blocks of one buffer, as the reference's merged q/k/v
+    Tensor part = ws.size() == 1 ? buf : buf.narrow(0, row, w.size(0));
+    if (w.grad().defined())
+      w.mutable_grad().add_(part);
+    else
+      w.mutable_grad() = part;
+    row += w.size(0);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- weight cache
+
+// FP8 copies of weights, remade only when a weight changes: in-place updates bump the tensor's version (fp8.h:18-38,
+// fp8.cpp:516-536). Used with the GIL held only.
+class WeightCache {
+ public:
+  explicit WeightCache(bool on) : enabled(on) {}
+  bool enabled;
+
+  py::object get(int kind, const std::vector<Tensor>& weights, const py::object& make) {
+    if (!enabled)
+      return make();
+    if (!hit(kind, weights)) {
+      py::object made = make();
+      store(kind, weights, made);
+    }
+    return value_;
+  }
+
+  bool hit(int kind, const std::vector<Tensor>& weights) const {
+    if (kind != kind_ || weights.size() != keys_.size())
+      return false;
+    for (size_t i = 0; i < weights.size(); ++i)
+      if (!(keys_[i] == Key(weights[i])))
+        return false;
+    return true;
+  }
+
+  void store(int kind, const std::vector<Tensor>& weights, py::object value) {
+    value_ = std::move(value);
+    kind_ = kind;
+    keys_.clear();
+    for (const Tensor& w : weights)
+      keys_.emplace_back(w);
+  }
+
+  Mx mx() const {
+    const auto t = value_.cast<std::vector<Tensor>>();
+    return {t.at(0), t.at(1), t.at(2), t.at(3)};
+  }
+
+ private:
+  struct Key {
+    const void* impl;
+    const void* data;
+    int64_t version;
+    explicit Key(const Tensor& w)
+        : impl(w.unsafeGetTensorImpl()), data(w.data_ptr()), version(static_cast<int64_t>(w._version())) {}
+    bool operator==(const Key& o) const { return impl == o.impl && data == o.data && version == o.version; }
+  };
+  int kind_ = -1;
+  std::vector<Key> keys_;
+  py::object value_;
+};
+
+// The quantized copy of a (merged) weight: from the cache when it holds it, else to be quantized by the caller, into
+// `keep` when a cache wants it afterwards and into unnamed buffers otherwise.
+struct WeightUse {
+  WeightCache* cache = nullptr;  // null: no caching
+  std::vector<Tensor> weights;
+  Mx mx;        // cached, or freshly made for the cache
+  bool ready = false;
+  Tensor rows_buffer, cols_buffer;  // without a cache
+
+  WeightUse(WeightCache* c, std::vector<Tensor> ws) : weights(std::move(ws)) {
+    if (c != nullptr && c->enabled) {
+      cache = c;
+      if (c->hit(1, weights))
+        mx = c->mx(), ready = true;
+    }
+  }
+
+  int64_t out_features() const {
+    int64_t n = 0;
+    for (const Tensor& w : weights)
+      n += w.size(0);
+    return n;
+  }
+  int64_t in_features() const { return weights[0].size(1); }
+
+  void allocate(at::Device device, bool need_cols) {
+    const int64_t n = out_features(), C = in_features();
+    if (cache != nullptr) {
+      mx = empty_mx(n, C, device);
+    } else {
+      rows_buffer = layout_buffer(n, C, device);
+      if (need_cols)
+        cols_buffer = layout_buffer(C, n, device);
+    }
+  }
+  Layout rows() const {
+    return rows_buffer.defined() ? layout_of(rows_buffer, out_features(), in_features()) : mx.rows();
+  }
+  Layout cols() const {
+    return cols_buffer.defined() ? layout_of(cols_buffer, in_features(), out_features())
+                                 : (mx.data_t.defined() ? mx.cols() : Layout{});
+  }
+  // what backward reads: {buffer} or {data_t, scale_t}
+  void save(variable_list& to) const {
+    if (cols_buffer.defined()) {
+      to.push_back(cols_buffer);
+      to.emplace_back();
+    } else {
+      to.push_back(mx.data_t);
+      to.push_back(mx.scale_t);
+    }
+  }
+  void publish() {
+    if (cache != nullptr && !ready) {
+      py::list l;
+      for (const Tensor& t : {mx.data, mx.data_t, mx.scale, mx.scale_t})
+        l.append(py::cast(t));
+      cache->store(1, weights, l);
+    }
+  }
+};
+
+// A saved layout: one buffer holding data then scales, or a data tensor and a scale tensor.
+inline Layout saved_layout(const Tensor& a, const Tensor& b, int64_t R, int64_t C) {
+  return b.defined() ? layout_of(a, b) : layout_of(a, R, C);
+}
+
+// ---------------------------------------------------------------------------------------------------- quantizer jobs
+
+// Quantizations that do not depend on one another, issued together.
+class QuantizeJobs {
+ public:
+  void add(const Tensor& x, const mxb200_mx_out& out, const mxb200_mx_out& out_t) {
+    check_quantizable(x);
+    jobs_[x.scalar_type() == at::kBFloat16].push_back({x.data_ptr(), x.size(0), x.size(1), out, out_t});
+    hold_.push_back(x);
+  }
+  void add(const Tensor& x, const Layout& rows, const Layout& cols, bool need_cols = true) {
+    add(x, view(rows, x.size(1)), need_cols ? view(cols, x.size(0)) : kNoLayout);
+  }
+  // a weight's parts into their row ranges of one buffer (fp8.cpp:155-171)
+  void add(WeightUse& w, at::Device device, bool need_cols) {
+    if (w.ready)
+      return;
+    w.allocate(device, need_cols);
+    const Layout rows = w.rows(), cols = w.cols();
+    const int64_t n = w.out_features(), C = w.in_features();
+    int64_t row = 0;
+    for (const Tensor& part : w.weights) {
+      const Tensor p = part.detach().contiguous();
+      add(p, view(rows, C, row, 0), cols.data != nullptr ? view(cols, n, 0, row) : kNoLayout);
+      row += part.size(0);
+    }
+  }
+  void run() {
+    for (int bf16 = 0; bf16 < 2; ++bf16) {
+      auto& j = jobs_[bf16];
+      if (j.size() == 1)
+        check(mxb200_quantize_mx(j[0].x, bf16, j[0].rows, j[0].cols, j[0].out, j[0].out_t, MXB200_PROLOGUE_NONE,
+                                 MXB200_SCALE_REFERENCE, stream()),
+              "quantize_mx");
+      else if (!j.empty())
+        check(mxb200_quantize_mx_batch(j.data(), static_cast<int>(j.size()), bf16, MXB200_SCALE_REFERENCE, stream()),
+              "quantize_mx");
+    }
+  }
+
+ private:
+  std::vector<mxb200_quantize_job> jobs_[2];
+  std::vector<Tensor> hold_;
+};
+
+// ---------------------------------------------------------------------------------------------------- Linear
+
+inline bool grad_mode(std::initializer_list<const Tensor*> inputs) {
+  if (!at::GradMode::is_enabled())
+    return false;
+  for (const Tensor* t : inputs)
+    if (t->requires_grad())
+      return true;
+  return false;
+}
+
+// One Linear under MX: y = x . w^T, dX = dY . w, dW = dY^T . x, every operand E4M3 with per-32 scales along the
+// contraction (fp8.cpp:240-260).
+Tensor linear_forward(const Tensor& x, WeightUse& w, bool grad, Tensor* x_cols) {
+  const auto device = x.device();
+  const int64_t N = x.size(0), C = x.size(1), O = w.out_features();
+  const Tensor x_rows = layout_buffer(N, C, device);
+  if (grad)
+    *x_cols = layout_buffer(C, N, device);
+  QuantizeJobs jobs;
+  jobs.add(x, layout_of(x_rows, N, C), grad ? layout_of(*x_cols, C, N) : Layout{}, grad);
+  jobs.add(w, device, grad);
+  jobs.run();
+  w.publish();
+  return gemm_bf16(layout_of(x_rows, N, C), w.rows(), N, O, C, device);
+}
+
+struct Float8Matmul : torch::autograd::Function<Float8Matmul> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, WeightUse* use) {
+    Tensor x_cols;
+    Tensor y = linear_forward(x, *use, true, &x_cols);
+    variable_list saved{x_cols};
+    use->save(saved);
+    ctx->save_for_backward(std::move(saved));
+    ctx->saved_data["w"] = w;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor w = ctx->saved_data["w"].toTensor();
+    const Tensor go = grads[0].contiguous();
+    const auto device = go.device();
+    const int64_t N = go.size(0), O = w.size(0), C = w.size(1);
+    const Tensor g_rows = layout_buffer(N, O, device), g_cols = layout_buffer(O, N, device);
+    QuantizeJobs jobs;
+    jobs.add(go, layout_of(g_rows, N, O), layout_of(g_cols, O, N));
+    jobs.run();
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0))
+      dx = gemm_bf16(layout_of(g_rows, N, O), saved_layout(saved[1], saved[2], C, O), N, C, O, device);
+    const Layout g_t = layout_of(g_cols, O, N), x_t = layout_of(saved[0], C, N);
+    if (grad_direct(w)) {
+      grad_weights(g_t, x_t, O, C, N, {w}, nullptr, device);
+    } else if (ctx->needs_input_grad(1)) {
+      dw = empty({O, C}, at::kFloat, device);
+      gemm(dw.data_ptr(), true, g_t, x_t, O, C, N, device);
+      dw = dw.to(w.scalar_type());
+    }
+    return {dx, dw, Tensor()};
+  }
+};
+
+Tensor fp8_matmul(const Tensor& input, const Tensor& w, WeightCache* cache) {
+  require(input.dim() == 2 && w.dim() == 2 && fits(input.size(0), input.size(1)) && fits(w.size(0), w.size(1)),
+          "fp8_matmul: MX needs N, in, out % 128");
+  require(input.size(1) == w.size(1), "mx_gemm: shape mismatch");
+  require_cuda(input, "quantize_mx");
+  const Tensor x = input.contiguous();
+  WeightUse use(cache, {w});
+  if (!grad_mode({&x, &w}))
+    return linear_forward(x, use, false, nullptr);
+  return Float8Matmul::apply(x, w, &use);
+}
+
+// ---------------------------------------------------------------------------------------------------- q, k, v
+
+// Attention's three projections of one input, merged: MX scales run along K, so the weights concatenate along their
+// rows and the output gradients along their columns (fp8.cpp:424-462).
+variable_list qkv_forward(const Tensor& x, WeightUse& w, int64_t gate_cols, const Mx* x_mx, bool grad, variable_list* saved) {
+  const auto device = x.device();
+  const int64_t N = x.size(0), C = x.size(1), n = w.out_features();
+  Tensor x_rows, x_cols;
+  QuantizeJobs jobs;
+  if (x_mx == nullptr) {
+    x_rows = layout_buffer(N, C, device);
+    if (grad)
+      x_cols = layout_buffer(C, N, device);
+    jobs.add(x, layout_of(x_rows, N, C), grad ? layout_of(x_cols, C, N) : Layout{}, grad);
+  }
+  jobs.add(w, device, grad);
+  jobs.run();
+  w.publish();
+  const Tensor qkv = gemm_bf16(x_mx != nullptr ? x_mx->rows() : layout_of(x_rows, N, C), w.rows(), N, n, C, device);
+  variable_list out;
+  int64_t row = 0;
+  for (const Tensor& part : w.weights) {
+    out.push_back(qkv.narrow(1, row, part.size(0)));
+    row += part.size(0);
+  }
+  if (gate_cols > 0)
+    out.push_back(x.narrow(1, 0, gate_cols).contiguous());
+  if (saved != nullptr) {
+    if (x_mx != nullptr)
+      *saved = {x_mx->data_t, x_mx->scale_t};
+    else
+      *saved = {x_cols, Tensor()};
+    w.save(*saved);
+  }
+  return out;
+}
+
+struct MxQkv : torch::autograd::Function<MxQkv> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv,
+                               int64_t gate_cols, WeightUse* use, const Mx* x_mx) {
+    variable_list saved;
+    variable_list out = qkv_forward(x, *use, gate_cols, x_mx, true, &saved);
+    ctx->save_for_backward(std::move(saved));
+    ctx->saved_data["w"] = std::vector<Tensor>{wq, wk, wv};
+    ctx->saved_data["gate_cols"] = gate_cols;
+    ctx->saved_data["tokens"] = x.size(0);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const std::vector<Tensor> ws = ctx->saved_data["w"].toTensorVector();
+    const int64_t gate_cols = ctx->saved_data["gate_cols"].toInt(), N = ctx->saved_data["tokens"].toInt();
+    const auto device = ws[0].device();
+    const int64_t C = ws[0].size(1);
+    int64_t n = 0;
+    bool direct = true;
+    for (const Tensor& w : ws)
+      n += w.size(0), direct &= grad_direct(w);
+    const Tensor g_rows = layout_buffer(N, n, device), g_cols = layout_buffer(n, N, device);
+    const Layout g = layout_of(g_rows, N, n), g_t = layout_of(g_cols, n, N);
+    QuantizeJobs jobs;
+    int64_t row = 0;
+    for (size_t i = 0; i < 3; ++i) {
+      const Tensor gi = grads[i].defined() ? grads[i].contiguous()
+                                           : at::zeros({N, ws[i].size(0)}, ws[i].options().dtype(at::kBFloat16));
+      jobs.add(gi, view(g, n, 0, row), view(g_t, N, row, 0));
+      row += ws[i].size(0);
+    }
+    jobs.run();
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) {
+      dx = gemm_bf16(g, saved_layout(saved[2], saved[3], C, n), N, C, n, device);
+      if (gate_cols > 0 && grads[3].defined())
+        dx.narrow(1, 0, gate_cols).add_(grads[3]);
+    }
+    const Layout x_t = saved_layout(saved[0], saved[1], C, N);
+    if (direct) {
+      grad_weights(g_t, x_t, n, C, N, ws, nullptr, device);
+      return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+    Tensor dw = empty({n, C}, at::kFloat, device);
+    gemm(dw.data_ptr(), true, g_t, x_t, n, C, N, device);
+    variable_list out{dx};
+    row = 0;
+    for (const Tensor& w : ws) {
+      out.push_back(dw.narrow(0, row, w.size(0)).to(w.scalar_type()));
+      row += w.size(0);
+    }
+    out.resize(7);
+    return out;
+  }
+};
+
+variable_list fp8_qkv(const Tensor& x_2d, const Tensor& wq, const Tensor& wk, const Tensor& wv, int64_t gate_cols,
+                      WeightCache* cache, const std::optional<std::vector<Tensor>>& x_mx) {
+  bool ok = x_2d.dim() == 2 && fits(x_2d.size(0), x_2d.size(1)) && gate_cols >= 0 && gate_cols <= x_2d.size(1);
+  for (const Tensor* w : {&wq, &wk, &wv})
+    ok &= w->dim() == 2 && w->size(0) % 128 == 0;
+  require(ok, "fp8_qkv: MX needs N, in and every weight's rows % 128");
+  require(wk.size(1) == wq.size(1) && wv.size(1) == wq.size(1), "q/k/v weights must share the input dim");
+  require(wq.size(1) == x_2d.size(1), "mx_gemm: shape mismatch");
+  require_cuda(x_2d, "quantize_mx");
+  const Tensor x = x_2d.contiguous();
+  Mx given;
+  if (x_mx.has_value()) {
+    const auto& t = *x_mx;
+    given = {t.at(0), t.at(1), t.at(2), t.at(3)};
+    require(given.data.sizes() == x.sizes() && given.data.scalar_type() == kE4M3 && given.data.is_contiguous() &&
+                  given.scale.numel() == x.numel() / 32 && given.data_t.numel() == x.numel() &&
+                  given.data_t.is_contiguous() && given.scale_t.numel() == x.numel() / 32,
+            "mx_gemm: shape mismatch");
+  }
+  WeightUse use(cache, {wq, wk, wv});
+  const Mx* mx = x_mx.has_value() ? &given : nullptr;
+  if (!grad_mode({&x, &wq, &wk, &wv}))
+    return qkv_forward(x, use, gate_cols, mx, false, nullptr);
+  return MxQkv::apply(x, wq, wk, wv, gate_cols, &use, mx);
+}
+
+// ---------------------------------------------------------------------------------------------------- relu^2 MLP
+
+// c_proj(relu(c_fc(x))^2): the forward quantizes relu(h)^2 in c_fc's epilogue, the backward quantizes
+// dh = (go . w_proj) * 2h in the dgrad GEMM's epilogue without writing it; h is what is saved (fp8.cpp:262-338).
+Tensor mlp_forward(const Tensor& x, WeightUse& fc, WeightUse& proj, const Mx* x_mx, bool grad, variable_list* saved) {
+  const auto device = x.device();
+  const int64_t N = x.size(0), C = x.size(1), H = fc.out_features(), O = proj.out_features();
+  Tensor x_rows, x_cols;
+  QuantizeJobs jobs;
+  if (x_mx == nullptr) {
+    x_rows = layout_buffer(N, C, device);
+    if (grad)
+      x_cols = layout_buffer(C, N, device);
+    jobs.add(x, layout_of(x_rows, N, C), grad ? layout_of(x_cols, C, N) : Layout{}, grad);
+  }
+  jobs.add(fc, device, grad);
+  jobs.add(proj, device, grad);
+  jobs.run();
+  fc.publish();
+  proj.publish();
+  const Tensor h = empty({N, H}, at::kBFloat16, device);
+  const Tensor a_rows = layout_buffer(N, H, device), a_cols = layout_buffer(H, N, device);
+  const Layout xq = x_mx != nullptr ? x_mx->rows() : layout_of(x_rows, N, C), w = fc.rows();
+  const Layout a = layout_of(a_rows, N, H), a_t = layout_of(a_cols, H, N);
+  check(mxb200_gemm_relu_square(xq.data, xq.scale, w.data, w.scale, h.data_ptr(), a.data, a.scale, a_t.data, a_t.scale, N,
+                                H, C, stream()),
+        "mx_gemm_relu_square");
+  if (saved != nullptr) {
+    if (x_mx != nullptr)
+      *saved = {x_mx->data_t, x_mx->scale_t};
+    else
+      *saved = {x_cols, Tensor()};
+    fc.save(*saved);
+    proj.save(*saved);
+    saved->push_back(h);
+    saved->push_back(a_cols);
+  }
+  return gemm_bf16(a, proj.rows(), N, O, H, device);
+}
+
+struct Fp8ReluSquareMlp : torch::autograd::Function<Fp8ReluSquareMlp> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_fc, const Tensor& w_proj, WeightUse* fc,
+                        WeightUse* proj, const Mx* x_mx) {
+    variable_list saved;
+    Tensor y = mlp_forward(x, *fc, *proj, x_mx, true, &saved);
+    ctx->save_for_backward(std::move(saved));
+    ctx->saved_data["w_fc"] = w_fc;
+    ctx->saved_data["w_proj"] = w_proj;
+    return y;
+  }
+  static Tensor weight_grad(const Layout& g_t, const Layout& in_t, int64_t n, int64_t C, int64_t K, const Tensor& w,
+                            bool needed) {
+    if (grad_direct(w)) {
+      grad_weights(g_t, in_t, n, C, K, {w}, nullptr, w.device());
+      return Tensor();
+    }
+    if (!needed)
+      return Tensor();
+    Tensor dw = empty({n, C}, at::kFloat, w.device());
+    gemm(dw.data_ptr(), true, g_t, in_t, n, C, K, w.device());
+    return dw.to(w.scalar_type());
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor w_fc = ctx->saved_data["w_fc"].toTensor(), w_proj = ctx->saved_data["w_proj"].toTensor();
+    const Tensor grad = grads[0].contiguous();
+    const auto device = grad.device();
+    const Tensor& h = saved[6];
+    const int64_t N = h.size(0), H = h.size(1), C = w_fc.size(1), O = w_proj.size(0);
+    const Tensor go_rows = layout_buffer(N, O, device), go_cols = layout_buffer(O, N, device);
+    const Layout go = layout_of(go_rows, N, O), go_t = layout_of(go_cols, O, N);
+    QuantizeJobs jobs;
+    jobs.add(grad, go, go_t);
+    jobs.run();
+    // the reference's order (fp8.cpp:299-337): fc's two GEMMs read dh while it is still in L2
+    const Tensor grad_proj =
+          weight_grad(go_t, layout_of(saved[7], H, N), O, H, N, w_proj, ctx->needs_input_grad(2));
+    const Tensor dh_rows = layout_buffer(N, H, device), dh_cols = layout_buffer(H, N, device);
+    const Layout dh = layout_of(dh_rows, N, H), dh_t = layout_of(dh_cols, H, N);
+    const Layout proj_t = saved_layout(saved[4], saved[5], H, O);
+    check(mxb200_gemm_relu_square_bwd(go.data, go.scale, proj_t.data, proj_t.scale, h.data_ptr(), dh.data, dh.scale,
+                                      dh_t.data, dh_t.scale, N, H, O, stream()),
+          "mx_gemm_relu_square_bwd");
+    Tensor dx;
+    if (ctx->needs_input_grad(0))
+      dx = gemm_bf16(dh, saved_layout(saved[2], saved[3], C, H), N, C, H, device);
+    const Tensor grad_fc = weight_grad(dh_t, saved_layout(saved[0], saved[1], C, N), H, C, N, w_fc, ctx->needs_input_grad(1));
+    return {dx, grad_fc, grad_proj, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor& w_proj, WeightCache* fc_cache,
+                           WeightCache* proj_cache, const std::optional<std::vector<Tensor>>& x_mx) {
+  require(x_2d.dim() == 2 && w_fc.dim() == 2 && w_proj.dim() == 2 && fits(x_2d.size(0), x_2d.size(1)) &&
+                fits(w_fc.size(0), w_fc.size(1)) && fits(w_proj.size(0), w_proj.size(1)) &&
+                w_fc.size(1) == x_2d.size(1) && w_proj.size(1) == w_fc.size(0),
+          "fp8_relu_square_mlp: MX needs N, in, hidden, out % 128");
+  require_cuda(x_2d, "quantize_mx");
+  const Tensor x = x_2d.contiguous();
+  Mx given;
+  if (x_mx.has_value()) {
+    const auto& t = *x_mx;
+    given = {t.at(0), t.at(1), t.at(2), t.at(3)};
+    require(given.data.sizes() == x.sizes() && given.data.scalar_type() == kE4M3 && given.data.is_contiguous() &&
+                  given.scale.numel() == x.numel() / 32 && given.data_t.numel() == x.numel() &&
+                  given.data_t.is_contiguous() && given.scale_t.numel() == x.numel() / 32,
+            "mx_gemm_relu_square: shape mismatch");
+  }
+  WeightUse fc(fc_cache, {w_fc}), proj(proj_cache, {w_proj});
+  const Mx* mx = x_mx.has_value() ? &given : nullptr;
+  if (!grad_mode({&x, &w_fc, &w_proj}))
+    return mlp_forward(x, fc, proj, mx, false, nullptr);
+  return Fp8ReluSquareMlp::apply(x, w_fc, w_proj, &fc, &proj, mx);
+}
+
+// ---------------------------------------------------------------------------------------------------- chunked lm_head
+
+struct LossArgs {
+  int64_t vocab, chunk_rows;
+  double softcap;
+};
+
+struct ChunkOutputs {
+  float* losses = nullptr;             // (N), or null
+  void* grad_x = nullptr;              // (N, C) bf16, or null: loss only
+  const float* grad_scale = nullptr;   // upstream gradient of the losses, one value or one per row
+  int64_t grad_scale_stride = 0;
+  const int64_t* num_valid = nullptr;  // divides the scale
+};
+
+// Per chunk of rows: logits = xq[chunk] . wq^T, the loss pass, the gradient quantized straight from the logits (row-wise
+// into a chunk buffer, transposed into one (padded, N) buffer), grad_x[chunk] = gq . wq_t^T (softcap_ce.cpp:27-110). With
+// grad_x, x_cols and g_cols receive the transposes: the operands of the single weight-gradient GEMM.
+void run_chunks(const Tensor& x, WeightUse& w, const Tensor& targets, const LossArgs& args, const ChunkOutputs& out,
+                Tensor* x_cols, Tensor* g_cols) {
+  const auto device = x.device();
+  const int64_t N = x.size(0), C = x.size(1), V = w.out_features();
+  const bool grad = out.grad_x != nullptr;
+  const Tensor x_rows = layout_buffer(N, C, device);
+  if (grad)
+    *x_cols = layout_buffer(C, N, device);
+  QuantizeJobs jobs;
+  jobs.add(x, layout_of(x_rows, N, C), grad ? layout_of(*x_cols, C, N) : Layout{}, grad);
+  jobs.add(w, device, grad);
+  jobs.run();
+  w.publish();
+  const int64_t rows_max = std::min(N, args.chunk_rows);
+  const Tensor logits = empty({rows_max, V}, at::kBFloat16, device);
+  const Tensor row_floats = empty({2, rows_max}, at::kFloat, device);  // lse, and the losses nobody asked for
+  auto* lse = static_cast<float*>(row_floats.data_ptr());
+  Tensor g_rows;
+  Layout g_t;
+  if (grad) {
+    g_rows = layout_buffer(rows_max, V, device);
+    *g_cols = layout_buffer(V, N, device);
+    g_t = layout_of(*g_cols, V, N);
+  }
+  const Layout xq = layout_of(x_rows, N, C), wq = w.rows();
+  const auto* t = static_cast<const int64_t*>(targets.data_ptr());
+  void* s = stream();
+  for (int64_t begin = 0; begin < N; begin += args.chunk_rows) {
+    const int64_t rows = std::min(N - begin, args.chunk_rows);
+    const mxb200_mx_out x_chunk = view(xq, C, begin);
+    gemm(logits.data_ptr(), false, {x_chunk.data, x_chunk.scale}, wq, rows, V, C, device);
+    check(mxb200_softcap_ce_loss(logits.data_ptr(), rows, V, t + begin, static_cast<int>(args.vocab), static_cast<int>(V),
+                                 static_cast<float>(args.softcap), out.losses != nullptr ? out.losses + begin : lse + rows_max,
+                                 lse, s),
+          "softcap_ce_loss");
+    if (!grad)
+      continue;
+    const Layout g = layout_of(g_rows, rows, V);
+    const float* scale = out.grad_scale != nullptr ? out.grad_scale + begin * out.grad_scale_stride : nullptr;
+    check(mxb200_softcap_ce_grad_mx(logits.data_ptr(), rows, V, t + begin, lse, static_cast<int>(args.vocab),
+                                    static_cast<int>(V), static_cast<float>(args.softcap), scale, out.grad_scale_stride,
+                                    out.num_valid, view(g, V), view(g_t, N, 0, begin), MXB200_SCALE_REFERENCE, s),
+          "softcap_ce_grad_mx");
+    gemm(static_cast<char*>(out.grad_x) + begin * C * 2, false, g, w.cols(), rows, C, V, device);
+  }
+}
+
+// For mean and sum the incoming gradient is a scalar, so the forward computes grad_x and the weight gradient's operands
+// at once and the backward only scales: one GEMM with alpha = that gradient, straight into .grad when the weight is an
+// fp32 leaf (softcap_ce.cpp:118-205).
+Tensor reduced_loss(const Tensor& losses, const Tensor& num_valid, bool mean) {
+  Tensor loss = empty({}, at::kFloat, losses.device());
+  check(mxb200_reduce_losses(static_cast<const float*>(losses.data_ptr()), losses.numel(),
+                             mean ? static_cast<const int64_t*>(num_valid.data_ptr()) : nullptr,
+                             static_cast<float*>(loss.data_ptr()), stream()),
+        "softcap_cross_entropy");
+  return loss;
+}
+
+Tensor count_valid(const Tensor& targets) {
+  Tensor n = empty({}, at::kLong, targets.device());
+  check(mxb200_count_valid(static_cast<const int64_t*>(targets.data_ptr()), targets.numel(),
+                           static_cast<int64_t*>(n.data_ptr()), stream()),
+        "softcap_cross_entropy");
+  return n;
+}
+
+struct SoftcapReduced : torch::autograd::Function<SoftcapReduced> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& targets,
+                        const LossArgs* args, bool mean, WeightUse* use) {
+    const Tensor num_valid = mean ? count_valid(targets) : Tensor();
+    const Tensor losses = empty({x.size(0)}, at::kFloat, x.device());
+    const Tensor grad_x = empty(x.sizes(), at::kBFloat16, x.device());
+    ChunkOutputs out;
+    out.losses = static_cast<float*>(losses.data_ptr());
+    out.grad_x = grad_x.data_ptr();
+    out.num_valid = mean ? static_cast<const int64_t*>(num_valid.data_ptr()) : nullptr;
+    Tensor x_cols, g_cols;
+    run_chunks(x, *use, targets, *args, out, &x_cols, &g_cols);
+    ctx->save_for_backward({grad_x, g_cols, x_cols});
+    ctx->saved_data["w"] = weight;
+    return reduced_loss(losses, num_valid, mean);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor weight = ctx->saved_data["w"].toTensor();
+    const Tensor& grad_x = saved[0];
+    const auto device = grad_x.device();
+    const int64_t N = grad_x.size(0), C = grad_x.size(1), V = weight.size(0);
+    const Tensor g = grads[0].to(at::kFloat).contiguous();
+    const auto* alpha = static_cast<const float*>(g.data_ptr());
+    const Layout g_t = layout_of(saved[1], V, N), x_t = layout_of(saved[2], C, N);
+    Tensor dw;
+    if (grad_direct(weight)) {
+      grad_weights(g_t, x_t, V, C, N, {weight}, alpha, device);
+    } else if (ctx->needs_input_grad(1)) {
+      dw = empty({V, C}, at::kFloat, device);
+      gemm(dw.data_ptr(), true, g_t, x_t, V, C, N, device, alpha, false);
+      dw = dw.to(weight.scalar_type());
+    }
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) {
+      dx = empty({N, C}, at::kBFloat16, device);
+      check(mxb200_scale_bf16(grad_x.data_ptr(), alpha, dx.data_ptr(), N * C, stream()), "softcap_cross_entropy");
+    }
+    return {dx, dw, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// A cache kept alive by a graph node, which may be destroyed without the GIL.
+struct CacheHolder : torch::CustomClassHolder {
+  PyObject* object;
+  explicit CacheHolder(py::object o) : object(o.release().ptr()) {}
+  ~CacheHolder() override {
+    py::gil_scoped_acquire gil;
+    Py_XDECREF(object);
+  }
+};
+
+// Reduction none: the backward re-runs the chunks with the per-row gradient.
+struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& targets,
+                        const LossArgs* args, WeightUse* use, py::object* cache) {
+    const Tensor losses = empty({x.size(0)}, at::kFloat, x.device());
+    ChunkOutputs out;
+    out.losses = static_cast<float*>(losses.data_ptr());
+    run_chunks(x, *use, targets, *args, out, nullptr, nullptr);
+    ctx->save_for_backward({x, weight, targets});
+    ctx->saved_data["vocab"] = args->vocab;
+    ctx->saved_data["chunk_rows"] = args->chunk_rows;
+    ctx->saved_data["softcap"] = args->softcap;
+    if (!cache->is_none())
+      ctx->saved_data["cache"] = c10::IValue::make_capsule(c10::make_intrusive<CacheHolder>(*cache));
+    return losses;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &weight = saved[1], &targets = saved[2];
+    const auto device = x.device();
+    const int64_t N = x.size(0), C = x.size(1), V = weight.size(0);
+    const LossArgs args{ctx->saved_data["vocab"].toInt(), ctx->saved_data["chunk_rows"].toInt(),
+                        ctx->saved_data["softcap"].toDouble()};
+    const Tensor g = grads[0].to(at::kFloat).contiguous();
+    const Tensor grad_x = empty({N, C}, at::kBFloat16, device);
+    ChunkOutputs out;
+    out.grad_x = grad_x.data_ptr();
+    out.grad_scale = static_cast<const float*>(g.data_ptr());
+    out.grad_scale_stride = 1;
+    Tensor x_cols, g_cols;
+    const auto cache = ctx->saved_data.find("cache");
+    if (cache != ctx->saved_data.end()) {
+      py::gil_scoped_acquire gil;
+      auto* holder = static_cast<CacheHolder*>(cache->second.toCapsule().get());
+      WeightUse use(py::handle(holder->object).cast<WeightCache*>(), {weight});
+      run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
+    } else {
+      WeightUse use(nullptr, {weight});
+      run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
+    }
+    Tensor dw = empty({V, C}, at::kFloat, device);
+    gemm(dw.data_ptr(), true, layout_of(g_cols, V, N), layout_of(x_cols, C, N), V, C, N, device);
+    return {grad_x, dw.to(weight.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor softcap_cross_entropy(const Tensor& x_in, const Tensor& weight, const Tensor& targets_in, int64_t vocab,
+                             double softcap, int64_t chunk_rows, int reduction, py::object cache_object) {
+  const Tensor x = x_in.contiguous(), targets = targets_in.to(at::kLong).contiguous();
+  require_cuda(targets, "softcap_cross_entropy");
+  auto* cache = cache_object.is_none() ? nullptr : cache_object.cast<WeightCache*>();
+  const LossArgs args{vocab, chunk_rows, softcap};
+  WeightUse use(cache, {weight});
+  const bool mean = reduction == 0, none = reduction == 2;
+  if (grad_mode({&x, &weight}))
+    return none ? SoftcapPerToken::apply(x, weight, targets, &args, &use, &cache_object)
+                : SoftcapReduced::apply(x, weight, targets, &args, mean, &use);
+  const Tensor losses = empty({x.size(0)}, at::kFloat, x.device());
+  ChunkOutputs out;
+  out.losses = static_cast<float*>(losses.data_ptr());
+  run_chunks(x, use, targets, args, out, nullptr, nullptr);
+  return none ? losses : reduced_loss(losses, mean ? count_valid(targets) : Tensor(), mean);
+}
+
+// ---------------------------------------------------------------------------------------------------- other entry points
+
+// Forward of the fused residual step with MX output (residual_norm.cpp:36-96). Returns (res, n, n_mx..., rstd, s).
+std::vector<std::optional<Tensor>> residual_norm_mx(const Tensor& x, const std::optional<Tensor>& r,
+                                                    const std::optional<Tensor>& x0, const std::optional<Tensor>& lr,
+                                                    const std::optional<Tensor>& l0, int64_t layer, int64_t gate_cols,
+                                                    double eps) {
+  const auto device = x.device();
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  const Tensor res = empty(x.sizes(), at::kBFloat16, device), n = empty(x.sizes(), at::kBFloat16, device);
+  const Tensor rstd = empty({rows}, at::kFloat, device);
+  std::optional<Tensor> s;
+  if (r.has_value() && x0.has_value())
+    s = empty(x.sizes(), at::kBFloat16, device);
+  const Mx q = empty_mx(rows, cols, device);
+  mxb200_residual_norm_mx a{};
+  a.x = x.data_ptr();
+  a.r = r.has_value() ? r->data_ptr() : nullptr;
+  if (x0.has_value()) {
+    a.x0 = x0->data_ptr();
+    a.lr = static_cast<const float*>(lr->data_ptr()) + layer;
+    a.l0 = static_cast<const float*>(l0->data_ptr()) + layer;
+  }
+  a.s = s.has_value() ? s->data_ptr() : nullptr;
+  a.res = res.data_ptr();
+  a.n = n.data_ptr();
+  a.rstd = static_cast<float*>(rstd.data_ptr());
+  a.rows = rows, a.cols = static_cast<int32_t>(cols), a.eps = static_cast<float>(eps);
+  a.out = view(q.rows(), cols), a.out_t = view(q.cols(), rows);
+  a.n_cols = static_cast<int32_t>(gate_cols);
+  check(mxb200_residual_norm_mx_fwd(&a, stream()), "residual_norm_mx");
+  return {res, n, q.data, q.data_t, q.scale, q.scale_t, rstd, s};
+}
+
+// (x, out, out_t) jobs; out and out_t are ctypes structures laid out as mxb200_mx_out.
+mxb200_mx_out mx_out_of(PyObject* o) {
+  Py_buffer b;
+  if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0)
+    throw py::error_already_set();
+  const bool ok = b.len == static_cast<Py_ssize_t>(sizeof(mxb200_mx_out));
+  mxb200_mx_out out = kNoLayout;
+  if (ok)
+    std::memcpy(&out, b.buf, sizeof(out));
+  PyBuffer_Release(&b);
+  require(ok, "MX: expected an MxOut");
+  return out;
+}
+
+void quantize_mx_batch_into(const py::sequence& jobs, int scale_rule) {
+  const size_t count = jobs.size();
+  if (count == 0)
+    return;
+  std::vector<mxb200_quantize_job> list;
+  list.reserve(count);
+  std::optional<at::ScalarType> dtype;
+  std::optional<at::Device> device;
+  for (size_t i = 0; i < count; ++i) {
+    const py::object item = jobs[i];
+    const auto job = py::reinterpret_borrow<py::sequence>(item);
+    require(job.size() == 3, "MX: a job is (x, out, out_t)");
+    const py::object px = job[0], po = job[1], pt = job[2];
+    const Tensor x = px.cast<Tensor>();
+    if (i == 0)
+      require_cuda(x, "quantize_mx_batch"), dtype = x.scalar_type(), device = x.device();
+    require(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && fits(x.size(0), x.size(1)) && x.scalar_type() == *dtype &&
+                  (*dtype == at::kBFloat16 || *dtype == at::kFloat) && x.device() == *device,
+            "MX: expected aligned, contiguous 2D tensors of one dtype with dims % 128");
+    list.push_back({x.data_ptr(), x.size(0), x.size(1), mx_out_of(po.ptr()), mx_out_of(pt.ptr())});
+  }
+  check(mxb200_quantize_mx_batch(list.data(), static_cast<int>(count), *dtype == at::kBFloat16, scale_rule, stream()),
+        "quantize_mx_batch");
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.doc() = "Native host path of nanochat_cpp_b200.engine.";
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p)
+        std::rethrow_exception(p);
+    } catch (const StatusError& e) {
+      const py::object type = py::module_::import("nanochat_cpp_b200.capi").attr("Mxb200Error");
+      const py::object error = type(e.status, e.what_failed);
+      PyErr_SetObject(type.ptr(), error.ptr());
+    }
+  });
+  py::class_<WeightCache>(m, "WeightCache")
+        .def(py::init<bool>(), py::arg("enabled") = false)
+        .def_readwrite("enabled", &WeightCache::enabled)
+        .def("get", &WeightCache::get, py::arg("kind"), py::arg("weights"), py::arg("make"));
+  m.def("fp8_matmul", &fp8_matmul);
+  m.def("fp8_qkv", &fp8_qkv);
+  m.def("fp8_relu_square_mlp", &fp8_relu_square_mlp);
+  m.def("softcap_cross_entropy", &softcap_cross_entropy);
+  m.def("residual_norm_mx", &residual_norm_mx);
+  m.def("quantize_mx_batch_into", &quantize_mx_batch_into);
+}

@@ -2,19 +2,22 @@
 
 Same names, argument meaning and error behaviour as the reference's fp8.h / mx_gemm.h (file:line cited per
 function, paths within nanochat-cpp), with torch tensors used only as owners of device memory. Every call
-goes to the CUDA library through the C ABI; nothing here computes on the CPU and nothing falls back.
+goes to the CUDA library through the C ABI; nothing here computes on the CPU and nothing falls back. The functions a
+model calls per layer (Linear, q/k/v, MLP, loss, residual step, weight refresh) run their host side in
+csrc/torch_engine.cpp; the single-kernel ones below go through ctypes.
 """
 from __future__ import annotations
 
 import ctypes
 import enum
 from dataclasses import dataclass
-from typing import Callable, List, Optional, Sequence
+from typing import List, Optional, Sequence
 
 import torch
 
 from . import capi
 from .capi import MxOut, check, lib
+from . import _torch_engine as native  # after capi, which builds and loads libmxb200.so
 
 __all__ = [
     "Fp8Tensor", "Fp8WeightCache", "MxGemmBackend", "set_mx_gemm_backend", "mx_gemm_backend", "mx_fits",
@@ -131,18 +134,7 @@ def quantize_mx_batch_into(jobs: Sequence[tuple], scale_rule: int = SCALE_REFERE
     """quantize_mx_into(x, False, out, out_t) for every (x, out, out_t) of jobs, all bf16 or all fp32, in as few
     launches as possible: the same bytes as one call each. For runs of small tensors, e.g. the parts of the merged
     q/k/v weight (src/nanochat/model/fp8/fp8.cpp:155-171) or a model's weights after an optimizer step."""
-    if not jobs:
-        return
-    x0 = jobs[0][0]
-    _require_cuda(x0, "quantize_mx_batch")
-    arr = (capi.QuantizeJob * len(jobs))()
-    for i, (x, out, out_t) in enumerate(jobs):
-        if not (x.is_cuda and x.dim() == 2 and x.is_contiguous() and mx_fits(x.size(0), x.size(1))
-                and x.dtype == x0.dtype and x.dtype in (torch.bfloat16, torch.float32) and x.device == x0.device):
-            raise RuntimeError("MX: expected aligned, contiguous 2D tensors of one dtype with dims % 128")
-        arr[i] = capi.QuantizeJob(x.data_ptr(), x.size(0), x.size(1), out, out_t)
-    check(lib.mxb200_quantize_mx_batch(arr, len(jobs), int(x0.dtype == torch.bfloat16), scale_rule, _stream()),
-          "quantize_mx_batch")
+    native.quantize_mx_batch_into(jobs, scale_rule)
 
 
 def quantize_mx(x: torch.Tensor, rows: bool = True, cols: bool = True, relu_square: bool = False,
@@ -198,17 +190,13 @@ def residual_norm_mx(x: torch.Tensor, r: Optional[torch.Tensor] = None, x0: Opti
     if blend and not (lr is not None and l0 is not None and lr.dtype == l0.dtype == torch.float32
                       and 0 <= layer < lr.numel() == l0.numel() and lr.is_contiguous() and l0.is_contiguous()):
         raise RuntimeError("residual_norm_mx: the blend needs fp32 lambdas")
-    if out is not None:
-        res, n, n_mx, rstd, s = out
-        if not (res.shape == x.shape and n.shape == x.shape and rstd.numel() == rows and n_mx.data.shape == (rows, cols)
-                and (s is not None) == (r is not None and blend)):
-            raise RuntimeError("residual_norm_mx: out does not match")
-    else:
-        res = torch.empty_like(x)
-        n = torch.empty_like(x)
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        s = torch.empty_like(x) if (r is not None and blend) else None
-        n_mx = empty_mx(rows, cols, x.device)
+    if out is None:
+        res, n, data, data_t, scale, scale_t, rstd, s = native.residual_norm_mx(x, r, x0, lr, l0, layer, gate_cols, eps)
+        return res, n, Fp8Tensor(data, data_t, scale, scale_t), rstd, s
+    res, n, n_mx, rstd, s = out
+    if not (res.shape == x.shape and n.shape == x.shape and rstd.numel() == rows and n_mx.data.shape == (rows, cols)
+            and (s is not None) == (r is not None and blend)):
+        raise RuntimeError("residual_norm_mx: out does not match")
     out, out_t = mx_outs(n_mx)
     args = capi.ResidualNormMx(x.data_ptr(), r.data_ptr() if r is not None else None,
                                x0.data_ptr() if blend else None,
@@ -219,24 +207,16 @@ def residual_norm_mx(x: torch.Tensor, r: Optional[torch.Tensor] = None, x0: Opti
     return res, n, n_mx, rstd, s
 
 
-class Fp8WeightCache:
+class Fp8WeightCache(native.WeightCache):
     """FP8 copies of weights, remade only when a weight changes: in-place updates bump the tensor's version
-    (src/nanochat/model/fp8/fp8.h:18-38, fp8.cpp:516-536)."""
+    (src/nanochat/model/fp8/fp8.h:18-38, fp8.cpp:516-536). `get(kind, weights, make)` returns make()'s list, kept while
+    `enabled` and until another kind or weight is asked for."""
 
     def __init__(self, enabled: bool = False):
-        self.enabled = enabled
-        self._kind = -1
-        self._keys: list = []
-        self._value: list = []
+        super().__init__(enabled)
 
-    def get(self, kind: int, weights: Sequence[torch.Tensor], make: Callable[[], List[torch.Tensor]]):
-        if not self.enabled:
-            return make()
-        keys = [(id(w), w.data_ptr(), w._version) for w in weights]
-        if kind != self._kind or keys != self._keys:
-            self._value = make()
-            self._kind, self._keys = kind, keys
-        return self._value
+    def __reduce__(self):  # a copy starts empty
+        return Fp8WeightCache, (self.enabled,)
 
 
 def quantize_fp8_weight(w: torch.Tensor, cache: Optional[Fp8WeightCache] = None) -> Fp8Tensor:
@@ -448,76 +428,8 @@ def mx_grad_weights(go_t: torch.Tensor, go_scale_t: torch.Tensor, in_t: torch.Te
         row += w.size(0)
 
 
-class _Float8Matmul(torch.autograd.Function):
-    """One Linear under MX: y = x . w^T, dX = dY . w, dW = dY^T . x, every operand E4M3 with per-32 scales
-    along the contraction (src/nanochat/model/fp8/fp8.cpp:240-260)."""
-
-    @staticmethod
-    def forward(ctx, x, w, cache):
-        xq = quantize_mx(x)
-        wq = quantize_fp8_weight(w, cache)
-        ctx.save_for_backward(xq.data_t, xq.inv_scale_t, wq.data_t, wq.inv_scale_t)
-        ctx.w = w
-        ctx.direct = mx_grad_direct(w)
-        return mx_gemm(xq.data, xq.inv_scale, wq.data, wq.inv_scale, torch.bfloat16)
-
-    @staticmethod
-    def backward(ctx, go):
-        x_t, x_scale_t, w_t, w_scale_t = ctx.saved_tensors
-        gq = quantize_mx(go.contiguous())
-        dx = mx_gemm(gq.data, gq.inv_scale, w_t, w_scale_t, torch.bfloat16)
-        if ctx.direct:
-            mx_grad_weights(gq.data_t, gq.inv_scale_t, x_t, x_scale_t, [ctx.w])
-            return dx, None, None
-        dw = mx_gemm(gq.data_t, gq.inv_scale_t, x_t, x_scale_t, torch.float32)
-        return dx, dw.to(ctx.w.dtype), None
-
-
-class _MxQkv(torch.autograd.Function):
-    """q, k, v = x . w_i^T with x quantized once and one GEMM each for the forward, the input gradient and the weight
-    gradients: MX scales run along K, so the three weights concatenate along their rows and the three output
-    gradients along their columns (src/nanochat/model/fp8/fp8.cpp:424-462)."""
-
-    @staticmethod
-    def forward(ctx, x, wq, wk, wv, gate_cols, cache, x_mx):
-        sizes = (wq.size(0), wk.size(0), wv.size(0))
-        xq = x_mx if x_mx is not None else quantize_mx(x)
-        w, w_t, w_scale, w_scale_t = mx_qkv_weights(wq, wk, wv, cache)
-        qkv = mx_gemm(xq.data, xq.inv_scale, w, w_scale, torch.bfloat16)
-        ctx.save_for_backward(xq.data_t, xq.inv_scale_t, w_t, w_scale_t)
-        ctx.ws, ctx.gate_cols, ctx.sizes = (wq, wk, wv), gate_cols, sizes
-        ctx.direct = all(mx_grad_direct(t) for t in (wq, wk, wv))
-        out = [qkv.narrow(1, 0, sizes[0]), qkv.narrow(1, sizes[0], sizes[1]), qkv.narrow(1, sizes[0] + sizes[1], sizes[2])]
-        if gate_cols > 0:
-            out.append(x.narrow(1, 0, gate_cols).contiguous())
-        return tuple(out)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        x_t, x_scale_t, w_t, w_scale_t = ctx.saved_tensors
-        N, sizes = x_t.size(1), ctx.sizes
-        n = sum(sizes)
-        dev = x_t.device
-        g = torch.empty((N, n), dtype=E4M3, device=dev)
-        g_t = torch.empty((n, N), dtype=E4M3, device=dev)
-        g_scale, g_scale_t = empty_mx_scale(N, n, dev), empty_mx_scale(n, N, dev)
-        row = 0
-        for i in range(3):
-            gi = grads[i] if grads[i] is not None else torch.zeros((N, sizes[i]), dtype=torch.bfloat16, device=dev)
-            quantize_mx_into(gi.contiguous(), False, mx_out(g, g_scale, 0, row), mx_out(g_t, g_scale_t, row, 0))
-            row += sizes[i]
-        dx = mx_gemm(g, g_scale, w_t, w_scale_t, torch.bfloat16)
-        if ctx.gate_cols > 0 and grads[3] is not None:
-            dx.narrow(1, 0, ctx.gate_cols).add_(grads[3])
-        if ctx.direct:
-            mx_grad_weights(g_t, g_scale_t, x_t, x_scale_t, list(ctx.ws))
-            return dx, None, None, None, None, None, None
-        dw = mx_gemm(g_t, g_scale_t, x_t, x_scale_t, torch.float32)
-        parts, row = [], 0
-        for w, rows in zip(ctx.ws, sizes):
-            parts.append(dw.narrow(0, row, rows).to(w.dtype))
-            row += rows
-        return (dx, *parts, None, None, None)
+def _mx_list(q: Optional[Fp8Tensor]):
+    return None if q is None else [q.data, q.data_t, q.inv_scale, q.inv_scale_t]
 
 
 def fp8_qkv(x_2d: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, wv: torch.Tensor, gate_cols: int = 0,
@@ -528,52 +440,9 @@ def fp8_qkv(x_2d: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, wv: torch.Te
     same pass). x_mx: x_2d already quantized in both layouts (residual_norm_mx), as the reference's attention path
     takes it (src/nanochat/model/attention/mx_attention.h:20, mx_attention.cpp:45); x_2d then carries autograd and the
     gate's columns only."""
-    n = wq.size(0) + wk.size(0) + wv.size(0)
-    if not (mx_fits(x_2d.size(0), x_2d.size(1)) and n % 128 == 0 and all(w.size(0) % 128 == 0 for w in (wq, wk, wv))
-            and 0 <= gate_cols <= x_2d.size(1)):
-        raise RuntimeError("fp8_qkv: MX needs N, in and every weight's rows % 128")
     if x_mx is not None and (x_mx.data is None or x_mx.data_t is None):
         raise RuntimeError("fp8_qkv: x_mx needs both layouts")
-    return _MxQkv.apply(x_2d.contiguous(), wq, wk, wv, gate_cols, cache, x_mx)
-
-
-class _Fp8ReluSquareMlp(torch.autograd.Function):
-    """c_proj(relu(c_fc(x))^2) as two MX Linears with relu^2 folded into the GEMM epilogues: the forward quantizes
-    relu(h)^2 in c_fc's epilogue, the backward quantizes dh = (go . w_proj) * 2h in the dgrad GEMM's epilogue without
-    writing it; h is what is saved (src/nanochat/model/fp8/fp8.cpp:262-338, MX branch)."""
-
-    @staticmethod
-    def forward(ctx, x, w_fc, w_proj, fc_cache, proj_cache, x_mx):
-        xq = x_mx if x_mx is not None else quantize_mx(x)
-        fcq = quantize_fp8_weight(w_fc, fc_cache)
-        h = torch.empty((x.size(0), w_fc.size(0)), dtype=torch.bfloat16, device=x.device)
-        aq = empty_mx(h.size(0), h.size(1), h.device)
-        mx_gemm_relu_square(h, aq.data, aq.inv_scale, aq.data_t, aq.inv_scale_t, xq.data, xq.inv_scale, fcq.data,
-                            fcq.inv_scale)
-        projq = quantize_fp8_weight(w_proj, proj_cache)
-        ctx.save_for_backward(xq.data_t, xq.inv_scale_t, fcq.data_t, fcq.inv_scale_t, h, aq.data_t, aq.inv_scale_t,
-                              projq.data_t, projq.inv_scale_t)
-        ctx.w_fc, ctx.w_proj = w_fc, w_proj
-        return mx_gemm(aq.data, aq.inv_scale, projq.data, projq.inv_scale, torch.bfloat16)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x_t, x_scale_t, fc_t, fc_scale_t, h, a_t, a_scale_t, proj_t, proj_scale_t = ctx.saved_tensors
-        go = quantize_mx(grad_output.contiguous())
-
-        def weight_grad(g_t, g_scale_t, in_t, in_scale_t, w):
-            if mx_grad_direct(w):
-                mx_grad_weights(g_t, g_scale_t, in_t, in_scale_t, [w])
-                return None
-            return mx_gemm(g_t, g_scale_t, in_t, in_scale_t, torch.float32).to(w.dtype)
-
-        grad_proj = weight_grad(go.data_t, go.inv_scale_t, a_t, a_scale_t, ctx.w_proj)
-        dhq = empty_mx(h.size(0), h.size(1), h.device)
-        mx_gemm_relu_square_bwd(go.data, go.inv_scale, proj_t, proj_scale_t, h, dhq.data, dhq.inv_scale, dhq.data_t,
-                                dhq.inv_scale_t)
-        grad_x = mx_gemm(dhq.data, dhq.inv_scale, fc_t, fc_scale_t, torch.bfloat16)
-        grad_fc = weight_grad(dhq.data_t, dhq.inv_scale_t, x_t, x_scale_t, ctx.w_fc)
-        return grad_x, grad_fc, grad_proj, None, None, None
+    return tuple(native.fp8_qkv(x_2d, wq, wk, wv, gate_cols, cache, _mx_list(x_mx)))
 
 
 def relu_square_mlp_mx(N: int, cin: int, w_fc: torch.Tensor, w_proj: torch.Tensor) -> bool:
@@ -589,20 +458,16 @@ def fp8_relu_square_mlp(x_2d: torch.Tensor, w_fc: torch.Tensor, w_proj: torch.Te
     """The MLP's c_proj(relu(c_fc(x)).square()) with both matmuls as fp8_matmul, bit for bit
     (src/nanochat/model/fp8/fp8.h:46-54). x_2d (N, in) bf16, w_fc (hidden, in), w_proj (out, hidden) -> (N, out).
     x_mx: x_2d already quantized in both layouts (residual_norm_mx); x_2d then only carries autograd."""
-    if not relu_square_mlp_mx(x_2d.size(0), x_2d.size(1), w_fc, w_proj):
-        raise RuntimeError("fp8_relu_square_mlp: MX needs N, in, hidden, out % 128")
     if x_mx is not None and (x_mx.data is None or x_mx.data_t is None):
         raise RuntimeError("fp8_relu_square_mlp: x_mx needs both layouts")
-    return _Fp8ReluSquareMlp.apply(x_2d.contiguous(), w_fc, w_proj, fc_cache, proj_cache, x_mx)
+    return native.fp8_relu_square_mlp(x_2d, w_fc, w_proj, fc_cache, proj_cache, _mx_list(x_mx))
 
 
 def fp8_matmul(input_2d: torch.Tensor, weight: torch.Tensor, cache: Optional[Fp8WeightCache] = None) -> torch.Tensor:
     """input_2d (N, in) bf16, weight (out, in) -> (N, out) bf16 under the MX recipe
     (src/nanochat/model/fp8/fp8.h:40-44, fp8.cpp:566-571). Dims must be % 128: the reference falls back to its
     tensorwise recipe otherwise, which is outside this library."""
-    if not (mx_fits(input_2d.size(0), input_2d.size(1)) and mx_fits(weight.size(0), weight.size(1))):
-        raise RuntimeError("fp8_matmul: MX needs N, in, out % 128")
-    return _Float8Matmul.apply(input_2d.contiguous(), weight, cache)
+    return native.fp8_matmul(input_2d, weight, cache)
 
 
 # ------------------------------------------------------------------------------------------------ chunked lm_head loss
@@ -647,92 +512,6 @@ def softcap_ce_grad_mx(logits: torch.Tensor, targets: torch.Tensor, lse: torch.T
                                         scale_rule, _stream()), "softcap_ce_grad_mx")
 
 
-def _run_chunks(x, weight, targets, vocab, softcap, chunk_rows, losses, grad_x, grad_scale, num_valid, cache):
-    """The MX branch of the reference's run_chunks (src/nanochat/model/ops/softcap_ce.cpp:27-110): per chunk of rows
-    logits = xq[chunk] . wq^T, the loss pass, the gradient quantized straight from the logits (row-wise into a chunk
-    buffer, transposed into one (padded, N) buffer), grad_x[chunk] = gq . wq_t^T. Returns (xq, g_all) whose transposes
-    are the operands of the single weight-gradient GEMM, or (None, None) without grad_x."""
-    N, C = x.shape
-    padded = weight.size(0)
-    grad = grad_x is not None
-    xq = quantize_mx(x, True, grad)
-    wq = quantize_fp8_weight(weight, cache)
-    rows_max = min(N, chunk_rows)
-    logits = torch.empty((rows_max, padded), dtype=torch.bfloat16, device=x.device)
-    lse = torch.empty(rows_max, dtype=torch.float32, device=x.device)
-    loss_scratch = torch.empty(rows_max, dtype=torch.float32, device=x.device) if losses is None else None
-    g_all = empty_mx(N, padded, x.device, False, True) if grad else None
-    blocks = C // 32
-    for begin in range(0, N, chunk_rows):
-        end = min(N, begin + chunk_rows)
-        rows = end - begin
-        buf = logits[:rows]
-        mx_gemm_out(buf, xq.data[begin:end], xq.inv_scale[begin * blocks:end * blocks], wq.data, wq.inv_scale)
-        softcap_ce_loss(buf, targets[begin:end], vocab, softcap,
-                        losses[begin:end] if losses is not None else loss_scratch[:rows], lse[:rows])
-        if not grad:
-            continue
-        gq = empty_mx(rows, padded, x.device, True, False)
-        scale = None
-        if grad_scale is not None:
-            scale = grad_scale[begin:end] if grad_scale.dim() == 1 and grad_scale.numel() == N else grad_scale
-        softcap_ce_grad_mx(buf, targets[begin:end], lse[:rows], vocab, softcap, mx_out(gq.data, gq.inv_scale, 0, 0),
-                           mx_out(g_all.data_t, g_all.inv_scale_t, 0, begin), scale, num_valid)
-        mx_gemm_out(grad_x[begin:end], gq.data, gq.inv_scale, wq.data_t, wq.inv_scale_t)
-    return (xq, g_all) if grad else (None, None)
-
-
-class _SoftcapCrossEntropy(torch.autograd.Function):
-    """src/nanochat/model/ops/softcap_ce.cpp:118-205, MX branch: for mean/sum the incoming gradient is a scalar, so the
-    forward computes grad_x and the weight gradient's operands at once and the backward only scales (one GEMM with
-    alpha = the incoming gradient, straight into .grad when the weight is an fp32 leaf); for none the backward re-runs
-    the chunks with the per-row gradient."""
-
-    @staticmethod
-    def forward(ctx, x, weight, targets, vocab, softcap, chunk_rows, reduction, needs_grad, cache):
-        num_valid = (targets >= 0).sum()
-        losses = torch.empty(x.size(0), dtype=torch.float32, device=x.device)
-        precompute = needs_grad and reduction != "none"
-        grad_x = torch.empty_like(x) if precompute else None
-        xq, g_all = _run_chunks(x, weight, targets, vocab, softcap, chunk_rows, losses, grad_x, None,
-                                num_valid if reduction == "mean" else None, cache)
-        ctx.precomputed, ctx.weight = precompute, weight
-        ctx.args = (vocab, softcap, chunk_rows, cache)
-        if precompute:
-            ctx.save_for_backward(grad_x, g_all.data_t, g_all.inv_scale_t, xq.data_t, xq.inv_scale_t)
-        elif needs_grad:
-            ctx.save_for_backward(x, weight, targets)
-        if reduction == "mean":
-            return losses.sum() / num_valid  # ignored targets have loss 0
-        if reduction == "sum":
-            return losses.sum()
-        return losses
-
-    @staticmethod
-    def backward(ctx, g):
-        saved = ctx.saved_tensors
-        if not saved:
-            raise RuntimeError("softcap_cross_entropy: backward without grad mode in forward")
-        weight = ctx.weight
-        if ctx.precomputed:
-            grad_x, g_t, g_scale_t, x_t, x_scale_t = saved
-            gw = g.to(torch.float32).reshape(1)
-            if mx_grad_direct(weight):  # .grad (+)= g * dlogits^T . x, one GEMM
-                mx_grad_weights(g_t, g_scale_t, x_t, x_scale_t, [weight], gw)
-                return grad_x * g, None, None, None, None, None, None, None, None
-            dw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)
-            mx_gemm_f32(g_t, g_scale_t, x_t, x_scale_t, dw, False, gw)
-            return grad_x * g, dw.to(weight.dtype), None, None, None, None, None, None, None
-        x, weight, targets = saved
-        vocab, softcap, chunk_rows, cache = ctx.args
-        grad_x = torch.empty_like(x)
-        xq, g_all = _run_chunks(x, weight, targets, vocab, softcap, chunk_rows, None, grad_x,
-                                g.to(torch.float32).contiguous(), None, cache)
-        dw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)
-        mx_gemm_f32(g_all.data_t, g_all.inv_scale_t, xq.data_t, xq.inv_scale_t, dw, False)
-        return grad_x, dw.to(weight.dtype), None, None, None, None, None, None, None
-
-
 def softcap_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor, vocab_size: int,
                           softcap: float, chunk_rows: int, reduction: str = "mean",
                           cache: Optional[Fp8WeightCache] = None) -> torch.Tensor:
@@ -752,6 +531,5 @@ def softcap_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.
     if not (mx_fits(x.size(0), x.size(1)) and chunk_rows % 128 == 0 and weight.size(0) % 128 == 0
             and weight.size(0) >= vocab_size and weight.size(1) == x.size(1)):
         raise RuntimeError("softcap_cross_entropy: MX needs N, C, chunk_rows and the padded vocab % 128")
-    needs_grad = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
-    return _SoftcapCrossEntropy.apply(x.contiguous(), weight, targets.to(torch.int64).contiguous(), int(vocab_size),
-                                      float(softcap), int(chunk_rows), reduction, needs_grad, cache)
+    return native.softcap_cross_entropy(x, weight, targets, int(vocab_size), float(softcap), int(chunk_rows),
+                                        ("mean", "sum", "none").index(reduction), cache)

@@ -1,0 +1,88 @@
+"""The native host path (csrc/torch_engine.cpp) and the small kernels it launches, against torch on the same inputs."""
+import pytest
+import torch
+
+import nanochat_cpp_b200 as nc
+
+pytestmark = pytest.mark.gpu
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 16384])
+def test_loss_reductions(n):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    targets = torch.randint(-1, 4, (n,), generator=g, device="cuda")
+    losses = torch.rand(n, generator=g, device="cuda") * (targets >= 0)
+    count = torch.empty((), dtype=torch.int64, device="cuda")
+    assert nc.lib.mxb200_count_valid(targets.data_ptr(), n, count.data_ptr(), _stream()) == 0
+    assert count.item() == (targets >= 0).sum().item()
+    total = torch.empty((), device="cuda")
+    assert nc.lib.mxb200_reduce_losses(losses.data_ptr(), n, None, total.data_ptr(), _stream()) == 0
+    # fp32 sum of n non-negative values: n / 1024 terms per thread, then 10 butterfly steps, half an ulp each
+    bound = (n / 1024 + 11) * 2 ** -24 * losses.double().sum().item()
+    assert abs(total.double() - losses.double().sum()).item() <= bound
+    if count.item():
+        mean = torch.empty((), device="cuda")
+        assert nc.lib.mxb200_reduce_losses(losses.data_ptr(), n, count.data_ptr(), mean.data_ptr(), _stream()) == 0
+        assert torch.equal(mean, total / count)
+
+
+@pytest.mark.parametrize("n", [8, 8 * 257, 128 * 1664, 16384 * 1536])
+def test_scale_bf16_matches_torch(n):
+    x = torch.randn(n, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda").to(torch.bfloat16)
+    x[:3] = torch.tensor([float("nan"), float("inf"), -0.0])
+    scale = torch.tensor(0.7312, device="cuda")
+    y = torch.empty_like(x)
+    assert nc.lib.mxb200_scale_bf16(x.data_ptr(), scale.data_ptr(), y.data_ptr(), n, _stream()) == 0
+    assert torch.equal(y.nan_to_num(7.0), (x * scale).nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("cached", [False, True])
+def test_no_grad_forward_equals_training_forward(cached):
+    """Without grad only the row-wise layouts are made; the output is the same, and a cache is filled or left alone."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(384, 256, generator=g, device="cuda").to(torch.bfloat16)
+    ws = [torch.randn(n, 256, generator=g, device="cuda").requires_grad_() for n in (256, 128, 128)]
+    caches = [nc.Fp8WeightCache(cached) for _ in range(3)]
+    with torch.no_grad():
+        y = nc.fp8_matmul(x, ws[0], caches[0])
+        qkv = nc.fp8_qkv(x, *ws, cache=caches[1])
+        mlp = nc.fp8_relu_square_mlp(x, ws[0], torch.eye(256, device="cuda"), caches[2])
+        again = nc.fp8_matmul(x, ws[0], caches[0])
+    assert not y.requires_grad and torch.equal(y, again)
+    assert torch.equal(y, nc.fp8_matmul(x, ws[0]).detach())
+    assert torch.equal(y, nc.fp8_matmul(x, ws[0], caches[0]).detach())
+    assert all(torch.equal(a, b.detach()) for a, b in zip(qkv, nc.fp8_qkv(x, *ws, cache=caches[1])))
+    assert torch.equal(mlp, nc.fp8_relu_square_mlp(x, ws[0], torch.eye(256, device="cuda")).detach())
+
+
+def test_per_token_loss_with_cache_matches_without():
+    """Reduction none holds its cache in the graph node and uses it again in backward."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x0 = torch.randn(256, 128, generator=g, device="cuda").to(torch.bfloat16)
+    w0 = torch.randn(384, 128, generator=g, device="cuda") * 0.1
+    t = torch.randint(-1, 380, (256,), generator=g, device="cuda")
+    up = torch.rand(256, generator=g, device="cuda")
+    got = []
+    for cache in (None, nc.Fp8WeightCache(True)):
+        x, w = x0.clone().requires_grad_(), w0.clone().requires_grad_()
+        loss = nc.softcap_cross_entropy(x, w, t, 380, 15.0, 128, "none", cache)
+        del cache
+        loss.backward(up)
+        got.append((loss.detach(), x.grad, w.grad))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_backward_twice_needs_retain_graph():
+    x = torch.randn(128, 128, device="cuda").to(torch.bfloat16).requires_grad_()
+    w = torch.randn(128, 128, device="cuda").requires_grad_()
+    y = nc.fp8_matmul(x, w)
+    y.backward(torch.ones_like(y), retain_graph=True)
+    first = w.grad.clone()
+    y.backward(torch.ones_like(y))
+    assert torch.equal(w.grad, 2 * first)
+    with pytest.raises(RuntimeError):
+        y.backward(torch.ones_like(y))
