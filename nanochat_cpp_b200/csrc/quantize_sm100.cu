@@ -25,6 +25,7 @@
 #include "internal.h"
 #include "mx_common.cuh"
 #include "ptx_sm100.cuh"
+#include "softcap_table_sm100.cuh"
 
 namespace mxb200 {
 
@@ -59,10 +60,9 @@ struct QuantParams {
   SoftcapGrad ce;   // softcap gradient prologue only
 };
 
-// d loss_row / d z of one logit, before rounding: p = softmax of the capped logits, th = tanh(z / softcap). The
+// d loss_row / d z of one logit, before rounding, from th = tanh(z / softcap): p = softmax of the capped logits. The
 // expressions are the reference's (softcap_ce_kernel.cu:49-54), so the compiler contracts them the same way.
-__device__ __forceinline__ float softcap_ce_grad(float z, bool is_target, float lse, float softcap, float scale) {
-  const float th = tanhf(z / softcap);
+__device__ __forceinline__ float softcap_ce_grad(float th, bool is_target, float lse, float softcap, float scale) {
   const float p = expf(softcap * th - lse);
   return (p - (is_target ? 1.f : 0.f)) * (1.f - th * th) * scale;
 }
@@ -276,37 +276,13 @@ __device__ __forceinline__ void quantize_tile(const QuantParams& p, int tile_ind
       } else {
         float m = 0.f;
         uint32_t pk[8];
-        if constexpr (kPro == kSoftcapGrad) {
-          // the gradient as the reference's grad kernel would have written it in bf16: 0 for ignored rows and for
-          // the padding columns
-          const int64_t grow = row0 + r;
-          const int64_t target = p.ce.targets[grow];
-          if (target < 0) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
-              v[k] = 0.f;
-          } else {
-            const float lse = p.ce.lse[grow];
-            float scale = p.ce.grad_scale != nullptr ? p.ce.grad_scale[grow * p.ce.grad_scale_stride] : 1.f;
-            if (p.ce.num_valid != nullptr)
-              scale /= static_cast<float>(*p.ce.num_valid);
-            const int64_t gcol = col0 + c;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const float g = gcol + k < p.ce.vocab ? softcap_ce_grad(v[k], gcol + k == target, lse, p.ce.softcap, scale) : 0.f;
-              v[k] = bf16_round(g);
-              m = fmaxf(m, fabsf(v[k]));
-            }
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            float hv = 0.f;
-            if constexpr (kPro == kReluSquareBwd)
-              hv = (k & 1) ? __uint_as_float(rawh[it][k >> 1] & 0xffff0000u) : __uint_as_float(rawh[it][k >> 1] << 16);
-            v[k] = prologue<kPro>(v[k], hv);
-            m = fmaxf(m, fabsf(v[k]));
-          }
+        for (int k = 0; k < 16; ++k) {
+          float hv = 0.f;
+          if constexpr (kPro == kReluSquareBwd)
+            hv = (k & 1) ? __uint_as_float(rawh[it][k >> 1] & 0xffff0000u) : __uint_as_float(rawh[it][k >> 1] << 16);
+          v[k] = prologue<kPro>(v[k], hv);
+          m = fmaxf(m, fabsf(v[k]));
         }
         m_bits = __float_as_uint(m);
 #pragma unroll
@@ -379,7 +355,13 @@ struct StreamBarriers {
 // One pair of words per launch in flight, taken round-robin: the next tile to hand out and the CTAs that have left.
 constexpr int kStreamSchedSlots = 256;
 
-constexpr size_t kStreamSmemBytes = kStreamStages * kStreamTileBytes + 4 * kScaleTileBytes + sizeof(StreamBarriers);
+// A group is 256 threads with tile buffers, scale staging and barriers of their own; a CTA holds one (plain form, three
+// CTAs per SM) or, where the groups share a table, three (softcap form, one CTA per SM).
+constexpr size_t kStreamGroupBytes =
+      (kStreamStages * kStreamTileBytes + 4 * kScaleTileBytes + sizeof(StreamBarriers) + 127) / 128 * 128;
+constexpr int kSoftcapGroups = 3;
+constexpr size_t kSoftcapSmemBytes = kSoftcapGroups * kStreamGroupBytes + kLogitEntries * 4;
+static_assert(kSoftcapSmemBytes <= 232448, "shared memory per CTA");
 
 }  // namespace
 
@@ -438,26 +420,148 @@ __device__ __forceinline__ void stream_row_pass(const __nv_bfloat16* tile, const
   }
 }
 
+// Eight logits (4 packed words) that the table path does not take: outside the table's range, beyond the vocabulary
+// (`left` of them are inside) or holding the target (number `hit`). Out of line: it is rare, and eight evaluations of
+// tanh inlined at every use push the row pass out of the instruction cache.
+__device__ __noinline__ uint4 softcap_grad_direct(uint4 z, int left, int hit, float lse, float softcap, float scale) {
+  uint32_t w[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float g[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float v = i != 0 ? hi_f32(w[k]) : lo_f32(w[k]);
+      const float th = v == 0.f ? 0.f : softcap_tanh(v, softcap);
+      g[i] = 2 * k + i < left ? softcap_ce_grad(th, 2 * k + i == hit, lse, softcap, scale) : 0.f;
+    }
+    w[k] = pack_bf16x2_rn(g[0], g[1]);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Row pass of the softcap form: the logits of the tile become the loss's gradient, rounded to bf16 as the reference's grad
+// kernel would have written it (0 for ignored rows and for the padding columns), in place for the column pass, and leave
+// quantized row-wise. tanh comes from the CTA's table (softcap_table_sm100.cuh); what is left per logit is one exp and
+// three multiplies.
+__device__ __forceinline__ void stream_row_pass_softcap(__nv_bfloat16* tile, const QuantParams& p, int64_t row0,
+                                                        int64_t col0, unsigned char* sc_rows, uint32_t table_base,
+                                                        int t) {
+  constexpr int kIters = kTile * (kTile / 16) / kThreads;
+  const int piece = t & 7, c = piece * 16, swap = piece >> 2;
+  const bool want_rows = p.out.data != nullptr;
+  const int64_t gcol = col0 + c;
+  const int left = static_cast<int>(p.ce.vocab - gcol < 0 ? 0 : (p.ce.vocab - gcol > 16 ? 16 : p.ce.vocab - gcol));
+  int64_t target[kIters];
+  float lse[kIters], scale[kIters];
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int64_t grow = row0 + ((it * kThreads + t) >> 3);
+    target[it] = p.ce.targets[grow];
+    lse[it] = p.ce.lse[grow];
+    scale[it] = p.ce.grad_scale != nullptr ? p.ce.grad_scale[grow * p.ce.grad_scale_stride] : 1.f;
+  }
+  const float valid = p.ce.num_valid != nullptr ? static_cast<float>(*p.ce.num_valid) : 1.f;
+  const float one_over_valid = 1.f / valid;  // the scale of every row without an upstream gradient
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int r = (it * kThreads + t) >> 3;
+    uint4* cell = reinterpret_cast<uint4*>(tile + r * kTile + c);
+    const uint4 v0 = cell[swap], v1 = cell[swap ^ 1];
+    uint32_t w[2][4] = {{v0.x, v0.y, v0.z, v0.w}, {v1.x, v1.y, v1.z, v1.w}};  // columns c + 8 swap.., c + 8 (swap ^ 1)..
+    if (target[it] < 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        w[k >> 2][k & 3] = 0u;
+    } else {
+      const float s = p.ce.grad_scale == nullptr ? one_over_valid : scale[it] / valid;
+      const int64_t off = target[it] - gcol;
+      const int hit = off >= 0 && off < 16 ? static_cast<int>(off) : -1;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int first = 8 * (swap ^ h);  // of these 8 columns, within the thread's 16
+        if (left - first >= 8 && hit >> 3 != (swap ^ h) && logits_in_table(w[h])) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float lo = softcap_ce_grad(logit_lookup(table_base, w[h][k], 0), false, lse[it], p.ce.softcap, s);
+            const float hi = softcap_ce_grad(logit_lookup(table_base, w[h][k], 1), false, lse[it], p.ce.softcap, s);
+            w[h][k] = pack_bf16x2_rn(lo, hi);
+          }
+        } else {
+          const uint4 g = softcap_grad_direct(make_uint4(w[h][0], w[h][1], w[h][2], w[h][3]), left - first,
+                                              hit >> 3 == (swap ^ h) ? hit & 7 : -1, lse[it], p.ce.softcap, s);
+          w[h][0] = g.x, w[h][1] = g.y, w[h][2] = g.z, w[h][3] = g.w;
+        }
+      }
+    }
+    cell[swap] = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
+    cell[swap ^ 1] = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
+    if (want_rows) {
+      uint32_t m = 0u;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        m = max_abs_skip_nan_bf16x2(m, w[k >> 2][k & 3]);
+      m &= 0x7fff7fffu;
+      uint32_t m_bits = max(m & 0xffffu, m >> 16) << 16;
+      m_bits = max(m_bits, __shfl_xor_sync(0xffffffffu, m_bits, 1));
+      const int e = mx_exponent(m_bits, p.floor_rule);
+      const uint16_t mb = static_cast<uint16_t>(mx_multiplier_bits(e) >> 16);
+      const uint32_t a0 = e4m3x4_scaled_fma(w[0][0], w[0][1], mb, mb), a1 = e4m3x4_scaled_fma(w[0][2], w[0][3], mb, mb);
+      const uint32_t b0 = e4m3x4_scaled_fma(w[1][0], w[1][1], mb, mb), b1 = e4m3x4_scaled_fma(w[1][2], w[1][3], mb, mb);
+      const uint4 o = swap ? make_uint4(b0, b1, a0, a1) : make_uint4(a0, a1, b0, b1);
+      *reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.out.data) + (row0 + r) * p.out.ld + col0 + c) = o;
+      if ((t & 1) == 0)
+        sc_rows[mx_scale_tile_offset(r, c >> 5)] = static_cast<unsigned char>(e);
+    }
+  }
+}
+
+// The 256 threads of one group: a barrier of their own, and one that tells all of them whether every one said yes.
+__device__ __forceinline__ void group_sync(int bar) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kThreads) : "memory");
+}
+
+__device__ __forceinline__ bool group_all(int bar, bool yes) {
+  int all;
+  asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(all)
+        : "r"(static_cast<int>(yes)), "r"(bar), "n"(kThreads)
+        : "memory");
+  return all != 0;
+}
+
 struct StreamParams {
   QuantParams q;
   int tiles;
   int slot;
 };
 
+template <int kPro>
 __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const StreamParams& sp) {
+  constexpr int kGroups = kPro == kSoftcapGrad ? kSoftcapGroups : 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* sc = smem_raw + kStreamStages * kStreamTileBytes;  // [2 tiles in turn][rows, columns][512]
+  const int group = kGroups == 1 ? 0 : static_cast<int>(threadIdx.x) / kThreads;
+  const int t = kGroups == 1 ? static_cast<int>(threadIdx.x) : static_cast<int>(threadIdx.x) % kThreads;
+  unsigned char* buffers = smem_raw + group * kStreamGroupBytes;
+  unsigned char* sc = buffers + kStreamStages * kStreamTileBytes;  // [2 tiles in turn][rows, columns][512]
   StreamBarriers* bars = reinterpret_cast<StreamBarriers*>(sc + 4 * kScaleTileBytes);
   const QuantParams& p = sp.q;
-  const int t = static_cast<int>(threadIdx.x);
   const bool want_rows = p.out.data != nullptr, want_cols = p.out_t.data != nullptr;
-  uint32_t* sched = g_quantize_sched + 2 * sp.slot;  // [0] next tile to hand out, [1] CTAs that have left
+  uint32_t* sched = g_quantize_sched + 2 * sp.slot;  // [0] next tile to hand out, [1] groups that have left
+  const uint32_t walkers = gridDim.x * kGroups;      // groups go round the SMs before an SM gets its second
 
   if (t == 0) {
     for (int s = 0; s < kStreamStages; ++s)
       mbar_init(&bars->full[s], 1);
     bars->abort_flag = 0;
     fence_mbar_init();
+  }
+  uint32_t table_base = 0;
+  if constexpr (kPro == kSoftcapGrad) {
+    float* table = reinterpret_cast<float*>(smem_raw + kGroups * kStreamGroupBytes);
+    for (uint32_t i = threadIdx.x; i < kLogitEntries; i += kThreads * kGroups)
+      table[i] = softcap_tanh(logit_of_entry(i), p.ce.softcap);
+    table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
   }
   __syncthreads();
 
@@ -479,13 +583,13 @@ __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const 
     }
     bars->tile_of[s] = tile;
     mbar_arrive_expect_tx(1u, &bars->full[s], kStreamTileBytes);
-    tma_load_2d_hint(1u, smem_raw + s * kStreamTileBytes, map_x, &bars->full[s], (tile % p.tiles_c) * kTile,
+    tma_load_2d_hint(1u, buffers + s * kStreamTileBytes, map_x, &bars->full[s], (tile % p.tiles_c) * kTile,
                      (tile / p.tiles_c) * kTile, l2_policy_evict_first());
   };
   if (t == 0) {
-    post(0, static_cast<int>(blockIdx.x));
+    post(0, static_cast<int>(blockIdx.x + group * gridDim.x));
     for (int i = 1; i < kStreamStages && drawing; ++i)
-      post(i, static_cast<int>(gridDim.x + atomicAdd(&sched[0], 1u)));
+      post(i, static_cast<int>(walkers + atomicAdd(&sched[0], 1u)));
   }
 
   int i = 0;
@@ -493,24 +597,31 @@ __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const 
     const int s = i % kStreamStages;
     int drawn = 0;  // thread 0: the tile of iteration i + stages, asked for now and posted after this tile
     if (t == 0 && drawing)
-      drawn = static_cast<int>(gridDim.x + atomicAdd(&sched[0], 1u));
+      drawn = static_cast<int>(walkers + atomicAdd(&sched[0], 1u));
     const bool landed = stream_wait(&bars->full[s], static_cast<uint32_t>(i / kStreamStages) & 1u, bars,
                                     kStreamWaitLimitNs, static_cast<uint32_t>(i));
     const int tile = landed ? *reinterpret_cast<volatile int*>(&bars->tile_of[s]) : -1;
+    if (kPro == kSoftcapGrad && !group_all(1 + group, tile >= 0))
+      break;  // the passes meet at a barrier below: the group goes in together or not at all
     const int tile_r = tile / p.tiles_c, tile_c = tile % p.tiles_c;
     const int64_t row0 = static_cast<int64_t>(tile_r) * kTile, col0 = static_cast<int64_t>(tile_c) * kTile;
-    const __nv_bfloat16* buf = reinterpret_cast<const __nv_bfloat16*>(smem_raw + s * kStreamTileBytes);
+    __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(buffers + s * kStreamTileBytes);
     unsigned char* sc_rows = sc + (i & 1) * 2 * kScaleTileBytes;
     unsigned char* sc_cols = sc_rows + kScaleTileBytes;
     if (tile >= 0) {
-      if (want_rows)
+      if constexpr (kPro == kSoftcapGrad) {
+        stream_row_pass_softcap(buf, p, row0, col0, sc_rows, table_base, t);
+        fence_proxy_async_smem();  // these writes come before the load that reuses the buffer
+        group_sync(1 + group);
+      } else if (want_rows) {
         stream_row_pass(buf, p, row0, col0, sc_rows, t);
+      }
       if (want_cols)
         column_pass<false>(buf, p, row0, col0, sc_cols, t);
     }
     // every thread is done with the buffer and the scale bytes are staged; the stop sign, or a wait that gave up,
     // ends the walk for all threads together
-    if (__syncthreads_and(tile >= 0) == 0)
+    if (!group_all(1 + group, tile >= 0))
       break;
     if (t == 0 && drawing)
       post(i + kStreamStages, drawn);
@@ -529,7 +640,7 @@ __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const 
     }
     // the last CTA to leave hands the slot back zeroed
     __threadfence();
-    if (atomicAdd(&sched[1], 1u) == gridDim.x - 1) {
+    if (atomicAdd(&sched[1], 1u) == walkers - 1) {
       sched[0] = 0u;
       sched[1] = 0u;
       __threadfence();
@@ -589,11 +700,15 @@ MXB200_QUANTIZE_KERNEL(mxb200_quantize_bf16, false, mxb200::kNone, 4)
 MXB200_QUANTIZE_KERNEL(mxb200_quantize_f32, true, mxb200::kNone, 2)
 MXB200_QUANTIZE_KERNEL(mxb200_quantize_relu_square, false, mxb200::kReluSquare, 4)
 MXB200_QUANTIZE_KERNEL(mxb200_quantize_relu_square_bwd, false, mxb200::kReluSquareBwd, 3)
-MXB200_QUANTIZE_KERNEL(mxb200_quantize_softcap_grad, false, mxb200::kSoftcapGrad, 2)
 // Streaming form: persistent, three CTAs per SM, each with two 32 KB tile buffers.
 __global__ void __launch_bounds__(mxb200::kThreads, MXB200_STREAM_CTAS_PER_SM)
     mxb200_quantize_bf16_stream(const __grid_constant__ CUtensorMap map_x, const mxb200::StreamParams sp) {
-  mxb200::quantize_stream(&map_x, sp);
+  mxb200::quantize_stream<mxb200::kNone>(&map_x, sp);
+}
+// Softcap form: one CTA of three groups per SM around one table of tanh.
+__global__ void __launch_bounds__(mxb200::kThreads * mxb200::kSoftcapGroups, 1)
+    mxb200_quantize_softcap_grad(const __grid_constant__ CUtensorMap map_x, const mxb200::StreamParams sp) {
+  mxb200::quantize_stream<mxb200::kSoftcapGrad>(&map_x, sp);
 }
 MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_bf16, false, 4)
 MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_f32, true, 2)
@@ -612,8 +727,6 @@ constexpr QuantKernel quantize_kernel() {
     return mxb200_quantize_relu_square;
   else if constexpr (kPro == kReluSquareBwd)
     return mxb200_quantize_relu_square_bwd;
-  else if constexpr (kPro == kSoftcapGrad)
-    return mxb200_quantize_softcap_grad;
   else
     return mxb200_quantize_bf16;
 }
@@ -652,7 +765,8 @@ int launch(const QuantParams& p, int64_t tiles, cudaStream_t stream) {
   return launch_status();
 }
 
-// The streaming kernel on a plain bf16 tensor: (rows, ld) row-major behind a tiled map with a 128 x 128 box.
+// A streaming kernel on a bf16 tensor: (rows, ld) row-major behind a tiled map with a 128 x 128 box.
+template <int kPro>
 int launch_stream(const QuantParams& p, int64_t rows, int64_t cols, int64_t tiles, int sms, cudaStream_t stream) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr)
@@ -666,19 +780,22 @@ int launch_stream(const QuantParams& p, int64_t rows, int64_t cols, int64_t tile
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return MXB200_ERR_DRIVER;
+  constexpr bool softcap = kPro == kSoftcapGrad;
+  constexpr auto kernel = softcap ? mxb200_quantize_softcap_grad : mxb200_quantize_bf16_stream;
+  constexpr size_t smem = softcap ? kSoftcapSmemBytes : kStreamGroupBytes;
   static std::atomic<int> configured_for{-1};
   int device = 0;
   cudaGetDevice(&device);
   if (configured_for.load() != device) {
-    if (cudaFuncSetAttribute(mxb200_quantize_bf16_stream, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kStreamSmemBytes)) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
       return MXB200_ERR_LAUNCH;
     configured_for.store(device);
   }
   static std::atomic<uint32_t> next_slot{0};
   const StreamParams sp{p, static_cast<int>(tiles), static_cast<int>(next_slot.fetch_add(1) % kStreamSchedSlots)};
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, kStreamCtasPerSm * static_cast<int64_t>(sms)));
-  mxb200_quantize_bf16_stream<<<grid, kThreads, kStreamSmemBytes, stream>>>(map, sp);
+  const int64_t most = softcap ? sms : kStreamCtasPerSm * static_cast<int64_t>(sms);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, most));
+  kernel<<<grid, softcap ? kThreads * kSoftcapGroups : kThreads, smem, stream>>>(map, sp);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return launch_status();
 }
@@ -722,14 +839,14 @@ int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t co
     case kNone:
       // more tiles than the one-shot kernel holds at once (4 CTAs per SM): stream them through persistent CTAs
       if (tiles > 4 * static_cast<int64_t>(dev.sms))
-        return launch_stream(p, rows, cols, tiles, dev.sms, s);
+        return launch_stream<kNone>(p, rows, cols, tiles, dev.sms, s);
       return launch<false, kNone>(p, tiles, s);
     case kReluSquare:
       return launch<false, kReluSquare>(p, tiles, s);
     case kReluSquareBwd:
       return launch<false, kReluSquareBwd>(p, tiles, s);
     case kSoftcapGrad:
-      return ce != nullptr ? launch<false, kSoftcapGrad>(p, tiles, s) : MXB200_ERR_NULL;
+      return ce != nullptr ? launch_stream<kSoftcapGrad>(p, rows, cols, tiles, dev.sms, s) : MXB200_ERR_NULL;
     default:
       return MXB200_ERR_ARGUMENT;
   }

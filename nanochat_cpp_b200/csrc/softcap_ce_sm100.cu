@@ -7,14 +7,13 @@
 // reference's: 256 threads per row, thread t adds columns t * 8 + 2048 * i + k in order of i then k, a butterfly
 // (xor 16..1) inside each warp, then the eight warp sums again by butterfly in warp 0. |capped| <= softcap, so
 // exp(capped - softcap) needs no running maximum.
-// A row of 32768 logits costs one tanh and one exp per element: the pass is bound by the SFU/ALU work, not by HBM
-// (64 KB per row).
 #include <algorithm>
 
 #include <cuda_bf16.h>
 
 #include "bf16x2_sm100.cuh"
 #include "internal.h"
+#include "softcap_table_sm100.cuh"
 
 namespace mxb200 {
 
@@ -23,56 +22,127 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kVec = 8;
 
-__device__ __forceinline__ float row_sum(float v, float* smem) {
+// The row's sum over its 256 threads in the reference's order. `bar`: the group's named barrier; smem: 8 floats per group.
+__device__ __forceinline__ float row_sum(float v, float* smem, int bar) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = static_cast<int>(threadIdx.x) & 31, warp = static_cast<int>(threadIdx.x) >> 5;
+  const int lane = static_cast<int>(threadIdx.x) & 31, warp = (static_cast<int>(threadIdx.x) >> 5) & 7;
   if (lane == 0)
     smem[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < kThreads / 32 ? smem[lane] : 0.f;
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(kThreads) : "memory");
+  v = lane < kThreads / 32 ? smem[lane] : 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0)
-      smem[0] = v;
-  }
-  __syncthreads();
-  return smem[0];
+  for (int o = 16; o > 0; o >>= 1)
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(kThreads) : "memory");  // before the next row's sums overwrite these
+  return v;
 }
 
-__global__ void __launch_bounds__(kThreads) mxb200_softcap_ce_loss_kernel(const __nv_bfloat16* logits, int64_t ld,
-                                                                          const int64_t* targets, int vocab, int padded,
-                                                                          float softcap, float* loss, float* lse_out) {
-  __shared__ float smem[kThreads / 32];
-  const int64_t row = blockIdx.x;
-  const __nv_bfloat16* z = logits + row * ld;
-  const int64_t target = targets[row];
-  if (target < 0) {  // ignored row: loss 0, lse left unset
-    if (loss != nullptr && threadIdx.x == 0)
-      loss[row] = 0.f;
-    return;
-  }
-  float sum = 0.f;
-  for (int j = static_cast<int>(threadIdx.x) * kVec; j < padded; j += kThreads * kVec) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(z + j);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+struct LossParams {
+  const __nv_bfloat16* logits;
+  int64_t ld;
+  const int64_t* targets;
+  int64_t rows;
+  int vocab, padded;
+  float softcap;
+  float* loss;
+  float* lse;
+};
+
+// Adds the terms of eight logits, the first `left` of them inside the vocabulary.
+__device__ __forceinline__ float add_direct(float sum, uint4 z, int left, float at_zero, float softcap) {
+  const uint32_t w[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
-    for (int k = 0; k < kVec; ++k) {
-      const float v = __uint_as_float((k & 1) ? (w[k >> 1] & 0xffff0000u) : (w[k >> 1] << 16));
-      if (j + k < vocab)
-        sum += expf(softcap * tanhf(v / softcap) - softcap);
+  for (int k = 0; k < kVec; ++k) {
+    const float v = (k & 1) ? hi_f32(w[k >> 1]) : lo_f32(w[k >> 1]);
+    if (k < left)
+      sum += v == 0.f ? at_zero : softcap_loss_term(v, softcap);
+  }
+  return sum;
+}
+
+// The same beside the table's path, where it is rare: out of the loop's registers and instructions.
+__device__ __noinline__ float add_direct_outlined(float sum, uint4 z, int left, float at_zero, float softcap) {
+  return add_direct(sum, z, left, at_zero, softcap);
+}
+
+constexpr uint32_t kLossTableBytes = kLogitEntries * 4;
+
+// A row per 256 threads, kGroups rows at a time per CTA, persistent over rows.
+//
+// kTable: exp(capped - softcap) comes from a table of the CTA's (softcap_table_sm100.cuh). Bound by shared memory: 32
+// random reads per instruction take about 3.5 bank cycles, so 2048 x 32768 logits need 27 us of them at 1.85 GHz against
+// 20 us for the bytes.
+template <bool kTable, int kGroups, int kCtas>
+__global__ void __launch_bounds__(kThreads * kGroups, kCtas) mxb200_softcap_ce_loss_kernel(const LossParams p) {
+  extern __shared__ __align__(16) float table[];
+  __shared__ float smem[kGroups][kThreads / 32];
+  const int group = static_cast<int>(threadIdx.x) / kThreads, t = static_cast<int>(threadIdx.x) % kThreads;
+  if constexpr (kTable) {
+    for (uint32_t i = threadIdx.x; i < kLogitEntries; i += kThreads * kGroups)
+      table[i] = softcap_loss_term(logit_of_entry(i), p.softcap);
+    __syncthreads();
+  }
+  const float at_zero = softcap_loss_term(0.f, p.softcap);
+  const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
+  // rows go round the CTAs first and their groups second, so that every SM gets the same number of rows
+  for (int64_t row = blockIdx.x + static_cast<int64_t>(group) * gridDim.x; row < p.rows;
+       row += static_cast<int64_t>(gridDim.x) * kGroups) {
+    const __nv_bfloat16* z = p.logits + row * p.ld;
+    const int64_t target = p.targets[row];
+    if (target < 0) {  // ignored row: loss 0, lse left unset
+      if (p.loss != nullptr && t == 0)
+        p.loss[row] = 0.f;
+      continue;
+    }
+    float sum = 0.f;
+    // two vectors ahead of the one being added up: the additions are a serial chain per thread
+    constexpr int kStep = kThreads * kVec;
+    const auto load = [&](int j) {
+      return j < p.padded ? *reinterpret_cast<const uint4*>(z + j) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    int j = t * kVec;
+    uint4 next[2] = {load(j), load(j + kStep)};
+    const auto add = [&](const uint4& raw) {
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+      if (kTable && j + kVec <= p.vocab && logits_in_table(w)) {
+#pragma unroll
+        for (int k = 0; k < kVec; ++k)
+          sum += logit_lookup(table_base, w[k >> 1], k & 1);
+      } else {
+        sum = kTable ? add_direct_outlined(sum, raw, p.vocab - j, at_zero, p.softcap)
+                     : add_direct(sum, raw, p.vocab - j, at_zero, p.softcap);
+      }
+      j += kStep;
+    };
+    while (j < p.padded) {
+      const uint4 a = next[0];
+      next[0] = load(j + 2 * kStep);
+      add(a);
+      if (j >= p.padded)
+        break;
+      const uint4 b = next[1];
+      next[1] = load(j + 2 * kStep);
+      add(b);
+    }
+    const float lse = p.softcap + logf(row_sum(sum, smem[group], 1 + group));
+    if (t == 0) {
+      if (p.loss != nullptr)
+        p.loss[row] = lse - p.softcap * tanhf(__bfloat162float(z[target]) / p.softcap);
+      if (p.lse != nullptr)
+        p.lse[row] = lse;
     }
   }
-  const float lse = softcap + logf(row_sum(sum, smem));
-  if (threadIdx.x == 0) {
-    if (loss != nullptr)
-      loss[row] = lse - softcap * tanhf(__bfloat162float(z[target]) / softcap);
-    if (lse_out != nullptr)
-      lse_out[row] = lse;
-  }
+}
+
+template <bool kTable, int kGroups, int kCtas>
+int launch_loss(const LossParams& p, int sms, cudaStream_t stream) {
+  const int64_t ctas = std::min<int64_t>((p.rows + kGroups - 1) / kGroups, static_cast<int64_t>(sms) * kCtas);
+  mxb200_softcap_ce_loss_kernel<kTable, kGroups, kCtas>
+        <<<static_cast<unsigned>(ctas), kThreads * kGroups, kTable ? kLossTableBytes : 0, stream>>>(p);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return launch_status();
 }
 
 // ---- the small reductions around the chunks: one block each, a few microseconds for any batch of tokens
@@ -147,10 +217,17 @@ extern "C" int mxb200_softcap_ce_loss(const void* logits, int64_t rows, int64_t 
     return MXB200_ERR_ARGUMENT;
   if (!aligned16(logits))
     return MXB200_ERR_ALIGNMENT;
-  mxb200_softcap_ce_loss_kernel<<<static_cast<unsigned>(rows), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(logits), ld, targets, vocab, padded, softcap, loss, lse);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  const LossParams p{static_cast<const __nv_bfloat16*>(logits), ld, targets, rows, vocab, padded, softcap, loss, lse};
+  auto* s = static_cast<cudaStream_t>(stream);
+  // The table is worth making where a CTA looks up at least twice its entries. With less than two rows per SM and group
+  // a CTA takes single rows, so that they spread over the SMs.
+  const auto pays = [&](int64_t ctas) { return rows * padded >= 2 * static_cast<int64_t>(kLogitEntries) * ctas; };
+  const int64_t sms = dev.sms;
+  if (rows >= 4 * sms && pays(3 * sms))
+    return launch_loss<true, 2, 3>(p, dev.sms, s);
+  if (pays(std::min<int64_t>(rows, 6 * sms)))
+    return launch_loss<true, 1, 6>(p, dev.sms, s);
+  return launch_loss<false, 1, 6>(p, dev.sms, s);
 }
 
 extern "C" int mxb200_count_valid(const int64_t* targets, int64_t n, int64_t* out, void* stream) {

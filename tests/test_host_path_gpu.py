@@ -17,16 +17,16 @@ def test_loss_reductions(n):
     targets = torch.randint(-1, 4, (n,), generator=g, device="cuda")
     losses = torch.rand(n, generator=g, device="cuda") * (targets >= 0)
     count = torch.empty((), dtype=torch.int64, device="cuda")
-    assert nc.lib.mxb200_count_valid(targets.data_ptr(), n, count.data_ptr(), _stream()) == 0
+    assert nc.capi.lib.mxb200_count_valid(targets.data_ptr(), n, count.data_ptr(), _stream()) == 0
     assert count.item() == (targets >= 0).sum().item()
     total = torch.empty((), device="cuda")
-    assert nc.lib.mxb200_reduce_losses(losses.data_ptr(), n, None, total.data_ptr(), _stream()) == 0
+    assert nc.capi.lib.mxb200_reduce_losses(losses.data_ptr(), n, None, total.data_ptr(), _stream()) == 0
     # fp32 sum of n non-negative values: n / 1024 terms per thread, then 10 butterfly steps, half an ulp each
     bound = (n / 1024 + 11) * 2 ** -24 * losses.double().sum().item()
     assert abs(total.double() - losses.double().sum()).item() <= bound
     if count.item():
         mean = torch.empty((), device="cuda")
-        assert nc.lib.mxb200_reduce_losses(losses.data_ptr(), n, count.data_ptr(), mean.data_ptr(), _stream()) == 0
+        assert nc.capi.lib.mxb200_reduce_losses(losses.data_ptr(), n, count.data_ptr(), mean.data_ptr(), _stream()) == 0
         assert torch.equal(mean, total / count)
 
 
@@ -36,7 +36,7 @@ def test_scale_bf16_matches_torch(n):
     x[:3] = torch.tensor([float("nan"), float("inf"), -0.0])
     scale = torch.tensor(0.7312, device="cuda")
     y = torch.empty_like(x)
-    assert nc.lib.mxb200_scale_bf16(x.data_ptr(), scale.data_ptr(), y.data_ptr(), n, _stream()) == 0
+    assert nc.capi.lib.mxb200_scale_bf16(x.data_ptr(), scale.data_ptr(), y.data_ptr(), n, _stream()) == 0
     assert torch.equal(y.nan_to_num(7.0), (x * scale).nan_to_num(7.0))
 
 
