@@ -32,14 +32,35 @@ int current_device(DeviceInfo* info) {
   return d.cc_major == 10 ? MXB200_OK : MXB200_ERR_DEVICE;
 }
 
+static EncodeTiledFn g_driver_encode = nullptr;
+
+// The driver's encode wants a context current on the calling thread. A thread whose first CUDA call this is (an autograd
+// worker whose buffers came out of a warm allocator) has none yet: the runtime then binds the device's own.
+static CUresult encode_bound(CUtensorMap* map, CUtensorMapDataType type, cuuint32_t rank, void* base,
+                             const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                             const cuuint32_t* element_strides, CUtensorMapInterleave interleave,
+                             CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion, CUtensorMapFloatOOBfill fill) {
+  const auto encode = [&] {
+    return g_driver_encode(map, type, rank, base, dims, strides, box, element_strides, interleave, swizzle, promotion, fill);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess)
+      r = encode();
+  }
+  return r;
+}
+
 EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
+  static const EncodeTiledFn fn = [] {
     void* f = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
         q != cudaDriverEntryPointSuccess)
       f = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
+    g_driver_encode = reinterpret_cast<EncodeTiledFn>(f);
+    return f != nullptr ? &encode_bound : EncodeTiledFn{nullptr};
   }();
   return fn;
 }

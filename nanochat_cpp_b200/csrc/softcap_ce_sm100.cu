@@ -67,69 +67,94 @@ __device__ __noinline__ float add_direct_outlined(float sum, uint4 z, int left, 
   return add_direct(sum, z, left, at_zero, softcap);
 }
 
-constexpr uint32_t kLossTableBytes = kLogitEntries * 4;
+// The table of exp(capped - softcap) (softcap_table_sm100.cuh says why) of this kernel covers |z| in [2^-25, 2^7), 4096
+// magnitudes, so that one packed subtraction and an or per two logits tell whether a lookup is allowed. Entries of positive
+// logits sit at the front of shared memory and those of negative ones 128 KB further on: the address is the logit's 16
+// bits times 4, a shift and a mask. That takes the SM's whole shared memory, so one CTA serves it.
+constexpr uint32_t kTermLow = (127 - 25) << 7;
+constexpr uint32_t kTermMagnitudes = 4096;
+constexpr uint32_t kLossTableBytes = 0x8000 * 4 + kTermMagnitudes * 4;
+static_assert(kTermLow + kTermMagnitudes == kLogitHigh && kLossTableBytes <= 232448);
 
-// A row per 256 threads, kGroups rows at a time per CTA, persistent over rows.
-//
-// kTable: exp(capped - softcap) comes from a table of the CTA's (softcap_table_sm100.cuh). Bound by shared memory: 32
-// random reads per instruction take about 3.5 bank cycles, so 2048 x 32768 logits need 27 us of them at 1.85 GHz against
-// 20 us for the bytes.
+// A row per 256 threads, kGroups rows at a time per CTA, persistent over rows. With the table it is bound by shared
+// memory: 32 random reads per instruction take about 3.6 bank cycles, so 2048 x 32768 logits need 27 us of them at 1.85
+// GHz against 20 us for the bytes; evaluated directly they took 106 us.
 template <bool kTable, int kGroups, int kCtas>
 __global__ void __launch_bounds__(kThreads * kGroups, kCtas) mxb200_softcap_ce_loss_kernel(const LossParams p) {
   extern __shared__ __align__(16) float table[];
   __shared__ float smem[kGroups][kThreads / 32];
   const int group = static_cast<int>(threadIdx.x) / kThreads, t = static_cast<int>(threadIdx.x) % kThreads;
+  // rows go round the CTAs first and their groups second, so that every SM gets the same number of rows
+  const int64_t first_row = blockIdx.x + static_cast<int64_t>(group) * gridDim.x;
+  const int64_t row_step = static_cast<int64_t>(gridDim.x) * kGroups;
+  constexpr int kStep = kThreads * kVec;
+  // vectors in flight ahead of the one being added up (the additions are a serial chain per thread); those of a row's
+  // start are asked for before the table is made or the row before is summed up
+  constexpr int kAhead = kTable ? 4 : 2;
+  uint4 next[kAhead];
+  const auto load = [&](int64_t row, int j) {
+    return row < p.rows && j < p.padded ? *reinterpret_cast<const uint4*>(p.logits + row * p.ld + j)
+                                        : make_uint4(0u, 0u, 0u, 0u);
+  };
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k)
+    next[k] = load(first_row, t * kVec + k * kStep);
   if constexpr (kTable) {
-    for (uint32_t i = threadIdx.x; i < kLogitEntries; i += kThreads * kGroups)
-      table[i] = softcap_loss_term(logit_of_entry(i), p.softcap);
+    for (uint32_t i = threadIdx.x; i < kTermMagnitudes; i += kThreads * kGroups) {
+      const float th = softcap_tanh(__uint_as_float((kTermLow + i) << 16), p.softcap);  // of -z: -th
+      table[i] = expf(p.softcap * th - p.softcap);
+      table[0x8000 + i] = expf(p.softcap * -th - p.softcap);
+    }
     __syncthreads();
   }
   const float at_zero = softcap_loss_term(0.f, p.softcap);
-  const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
-  // rows go round the CTAs first and their groups second, so that every SM gets the same number of rows
-  for (int64_t row = blockIdx.x + static_cast<int64_t>(group) * gridDim.x; row < p.rows;
-       row += static_cast<int64_t>(gridDim.x) * kGroups) {
-    const __nv_bfloat16* z = p.logits + row * p.ld;
+  const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 4 * kTermLow;
+  for (int64_t row = first_row; row < p.rows; row += row_step) {
     const int64_t target = p.targets[row];
+    float sum = 0.f;
+    const auto add = [&](const uint4& raw, int j) {
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+      // no bit above the 12 of a table index may be set in any (magnitude - low); a borrow out of the low half sets its
+      // own upper bits
+      uint32_t outside = 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        outside |= (w[k] & 0x7fff7fffu) - kTermLow * 0x10001u;
+      if (kTable && j + kVec <= p.vocab && (outside & 0xf000f000u) == 0u) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          sum += load_shared_f32(table_base + ((w[k] << 2) & 0x3fffcu));
+          sum += load_shared_f32(table_base + ((w[k] >> 14) & 0x3fffcu));
+        }
+      } else {
+        sum = kTable ? add_direct_outlined(sum, raw, p.vocab - j, at_zero, p.softcap)
+                     : add_direct(sum, raw, p.vocab - j, at_zero, p.softcap);
+      }
+    };
+    if (target >= 0) {
+      for (int j = t * kVec; j < p.padded; j += kAhead * kStep) {
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          const int at = j + k * kStep;
+          const uint4 raw = next[k];
+          next[k] = load(row, at + kAhead * kStep);
+          if (at < p.padded)
+            add(raw, at);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      next[k] = load(row + row_step, t * kVec + k * kStep);
     if (target < 0) {  // ignored row: loss 0, lse left unset
       if (p.loss != nullptr && t == 0)
         p.loss[row] = 0.f;
       continue;
     }
-    float sum = 0.f;
-    // two vectors ahead of the one being added up: the additions are a serial chain per thread
-    constexpr int kStep = kThreads * kVec;
-    const auto load = [&](int j) {
-      return j < p.padded ? *reinterpret_cast<const uint4*>(z + j) : make_uint4(0u, 0u, 0u, 0u);
-    };
-    int j = t * kVec;
-    uint4 next[2] = {load(j), load(j + kStep)};
-    const auto add = [&](const uint4& raw) {
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-      if (kTable && j + kVec <= p.vocab && logits_in_table(w)) {
-#pragma unroll
-        for (int k = 0; k < kVec; ++k)
-          sum += logit_lookup(table_base, w[k >> 1], k & 1);
-      } else {
-        sum = kTable ? add_direct_outlined(sum, raw, p.vocab - j, at_zero, p.softcap)
-                     : add_direct(sum, raw, p.vocab - j, at_zero, p.softcap);
-      }
-      j += kStep;
-    };
-    while (j < p.padded) {
-      const uint4 a = next[0];
-      next[0] = load(j + 2 * kStep);
-      add(a);
-      if (j >= p.padded)
-        break;
-      const uint4 b = next[1];
-      next[1] = load(j + 2 * kStep);
-      add(b);
-    }
     const float lse = p.softcap + logf(row_sum(sum, smem[group], 1 + group));
     if (t == 0) {
       if (p.loss != nullptr)
-        p.loss[row] = lse - p.softcap * tanhf(__bfloat162float(z[target]) / p.softcap);
+        p.loss[row] = lse - p.softcap * tanhf(__bfloat162float(p.logits[row * p.ld + target]) / p.softcap);
       if (p.lse != nullptr)
         p.lse[row] = lse;
     }
@@ -137,10 +162,17 @@ __global__ void __launch_bounds__(kThreads * kGroups, kCtas) mxb200_softcap_ce_l
 }
 
 template <bool kTable, int kGroups, int kCtas>
-int launch_loss(const LossParams& p, int sms, cudaStream_t stream) {
-  const int64_t ctas = std::min<int64_t>((p.rows + kGroups - 1) / kGroups, static_cast<int64_t>(sms) * kCtas);
-  mxb200_softcap_ce_loss_kernel<kTable, kGroups, kCtas>
-        <<<static_cast<unsigned>(ctas), kThreads * kGroups, kTable ? kLossTableBytes : 0, stream>>>(p);
+int launch_loss(const LossParams& p, const DeviceInfo& dev, cudaStream_t stream) {
+  constexpr auto kernel = mxb200_softcap_ce_loss_kernel<kTable, kGroups, kCtas>;
+  constexpr size_t smem = kTable ? kLossTableBytes : 0;
+  static std::atomic<int> configured_for{-1};
+  if (kTable && configured_for.load() != dev.device) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+      return MXB200_ERR_LAUNCH;
+    configured_for.store(dev.device);
+  }
+  const int64_t ctas = std::min<int64_t>(p.rows, static_cast<int64_t>(dev.sms) * kCtas);
+  kernel<<<static_cast<unsigned>(ctas), kThreads * kGroups, smem, stream>>>(p);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return launch_status();
 }
@@ -219,15 +251,10 @@ extern "C" int mxb200_softcap_ce_loss(const void* logits, int64_t rows, int64_t 
     return MXB200_ERR_ALIGNMENT;
   const LossParams p{static_cast<const __nv_bfloat16*>(logits), ld, targets, rows, vocab, padded, softcap, loss, lse};
   auto* s = static_cast<cudaStream_t>(stream);
-  // The table is worth making where a CTA looks up at least twice its entries. With less than two rows per SM and group
-  // a CTA takes single rows, so that they spread over the SMs.
-  const auto pays = [&](int64_t ctas) { return rows * padded >= 2 * static_cast<int64_t>(kLogitEntries) * ctas; };
-  const int64_t sms = dev.sms;
-  if (rows >= 4 * sms && pays(3 * sms))
-    return launch_loss<true, 2, 3>(p, dev.sms, s);
-  if (pays(std::min<int64_t>(rows, 6 * sms)))
-    return launch_loss<true, 1, 6>(p, dev.sms, s);
-  return launch_loss<false, 1, 6>(p, dev.sms, s);
+  // the table is worth making where a CTA looks up at least three times its entries (a CTA makes 8 per thread)
+  if (rows * padded >= 3 * 2 * static_cast<int64_t>(kTermMagnitudes) * std::min<int64_t>(rows, dev.sms))
+    return launch_loss<true, 4, 1>(p, dev, s);
+  return launch_loss<false, 1, 6>(p, dev, s);
 }
 
 extern "C" int mxb200_count_valid(const int64_t* targets, int64_t n, int64_t* out, void* stream) {

@@ -86,3 +86,22 @@ def test_backward_twice_needs_retain_graph():
     assert torch.equal(w.grad, 2 * first)
     with pytest.raises(RuntimeError):
         y.backward(torch.ones_like(y))
+
+
+def test_first_call_of_a_fresh_thread_may_be_a_gemm():
+    """A thread without a CUDA context of its own yet (an autograd worker) can start with a launch that encodes tensor
+    maps: its buffers come out of the allocator's cache without a CUDA call."""
+    import threading
+    q = nc.quantize_mx(torch.randn(256, 256, device="cuda"))
+    want, got = torch.empty(256, 256, device="cuda"), torch.zeros(256, 256, device="cuda")
+    args = (q.data.data_ptr(), q.inv_scale.data_ptr()) * 2
+    stream, status = _stream(), []
+    lib = nc.capi.lib
+    assert lib.mxb200_gemm_f32(*args, want.data_ptr(), 256, 256, 256, None, 0, stream) == 0
+    torch.cuda.synchronize()
+    t = threading.Thread(target=lambda: status.append(
+        lib.mxb200_gemm_f32(*args, got.data_ptr(), 256, 256, 256, None, 0, stream)))
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert status == [0] and torch.equal(got, want)
