@@ -217,6 +217,30 @@ MXB200_API int mxb200_gemm_splitk_static(const void* a, const void* a_scale, con
                                          int out_kind, const void* resid, int64_t M, int64_t N, int64_t K,
                                          const float* alpha, int accumulate, int splits, void* stream);
 
+/* One GEMM of a group: the arguments of mxb200_gemm_bf16 (out_kind BF16, resid optional) or mxb200_gemm_f32 (out_kind
+ * F32, alpha and accumulate). */
+typedef struct mxb200_gemm_desc {
+  const void* a;
+  const void* a_scale;
+  const void* b;
+  const void* b_scale;
+  void* d;
+  const void* resid;
+  const float* alpha;
+  int64_t M, N, K;
+  int32_t out_kind;
+  int32_t accumulate;
+} mxb200_gemm_desc;
+
+/* n independent GEMMs in as few launches as possible, bit for bit what n calls of mxb200_gemm_bf16 / mxb200_gemm_f32 (or
+ * mxb200_gemm_splitk, where the library splits K) give. For the GEMMs a backward runs on the same operands (the
+ * reference launches them one after another, fp8.cpp:299-337, 456-460): the tiles of up to three share one launch, so
+ * that shapes with fewer tiles than the machine has CTA pairs fill it together. They run in the order given as far as
+ * their tiles are taken up in order. workspace: mxb200_gemm_group_workspace_bytes (0: none needed), 256-byte aligned,
+ * uninitialised, reusable by later calls on the same stream. */
+MXB200_API size_t mxb200_gemm_group_workspace_bytes(const mxb200_gemm_desc* g, int n);
+MXB200_API int mxb200_gemm_group(const mxb200_gemm_desc* g, int n, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Static message for a status (the reference's seam returns const char* messages, mx_gemm_kernel.h:12). */
 MXB200_API const char* mxb200_strerror(int status);
 
@@ -232,7 +256,7 @@ MXB200_API int mxb200_device_status(uint32_t* word);
 MXB200_API int mxb200_selftest_bounded_wait(uint64_t limit_ns, void* stream);
 
 /* Tuning knobs for measurement, process-wide. tile_n: 128 or 256 = the one-CTA kernel with 128 x tile_n tiles;
- * 384 / 512 = the CTA-pair kernel (256 x 192 / 256 x 256 tile over two SMs); 0 = choose per shape. max_ctas: CTAs of the persistent
+ * 384 / 512 / 640 = the CTA-pair kernel (256 x 192 / 256 x 256 / 256 x 128 tile over two SMs); 0 = choose per shape. max_ctas: CTAs of the persistent
  * grid (0 = one per SM). Not part of the reference interface. */
 MXB200_API int mxb200_set_gemm_config(int tile_n, int max_ctas);
 

@@ -24,6 +24,7 @@ SYMBOLS = (
     "mxb200_gemm_relu_square", "mxb200_gemm_relu_square_bwd", "mxb200_residual_norm_mx_fwd",
     "mxb200_softcap_ce_loss", "mxb200_softcap_ce_grad_mx",
     "mxb200_count_valid", "mxb200_reduce_losses", "mxb200_scale_bf16",
+    "mxb200_gemm_group_workspace_bytes", "mxb200_gemm_group",
     "mxb200_gemm_splits", "mxb200_gemm_workspace_bytes", "mxb200_gemm_splitk", "mxb200_gemm_splitk_static",
     "mxb200_strerror",
     "mxb200_device_status", "mxb200_selftest_bounded_wait", "mxb200_set_gemm_config", "mxb200_launch_count", "mxb200_version",
@@ -50,6 +51,13 @@ class ResidualNormMx(ctypes.Structure):
                 ("out", MxOut), ("out_t", MxOut), ("n_cols", ctypes.c_int32)]
 
 
+class GemmDesc(ctypes.Structure):
+    """mxb200_gemm_desc."""
+    _fields_ = [("a", ctypes.c_void_p), ("a_scale", ctypes.c_void_p), ("b", ctypes.c_void_p), ("b_scale", ctypes.c_void_p),
+                ("d", ctypes.c_void_p), ("resid", ctypes.c_void_p), ("alpha", ctypes.c_void_p), ("M", ctypes.c_int64),
+                ("N", ctypes.c_int64), ("K", ctypes.c_int64), ("out_kind", ctypes.c_int32), ("accumulate", ctypes.c_int32)]
+
+
 class Mxb200Error(RuntimeError):
     def __init__(self, status: int, what: str):
         self.status = status
@@ -73,6 +81,9 @@ def _load() -> ctypes.CDLL:
     f32 = ctypes.c_float
     lib.mxb200_softcap_ce_loss.argtypes = [vp, i64, i64, vp, i32, i32, f32, vp, vp, vp]
     lib.mxb200_softcap_ce_grad_mx.argtypes = [vp, i64, i64, vp, vp, i32, i32, f32, vp, i64, vp, MxOut, MxOut, i32, vp]
+    lib.mxb200_gemm_group_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc), i32]
+    lib.mxb200_gemm_group_workspace_bytes.restype = ctypes.c_size_t
+    lib.mxb200_gemm_group.argtypes = [ctypes.POINTER(GemmDesc), i32, vp, ctypes.c_size_t, vp]
     lib.mxb200_count_valid.argtypes = [vp, i64, vp, vp]
     lib.mxb200_reduce_losses.argtypes = [vp, i64, vp, vp, vp]
     lib.mxb200_scale_bf16.argtypes = [vp, vp, vp, i64, vp]

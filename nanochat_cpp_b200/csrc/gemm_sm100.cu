@@ -122,7 +122,27 @@ struct GemmParams {
   int q_scale_tiles, qt_scale_tiles;
   const void* h_in;
   bool floor_rule;
-  int sched_slot;  // CTA-pair kernel: this launch's pair of words in g_sched_words
+};
+
+// Up to kMaxGroup independent GEMMs share one launch of the CTA-pair kernel: their output tiles form one list of units,
+// the first GEMM's first. The backward of a Linear is two GEMMs (input and weight gradient) that often have fewer tiles
+// than the machine has CTA pairs, or a round and a bit; together they fill it, and one launch is saved.
+constexpr int kMaxGroup = 3;
+
+struct PairMaps {
+  CUtensorMap a, b, sfa, sfb, d, part;
+};
+
+template <int kProblems>
+struct PairArgs {
+  PairMaps maps[kProblems];
+  GemmParams p[kProblems];
+  int end[kProblems];  // one past the last unit of each
+  int sched_slot;      // this launch's pair of words in g_sched_words
+};
+
+struct FuseMaps {
+  CUtensorMap q, qt;
 };
 
 struct Barriers {
@@ -876,7 +896,7 @@ constexpr int kEpiFusedBytes = 6144;       // ... with a fused quantizer: output
 
 template <int TN, int kFuse = kFuseNone>
 struct PairConfig {
-  static_assert(TN == 192 || TN == 256, "tile width");
+  static_assert(TN == 128 || TN == 192 || TN == 256, "tile width");
   static constexpr int kEpiBytes = kFuse == kFuseNone ? kEpiStageBytes : kEpiFusedBytes;
   static constexpr int kParts = kFuse == kFuseNone ? 2 : 3;
   static constexpr int kEpiWarps = 4 * kParts;
@@ -884,12 +904,12 @@ struct PairConfig {
   static constexpr int kThreads = 64 + kEpiThreads;
   static constexpr int kTileM = 256, kTileN = TN;
   static constexpr int kBRows = TN / 2;                // this CTA's rows of B
-  static constexpr int kSfbTiles = 2;
+  static constexpr int kSfbTiles = TN == 128 ? 1 : 2;
   static constexpr uint32_t kABytes = 128 * kBK;       // this CTA's 128 rows of A
   static constexpr uint32_t kBBytes = kBRows * kBK;
   static constexpr uint32_t kSfBytes = kScaleTileBytes * (1 + kSfbTiles);  // A: own 128 rows; B: all its tiles
   static constexpr uint32_t kTxPerCta = kABytes + kBBytes + kSfBytes;
-  static constexpr int kStages = (TN == 192 ? 7 : 6) - (kFuse == kFuseNone ? 0 : 2);
+  static constexpr int kStages = (TN == 128 ? 8 : TN == 192 ? 7 : 6) - (kFuse == kFuseNone ? 0 : 2);
   static constexpr bool kOverlap = TN == 256;
   static constexpr uint32_t kAcc0 = 0, kAcc1 = kOverlap ? 224 : TN;
   static constexpr uint32_t kSfaCol = kOverlap ? 480 : 2 * TN, kSfbCol = kSfaCol + 4;
@@ -905,12 +925,9 @@ struct PairConfig {
 
 // The kernel body; the kernels themselves are the non-template functions at the end of this file (plain global
 // names read the same in every profiler). The tensor maps stay in the kernels' parameter space and come by address.
-template <int TN, int kFuse>
-__device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const CUtensorMap* map_b,
-                                                 const CUtensorMap* map_sfa, const CUtensorMap* map_sfb,
-                                                 const CUtensorMap* map_d, const CUtensorMap* map_part,
-                                                 const CUtensorMap* map_q, const CUtensorMap* map_qt,
-                                                 const GemmParams& p) {
+template <int TN, int kFuse, int kProblems>
+__device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args, const CUtensorMap* map_q,
+                                                 const CUtensorMap* map_qt) {
   using C = PairConfig<TN, kFuse>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -925,7 +942,17 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int num_pairs = static_cast<int>(gridDim.x) >> 1;
-  const int total_units = p.tiles_m * p.tiles_n * p.splits;
+  const int total_units = args.end[kProblems - 1];
+  // which GEMM a unit belongs to; `unit` becomes its number within that one
+  const auto problem_of = [&](int* unit) {
+    int g = 0;
+#pragma unroll
+    for (int k = 0; k + 1 < kProblems; ++k)
+      g += *unit >= args.end[k] ? 1 : 0;
+    if (g > 0)
+      *unit -= args.end[g - 1];
+    return g;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
@@ -949,13 +976,16 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
     fence_mbar_init();
   }
   if (warp == 0 && lane == 0) {
-    prefetch_tensormap(map_a);
-    prefetch_tensormap(map_b);
-    prefetch_tensormap(map_sfa);
-    prefetch_tensormap(map_sfb);
-    prefetch_tensormap(map_d);
-    if (p.splits > 1)
-      prefetch_tensormap(map_part);
+#pragma unroll
+    for (int g = 0; g < kProblems; ++g) {
+      prefetch_tensormap(&args.maps[g].a);
+      prefetch_tensormap(&args.maps[g].b);
+      prefetch_tensormap(&args.maps[g].sfa);
+      prefetch_tensormap(&args.maps[g].sfb);
+      prefetch_tensormap(&args.maps[g].d);
+      if (args.p[g].splits > 1)
+        prefetch_tensormap(&args.maps[g].part);
+    }
     if (kFuse != kFuseNone) {
       prefetch_tensormap(map_q);
       prefetch_tensormap(map_qt);
@@ -984,7 +1014,7 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
       const uint32_t full_leader0 = map_to_cta(full0, 0);
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      uint32_t* const sched = g_sched_words + 2 * p.sched_slot;
+      uint32_t* const sched = g_sched_words + 2 * args.sched_slot;
       const uint32_t sched_empty_leader0 = map_to_cta(smem_u32(&bars->sched_empty[0]), 0);
       const uint32_t sched_full_peer0 = map_to_cta(smem_u32(&bars->sched_full[0]), 1);
       const uint32_t sched_unit_peer0 = map_to_cta(smem_u32(&bars->sched_unit[0]), 1);
@@ -1018,6 +1048,9 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
         }
         if (unit >= total_units)
           break;
+        const int g = problem_of(&unit);
+        const GemmParams& p = args.p[g];
+        const PairMaps& maps = args.maps[g];
         const TileCoord tc = decode_unit(p, unit);
         const int k_begin = tc.split * p.k_tiles_split;
         const int k_end = min(k_begin + p.k_tiles_split, p.k_tiles_total);
@@ -1032,10 +1065,10 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
           mbar_arrive_expect_tx(el_leader, full0 + stage * 8, 2 * C::kTxPerCta);
           const uint32_t full = full_leader0 + stage * 8;
           const uint32_t sf = sf0 + stage * C::kSfBytes;
-          tma_load_2d_pair(el, a0 + stage * C::kABytes, map_a, full, kt * kBK, row_a);
-          tma_load_2d_pair(el, b0 + stage * C::kBBytes, map_b, full, kt * kBK, row_b);
-          tma_load_4d_pair(el, sf, map_sfa, full, 0, 0, kt, sfa_tile);
-          tma_load_4d_pair(el, sf + kScaleTileBytes, map_sfb, full, 0, 0, kt, sfb_tile);
+          tma_load_2d_pair(el, a0 + stage * C::kABytes, &maps.a, full, kt * kBK, row_a);
+          tma_load_2d_pair(el, b0 + stage * C::kBBytes, &maps.b, full, kt * kBK, row_b);
+          tma_load_4d_pair(el, sf, &maps.sfa, full, 0, 0, kt, sfa_tile);
+          tma_load_4d_pair(el, sf + kScaleTileBytes, &maps.sfb, full, 0, 0, kt, sfb_tile);
           if (++stage == C::kStages) {
             stage = 0;
             phase ^= 1u;
@@ -1076,6 +1109,7 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
         }
         if (unit >= total_units)
           break;
+        const GemmParams& p = args.p[problem_of(&unit)];
         const TileCoord tc = decode_unit(p, unit);
         const uint32_t buf = local & 1u, use = local >> 1;
         if (!wait_bounded_warp(&bars->tmem_empty[buf], (use & 1u) ^ 1u, bars, kSiteMmaTmemEmpty)) {
@@ -1131,7 +1165,6 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
     const int quarter = warp & 3;
     const int col_part = (warp - 2) >> 2;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? *p.alpha : 1.f;
     uint32_t local = 0, sync_phase = 0;
     bool ok = true;
     constexpr int kChunks = C::kTileN / 32;
@@ -1154,6 +1187,10 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
       }
       if (unit >= total_units)
         break;
+      const int g = problem_of(&unit);
+      const GemmParams& p = args.p[g];
+      const PairMaps& maps = args.maps[g];
+      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
       // the relu^2 backward form reads h: the first chunk's block is requested before the accumulator is waited for
@@ -1205,10 +1242,10 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
         if (part != nullptr) {
           // split-K partials take the same TMA store path: the workspace is a (half tiles x 128 rows, TN) matrix
           const int part_row0 = static_cast<int>(half_index) * 128 + quarter * 32;
-          store_rows_tma(map_part, stage, lane, r[i & 1], c * 32, part_row0, true);
-          store_rows_tma(map_part, stage, lane, r[i & 1] + 16, c * 32 + 16, part_row0, true);
+          store_rows_tma(&maps.part, stage, lane, r[i & 1], c * 32, part_row0, true);
+          store_rows_tma(&maps.part, stage, lane, r[i & 1] + 16, c * 32 + 16, part_row0, true);
         } else if constexpr (kFuse != kFuseNone) {
-          fused_quantize_chunk<kFuse>(p, map_d, map_q, map_qt, stage, lane, reinterpret_cast<const float*>(r[i & 1]),
+          fused_quantize_chunk<kFuse>(p, &maps.d, map_q, map_qt, stage, lane, reinterpret_cast<const float*>(r[i & 1]),
                                       row, col, warp_row0, row_ok && col < p.N, h_pieces,
                                       i + 1 < n_mine ? col0 + chunk_of(i + 1) * 32 : -1,
                                       C::kStageScales ? s_scales + buf * (4 * kScaleTileBytes) : nullptr, c);
@@ -1217,9 +1254,9 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
           const bool issue = warp_row0 < p.M && col < p.N;
           uint32_t o[32];
           compute_chunk(p, alpha, row, col, reinterpret_cast<const float*>(r[i & 1]), valid, o);
-          store_rows_tma(map_d, stage, lane, o, col, warp_row0, issue);
+          store_rows_tma(&maps.d, stage, lane, o, col, warp_row0, issue);
           if (p.out_kind == kOutF32)
-            store_rows_tma(map_d, stage, lane, o + 16, col + 16, warp_row0, issue);
+            store_rows_tma(&maps.d, stage, lane, o + 16, col + 16, warp_row0, issue);
         }
       }
       if constexpr (C::kStageScales) {
@@ -1354,45 +1391,55 @@ __device__ __forceinline__ void pair_kernel_body(const CUtensorMap* map_a, const
     mxb200::one_cta_kernel_body<BN>(&map_a, &map_b, p);                                                                \
   }
 
-#define MXB200_GEMM_PAIR_KERNEL(name, TN, FUSE)                                                                        \
+#define MXB200_GEMM_PAIR_KERNEL(name, TN, PROBLEMS)                                                                    \
+  __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(mxb200::PairConfig<TN>::kThreads, 1)                     \
+        name(const __grid_constant__ mxb200::PairArgs<PROBLEMS> args) {                                                \
+    mxb200::pair_kernel_body<TN, mxb200::kFuseNone, PROBLEMS>(args, nullptr, nullptr);                                 \
+  }
+
+#define MXB200_GEMM_FUSED_KERNEL(name, TN, FUSE)                                                                       \
   __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(mxb200::PairConfig<TN, FUSE>::kThreads, 1)               \
-        name(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,                     \
-             const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,                 \
-             const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_part,                  \
-             const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qt,                    \
-             const mxb200::GemmParams p) {                                                                             \
-    mxb200::pair_kernel_body<TN, FUSE>(&map_a, &map_b, &map_sfa, &map_sfb, &map_d, &map_part, &map_q, &map_qt, p);     \
+        name(const __grid_constant__ mxb200::PairArgs<1> args, const __grid_constant__ mxb200::FuseMaps fuse) {        \
+    mxb200::pair_kernel_body<TN, FUSE, 1>(args, &fuse.q, &fuse.qt);                                                    \
   }
 
 MXB200_GEMM_KERNEL(mxb200_gemm_128x128, 128)
 MXB200_GEMM_KERNEL(mxb200_gemm_128x256, 256)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x192, 192, mxb200::kFuseNone)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x256, 256, mxb200::kFuseNone)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x192_relu_square, 192, mxb200::kFuseReluSquare)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x256_relu_square, 256, mxb200::kFuseReluSquare)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x192_relu_square_bwd, 192, mxb200::kFuseReluSquareBwd)
-MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x256_relu_square_bwd, 256, mxb200::kFuseReluSquareBwd)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x128, 128, 1)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x192, 192, 1)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x256, 256, 1)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_group_256x128, 128, mxb200::kMaxGroup)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_group_256x192, 192, mxb200::kMaxGroup)
+MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_group_256x256, 256, mxb200::kMaxGroup)
+MXB200_GEMM_FUSED_KERNEL(mxb200_gemm_pair_256x192_relu_square, 192, mxb200::kFuseReluSquare)
+MXB200_GEMM_FUSED_KERNEL(mxb200_gemm_pair_256x256_relu_square, 256, mxb200::kFuseReluSquare)
+MXB200_GEMM_FUSED_KERNEL(mxb200_gemm_pair_256x192_relu_square_bwd, 192, mxb200::kFuseReluSquareBwd)
+MXB200_GEMM_FUSED_KERNEL(mxb200_gemm_pair_256x256_relu_square_bwd, 256, mxb200::kFuseReluSquareBwd)
 
 namespace mxb200 {
 namespace {
 
 using GemmKernel = void (*)(CUtensorMap, CUtensorMap, GemmParams);
-using GemmPairKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
-                                CUtensorMap, GemmParams);
 
 template <int BN>
 constexpr GemmKernel one_cta_kernel() {
   return BN == 256 ? mxb200_gemm_128x256 : mxb200_gemm_128x128;
 }
 
+template <int TN, int kProblems>
+constexpr auto pair_kernel() {
+  if constexpr (kProblems == 1)
+    return TN == 256 ? mxb200_gemm_pair_256x256 : TN == 192 ? mxb200_gemm_pair_256x192 : mxb200_gemm_pair_256x128;
+  else
+    return TN == 256 ? mxb200_gemm_group_256x256 : TN == 192 ? mxb200_gemm_group_256x192 : mxb200_gemm_group_256x128;
+}
+
 template <int TN, int kFuse>
-constexpr GemmPairKernel pair_kernel() {
+constexpr auto fused_kernel() {
   if constexpr (kFuse == kFuseReluSquare)
     return TN == 256 ? mxb200_gemm_pair_256x256_relu_square : mxb200_gemm_pair_256x192_relu_square;
-  else if constexpr (kFuse == kFuseReluSquareBwd)
-    return TN == 256 ? mxb200_gemm_pair_256x256_relu_square_bwd : mxb200_gemm_pair_256x192_relu_square_bwd;
   else
-    return TN == 256 ? mxb200_gemm_pair_256x256 : mxb200_gemm_pair_256x192;
+    return TN == 256 ? mxb200_gemm_pair_256x256_relu_square_bwd : mxb200_gemm_pair_256x192_relu_square_bwd;
 }
 
 // ------------------------------------------------------------------------------------------------ host side
@@ -1449,66 +1496,80 @@ int make_scale_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k, 
   return r == CUDA_SUCCESS ? MXB200_OK : MXB200_ERR_DRIVER;
 }
 
-// How a shape is tiled: one-CTA kernel with 128 x 128 or 128 x 256 tiles, or the CTA-pair kernel with 256 x 192
-// or 256 x 256.
+// One GEMM of a launch, as the entry points take it.
+using GemmDesc = mxb200_gemm_desc;
+
+// How a launch is tiled: one-CTA kernel with 128 x 128 or 128 x 256 tiles, or the CTA-pair kernel with 256 x 128, 192 or
+// 256, and into how many slices the K of each of its GEMMs is cut.
 struct TilePlan {
   bool pair;
   int tile_m, tile_n;
-  int slots;         // tiles the machine runs at once
-  int64_t tiles_m, tiles_n;
-  int64_t tiles() const { return tiles_m * tiles_n; }
+  int splits[kMaxGroup] = {1, 1, 1};
+  int64_t tiles(int64_t M, int64_t N) const { return (M + tile_m - 1) / tile_m * ((N + tile_n - 1) / tile_n); }
   size_t tile_bytes() const { return static_cast<size_t>(tile_m) * tile_n * sizeof(float); }
-  int64_t counters() const { return tiles() * (pair ? 2 : 1); }
+  int64_t counters(int64_t M, int64_t N) const { return tiles(M, N) * (pair ? 2 : 1); }
 };
 
-TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, bool need_pair = false) {
+// Estimated cycles of one unit of the CTA-pair kernel with `k_iters` K steps of 128, besides what the launch costs anyway.
+// A step runs at the slower of MMA execution (2 TN cycles) and what an SM can ingest (about 58 bytes per cycle in
+// practice); 256-wide tiles pay an overlap bubble of about 1500 cycles per tile.
+double unit_cycles(int tn, int64_t k_iters) {
+  const double ingest = (16384.0 + tn * 64.0 + 1536.0) / 58.0;  // bytes a CTA loads per K step / (B/clk)
+  return static_cast<double>(k_iters) * std::max(2.0 * tn, ingest) + (tn == 256 ? 1500.0 : 300.0);
+}
+
+TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair = false) {
   int forced = g_tile_n.load();
   if (need_pair && (forced == 128 || forced == 256))
     forced = 0;  // the fused-quantize epilogues exist in the CTA-pair kernel only
   TilePlan t{};
-  if (forced == 512 || forced == 384 || need_pair || (forced == 0 && M >= 256 && N >= 256)) {
-    t.pair = true, t.tile_m = 256, t.slots = std::max(sms / 2, 1);
-    if (forced == 512) {
-      t.tile_n = 256;
-    } else if (forced == 384) {
-      t.tile_n = 192;
-    } else {
-      // Estimated cycles: waves x (main loop + the hand-over between tiles). The main loop runs at the slower of
-      // MMA execution (2 TN cycles per K step of 128) and what an SM can ingest (about 64 bytes per cycle); 256
-      // pays an overlap bubble per tile. Measured on the d24 shapes this picks the faster width in every case,
-      // including the long-K weight gradients whose tile count it raises past one wave (splitting K instead costs
-      // more than it gains, see mxb200_gemm_splits).
-      const int64_t k_iters = K / 128;
-      double best = 0.0;
-      for (int tn : {256, 192}) {
-        const int64_t tiles = ((M + 255) / 256) * ((N + tn - 1) / tn);
-        const int64_t units = tiles, iters = k_iters;
-        // Pairs draw their tiles from a counter, so with many short tiles per pair the launch ends within a fraction
-        // of a tile of the average share; with few long ones (the weight gradients) it ends on a whole round.
-        const double share = static_cast<double>(units) / t.slots;
-        const double waves = share >= 4.0 ? share + 0.25 : std::ceil(share);
-        const double ingest = (16384.0 + tn * 64.0 + 1536.0) / 58.0;  // bytes a CTA loads per K step / (B/clk)
-        const double per_tile = static_cast<double>(iters) * std::max(2.0 * tn, ingest) + (tn == 256 ? 1500.0 : 300.0);
-        const double cost = waves * per_tile;
-        if (best == 0.0 || cost < best * 0.995)
-          best = cost, t.tile_n = tn;
-      }
-    }
-  } else {
-    t.pair = false, t.tile_m = 128, t.slots = std::max(sms, 1);
-    t.tile_n = (forced == 128 || forced == 256) ? forced : (N >= 256 ? 256 : 128);
+  bool wide = true;
+  for (int i = 0; i < n; ++i)
+    wide &= g[i].M >= 256 && g[i].N >= 256;
+  if (!(forced >= 384 || need_pair || (forced == 0 && wide))) {
+    t.pair = false, t.tile_m = 128;
+    t.tile_n = (forced == 128 || forced == 256) ? forced : (g[0].N >= 256 ? 256 : 128);
+    return t;
   }
-  t.tiles_m = (M + t.tile_m - 1) / t.tile_m;
-  t.tiles_n = (N + t.tile_n - 1) / t.tile_n;
+  t.pair = true, t.tile_m = 256;
+  if (forced >= 384) {
+    t.tile_n = forced == 512 ? 256 : forced == 384 ? 192 : 128;
+    return t;
+  }
+  const double slots = std::max(sms / 2, 1);
+  double best = 0.0;
+  for (int tn : {256, 192, 128}) {
+    if (need_pair && tn == 128)
+      continue;
+    double units = 0.0, work = 0.0, longest = 0.0;
+    for (int i = 0; i < n; ++i) {
+      const double u = static_cast<double>((g[i].M + 255) / 256 * ((g[i].N + tn - 1) / tn));
+      const double c = unit_cycles(tn, g[i].K / 128);
+      units += u, work += u * c;
+      longest = std::max(longest, c);
+    }
+    // Pairs draw their tiles from a counter, so with many short tiles per pair the launch ends within a fraction of a
+    // tile of the average share; with few long ones (the weight gradients) it ends on a whole round.
+    const double share = units / slots;
+    const double cost = share >= 4.0 ? work / slots + 0.25 * longest : std::ceil(share) * (work / units);
+    if (best == 0.0 || cost < best * 0.995)
+      best = cost, t.tile_n = tn;
+  }
   return t;
+}
+
+TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, bool need_pair = false) {
+  GemmDesc g{};
+  g.M = M, g.N = N, g.K = K;
+  return plan_tiles(&g, 1, sms, need_pair);
 }
 
 size_t counters_bytes(int64_t counters) {
   return static_cast<size_t>((counters * 4 + 255) / 256 * 256);
 }
 
-size_t workspace_bytes_for(const TilePlan& t, int splits) {
-  return splits <= 1 ? 0 : counters_bytes(t.counters()) + static_cast<size_t>(t.tiles()) * splits * t.tile_bytes();
+size_t workspace_bytes_for(const TilePlan& t, int64_t M, int64_t N, int splits) {
+  return splits <= 1 ? 0 : counters_bytes(t.counters(M, N)) + static_cast<size_t>(t.tiles(M, N)) * splits * t.tile_bytes();
 }
 
 template <typename Kernel>
@@ -1535,25 +1596,33 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, in
   return launch_status();
 }
 
-struct PairMaps {
-  CUtensorMap a, b, sfa, sfb, d, part, q, qt;
-};
-
-template <int TN, int kFuse>
-int launch_pair(const PairMaps& m, const GemmParams& p, int pairs, cudaStream_t stream) {
-  using C = PairConfig<TN, kFuse>;
+template <int TN, int kProblems>
+int launch_pair(const PairArgs<kProblems>& args, int pairs, cudaStream_t stream) {
+  using C = PairConfig<TN>;
   static bool configured[64] = {};
-  if (int st = set_smem_once(pair_kernel<TN, kFuse>(), C::kSmemBytes, configured); st != MXB200_OK)
+  if (int st = set_smem_once(pair_kernel<TN, kProblems>(), C::kSmemBytes, configured); st != MXB200_OK)
     return st;
-  pair_kernel<TN, kFuse>()<<<2 * pairs, C::kThreads, C::kSmemBytes, stream>>>(m.a, m.b, m.sfa, m.sfb, m.d,
-                                                                                          m.part, m.q, m.qt, p);
+  pair_kernel<TN, kProblems>()<<<2 * pairs, C::kThreads, C::kSmemBytes, stream>>>(args);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return launch_status();
 }
 
-template <int kFuse>
-int launch_pair_width(int tile_n, const PairMaps& m, const GemmParams& p, int pairs, cudaStream_t stream) {
-  return tile_n == 256 ? launch_pair<256, kFuse>(m, p, pairs, stream) : launch_pair<192, kFuse>(m, p, pairs, stream);
+template <int kProblems>
+int launch_pair_width(int tile_n, const PairArgs<kProblems>& args, int pairs, cudaStream_t stream) {
+  return tile_n == 256   ? launch_pair<256, kProblems>(args, pairs, stream)
+         : tile_n == 192 ? launch_pair<192, kProblems>(args, pairs, stream)
+                         : launch_pair<128, kProblems>(args, pairs, stream);
+}
+
+template <int TN, int kFuse>
+int launch_fused(const PairArgs<1>& args, const FuseMaps& fuse, int pairs, cudaStream_t stream) {
+  using C = PairConfig<TN, kFuse>;
+  static bool configured[64] = {};
+  if (int st = set_smem_once(fused_kernel<TN, kFuse>(), C::kSmemBytes, configured); st != MXB200_OK)
+    return st;
+  fused_kernel<TN, kFuse>()<<<2 * pairs, C::kThreads, C::kSmemBytes, stream>>>(args, fuse);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return launch_status();
 }
 
 // (rows, cols) row-major bytes, box = 32 rows x 32 bytes: what one epilogue warp stores of a quantized layout
@@ -1581,15 +1650,10 @@ struct FusedOut {
   const void* h_in = nullptr;
 };
 
-int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale, void* d, int out_kind,
-         const void* resid, int64_t M, int64_t N, int64_t K, const float* alpha, int accumulate, int splits,
-         void* workspace, size_t workspace_bytes, void* stream, const FusedOut& fused = FusedOut{}) {
-  DeviceInfo dev;
-  if (int s = current_device(&dev); s != MXB200_OK)
-    return s;
+int check_gemm(const GemmDesc& g, const FusedOut& fused, int splits) {
   const bool fusing = fused.fuse != kFuseNone;
-  if (a == nullptr || a_scale == nullptr || b == nullptr || b_scale == nullptr ||
-      (d == nullptr && fused.fuse != kFuseReluSquareBwd))
+  if (g.a == nullptr || g.a_scale == nullptr || g.b == nullptr || g.b_scale == nullptr ||
+      (g.d == nullptr && fused.fuse != kFuseReluSquareBwd))
     return MXB200_ERR_NULL;
   if (fusing) {
     if (fused.q == nullptr || fused.q_scale == nullptr || fused.q_t == nullptr || fused.q_t_scale == nullptr ||
@@ -1598,108 +1662,230 @@ int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale,
     if (!aligned16(fused.q) || !aligned16(fused.q_scale) || !aligned16(fused.q_t) || !aligned16(fused.q_t_scale) ||
         (fused.h_in != nullptr && !aligned16(fused.h_in)))
       return MXB200_ERR_ALIGNMENT;
-    if (out_kind != kOutBf16 || resid != nullptr || splits != 1)
+    if (g.out_kind != kOutBf16 || g.resid != nullptr || splits != 1)
       return MXB200_ERR_ARGUMENT;
   }
-  if (M <= 0 || N <= 0 || K <= 0 || M % 128 != 0 || N % 128 != 0 || K % 128 != 0 || M > (1 << 30) || N > (1 << 30) ||
-      K > (1 << 30))
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.M % 128 != 0 || g.N % 128 != 0 || g.K % 128 != 0 || g.M > (1 << 30) ||
+      g.N > (1 << 30) || g.K > (1 << 30))
     return MXB200_ERR_SHAPE;
-  if (!aligned16(a) || !aligned16(a_scale) || !aligned16(b) || !aligned16(b_scale) || (d != nullptr && !aligned16(d)) ||
-      (resid != nullptr && !aligned16(resid)))
+  if (!aligned16(g.a) || !aligned16(g.a_scale) || !aligned16(g.b) || !aligned16(g.b_scale) ||
+      (g.d != nullptr && !aligned16(g.d)) || (g.resid != nullptr && !aligned16(g.resid)))
     return MXB200_ERR_ALIGNMENT;
-  if (out_kind != kOutBf16 && out_kind != kOutF32)
+  if (g.out_kind != kOutBf16 && g.out_kind != kOutF32)
     return MXB200_ERR_ARGUMENT;
-  if (out_kind == kOutF32 && resid != nullptr)
+  if (g.out_kind == kOutF32 && g.resid != nullptr)
     return MXB200_ERR_ARGUMENT;
-  const int k_tiles = static_cast<int>(K / kBK);
-  if (splits < 1 || splits > k_tiles || splits > 64)
+  if (splits < 1 || splits > g.K / kBK || splits > 64)
     return MXB200_ERR_ARGUMENT;
+  return MXB200_OK;
+}
 
-  const TilePlan plan = plan_tiles(M, N, K, dev.sms, fusing);
+GemmParams gemm_params(const GemmDesc& g, const TilePlan& plan, int splits, const FusedOut& fused) {
   GemmParams p{};
-  p.a_scale = static_cast<const uint8_t*>(a_scale);
-  p.b_scale = static_cast<const uint8_t*>(b_scale);
-  p.d = d;
-  p.resid = out_kind == kOutBf16 ? resid : nullptr;
-  p.alpha = out_kind == kOutF32 ? alpha : nullptr;
-  p.M = static_cast<int>(M), p.N = static_cast<int>(N), p.K = static_cast<int>(K);
-  p.tiles_m = static_cast<int>(plan.tiles_m);
-  p.tiles_n = static_cast<int>(plan.tiles_n);
-  p.k_tiles_total = k_tiles;
-  p.k_tiles_split = (k_tiles + splits - 1) / splits;
-  p.splits = (k_tiles + p.k_tiles_split - 1) / p.k_tiles_split;  // no empty slices
+  p.a_scale = static_cast<const uint8_t*>(g.a_scale);
+  p.b_scale = static_cast<const uint8_t*>(g.b_scale);
+  p.d = g.d;
+  p.resid = g.out_kind == kOutBf16 ? g.resid : nullptr;
+  p.alpha = g.out_kind == kOutF32 ? g.alpha : nullptr;
+  p.M = static_cast<int>(g.M), p.N = static_cast<int>(g.N), p.K = static_cast<int>(g.K);
+  p.tiles_m = static_cast<int>((g.M + plan.tile_m - 1) / plan.tile_m);
+  p.tiles_n = static_cast<int>((g.N + plan.tile_n - 1) / plan.tile_n);
+  p.k_tiles_total = static_cast<int>(g.K / kBK);
+  p.k_tiles_split = (p.k_tiles_total + splits - 1) / splits;
+  p.splits = (p.k_tiles_total + p.k_tiles_split - 1) / p.k_tiles_split;  // no empty slices
   p.panel = std::min(p.tiles_n, 8);
-  p.out_kind = out_kind;
-  p.accumulate = out_kind == kOutF32 ? (accumulate != 0) : 0;
-  p.wide = (reinterpret_cast<uintptr_t>(d) & 31u) == 0 && (reinterpret_cast<uintptr_t>(resid) & 31u) == 0 &&
+  p.out_kind = g.out_kind;
+  p.accumulate = g.out_kind == kOutF32 ? (g.accumulate != 0) : 0;
+  p.wide = (reinterpret_cast<uintptr_t>(g.d) & 31u) == 0 && (reinterpret_cast<uintptr_t>(g.resid) & 31u) == 0 &&
            (reinterpret_cast<uintptr_t>(fused.h_in) & 31u) == 0;
   p.q_scale = static_cast<uint8_t*>(fused.q_scale);
   p.qt_scale = static_cast<uint8_t*>(fused.q_t_scale);
-  p.q_scale_tiles = static_cast<int>(N / 128);
-  p.qt_scale_tiles = static_cast<int>(M / 128);
+  p.q_scale_tiles = static_cast<int>(g.N / 128);
+  p.qt_scale_tiles = static_cast<int>(g.M / 128);
   p.h_in = fused.h_in;
   p.floor_rule = false;
-  const int64_t tiles = plan.tiles();
-  if (tiles * p.splits > 0x7fffffffLL)
-    return MXB200_ERR_SHAPE;
-  auto* s = static_cast<cudaStream_t>(stream);
+  return p;
+}
+
+int pair_maps(PairMaps* m, const GemmDesc& g, const TilePlan& plan, const GemmParams& p) {
+  if (int st = make_operand_map(&m->a, g.a, g.M, g.K, 128); st != MXB200_OK)
+    return st;
+  if (int st = make_operand_map(&m->b, g.b, g.N, g.K, plan.tile_n / 2); st != MXB200_OK)
+    return st;
+  if (int st = make_scale_map(&m->sfa, g.a_scale, g.M, g.K, 1); st != MXB200_OK)
+    return st;
+  if (int st = make_scale_map(&m->sfb, g.b_scale, g.N, g.K, plan.tile_n == 128 ? 1 : 2); st != MXB200_OK)
+    return st;
+  if (g.d != nullptr) {
+    if (int st = make_output_map(&m->d, g.d, g.M, g.N, g.out_kind == kOutF32); st != MXB200_OK)
+      return st;
+  } else {
+    m->d = m->a;  // never used: the relu^2 backward form writes no plain output
+  }
+  m->part = m->d;  // unused without a K split
   if (p.splits > 1) {
-    const size_t need = workspace_bytes_for(plan, p.splits);
-    if (workspace == nullptr || workspace_bytes < need)
+    // partial half tiles, stacked: (tiles x splits x 2 halves x 128 rows, TN) fp32
+    const int64_t rows = static_cast<int64_t>(p.tiles_m) * p.tiles_n * p.splits * 256;
+    if (int st = make_output_map(&m->part, p.partials, rows, plan.tile_n, true); st != MXB200_OK)
+      return st;
+  }
+  return MXB200_OK;
+}
+
+int next_sched_slot() {
+  static std::atomic<uint32_t> launch_seq{0};
+  return static_cast<int>(launch_seq.fetch_add(1, std::memory_order_relaxed) % kSchedLaunchSlots);
+}
+
+// n independent GEMMs, each with its slices; one launch of the CTA-pair kernel where the plan is for it (always with n > 1).
+template <int kProblems>
+int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInfo& dev, void* workspace,
+                 size_t workspace_bytes, cudaStream_t s, const FusedOut& fused) {
+  PairArgs<kProblems> args{};
+  int64_t units = 0;
+  size_t counters = 0, need = 0;
+  bool split = false;
+  for (int i = 0; i < n; ++i) {
+    args.p[i] = gemm_params(g[i], plan, plan.splits[i], fused);
+    const int64_t tiles = plan.tiles(g[i].M, g[i].N);
+    units += tiles * args.p[i].splits;
+    if (units > 0x7fffffffLL)
+      return MXB200_ERR_SHAPE;
+    args.end[i] = static_cast<int>(units);
+    if (args.p[i].splits > 1) {
+      split = true;
+      counters += static_cast<size_t>(plan.counters(g[i].M, g[i].N));
+      need += static_cast<size_t>(tiles) * args.p[i].splits * plan.tile_bytes();
+    }
+  }
+  for (int i = n; i < kProblems; ++i)
+    args.p[i] = args.p[n - 1], args.end[i] = static_cast<int>(units);
+  if (split) {
+    // all counters first, zeroed together, then each GEMM's partial tiles
+    const size_t head = counters_bytes(static_cast<int64_t>(counters));
+    if (workspace == nullptr || workspace_bytes < head + need)
       return MXB200_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
       return MXB200_ERR_ALIGNMENT;
-    p.counters = static_cast<uint32_t*>(workspace);
-    p.partials = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + counters_bytes(plan.counters()));
-    if (cudaMemsetAsync(p.counters, 0, counters_bytes(plan.counters()), s) != cudaSuccess)
+    auto* counter = static_cast<uint32_t*>(workspace);
+    auto* partial = static_cast<unsigned char*>(workspace) + head;
+    if (cudaMemsetAsync(counter, 0, head, s) != cudaSuccess)
       return MXB200_ERR_LAUNCH;
+    for (int i = 0; i < n; ++i) {
+      if (args.p[i].splits == 1)
+        continue;
+      args.p[i].counters = counter;
+      args.p[i].partials = reinterpret_cast<float*>(partial);
+      counter += plan.counters(g[i].M, g[i].N);
+      partial += static_cast<size_t>(plan.tiles(g[i].M, g[i].N)) * args.p[i].splits * plan.tile_bytes();
+    }
   }
   const int cap = g_max_ctas.load() > 0 ? g_max_ctas.load() : dev.sms;
-  CUtensorMap ma, mb;
-  if (plan.pair) {
-    PairMaps m;
-    if (int st = make_operand_map(&m.a, a, M, K, 128); st != MXB200_OK)
+  if (!plan.pair) {
+    CUtensorMap ma, mb;
+    if (int st = make_operand_map(&ma, g[0].a, g[0].M, g[0].K, kBM); st != MXB200_OK)
       return st;
-    if (int st = make_operand_map(&m.b, b, N, K, plan.tile_n / 2); st != MXB200_OK)
+    if (int st = make_operand_map(&mb, g[0].b, g[0].N, g[0].K, plan.tile_n); st != MXB200_OK)
       return st;
-    if (int st = make_scale_map(&m.sfa, a_scale, M, K, 1); st != MXB200_OK)
-      return st;
-    if (int st = make_scale_map(&m.sfb, b_scale, N, K, 2); st != MXB200_OK)
-      return st;
-    if (d != nullptr) {
-      if (int st = make_output_map(&m.d, d, M, N, out_kind == kOutF32); st != MXB200_OK)
-        return st;
-    } else {
-      m.d = m.a;  // never used: the relu^2 backward form writes no plain output
-    }
-    m.part = m.d;  // unused without a K split
-    if (p.splits > 1) {
-      // partial half tiles, stacked: (tiles x splits x 2 halves x 128 rows, TN) fp32
-      if (int st = make_output_map(&m.part, p.partials, tiles * p.splits * 256, plan.tile_n, true); st != MXB200_OK)
-        return st;
-    }
-    m.q = m.qt = m.d;
-    if (fusing) {
-      if (int st = make_bytes_map(&m.q, fused.q, M, N); st != MXB200_OK)
-        return st;
-      if (int st = make_bytes_map(&m.qt, fused.q_t, N, M); st != MXB200_OK)
-        return st;
-    }
-    const int pairs = static_cast<int>(std::min<int64_t>(tiles * p.splits, std::max(cap / 2, 1)));
-    static std::atomic<uint32_t> launch_seq{0};
-    p.sched_slot = static_cast<int>(launch_seq.fetch_add(1, std::memory_order_relaxed) % kSchedLaunchSlots);
-    if (fused.fuse == kFuseReluSquare)
-      return launch_pair_width<kFuseReluSquare>(plan.tile_n, m, p, pairs, s);
-    if (fused.fuse == kFuseReluSquareBwd)
-      return launch_pair_width<kFuseReluSquareBwd>(plan.tile_n, m, p, pairs, s);
-    return launch_pair_width<kFuseNone>(plan.tile_n, m, p, pairs, s);
+    const int grid = static_cast<int>(std::min<int64_t>(units, cap));
+    return plan.tile_n == 256 ? launch<256>(ma, mb, args.p[0], grid, s) : launch<128>(ma, mb, args.p[0], grid, s);
   }
-  if (int st = make_operand_map(&ma, a, M, K, kBM); st != MXB200_OK)
-    return st;
-  if (int st = make_operand_map(&mb, b, N, K, plan.tile_n); st != MXB200_OK)
-    return st;
-  const int grid = static_cast<int>(std::min<int64_t>(tiles * p.splits, cap));
-  return plan.tile_n == 256 ? launch<256>(ma, mb, p, grid, s) : launch<128>(ma, mb, p, grid, s);
+  for (int i = 0; i < n; ++i)
+    if (int st = pair_maps(&args.maps[i], g[i], plan, args.p[i]); st != MXB200_OK)
+      return st;
+  for (int i = n; i < kProblems; ++i)
+    args.maps[i] = args.maps[n - 1];
+  const int pairs = static_cast<int>(std::min<int64_t>(units, std::max(cap / 2, 1)));
+  args.sched_slot = next_sched_slot();
+  if constexpr (kProblems == 1) {
+    if (fused.fuse != kFuseNone) {
+      FuseMaps fuse;
+      if (int st = make_bytes_map(&fuse.q, fused.q, g[0].M, g[0].N); st != MXB200_OK)
+        return st;
+      if (int st = make_bytes_map(&fuse.qt, fused.q_t, g[0].N, g[0].M); st != MXB200_OK)
+        return st;
+      if (fused.fuse == kFuseReluSquare)
+        return plan.tile_n == 256 ? launch_fused<256, kFuseReluSquare>(args, fuse, pairs, s)
+                                  : launch_fused<192, kFuseReluSquare>(args, fuse, pairs, s);
+      return plan.tile_n == 256 ? launch_fused<256, kFuseReluSquareBwd>(args, fuse, pairs, s)
+                                : launch_fused<192, kFuseReluSquareBwd>(args, fuse, pairs, s);
+    }
+  }
+  return launch_pair_width<kProblems>(plan.tile_n, args, pairs, s);
+}
+
+int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale, void* d, int out_kind,
+         const void* resid, int64_t M, int64_t N, int64_t K, const float* alpha, int accumulate, int splits,
+         void* workspace, size_t workspace_bytes, void* stream, const FusedOut& fused = FusedOut{}) {
+  DeviceInfo dev;
+  if (int s = current_device(&dev); s != MXB200_OK)
+    return s;
+  const GemmDesc g{a, a_scale, b, b_scale, d, resid, alpha, M, N, K, out_kind, accumulate};
+  if (int s = check_gemm(g, fused, splits); s != MXB200_OK)
+    return s;
+  TilePlan plan = plan_tiles(&g, 1, dev.sms, fused.fuse != kFuseNone);
+  plan.splits[0] = splits;
+  return launch_gemms<1>(&g, 1, plan, dev, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), fused);
+}
+
+// Whether GEMMs i.. of a list go together, and how many: the CTA-pair kernel takes up to kMaxGroup of them.
+int group_size(const GemmDesc* g, int n) {
+  const int forced = g_tile_n.load();
+  int k = 0;
+  while (k < n && k < kMaxGroup && (forced >= 384 || (forced == 0 && g[k].M >= 256 && g[k].N >= 256)))
+    ++k;
+  return std::max(k, 1);
+}
+
+TilePlan plan_group(const GemmDesc* g, int n, int sms) {
+  TilePlan plan = plan_tiles(g, n, sms);
+  for (int i = 0; i < n; ++i)
+    plan.splits[i] = n == 1 ? mxb200_gemm_splits(g[i].M, g[i].N, g[i].K) : 1;
+  return plan;
+}
+
+size_t plan_workspace_bytes(const GemmDesc* g, int n, const TilePlan& plan) {
+  size_t counters = 0, partials = 0;
+  for (int i = 0; i < n; ++i) {
+    if (plan.splits[i] <= 1)
+      continue;
+    counters += static_cast<size_t>(plan.counters(g[i].M, g[i].N));
+    partials += static_cast<size_t>(plan.tiles(g[i].M, g[i].N)) * plan.splits[i] * plan.tile_bytes();
+  }
+  return partials == 0 ? 0 : counters_bytes(static_cast<int64_t>(counters)) + partials;
+}
+
+size_t group_workspace_bytes(const GemmDesc* g, int n, int sms) {
+  size_t most = 0;
+  for (int i = 0; i < n;) {
+    const int k = group_size(g + i, n - i);
+    most = std::max(most, plan_workspace_bytes(g + i, k, plan_group(g + i, k, sms)));
+    i += k;
+  }
+  return most;
+}
+
+int gemm_group(const GemmDesc* g, int n, void* workspace, size_t workspace_bytes, void* stream) {
+  DeviceInfo dev;
+  if (int s = current_device(&dev); s != MXB200_OK)
+    return s;
+  if (n < 0 || (n > 0 && g == nullptr))
+    return MXB200_ERR_NULL;
+  const FusedOut none;
+  for (int i = 0; i < n; ++i)  // every one is checked before anything is launched
+    if (int s = check_gemm(g[i], none, 1); s != MXB200_OK)
+      return s;
+  for (int i = 0; i < n;) {
+    const int k = group_size(g + i, n - i);
+    const TilePlan plan = plan_group(g + i, k, dev.sms);
+    auto* s = static_cast<cudaStream_t>(stream);
+    const int st = k == 1 ? launch_gemms<1>(g + i, 1, plan, dev, workspace, workspace_bytes, s, none)
+                          : launch_gemms<kMaxGroup>(g + i, k, plan, dev, workspace, workspace_bytes, s, none);
+    if (st != MXB200_OK)
+      return st;
+    i += k;
+  }
+  return MXB200_OK;
 }
 
 }  // namespace
@@ -1722,7 +1908,7 @@ extern "C" int mxb200_gemm_splits(int64_t M, int64_t N, int64_t K) {
   if (mxb200::current_device(&dev) != MXB200_OK || M <= 0 || N <= 0 || K <= 0)
     return 1;
   const mxb200::TilePlan plan = mxb200::plan_tiles(M, N, K, dev.sms);
-  const int64_t tiles = plan.tiles(), slots = plan.slots;
+  const int64_t tiles = plan.tiles(M, N), slots = plan.pair ? std::max(dev.sms / 2, 1) : dev.sms;
   const int64_t k_tiles = K / 128;
   // Splitting K costs a round trip of fp32 partial tiles through the workspace plus a serial reduction, and on
   // the d12-d26 shapes a narrower tile that fills a wave beat every split measured. It is kept for shapes that
@@ -1745,7 +1931,7 @@ extern "C" size_t mxb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, i
     return 0;
   if (mxb200::current_device(&dev) != MXB200_OK)
     dev.sms = 148;
-  return mxb200::workspace_bytes_for(mxb200::plan_tiles(M, N, K, dev.sms), splits);
+  return mxb200::workspace_bytes_for(mxb200::plan_tiles(M, N, K, dev.sms), M, N, splits);
 }
 
 extern "C" int mxb200_gemm_splitk(const void* a, const void* a_scale, const void* b, const void* b_scale, void* d,
@@ -1755,8 +1941,21 @@ extern "C" int mxb200_gemm_splitk(const void* a, const void* a_scale, const void
                       workspace_bytes, stream);
 }
 
+extern "C" size_t mxb200_gemm_group_workspace_bytes(const mxb200_gemm_desc* g, int n) {
+  mxb200::DeviceInfo dev;
+  if (g == nullptr || n <= 0)
+    return 0;
+  if (mxb200::current_device(&dev) != MXB200_OK)
+    dev.sms = 148;
+  return mxb200::group_workspace_bytes(g, n, dev.sms);
+}
+
+extern "C" int mxb200_gemm_group(const mxb200_gemm_desc* g, int n, void* workspace, size_t workspace_bytes, void* stream) {
+  return mxb200::gemm_group(g, n, workspace, workspace_bytes, stream);
+}
+
 extern "C" int mxb200_set_gemm_config(int tile_n, int max_ctas) {
-  if ((tile_n != 0 && tile_n != 128 && tile_n != 256 && tile_n != 384 && tile_n != 512) || max_ctas < 0)
+  if ((tile_n != 0 && tile_n != 128 && tile_n != 256 && tile_n != 384 && tile_n != 512 && tile_n != 640) || max_ctas < 0)
     return MXB200_ERR_ARGUMENT;
   mxb200::g_tile_n.store(tile_n);
   mxb200::g_max_ctas.store(max_ctas);
