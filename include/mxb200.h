@@ -185,9 +185,9 @@ MXB200_API int mxb200_gemm_relu_square_bwd(const void* a, const void* a_scale, c
 typedef enum mxb200_out_kind { MXB200_OUT_BF16 = 0, MXB200_OUT_F32 = 1 } mxb200_out_kind;
 
 /* Deterministic split-K for long-K, few-tile shapes (the weight gradients: K = tokens). The K range is cut
- * into `splits` slices run by different CTAs; partial tiles go through `workspace` and are summed in slice
- * order by whichever CTA finishes last, so results do not depend on timing. Counterpart of the reference's
- * split-K choice for these shapes (src/nanochat/model/fp8/mx_gemm.cpp:269-274, 293-314).
+ * into `splits` slices run by different CTAs, each of which writes an fp32 (M, N) matrix to `workspace`; a second launch
+ * sums them in slice order, so results do not depend on timing. Counterpart of the reference's split-K choice for these
+ * shapes (src/nanochat/model/fp8/mx_gemm.cpp:269-274, 293-314).
  * mxb200_gemm_splits picks a slice count for a shape on the current device (1 = not worth splitting);
  * mxb200_gemm_workspace_bytes gives the bytes `workspace` must hold for that count (0 when splits == 1).
  * The workspace needs no initialisation and may be reused by later calls on the same stream. */
@@ -202,14 +202,14 @@ MXB200_API int mxb200_gemm_splitk(const void* a, const void* a_scale, const void
  * must not trigger an allocation: a backend wired in at the reference's kernel seam gets plain pointers and a
  * stream but no workspace argument, runs on autograd worker threads in the middle of backward where a
  * cudaMalloc would stall the whole device, and in a trainer whose caching allocator already owns all of HBM a
- * raw allocation simply fails. The partial tiles and tile counters go to an array of
+ * raw allocation simply fails. The slices go to an array of
  * MXB200_STATIC_SCRATCH_BYTES that is part of the library's device image (each GPU that loads the library
  * carries it for the life of the process). The call itself allocates nothing, on the device or through any
  * library. Shapes whose mxb200_gemm_workspace_bytes(M, N, K, splits) exceeds that size are refused with
  * MXB200_ERR_WORKSPACE; pick fewer splits or use mxb200_gemm_splitk. The first call on each device looks up
  * the array's device address; make that first call outside any stream capture. All calls on a device share
- * the one array and it keeps whatever the previous call left: the tile counters are cleared on the stream at
- * the start of every call, the partial tiles are fully rewritten before they are read. Two calls whose kernels
+ * the one array and it keeps whatever the previous call left: the slices are fully rewritten before they are
+ * read. Two calls whose kernels
  * may overlap on the GPU (different streams, no dependency) would race on it; serialise them. Same arguments
  * and results as mxb200_gemm_splitk, bit for bit. */
 #define MXB200_STATIC_SCRATCH_BYTES (32u << 20)

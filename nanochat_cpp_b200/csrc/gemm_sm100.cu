@@ -16,8 +16,8 @@
 // Two accumulator buffers let the epilogue of tile i overlap the main loop of tile i+1. With BN = 256 they
 // overlap by 32 TMEM columns ([0,256) and [224,480), scales at [480,492)); the epilogue drains the shared
 // columns first and signals that separately, so the next main loop starts after one 32-column read.
-// Split-K (weight gradients, K = tokens): partial tiles go to a caller-provided workspace and the CTA that
-// finishes a tile last sums the slices in fixed order, so results are deterministic.
+// Split-K (weight gradients, K = tokens): every slice writes an fp32 (M, N) matrix of its own to a workspace and a second
+// kernel sums them in slice order, so results are deterministic.
 // Every wait is bounded: after kWaitLimitNs a wait records its site in a device word, raises a CTA-wide abort
 // flag that all other waits poll, and the kernel drains and returns.
 #include <algorithm>
@@ -76,7 +76,6 @@ enum WaitSite : uint32_t {
   kSiteMmaTmemEmpty = 3,
   kSiteMmaOverlap = 4,
   kSiteEpilogueFull = 5,
-  kSiteEpilogueSync = 6,
   kSiteSchedEmpty = 7,
   kSiteSchedFull = 8,
 };
@@ -104,13 +103,11 @@ struct GemmParams {
   void* d;
   const void* resid;
   const float* alpha;
-  float* partials;     // split-K: [tile][split][128 * BN] fp32
-  uint32_t* counters;  // split-K: [tile], zero on entry, zero on exit
   int M, N, K;
   int tiles_m, tiles_n;
   int k_tiles_total;   // K / 128
   int k_tiles_split;   // K tiles per split
-  int splits;
+  int splits;          // K slices: slice s of the output goes to rows s * M.. of d (fp32), summed by the reduction kernel
   int panel;           // n-tiles per raster panel
   int out_kind;
   int accumulate;
@@ -130,7 +127,7 @@ struct GemmParams {
 constexpr int kMaxGroup = 3;
 
 struct PairMaps {
-  CUtensorMap a, b, sfa, sfb, d, part;
+  CUtensorMap a, b, sfa, sfb, d;
 };
 
 template <int kProblems>
@@ -151,10 +148,8 @@ struct Barriers {
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t overlap_free;
-  uint64_t epi_sync;
   uint32_t tmem_base;
   uint32_t abort_flag;
-  uint32_t last_flag;
   uint32_t scale_done[2];  // fused quantizer, 256-wide tile: epilogue warps done with the tile in accumulator buffer 0 / 1
   // CTA-pair kernel, tile scheduler: the leader CTA's producer draws unit indices from a global counter and posts each
   // to both CTAs (sched_unit, sched_full); every other role of the pair reads it and reports to the leader's sched_empty
@@ -251,14 +246,6 @@ __device__ __forceinline__ void load_u32x8(const void* p, uint32_t* w, bool wide
     const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
     w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
   }
-}
-
-// L2-coherent read (partials written by other SMs)
-__device__ __forceinline__ void load_u32x8_cg(const void* p, uint32_t* w) {
-  asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-               : "l"(p)
-               : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
@@ -413,9 +400,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
       mbar_init(&bars->tmem_empty[a], kEpilogueThreads);
     }
     mbar_init(&bars->overlap_free, kEpilogueThreads);
-    mbar_init(&bars->epi_sync, kEpilogueThreads);
     bars->abort_flag = 0;
-    bars->last_flag = 0;
     fence_mbar_init();
   }
   if (warp == 0 && lane == 0) {
@@ -536,7 +521,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: 32 * (warp id % 4) ...
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? *p.alpha : 1.f;
-    uint32_t local = 0, sync_phase = 0;
+    uint32_t local = 0;
     bool ok = true;
     constexpr int kChunks = BN / 32;
     for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x, ++local) {
@@ -548,12 +533,8 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
       }
       tcgen05_fence_after_sync();
       const uint32_t acc_t = tmem_base + lane_base + (buf ? C::kAcc1 : C::kAcc0);
-      const int64_t row = static_cast<int64_t>(tc.m) * kBM + quarter * 32 + lane;
+      const int64_t row = static_cast<int64_t>(tc.split) * p.M + tc.m * kBM + quarter * 32 + lane;
       const int col0 = tc.n * BN;
-      float* part = p.splits > 1
-                          ? p.partials + (static_cast<int64_t>(tc.tile) * p.splits + tc.split) * (kBM * BN) +
-                                  static_cast<int64_t>(quarter * 32 + lane) * BN
-                          : nullptr;
 #pragma unroll 1
       for (int i = 0; i < kChunks; ++i) {
         // overlapping buffers: buffer 0 shares its last 32 columns, buffer 1 its first 32; drain those first
@@ -565,76 +546,11 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
           tcgen05_fence_before_sync();
           mbar_arrive(&bars->overlap_free);
         }
-        if (col0 + c * 32 < p.N) {
-          if (part != nullptr) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-              store_u32x8(part + c * 32 + 8 * g, r + 8 * g, true);
-          } else {
-            write_chunk(p, alpha, row, col0 + c * 32, reinterpret_cast<const float*>(r));
-          }
-        }
+        if (col0 + c * 32 < p.N)
+          write_chunk(p, alpha, row, col0 + c * 32, reinterpret_cast<const float*>(r));
       }
       tcgen05_fence_before_sync();
       mbar_arrive(&bars->tmem_empty[buf]);
-
-      if (part != nullptr) {
-        // split-K: publish this slice, then the last CTA to arrive for the tile sums all slices in order
-        __threadfence();
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-        if (threadIdx.x == 64) {
-          const uint32_t prev = atomicAdd(&p.counters[tc.tile], 1u);
-          const bool last = prev + 1 == static_cast<uint32_t>(p.splits);
-          if (last)
-            p.counters[tc.tile] = 0;  // ready for the next call
-          *reinterpret_cast<volatile uint32_t*>(&bars->last_flag) = last ? 1u : 0u;
-        }
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-        const bool last = *reinterpret_cast<volatile uint32_t*>(&bars->last_flag) != 0;
-        if (last) {
-          __threadfence();
-          const float* tile_part = p.partials + static_cast<int64_t>(tc.tile) * p.splits * (kBM * BN) +
-                                   static_cast<int64_t>(quarter * 32 + lane) * BN;
-#pragma unroll 1
-          for (int c = 0; c < kChunks; ++c) {
-            if (col0 + c * 32 >= p.N)
-              break;
-            float acc[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-              acc[k] = 0.f;
-            for (int s = 0; s < p.splits; ++s) {
-              const float* src = tile_part + static_cast<int64_t>(s) * (kBM * BN) + c * 32;
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                uint32_t w[8];
-                load_u32x8_cg(src + 8 * g, w);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  acc[8 * g + k] += __uint_as_float(w[k]);
-              }
-            }
-            write_chunk(p, alpha, row, col0 + c * 32, acc);
-          }
-        }
-        // the flag is rewritten only after every thread has read it
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-      }
     }
   }
 
@@ -964,14 +880,12 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
       mbar_init(&bars->tmem_empty[a], 2 * C::kEpiWarps);  // one arrival per epilogue warp of either CTA (leader's copy is used)
     }
     mbar_init(&bars->overlap_free, 8);  // the four warps per CTA that own the shared columns
-    mbar_init(&bars->epi_sync, C::kEpiThreads);
     for (int i = 0; i < kSchedSlots; ++i) {
       mbar_init(&bars->sched_full[i], 1);
       // readers of a posted unit: the MMA warp, the peer's producer, and both CTAs' epilogue warps (leader's copy)
       mbar_init(&bars->sched_empty[i], 2 * C::kEpiWarps + 2);
     }
     bars->abort_flag = 0;
-    bars->last_flag = 0;
     bars->scale_done[0] = bars->scale_done[1] = 0;
     fence_mbar_init();
   }
@@ -983,8 +897,6 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
       prefetch_tensormap(&args.maps[g].sfa);
       prefetch_tensormap(&args.maps[g].sfb);
       prefetch_tensormap(&args.maps[g].d);
-      if (args.p[g].splits > 1)
-        prefetch_tensormap(&args.maps[g].part);
     }
     if (kFuse != kFuseNone) {
       prefetch_tensormap(map_q);
@@ -1165,11 +1077,10 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
     const int quarter = warp & 3;
     const int col_part = (warp - 2) >> 2;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    uint32_t local = 0, sync_phase = 0;
+    uint32_t local = 0;
     bool ok = true;
     constexpr int kChunks = C::kTileN / 32;
     constexpr int kMine = (kChunks + C::kParts - 1) / C::kParts;  // the most chunks any part takes
-    constexpr int kHalf = 128 * C::kTileN;                        // elements of one CTA's half tile
     // part p takes chunks [first, first + n_mine): the remainder of kChunks / kParts goes to the leading parts
     const int n_mine = kChunks / C::kParts + (col_part < kChunks % C::kParts ? 1 : 0);
     const int first = col_part * (kChunks / C::kParts) + min(col_part, kChunks % C::kParts);
@@ -1210,9 +1121,7 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
       const bool row_ok = row < p.M;
       const int warp_row0 = tc.m * C::kTileM + static_cast<int>(rank) * 128 + quarter * 32;
       const int col0 = tc.n * C::kTileN;
-      const int64_t half_index = (static_cast<int64_t>(tc.tile) * p.splits + tc.split) * 2 + rank;
-      float* part = p.splits > 1 ? p.partials + half_index * kHalf + static_cast<int64_t>(quarter * 32 + lane) * C::kTileN
-                                 : nullptr;
+      const int out_row0 = tc.split * p.M + warp_row0;  // a K slice writes an (M, N) matrix of its own
       // Overlapping buffers: buffer 0 shares its last 32 columns (owned by the last part), buffer 1 its first 32
       // (part 0). The owning warps read those first and hand them over before anything else.
       const bool owns_shared = C::kOverlap && (buf == 0 ? col_part == kLast : col_part == 0);
@@ -1239,12 +1148,7 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
             mbar_arrive_cluster(overlap_leader);
         }
         const int col = col0 + c * 32;
-        if (part != nullptr) {
-          // split-K partials take the same TMA store path: the workspace is a (half tiles x 128 rows, TN) matrix
-          const int part_row0 = static_cast<int>(half_index) * 128 + quarter * 32;
-          store_rows_tma(&maps.part, stage, lane, r[i & 1], c * 32, part_row0, true);
-          store_rows_tma(&maps.part, stage, lane, r[i & 1] + 16, c * 32 + 16, part_row0, true);
-        } else if constexpr (kFuse != kFuseNone) {
+        if constexpr (kFuse != kFuseNone) {
           fused_quantize_chunk<kFuse>(p, &maps.d, map_q, map_qt, stage, lane, reinterpret_cast<const float*>(r[i & 1]),
                                       row, col, warp_row0, row_ok && col < p.N, h_pieces,
                                       i + 1 < n_mine ? col0 + chunk_of(i + 1) * 32 : -1,
@@ -1254,9 +1158,9 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
           const bool issue = warp_row0 < p.M && col < p.N;
           uint32_t o[32];
           compute_chunk(p, alpha, row, col, reinterpret_cast<const float*>(r[i & 1]), valid, o);
-          store_rows_tma(&maps.d, stage, lane, o, col, warp_row0, issue);
+          store_rows_tma(&maps.d, stage, lane, o, col, out_row0, issue);
           if (p.out_kind == kOutF32)
-            store_rows_tma(&maps.d, stage, lane, o + 16, col + 16, warp_row0, issue);
+            store_rows_tma(&maps.d, stage, lane, o + 16, col + 16, out_row0, issue);
         }
       }
       if constexpr (C::kStageScales) {
@@ -1292,68 +1196,6 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
       if (lane == 0)
         mbar_arrive_cluster(empty_leader[buf]);
 
-      if (part != nullptr) {
-        // split-K, per half tile: the rows of this CTA are reduced by whichever CTA finishes them last
-        if (lane == 0) {
-          tma_store_wait_all<0>();                       // this warp's partial stores have completed ...
-          asm volatile("fence.proxy.async;" ::: "memory");  // ... and are ordered before generic-proxy traffic
-        }
-        __threadfence();
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-        if (threadIdx.x == 64) {
-          uint32_t* counter = &p.counters[tc.tile * 2 + rank];
-          const uint32_t prev = atomicAdd(counter, 1u);
-          const bool last = prev + 1 == static_cast<uint32_t>(p.splits);
-          if (last)
-            *counter = 0;
-          *reinterpret_cast<volatile uint32_t*>(&bars->last_flag) = last ? 1u : 0u;
-        }
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-        const bool last = *reinterpret_cast<volatile uint32_t*>(&bars->last_flag) != 0;
-        if (last) {
-          // The reduction reads only the workspace, so it need not follow the TMEM lane mapping: a warp takes whole
-          // rows, a lane 8 consecutive columns, and every load and store is a contiguous run across the warp.
-          __threadfence();
-          const float* half_base = p.partials + (static_cast<int64_t>(tc.tile) * p.splits * 2 + rank) * kHalf;
-          const int sub = lane * 8;
-          if (sub < C::kTileN && col0 + sub < p.N) {
-#pragma unroll 1
-            for (int rr = warp - 2; rr < 128; rr += C::kEpiWarps) {
-              const int64_t grow = static_cast<int64_t>(tc.m) * C::kTileM + rank * 128 + rr;
-              if (grow >= p.M)
-                break;
-              float acc[8];
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                acc[k] = 0.f;
-              for (int sl = 0; sl < p.splits; ++sl) {  // slice order: the sum does not depend on who arrived last
-                uint32_t w[8];
-                load_u32x8_cg(half_base + static_cast<int64_t>(sl) * 2 * kHalf + rr * C::kTileN + sub, w);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  acc[k] += __uint_as_float(w[k]);
-              }
-              write_octet(p, alpha, grow, col0 + sub, acc);
-            }
-          }
-        }
-        mbar_arrive(&bars->epi_sync);
-        if (!wait_bounded(&bars->epi_sync, sync_phase, bars, kSiteEpilogueSync)) {
-          ok = false;
-          break;
-        }
-        sync_phase ^= 1u;
-      }
     }
   }
 
@@ -1377,6 +1219,54 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
 
 }  // namespace
 }  // namespace mxb200
+
+// ------------------------------------------------------------------------------------------------ K slices
+//
+// Sum of a GEMM's K slices, fp32 (M, N) matrices one after another, in slice order, with the output step of the unsplit
+// kernel (alpha, +=, or bf16 with the residual). A kernel of its own behind the GEMM: all SMs take part, where the CTA
+// that finished a tile last used to sum it alone at the launch's end (13 of 31 us on 768 x 768 x 16384).
+namespace mxb200 {
+namespace {
+
+struct ReduceJob {
+  GemmParams p;  // d, resid, alpha, N, out_kind, accumulate
+  const float* slices;
+  int64_t elements;
+  int splits;
+  int first_block;
+};
+
+struct ReduceParams {
+  ReduceJob jobs[kMaxGroup];
+  int n;
+};
+
+constexpr int kReduceThreads = 256;
+
+}  // namespace
+}  // namespace mxb200
+
+__global__ void __launch_bounds__(mxb200::kReduceThreads) mxb200_gemm_sum_slices(const __grid_constant__ mxb200::ReduceParams r) {
+  using namespace mxb200;
+  int j = 0;
+  while (j + 1 < r.n && static_cast<int>(blockIdx.x) >= r.jobs[j + 1].first_block)
+    ++j;
+  const ReduceJob& job = r.jobs[j];
+  const int64_t at = (static_cast<int64_t>(static_cast<int>(blockIdx.x) - job.first_block) * kReduceThreads + threadIdx.x) * 8;
+  if (at >= job.elements)
+    return;
+  const float alpha = job.p.out_kind == kOutF32 && job.p.alpha != nullptr ? __ldg(job.p.alpha) : 1.f;
+  float acc[8] = {};
+#pragma unroll 4
+  for (int s = 0; s < job.splits; ++s) {
+    uint32_t w[8];
+    load_u32x8(job.slices + s * job.elements + at, w, true);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      acc[k] += __uint_as_float(w[k]);
+  }
+  write_octet(job.p, alpha, at / job.p.N, static_cast<int>(at % job.p.N), acc);
+}
 
 // ------------------------------------------------------------------------------------------------ kernels
 //
@@ -1506,19 +1396,55 @@ struct TilePlan {
   int tile_m, tile_n;
   int splits[kMaxGroup] = {1, 1, 1};
   int64_t tiles(int64_t M, int64_t N) const { return (M + tile_m - 1) / tile_m * ((N + tile_n - 1) / tile_n); }
-  size_t tile_bytes() const { return static_cast<size_t>(tile_m) * tile_n * sizeof(float); }
-  int64_t counters(int64_t M, int64_t N) const { return tiles(M, N) * (pair ? 2 : 1); }
 };
 
-// Estimated cycles of one unit of the CTA-pair kernel with `k_iters` K steps of 128, besides what the launch costs anyway.
-// A step runs at the slower of MMA execution (2 TN cycles) and what an SM can ingest (about 58 bytes per cycle in
-// practice); 256-wide tiles pay an overlap bubble of about 1500 cycles per tile.
-double unit_cycles(int tn, int64_t k_iters) {
-  const double ingest = (16384.0 + tn * 64.0 + 1536.0) / 58.0;  // bytes a CTA loads per K step / (B/clk)
-  return static_cast<double>(k_iters) * std::max(2.0 * tn, ingest) + (tn == 256 ? 1500.0 : 300.0);
+// What the planner expects of the CTA-pair kernel, in SM cycles.
+//   A K step of 128 costs a CTA its share of the operands over the path from L2, about 50 bytes per cycle when all SMs pull
+//   (16384 + 64 TN + scales; the MMA's own 2 TN cycles stay below that at every width), an output tile its bytes over the
+//   same path; 256-wide tiles pay a hand-over bubble between tiles. Fitted to singles and groups from 256 x 768 x 768 to
+//   16384 x 6144 x 1536 at the clocks those run at.
+//   A K slice writes an fp32 tile, and the launch that sums the slices comes on top.
+double step_cycles(int tn) {
+  return (16384.0 + tn * 64.0 + (tn == 128 ? 1024.0 : 1536.0)) / 50.0;
+}
+double out_cycles(int tn, const GemmDesc& g) {
+  const double bytes = g.out_kind == kOutF32 ? (g.accumulate ? 8.0 : 4.0) : (g.resid != nullptr ? 4.0 : 2.0);
+  return 128.0 * tn * bytes / 50.0;
+}
+constexpr double kBubbleCycles = 1200.0, kTileCycles = 300.0;
+double sum_cycles(const GemmDesc& g, int splits) {
+  return 4500.0 + static_cast<double>(g.M) * g.N * 4.0 * splits / 3500.0;
 }
 
-TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair = false) {
+// Expected cycles of n GEMMs in one launch with TN-wide tiles and the given slices, taken up in the order given. Pairs draw
+// their units from a counter: with many short units per pair a launch ends within a fraction of one of the average share,
+// with few long ones on a whole round.
+double launch_cycles(const GemmDesc* g, int n, int tn, const int* splits, double slots) {
+  double work = 0.0, least = 0.0, last = 0.0, units = 0.0, tail = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const int64_t k = g[i].K / 128, slice = (k + splits[i] - 1) / splits[i];
+    const double u = static_cast<double>((g[i].M + 255) / 256 * ((g[i].N + tn - 1) / tn)) * static_cast<double>((k + slice - 1) / slice);
+    double c = static_cast<double>(slice) * step_cycles(tn) + kTileCycles;
+    c += splits[i] > 1 ? 128.0 * tn * 4.0 / 50.0 : out_cycles(tn, g[i]);
+    if (tn == 256)
+      c += kBubbleCycles;
+    work += u * c;
+    units += u;
+    // units of this GEMM alone, behind what came before it
+    const double before = (work - u * c) / slots;
+    const double rounds = u / slots < 4.0 ? std::ceil(u / slots) : u / slots + 0.25;
+    least = std::max(least, i == 0 ? rounds * c : before + c);
+    last = c;
+    if (splits[i] > 1)
+      tail += sum_cycles(g[i], splits[i]);
+  }
+  if (n == 1)
+    return least + tail;
+  return std::max(least, work / slots + (units > slots ? 0.5 * last : 0.0)) + tail;
+}
+
+// Tile width and slices with the least expected time. `fixed`: slices of a single GEMM given by the caller.
+TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed) {
   int forced = g_tile_n.load();
   if (need_pair && (forced == 128 || forced == 256))
     forced = 0;  // the fused-quantize epilogues exist in the CTA-pair kernel only
@@ -1529,47 +1455,56 @@ TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair = false) {
   if (!(forced >= 384 || need_pair || (forced == 0 && wide))) {
     t.pair = false, t.tile_m = 128;
     t.tile_n = (forced == 128 || forced == 256) ? forced : (g[0].N >= 256 ? 256 : 128);
+    t.splits[0] = std::max(fixed, 1);
     return t;
   }
   t.pair = true, t.tile_m = 256;
-  if (forced >= 384) {
-    t.tile_n = forced == 512 ? 256 : forced == 384 ? 192 : 128;
-    return t;
-  }
   const double slots = std::max(sms / 2, 1);
   double best = 0.0;
   for (int tn : {256, 192, 128}) {
-    if (need_pair && tn == 128)
+    if ((need_pair && tn == 128) || (forced >= 384 && tn != (forced == 512 ? 256 : forced == 384 ? 192 : 128)))
       continue;
-    double units = 0.0, work = 0.0, longest = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double u = static_cast<double>((g[i].M + 255) / 256 * ((g[i].N + tn - 1) / tn));
-      const double c = unit_cycles(tn, g[i].K / 128);
-      units += u, work += u * c;
-      longest = std::max(longest, c);
+    int splits[kMaxGroup] = {1, 1, 1};
+    const auto consider = [&] {
+      const double cost = launch_cycles(g, n, tn, splits, slots);
+      if (best == 0.0 || cost < best * 0.99) {
+        best = cost, t.tile_n = tn;
+        std::copy(splits, splits + kMaxGroup, t.splits);
+      }
+    };
+    if (fixed > 0 || need_pair) {
+      splits[0] = std::max(fixed, 1);
+      consider();
+      continue;
     }
-    // Pairs draw their tiles from a counter, so with many short tiles per pair the launch ends within a fraction of a
-    // tile of the average share; with few long ones (the weight gradients) it ends on a whole round.
-    const double share = units / slots;
-    const double cost = share >= 4.0 ? work / slots + 0.25 * longest : std::ceil(share) * (work / units);
-    if (best == 0.0 || cost < best * 0.995)
-      best = cost, t.tile_n = tn;
+    consider();
+    // K slices, one GEMM at a time: each takes the count that helps most given the others
+    for (int i = 0; i < n; ++i) {
+      int kept = 1;
+      double least = launch_cycles(g, n, tn, splits, slots);
+      for (int s = 2; s <= 8; s *= 2) {
+        if (g[i].K / 128 / s < 8)
+          break;
+        splits[i] = s;
+        if (const double c = launch_cycles(g, n, tn, splits, slots); c < least * 0.97)
+          least = c, kept = s;
+      }
+      splits[i] = kept;
+    }
+    consider();
   }
   return t;
 }
 
-TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, bool need_pair = false) {
+TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, int fixed) {
   GemmDesc g{};
-  g.M = M, g.N = N, g.K = K;
-  return plan_tiles(&g, 1, sms, need_pair);
+  g.M = M, g.N = N, g.K = K, g.out_kind = kOutF32;
+  return plan_tiles(&g, 1, sms, false, fixed);
 }
 
-size_t counters_bytes(int64_t counters) {
-  return static_cast<size_t>((counters * 4 + 255) / 256 * 256);
-}
-
-size_t workspace_bytes_for(const TilePlan& t, int64_t M, int64_t N, int splits) {
-  return splits <= 1 ? 0 : counters_bytes(t.counters(M, N)) + static_cast<size_t>(t.tiles(M, N)) * splits * t.tile_bytes();
+// Bytes of a GEMM's K slices; 0 when K is not split.
+size_t slice_bytes(const GemmDesc& g, int splits) {
+  return splits <= 1 ? 0 : static_cast<size_t>(g.M) * g.N * splits * sizeof(float);
 }
 
 template <typename Kernel>
@@ -1717,17 +1652,10 @@ int pair_maps(PairMaps* m, const GemmDesc& g, const TilePlan& plan, const GemmPa
   if (int st = make_scale_map(&m->sfb, g.b_scale, g.N, g.K, plan.tile_n == 128 ? 1 : 2); st != MXB200_OK)
     return st;
   if (g.d != nullptr) {
-    if (int st = make_output_map(&m->d, g.d, g.M, g.N, g.out_kind == kOutF32); st != MXB200_OK)
+    if (int st = make_output_map(&m->d, p.d, g.M * p.splits, g.N, p.out_kind == kOutF32); st != MXB200_OK)
       return st;
   } else {
     m->d = m->a;  // never used: the relu^2 backward form writes no plain output
-  }
-  m->part = m->d;  // unused without a K split
-  if (p.splits > 1) {
-    // partial half tiles, stacked: (tiles x splits x 2 halves x 128 rows, TN) fp32
-    const int64_t rows = static_cast<int64_t>(p.tiles_m) * p.tiles_n * p.splits * 256;
-    if (int st = make_output_map(&m->part, p.partials, rows, plan.tile_n, true); st != MXB200_OK)
-      return st;
   }
   return MXB200_OK;
 }
@@ -1743,43 +1671,44 @@ int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInf
                  size_t workspace_bytes, cudaStream_t s, const FusedOut& fused) {
   PairArgs<kProblems> args{};
   int64_t units = 0;
-  size_t counters = 0, need = 0;
-  bool split = false;
+  ReduceParams sums{};
+  int sum_blocks = 0;
+  size_t used = 0;
   for (int i = 0; i < n; ++i) {
-    args.p[i] = gemm_params(g[i], plan, plan.splits[i], fused);
+    GemmParams& p = args.p[i];
+    p = gemm_params(g[i], plan, plan.splits[i], fused);
     const int64_t tiles = plan.tiles(g[i].M, g[i].N);
-    units += tiles * args.p[i].splits;
-    if (units > 0x7fffffffLL)
+    units += tiles * p.splits;
+    if (units > 0x7fffffffLL || g[i].M * p.splits > 0x7fffffffLL)
       return MXB200_ERR_SHAPE;
     args.end[i] = static_cast<int>(units);
-    if (args.p[i].splits > 1) {
-      split = true;
-      counters += static_cast<size_t>(plan.counters(g[i].M, g[i].N));
-      need += static_cast<size_t>(tiles) * args.p[i].splits * plan.tile_bytes();
+    if (p.splits > 1) {
+      // the slices go to the workspace as plain fp32 outputs; the reduction does the output step
+      ReduceJob& sum = sums.jobs[sums.n++];
+      sum.p = p;
+      sum.elements = g[i].M * g[i].N;
+      sum.splits = p.splits;
+      sum.first_block = sum_blocks;
+      sum_blocks += static_cast<int>((sum.elements / 8 + kReduceThreads - 1) / kReduceThreads);
+      if (workspace == nullptr || workspace_bytes < used + slice_bytes(g[i], p.splits))
+        return MXB200_ERR_WORKSPACE;
+      if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+        return MXB200_ERR_ALIGNMENT;
+      p.d = static_cast<unsigned char*>(workspace) + used;
+      used += slice_bytes(g[i], p.splits);
+      sum.slices = static_cast<const float*>(p.d);
+      p.resid = nullptr, p.alpha = nullptr, p.out_kind = kOutF32, p.accumulate = 0, p.wide = true;
     }
   }
   for (int i = n; i < kProblems; ++i)
     args.p[i] = args.p[n - 1], args.end[i] = static_cast<int>(units);
-  if (split) {
-    // all counters first, zeroed together, then each GEMM's partial tiles
-    const size_t head = counters_bytes(static_cast<int64_t>(counters));
-    if (workspace == nullptr || workspace_bytes < head + need)
-      return MXB200_ERR_WORKSPACE;
-    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
-      return MXB200_ERR_ALIGNMENT;
-    auto* counter = static_cast<uint32_t*>(workspace);
-    auto* partial = static_cast<unsigned char*>(workspace) + head;
-    if (cudaMemsetAsync(counter, 0, head, s) != cudaSuccess)
-      return MXB200_ERR_LAUNCH;
-    for (int i = 0; i < n; ++i) {
-      if (args.p[i].splits == 1)
-        continue;
-      args.p[i].counters = counter;
-      args.p[i].partials = reinterpret_cast<float*>(partial);
-      counter += plan.counters(g[i].M, g[i].N);
-      partial += static_cast<size_t>(plan.tiles(g[i].M, g[i].N)) * args.p[i].splits * plan.tile_bytes();
-    }
-  }
+  const auto sum_slices = [&](int status) {
+    if (status != MXB200_OK || sums.n == 0)
+      return status;
+    mxb200_gemm_sum_slices<<<static_cast<unsigned>(sum_blocks), kReduceThreads, 0, s>>>(sums);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return launch_status();
+  };
   const int cap = g_max_ctas.load() > 0 ? g_max_ctas.load() : dev.sms;
   if (!plan.pair) {
     CUtensorMap ma, mb;
@@ -1788,7 +1717,7 @@ int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInf
     if (int st = make_operand_map(&mb, g[0].b, g[0].N, g[0].K, plan.tile_n); st != MXB200_OK)
       return st;
     const int grid = static_cast<int>(std::min<int64_t>(units, cap));
-    return plan.tile_n == 256 ? launch<256>(ma, mb, args.p[0], grid, s) : launch<128>(ma, mb, args.p[0], grid, s);
+    return sum_slices(plan.tile_n == 256 ? launch<256>(ma, mb, args.p[0], grid, s) : launch<128>(ma, mb, args.p[0], grid, s));
   }
   for (int i = 0; i < n; ++i)
     if (int st = pair_maps(&args.maps[i], g[i], plan, args.p[i]); st != MXB200_OK)
@@ -1811,7 +1740,7 @@ int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInf
                                 : launch_fused<192, kFuseReluSquareBwd>(args, fuse, pairs, s);
     }
   }
-  return launch_pair_width<kProblems>(plan.tile_n, args, pairs, s);
+  return sum_slices(launch_pair_width<kProblems>(plan.tile_n, args, pairs, s));
 }
 
 int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale, void* d, int out_kind,
@@ -1823,8 +1752,8 @@ int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale,
   const GemmDesc g{a, a_scale, b, b_scale, d, resid, alpha, M, N, K, out_kind, accumulate};
   if (int s = check_gemm(g, fused, splits); s != MXB200_OK)
     return s;
-  TilePlan plan = plan_tiles(&g, 1, dev.sms, fused.fuse != kFuseNone);
-  plan.splits[0] = splits;
+  // the plan of a single GEMM depends on its shape and slices only, as the workspace query's does
+  const TilePlan plan = fused.fuse != kFuseNone ? plan_tiles(&g, 1, dev.sms, true, 1) : plan_tiles(M, N, K, dev.sms, splits);
   return launch_gemms<1>(&g, 1, plan, dev, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), fused);
 }
 
@@ -1837,29 +1766,18 @@ int group_size(const GemmDesc* g, int n) {
   return std::max(k, 1);
 }
 
-TilePlan plan_group(const GemmDesc* g, int n, int sms) {
-  TilePlan plan = plan_tiles(g, n, sms);
-  for (int i = 0; i < n; ++i)
-    plan.splits[i] = n == 1 ? mxb200_gemm_splits(g[i].M, g[i].N, g[i].K) : 1;
-  return plan;
-}
-
 size_t plan_workspace_bytes(const GemmDesc* g, int n, const TilePlan& plan) {
-  size_t counters = 0, partials = 0;
-  for (int i = 0; i < n; ++i) {
-    if (plan.splits[i] <= 1)
-      continue;
-    counters += static_cast<size_t>(plan.counters(g[i].M, g[i].N));
-    partials += static_cast<size_t>(plan.tiles(g[i].M, g[i].N)) * plan.splits[i] * plan.tile_bytes();
-  }
-  return partials == 0 ? 0 : counters_bytes(static_cast<int64_t>(counters)) + partials;
+  size_t bytes = 0;
+  for (int i = 0; i < n; ++i)
+    bytes += slice_bytes(g[i], plan.splits[i]);
+  return bytes;
 }
 
 size_t group_workspace_bytes(const GemmDesc* g, int n, int sms) {
   size_t most = 0;
   for (int i = 0; i < n;) {
     const int k = group_size(g + i, n - i);
-    most = std::max(most, plan_workspace_bytes(g + i, k, plan_group(g + i, k, sms)));
+    most = std::max(most, plan_workspace_bytes(g + i, k, plan_tiles(g + i, k, sms, false, 0)));
     i += k;
   }
   return most;
@@ -1877,7 +1795,7 @@ int gemm_group(const GemmDesc* g, int n, void* workspace, size_t workspace_bytes
       return s;
   for (int i = 0; i < n;) {
     const int k = group_size(g + i, n - i);
-    const TilePlan plan = plan_group(g + i, k, dev.sms);
+    const TilePlan plan = plan_tiles(g + i, k, dev.sms, false, 0);
     auto* s = static_cast<cudaStream_t>(stream);
     const int st = k == 1 ? launch_gemms<1>(g + i, 1, plan, dev, workspace, workspace_bytes, s, none)
                           : launch_gemms<kMaxGroup>(g + i, k, plan, dev, workspace, workspace_bytes, s, none);
@@ -1907,31 +1825,13 @@ extern "C" int mxb200_gemm_splits(int64_t M, int64_t N, int64_t K) {
   mxb200::DeviceInfo dev;
   if (mxb200::current_device(&dev) != MXB200_OK || M <= 0 || N <= 0 || K <= 0)
     return 1;
-  const mxb200::TilePlan plan = mxb200::plan_tiles(M, N, K, dev.sms);
-  const int64_t tiles = plan.tiles(M, N), slots = plan.pair ? std::max(dev.sms / 2, 1) : dev.sms;
-  const int64_t k_tiles = K / 128;
-  // Splitting K costs a round trip of fp32 partial tiles through the workspace plus a serial reduction, and on
-  // the d12-d26 shapes a narrower tile that fills a wave beat every split measured. It is kept for shapes that
-  // cannot fill even a quarter of the machine with tiles alone and have a deep K to share out (d12's 768 x 768
-  // weight gradient: 40 us with four splits against 47 us; with half the machine filled a split already loses).
-  if (tiles * 4 > slots)
-    return 1;
-  int best = 1;
-  for (int s = 2; s <= 4; s *= 2) {
-    if (k_tiles / s < 32 || tiles * s > slots)
-      break;
-    best = s;
-  }
-  return best;
+  return mxb200::plan_tiles(M, N, K, dev.sms, 0).splits[0];
 }
 
 extern "C" size_t mxb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int splits) {
-  mxb200::DeviceInfo dev;
   if (splits <= 1 || M <= 0 || N <= 0 || K <= 0)
     return 0;
-  if (mxb200::current_device(&dev) != MXB200_OK)
-    dev.sms = 148;
-  return mxb200::workspace_bytes_for(mxb200::plan_tiles(M, N, K, dev.sms), M, N, splits);
+  return static_cast<size_t>(M) * N * splits * sizeof(float);
 }
 
 extern "C" int mxb200_gemm_splitk(const void* a, const void* a_scale, const void* b, const void* b_scale, void* d,
