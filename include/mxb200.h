@@ -65,7 +65,7 @@ typedef struct mxb200_mx_out {
  * x: (rows, cols) contiguous bf16 (x_bf16 != 0) or fp32. out: x scaled along its rows; out_t: x's transpose
  * (cols, rows) scaled along its own rows. rows, cols % 128 == 0 (the callers' mx_fits, fp8.h:86-88);
  * x, data pointers and lds 16-byte aligned. prologue RELU_SQUARE quantizes bf16(relu(x)^2), bf16 x only.
- * Plain bf16 tensors of more than four tiles of 128 x 128 per SM run as persistent CTAs that draw their tiles from a
+ * Tensors of more than four bf16 or two fp32 tiles of 128 x 128 per SM run as persistent CTAs that draw their tiles from a
  * counter in the library's device image; at most 256 such launches may be in flight on a device at once (launches on
  * one stream never overlap; this bounds launches spread over many streams). */
 MXB200_API int mxb200_quantize_mx(const void* x, int x_bf16, int64_t rows, int64_t cols, mxb200_mx_out out, mxb200_mx_out out_t,
@@ -78,13 +78,28 @@ typedef struct mxb200_quantize_job {
   mxb200_mx_out out, out_t;
 } mxb200_quantize_job;
 
-/* mxb200_quantize_mx (no prologue) of n_jobs tensors of one input type in as few launches as possible (32 tensors
+/* mxb200_quantize_mx (no prologue) of n_jobs tensors of one input type in as few launches as possible (32 or 64 tensors
  * each), bit for bit what n_jobs separate calls give. It stands for the runs of quantize_mx calls the reference makes
  * on small tensors: the three parts of the merged q/k/v weight (src/nanochat/model/fp8/fp8.cpp:155-171) and a model's
  * weights after an optimizer step (Fp8WeightCache, fp8.cpp:516-536), where a launch per matrix of one or two waves of
  * tiles is bound by its own ramp-up and tail. jobs is read on the host during the call. */
 MXB200_API int mxb200_quantize_mx_batch(const mxb200_quantize_job* jobs, int n_jobs, int x_bf16, int scale_rule,
                                         void* stream);
+
+/* The same for tensors of both input types in one list (what one Linear quantizes together: its activation in bf16 and
+ * its fp32 weight). */
+typedef struct mxb200_quantize_item {
+  mxb200_quantize_job job;
+  int32_t x_bf16;
+} mxb200_quantize_item;
+MXB200_API int mxb200_quantize_mx_items(const mxb200_quantize_item* items, int n, int scale_rule, void* stream);
+
+/* The value-embedding gate's columns of a Linear's input and of its gradient (torch ops in the reference, fp8.cpp:436-438,
+ * 457): dst (rows, cols) = src and dst += src (bf16), row strides in elements. */
+MXB200_API int mxb200_copy_columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t rows, int64_t cols,
+                                   void* stream);
+MXB200_API int mxb200_add_columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t rows, int64_t cols,
+                                  void* stream);
 
 /* Replaces nanochat::kernels::quantize_mx_relu_square_bwd (fp8_kernel.h:41-43, fp8_kernel.cu:207-210):
  * quantizes dh = bf16(h > 0 ? g * 2h : 0) from bf16 g, h (rows, cols) without writing dh. */

@@ -20,7 +20,8 @@ STATIC_SCRATCH_BYTES = 32 << 20
 
 # every symbol include/mxb200.h declares
 SYMBOLS = (
-    "mxb200_quantize_mx", "mxb200_quantize_mx_batch", "mxb200_quantize_mx_relu_square_bwd", "mxb200_gemm_bf16", "mxb200_gemm_f32",
+    "mxb200_quantize_mx", "mxb200_quantize_mx_batch", "mxb200_quantize_mx_items",
+    "mxb200_copy_columns", "mxb200_add_columns", "mxb200_quantize_mx_relu_square_bwd", "mxb200_gemm_bf16", "mxb200_gemm_f32",
     "mxb200_gemm_relu_square", "mxb200_gemm_relu_square_bwd", "mxb200_residual_norm_mx_fwd",
     "mxb200_softcap_ce_loss", "mxb200_softcap_ce_grad_mx",
     "mxb200_count_valid", "mxb200_reduce_losses", "mxb200_scale_bf16",
@@ -41,6 +42,11 @@ class QuantizeJob(ctypes.Structure):
     """mxb200_quantize_job."""
     _fields_ = [("x", ctypes.c_void_p), ("rows", ctypes.c_int64), ("cols", ctypes.c_int64), ("out", MxOut),
                 ("out_t", MxOut)]
+
+
+class QuantizeItem(ctypes.Structure):
+    """mxb200_quantize_item."""
+    _fields_ = [("job", QuantizeJob), ("x_bf16", ctypes.c_int32)]
 
 
 class ResidualNormMx(ctypes.Structure):
@@ -72,6 +78,8 @@ def _load() -> ctypes.CDLL:
     vp, i64, i32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
     lib.mxb200_quantize_mx.argtypes = [vp, i32, i64, i64, MxOut, MxOut, i32, i32, vp]
     lib.mxb200_quantize_mx_batch.argtypes = [ctypes.POINTER(QuantizeJob), i32, i32, i32, vp]
+    lib.mxb200_copy_columns.argtypes = lib.mxb200_add_columns.argtypes = [vp, i64, vp, i64, i64, i64, vp]
+    lib.mxb200_quantize_mx_items.argtypes = [ctypes.POINTER(QuantizeItem), i32, i32, vp]
     lib.mxb200_quantize_mx_relu_square_bwd.argtypes = [vp, vp, i64, i64, MxOut, MxOut, i32, vp]
     lib.mxb200_gemm_bf16.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, i64, vp]
     lib.mxb200_gemm_f32.argtypes = [vp, vp, vp, vp, vp, i64, i64, i64, vp, i32, vp]

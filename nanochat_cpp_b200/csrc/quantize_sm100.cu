@@ -17,6 +17,7 @@
 // tensors of more than one wave persistent CTAs that draw tiles from a counter and bring them in by TMA a tile ahead.
 // HBM traffic is the algorithmic minimum: every input byte read once, every output byte written once.
 #include <algorithm>
+#include <vector>
 
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -349,6 +350,7 @@ constexpr uint64_t kStreamDrainLimitNs = 50000000ull;
 struct StreamBarriers {
   uint64_t full[kStreamStages];
   int tile_of[kStreamStages];  // the tile whose load completes full[s]; -1 is the stop sign
+  int job_of[kStreamStages];   // and the tensor it belongs to
   uint32_t abort_flag;
 };
 
@@ -389,6 +391,25 @@ __device__ __forceinline__ bool stream_wait(uint64_t* bar, uint32_t parity, Stre
     }
   }
   return true;
+}
+
+// The end of a walk that stopped before its i-th tile. Loads drawn and not taken (a wait gave up) may still land in this
+// CTA's shared memory: they get a bounded time before it leaves. The last walker out hands the slot back zeroed.
+__device__ __forceinline__ void stream_leave(StreamBarriers* bars, int i, uint32_t* sched, uint32_t walkers) {
+  if (*reinterpret_cast<volatile uint32_t*>(&bars->abort_flag) != 0) {
+    for (int j = i; j < i + kStreamStages; ++j) {
+      const uint64_t t0 = global_timer_ns();
+      while (!mbar_try_wait(&bars->full[j % kStreamStages], static_cast<uint32_t>(j / kStreamStages) & 1u))
+        if (global_timer_ns() - t0 > kStreamDrainLimitNs)
+          break;
+    }
+  }
+  __threadfence();
+  if (atomicAdd(&sched[1], 1u) == walkers - 1) {
+    sched[0] = 0u;
+    sched[1] = 0u;
+    __threadfence();
+  }
 }
 
 // Row pass from a tile in shared memory. A thread owns 16 consecutive values (32 bytes) and reads them as two 16-byte
@@ -536,17 +557,15 @@ struct StreamParams {
   int slot;
 };
 
-template <int kPro>
-__device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const StreamParams& sp) {
-  constexpr int kGroups = kPro == kSoftcapGrad ? kSoftcapGroups : 1;
+__device__ __forceinline__ void quantize_stream_softcap(const CUtensorMap* map_x, const StreamParams& sp) {
+  constexpr int kGroups = kSoftcapGroups;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int group = kGroups == 1 ? 0 : static_cast<int>(threadIdx.x) / kThreads;
-  const int t = kGroups == 1 ? static_cast<int>(threadIdx.x) : static_cast<int>(threadIdx.x) % kThreads;
+  const int group = static_cast<int>(threadIdx.x) / kThreads;
+  const int t = static_cast<int>(threadIdx.x) % kThreads;
   unsigned char* buffers = smem_raw + group * kStreamGroupBytes;
   unsigned char* sc = buffers + kStreamStages * kStreamTileBytes;  // [2 tiles in turn][rows, columns][512]
   StreamBarriers* bars = reinterpret_cast<StreamBarriers*>(sc + 4 * kScaleTileBytes);
   const QuantParams& p = sp.q;
-  const bool want_rows = p.out.data != nullptr, want_cols = p.out_t.data != nullptr;
   uint32_t* sched = g_quantize_sched + 2 * sp.slot;  // [0] next tile to hand out, [1] groups that have left
   const uint32_t walkers = gridDim.x * kGroups;      // groups go round the SMs before an SM gets its second
 
@@ -556,13 +575,10 @@ __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const 
     bars->abort_flag = 0;
     fence_mbar_init();
   }
-  uint32_t table_base = 0;
-  if constexpr (kPro == kSoftcapGrad) {
-    float* table = reinterpret_cast<float*>(smem_raw + kGroups * kStreamGroupBytes);
-    for (uint32_t i = threadIdx.x; i < kLogitEntries; i += kThreads * kGroups)
-      table[i] = softcap_tanh(logit_of_entry(i), p.ce.softcap);
-    table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
-  }
+  float* table = reinterpret_cast<float*>(smem_raw + kGroups * kStreamGroupBytes);
+  for (uint32_t i = threadIdx.x; i < kLogitEntries; i += kThreads * kGroups)
+    table[i] = softcap_tanh(logit_of_entry(i), p.ce.softcap);
+  const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
   __syncthreads();
 
   // Thread 0 posts this CTA's i-th tile and starts its load into buffer i % stages. A number past the last tile is the
@@ -601,56 +617,220 @@ __device__ __forceinline__ void quantize_stream(const CUtensorMap* map_x, const 
     const bool landed = stream_wait(&bars->full[s], static_cast<uint32_t>(i / kStreamStages) & 1u, bars,
                                     kStreamWaitLimitNs, static_cast<uint32_t>(i));
     const int tile = landed ? *reinterpret_cast<volatile int*>(&bars->tile_of[s]) : -1;
-    if (kPro == kSoftcapGrad && !group_all(1 + group, tile >= 0))
+    if (!group_all(1 + group, tile >= 0))
       break;  // the passes meet at a barrier below: the group goes in together or not at all
     const int tile_r = tile / p.tiles_c, tile_c = tile % p.tiles_c;
     const int64_t row0 = static_cast<int64_t>(tile_r) * kTile, col0 = static_cast<int64_t>(tile_c) * kTile;
     __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(buffers + s * kStreamTileBytes);
     unsigned char* sc_rows = sc + (i & 1) * 2 * kScaleTileBytes;
     unsigned char* sc_cols = sc_rows + kScaleTileBytes;
-    if (tile >= 0) {
-      if constexpr (kPro == kSoftcapGrad) {
-        stream_row_pass_softcap(buf, p, row0, col0, sc_rows, table_base, t);
-        fence_proxy_async_smem();  // these writes come before the load that reuses the buffer
-        group_sync(1 + group);
-      } else if (want_rows) {
-        stream_row_pass(buf, p, row0, col0, sc_rows, t);
-      }
-      if (want_cols)
-        column_pass<false>(buf, p, row0, col0, sc_cols, t);
-    }
-    // every thread is done with the buffer and the scale bytes are staged; the stop sign, or a wait that gave up,
-    // ends the walk for all threads together
-    if (!group_all(1 + group, tile >= 0))
-      break;
+    stream_row_pass_softcap(buf, p, row0, col0, sc_rows, table_base, t);
+    fence_proxy_async_smem();  // these writes come before the load that reuses the buffer
+    group_sync(1 + group);
+    if (p.out_t.data != nullptr)
+      column_pass<false>(buf, p, row0, col0, sc_cols, t);
+    group_sync(1 + group);  // every thread is done with the buffer and the scale bytes are staged
     if (t == 0 && drawing)
       post(i + kStreamStages, drawn);
     // the next tile stages its scale bytes in the other half, and the one after that comes after another barrier
     write_scale_tiles(p, tile_r, tile_c, sc_rows, sc_cols, t);
   }
-  if (t == 0) {
-    if (*reinterpret_cast<volatile uint32_t*>(&bars->abort_flag) != 0) {
-      // loads drawn and not taken may still land in this CTA's shared memory: give them a bounded time before leaving
-      for (int j = i; j < i + kStreamStages; ++j) {
-        const uint64_t t0 = global_timer_ns();
-        while (!mbar_try_wait(&bars->full[j % kStreamStages], static_cast<uint32_t>(j / kStreamStages) & 1u))
-          if (global_timer_ns() - t0 > kStreamDrainLimitNs)
-            break;
-      }
+  if (t == 0)
+    stream_leave(bars, i, sched, walkers);
+}
+
+// ---- plain input, one or several tensors: the streaming form over a list of tensors
+//
+// A stage holds 32 KB of input: a whole 128 x 128 tile of bf16, or the upper or lower 64 rows of a tile of fp32 (half of
+// its scale tiles: 8 of every 16 bytes row-wise, 2 of every 4 column-wise). Both kinds may be in one list, so what a
+// Linear quantizes together (activation and fp32 weight) is one launch.
+struct StreamJob {
+  mxb200_mx_out out, out_t;
+  int tiles_c;
+  int first_unit;
+  bool f32, wide_out_t;
+};
+
+// What a layer quantizes together, and what a model's weights take (kernel parameters: 1 and 15 KB).
+constexpr int kFewJobs = 4, kManyJobs = 64;
+
+template <int kMaxJobs>
+struct StreamBatch {
+  CUtensorMap maps[kMaxJobs];
+  StreamJob jobs[kMaxJobs];
+  int n, units, slot;
+  bool floor_rule;
+};
+
+// fp32 row pass over 64 rows in shared memory: a thread owns 16 consecutive values, read as four 16-byte vectors in an
+// order rotated by its pair of lanes, so that the eight lanes of a request cover all 32 banks.
+__device__ __forceinline__ void stream_row_pass_f32(const float* tile, const QuantParams& p, int64_t row0, int64_t col0,
+                                                    int half, unsigned char* sc_rows, int t) {
+  constexpr int kIters = (kTile / 2) * (kTile / 16) / kThreads;
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int q = it * kThreads + t, r = q >> 3, piece = q & 7, c = piece * 16, rot = (piece >> 1) & 3;
+    const float4* src = reinterpret_cast<const float4*>(tile + r * kTile + c);
+    float4 v[4];
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[i] = src[(i + rot) & 3];
+      m = fmaxf(fmaxf(fmaxf(m, fabsf(v[i].x)), fmaxf(fabsf(v[i].y), fabsf(v[i].z))), fabsf(v[i].w));  // drops NaN
     }
-    // the last CTA to leave hands the slot back zeroed
-    __threadfence();
-    if (atomicAdd(&sched[1], 1u) == walkers - 1) {
-      sched[0] = 0u;
-      sched[1] = 0u;
-      __threadfence();
+    uint32_t m_bits = __float_as_uint(m);
+    m_bits = max(m_bits, __shfl_xor_sync(0xffffffffu, m_bits, 1));
+    const int e = mx_exponent(m_bits, p.floor_rule);
+    const float mul = __uint_as_float(mx_multiplier_bits(e));
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      o[i] = cvt_e4m3x4(v[i].x * mul, v[i].y * mul, v[i].z * mul, v[i].w * mul);
+    // o[i] belongs at word (i + rot) & 3
+    const bool one = (rot & 1) != 0, two = (rot & 2) != 0;
+    const uint32_t a0 = one ? o[3] : o[0], a1 = one ? o[0] : o[1], a2 = one ? o[1] : o[2], a3 = one ? o[2] : o[3];
+    *reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.out.data) + (row0 + r) * p.out.ld + col0 + c) =
+          two ? make_uint4(a2, a3, a0, a1) : make_uint4(a0, a1, a2, a3);
+    if ((t & 1) == 0)
+      sc_rows[mx_scale_tile_offset(half * 64 + r, c >> 5)] = static_cast<unsigned char>(e);
+  }
+}
+
+// fp32 column pass over 64 rows: a thread owns one column of a 32-row block (a warp reads 128 contiguous bytes per row).
+__device__ __forceinline__ void stream_column_pass_f32(const float* tile, const QuantParams& p, int64_t row0,
+                                                       int64_t col0, int half, unsigned char* sc_cols, int t) {
+  const int c = t & (kTile - 1), rb = t >> 7;
+  float v[32];
+  float m = 0.f;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    v[k] = tile[(rb * 32 + k) * kTile + c];
+    m = fmaxf(m, fabsf(v[k]));
+  }
+  const int e = mx_exponent(__float_as_uint(m), p.floor_rule);
+  const float mul = __uint_as_float(mx_multiplier_bits(e));
+  uint32_t w[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    w[k] = cvt_e4m3x4(v[4 * k] * mul, v[4 * k + 1] * mul, v[4 * k + 2] * mul, v[4 * k + 3] * mul);
+  store_u32x8(static_cast<unsigned char*>(p.out_t.data) + (col0 + c) * p.out_t.ld + row0 + rb * 32, w, p.wide_out_t);
+  sc_cols[mx_scale_tile_offset(c, half * 2 + rb)] = static_cast<unsigned char>(e);
+}
+
+// This half's bytes of the two scale tiles.
+__device__ __forceinline__ void write_half_scale_tiles(const QuantParams& p, int tile_r, int tile_c, int half,
+                                                       const unsigned char* sc_rows, const unsigned char* sc_cols, int t) {
+  if (t < 32) {
+    if (p.out.data != nullptr) {
+      const int at = t * 16 + half * 8;
+      *reinterpret_cast<uint2*>(static_cast<unsigned char*>(p.out.scale) +
+                                (static_cast<int64_t>(tile_r) * p.out.scale_tiles + tile_c) * kScaleTileBytes + at) =
+            *reinterpret_cast<const uint2*>(sc_rows + at);
+    }
+  } else if (t >= 128) {
+    if (p.out_t.data != nullptr) {
+      const int at = (t - 128) * 4 + half * 2;
+      *reinterpret_cast<uint16_t*>(static_cast<unsigned char*>(p.out_t.scale) +
+                                   (static_cast<int64_t>(tile_c) * p.out_t.scale_tiles + tile_r) * kScaleTileBytes + at) =
+            *reinterpret_cast<const uint16_t*>(sc_cols + at);
     }
   }
 }
 
-// Several tensors in one launch: a weight matrix of a d12-d26 model is 36 to 700 tiles, under one or two waves of
-// the machine, so a launch per weight is bound by its own ramp-up and tail (12 us for 14 MB). The tiles of up to
-// kMaxBatch tensors are numbered through; a CTA finds its tensor by its first tile.
+template <int kMaxJobs>
+__device__ __forceinline__ void quantize_stream_batch(const StreamBatch<kMaxJobs>& b) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* sc = smem_raw + kStreamStages * kStreamTileBytes;  // [2 units in turn][rows, columns][512]
+  StreamBarriers* bars = reinterpret_cast<StreamBarriers*>(sc + 4 * kScaleTileBytes);
+  const int t = static_cast<int>(threadIdx.x);
+  uint32_t* sched = g_quantize_sched + 2 * b.slot;
+
+  if (t == 0) {
+    for (int s = 0; s < kStreamStages; ++s)
+      mbar_init(&bars->full[s], 1);
+    bars->abort_flag = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+
+  // as in the softcap form: the first unit is the CTA's own number, later ones are drawn a whole unit ahead
+  bool drawing = true;
+  auto post = [&](int i, int unit) {
+    const int s = i % kStreamStages;
+    if (unit >= b.units) {
+      bars->tile_of[s] = -1;
+      mbar_arrive(&bars->full[s]);
+      drawing = false;
+      return;
+    }
+    int lo = 0, hi = b.n;  // the tensor whose units include this one
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (unit >= b.jobs[mid].first_unit)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    const StreamJob& job = b.jobs[lo];
+    const int u = unit - job.first_unit, tile = job.f32 ? u >> 1 : u;
+    bars->tile_of[s] = u;
+    bars->job_of[s] = lo;
+    mbar_arrive_expect_tx(1u, &bars->full[s], kStreamTileBytes);
+    tma_load_2d_hint(1u, smem_raw + s * kStreamTileBytes, &b.maps[lo], &bars->full[s], (tile % job.tiles_c) * kTile,
+                     (tile / job.tiles_c) * kTile + (job.f32 ? (u & 1) * (kTile / 2) : 0), l2_policy_evict_first());
+  };
+  if (t == 0) {
+    post(0, static_cast<int>(blockIdx.x));
+    for (int i = 1; i < kStreamStages && drawing; ++i)
+      post(i, static_cast<int>(gridDim.x + atomicAdd(&sched[0], 1u)));
+  }
+
+  int i = 0;
+  for (;; ++i) {
+    const int s = i % kStreamStages;
+    int drawn = 0;
+    if (t == 0 && drawing)
+      drawn = static_cast<int>(gridDim.x + atomicAdd(&sched[0], 1u));
+    const bool landed = stream_wait(&bars->full[s], static_cast<uint32_t>(i / kStreamStages) & 1u, bars,
+                                    kStreamWaitLimitNs, static_cast<uint32_t>(i));
+    const int u = landed ? *reinterpret_cast<volatile int*>(&bars->tile_of[s]) : -1;
+    const StreamJob& job = b.jobs[u >= 0 ? *reinterpret_cast<volatile int*>(&bars->job_of[s]) : 0];
+    const bool f32 = job.f32;
+    const int tile = f32 ? u >> 1 : u, half = u & 1;
+    const int tile_r = tile / job.tiles_c, tile_c = tile % job.tiles_c;
+    const int64_t row0 = static_cast<int64_t>(tile_r) * kTile + (f32 ? half * (kTile / 2) : 0);
+    const int64_t col0 = static_cast<int64_t>(tile_c) * kTile;
+    const QuantParams p{nullptr, nullptr, 0, job.out, job.out_t, job.tiles_c, b.floor_rule, false, job.wide_out_t, SoftcapGrad{}};
+    const unsigned char* buf = smem_raw + s * kStreamTileBytes;
+    unsigned char* sc_rows = sc + (i & 1) * 2 * kScaleTileBytes;
+    unsigned char* sc_cols = sc_rows + kScaleTileBytes;
+    if (u >= 0) {
+      if (f32) {
+        if (p.out.data != nullptr)
+          stream_row_pass_f32(reinterpret_cast<const float*>(buf), p, row0, col0, half, sc_rows, t);
+        if (p.out_t.data != nullptr)
+          stream_column_pass_f32(reinterpret_cast<const float*>(buf), p, row0, col0, half, sc_cols, t);
+      } else {
+        if (p.out.data != nullptr)
+          stream_row_pass(reinterpret_cast<const __nv_bfloat16*>(buf), p, row0, col0, sc_rows, t);
+        if (p.out_t.data != nullptr)
+          column_pass<false>(reinterpret_cast<const __nv_bfloat16*>(buf), p, row0, col0, sc_cols, t);
+      }
+    }
+    if (__syncthreads_and(u >= 0) == 0)
+      break;
+    if (t == 0 && drawing)
+      post(i + kStreamStages, drawn);
+    if (f32)
+      write_half_scale_tiles(p, tile_r, tile_c, half, sc_rows, sc_cols, t);
+    else
+      write_scale_tiles(p, tile_r, tile_c, sc_rows, sc_cols, t);
+  }
+  if (t == 0)
+    stream_leave(bars, i, sched, gridDim.x);
+}
+
+// Small lists (no more units than the machine holds at once): a CTA per tile, which finds its tensor by its first tile.
 constexpr int kMaxBatch = 32;
 
 struct BatchJob {
@@ -659,7 +839,7 @@ struct BatchJob {
   mxb200_mx_out out, out_t;
   int tiles_c;
   int first_tile;
-  bool wide_in, wide_out_t;
+  bool f32, wide_in, wide_out_t;
 };
 
 struct BatchParams {
@@ -668,8 +848,9 @@ struct BatchParams {
   bool floor_rule;
 };
 
-// One CTA of the batched launch: finds its tensor by its first tile.
-template <bool kIn32>
+enum InputKinds : int { kAllBf16 = 0, kAllF32 = 1, kMixed = 2 };
+
+template <int kKinds>
 __device__ __forceinline__ void quantize_batch_tile(const BatchParams& bp) {
   int j = 0;
   const int tile = static_cast<int>(blockIdx.x);
@@ -678,7 +859,10 @@ __device__ __forceinline__ void quantize_batch_tile(const BatchParams& bp) {
   const BatchJob& job = bp.jobs[j];
   QuantParams p{job.x,      nullptr,         job.ld, job.out, job.out_t, job.tiles_c, bp.floor_rule,
                 job.wide_in, job.wide_out_t, SoftcapGrad{}};
-  quantize_tile<kIn32, kNone>(p, tile - job.first_tile);
+  if (kKinds == kAllF32 || (kKinds == kMixed && job.f32))
+    quantize_tile<true, kNone>(p, tile - job.first_tile);
+  else
+    quantize_tile<false, kNone>(p, tile - job.first_tile);
 }
 
 }  // namespace
@@ -691,49 +875,49 @@ __device__ __forceinline__ void quantize_batch_tile(const BatchParams& bp) {
   __global__ void __launch_bounds__(mxb200::kThreads, CTAS) name(const mxb200::QuantParams p) {                        \
     mxb200::quantize_tile<IN32, PRO>(p, static_cast<int>(blockIdx.x));                                                 \
   }
-#define MXB200_QUANTIZE_BATCH_KERNEL(name, IN32, CTAS)                                                                 \
+#define MXB200_QUANTIZE_BATCH_KERNEL(name, KINDS, CTAS)                                                                \
   __global__ void __launch_bounds__(mxb200::kThreads, CTAS) name(const __grid_constant__ mxb200::BatchParams bp) {     \
-    mxb200::quantize_batch_tile<IN32>(bp);                                                                             \
+    mxb200::quantize_batch_tile<KINDS>(bp);                                                                            \
+  }
+#define MXB200_QUANTIZE_STREAM_KERNEL(name, JOBS)                                                                      \
+  __global__ void __launch_bounds__(mxb200::kThreads, MXB200_STREAM_CTAS_PER_SM)                                       \
+        name(const __grid_constant__ mxb200::StreamBatch<JOBS> batch) {                                                \
+    mxb200::quantize_stream_batch<JOBS>(batch);                                                                        \
   }
 
-MXB200_QUANTIZE_KERNEL(mxb200_quantize_bf16, false, mxb200::kNone, 4)
-MXB200_QUANTIZE_KERNEL(mxb200_quantize_f32, true, mxb200::kNone, 2)
 MXB200_QUANTIZE_KERNEL(mxb200_quantize_relu_square, false, mxb200::kReluSquare, 4)
 MXB200_QUANTIZE_KERNEL(mxb200_quantize_relu_square_bwd, false, mxb200::kReluSquareBwd, 3)
 // Streaming form: persistent, three CTAs per SM, each with two 32 KB tile buffers.
-__global__ void __launch_bounds__(mxb200::kThreads, MXB200_STREAM_CTAS_PER_SM)
-    mxb200_quantize_bf16_stream(const __grid_constant__ CUtensorMap map_x, const mxb200::StreamParams sp) {
-  mxb200::quantize_stream<mxb200::kNone>(&map_x, sp);
+MXB200_QUANTIZE_STREAM_KERNEL(mxb200_quantize_stream, mxb200::kFewJobs)
+MXB200_QUANTIZE_STREAM_KERNEL(mxb200_quantize_stream_many, mxb200::kManyJobs)
+// A few columns of a matrix (the value-embedding gate reads 12), copied or added; bound by the launch.
+__global__ void __launch_bounds__(256) mxb200_columns_bf16(__nv_bfloat16* dst, int64_t dst_ld, const __nv_bfloat16* src,
+                                                           int64_t src_ld, int64_t n, int cols, bool add) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n)
+    return;
+  const int64_t r = i / cols, c = i % cols;
+  const __nv_bfloat16 v = src[r * src_ld + c];
+  __nv_bfloat16* d = dst + r * dst_ld + c;
+  *d = add ? __float2bfloat16(__bfloat162float(*d) + __bfloat162float(v)) : v;
 }
 // Softcap form: one CTA of three groups per SM around one table of tanh.
 __global__ void __launch_bounds__(mxb200::kThreads * mxb200::kSoftcapGroups, 1)
     mxb200_quantize_softcap_grad(const __grid_constant__ CUtensorMap map_x, const mxb200::StreamParams sp) {
-  mxb200::quantize_stream<mxb200::kSoftcapGrad>(&map_x, sp);
+  mxb200::quantize_stream_softcap(&map_x, sp);
 }
-MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_bf16, false, 4)
-MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_f32, true, 2)
+MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_bf16, mxb200::kAllBf16, 4)
+MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_f32, mxb200::kAllF32, 2)
+MXB200_QUANTIZE_BATCH_KERNEL(mxb200_quantize_batch_mixed, mxb200::kMixed, 2)
 
 namespace mxb200 {
 namespace {
 
 using QuantKernel = void (*)(QuantParams);
-using QuantBatchKernel = void (*)(BatchParams);
 
-template <bool kIn32, int kPro>
+template <int kPro>
 constexpr QuantKernel quantize_kernel() {
-  if constexpr (kIn32)
-    return mxb200_quantize_f32;
-  else if constexpr (kPro == kReluSquare)
-    return mxb200_quantize_relu_square;
-  else if constexpr (kPro == kReluSquareBwd)
-    return mxb200_quantize_relu_square_bwd;
-  else
-    return mxb200_quantize_bf16;
-}
-
-template <bool kIn32>
-constexpr QuantBatchKernel quantize_batch_kernel() {
-  return kIn32 ? mxb200_quantize_batch_f32 : mxb200_quantize_batch_bf16;
+  return kPro == kReluSquare ? mxb200_quantize_relu_square : mxb200_quantize_relu_square_bwd;
 }
 
 int check_out(const mxb200_mx_out& o, int64_t ld_min) {
@@ -748,42 +932,31 @@ int check_out(const mxb200_mx_out& o, int64_t ld_min) {
   return MXB200_OK;
 }
 
-template <bool kIn32, int kPro>
+template <int kPro>
 int launch(const QuantParams& p, int64_t tiles, cudaStream_t stream) {
-  constexpr size_t smem = (kIn32 ? 4 : 2) * kTile * kTile + 2 * kScaleTileBytes;
-  static std::atomic<int> configured_for{-1};
-  int device = 0;
-  cudaGetDevice(&device);
-  if (smem > 48 * 1024 && configured_for.load() != device) {
-    if (cudaFuncSetAttribute(quantize_kernel<kIn32, kPro>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return MXB200_ERR_LAUNCH;
-    configured_for.store(device);
-  }
-  quantize_kernel<kIn32, kPro>()<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(p);
+  constexpr size_t smem = 2 * kTile * kTile + 2 * kScaleTileBytes;
+  quantize_kernel<kPro>()<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(p);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return launch_status();
 }
 
-// A streaming kernel on a bf16 tensor: (rows, ld) row-major behind a tiled map with a 128 x 128 box.
-template <int kPro>
-int launch_stream(const QuantParams& p, int64_t rows, int64_t cols, int64_t tiles, int sms, cudaStream_t stream) {
+// (rows, ld) row-major, a box of one stage: 128 x 128 of bf16 or 64 x 128 of fp32.
+int make_input_map(CUtensorMap* map, const void* x, bool f32, int64_t rows, int64_t cols, int64_t ld) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr)
     return MXB200_ERR_DRIVER;
-  CUtensorMap map;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.cols) * 2};
-  const cuuint32_t box[2] = {kTile, kTile};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * (f32 ? 4 : 2)};
+  const cuuint32_t box[2] = {kTile, f32 ? kTile / 2 : kTile};
   const cuuint32_t estr[2] = {1, 1};
-  if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p.x), dims, strides, box, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return MXB200_ERR_DRIVER;
-  constexpr bool softcap = kPro == kSoftcapGrad;
-  constexpr auto kernel = softcap ? mxb200_quantize_softcap_grad : mxb200_quantize_bf16_stream;
-  constexpr size_t smem = softcap ? kSoftcapSmemBytes : kStreamGroupBytes;
-  static std::atomic<int> configured_for{-1};
+  const CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                        const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? MXB200_OK : MXB200_ERR_DRIVER;
+}
+
+template <typename Kernel>
+int configure_once(Kernel kernel, size_t smem, std::atomic<int>& configured_for) {
   int device = 0;
   cudaGetDevice(&device);
   if (configured_for.load() != device) {
@@ -791,13 +964,145 @@ int launch_stream(const QuantParams& p, int64_t rows, int64_t cols, int64_t tile
       return MXB200_ERR_LAUNCH;
     configured_for.store(device);
   }
+  return MXB200_OK;
+}
+
+int next_stream_slot() {
   static std::atomic<uint32_t> next_slot{0};
-  const StreamParams sp{p, static_cast<int>(tiles), static_cast<int>(next_slot.fetch_add(1) % kStreamSchedSlots)};
-  const int64_t most = softcap ? sms : kStreamCtasPerSm * static_cast<int64_t>(sms);
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, most));
-  kernel<<<grid, softcap ? kThreads * kSoftcapGroups : kThreads, smem, stream>>>(map, sp);
+  return static_cast<int>(next_slot.fetch_add(1) % kStreamSchedSlots);
+}
+
+int launch_softcap(const QuantParams& p, int64_t rows, int64_t cols, int64_t tiles, int sms, cudaStream_t stream) {
+  CUtensorMap map;
+  if (int s = make_input_map(&map, p.x, false, rows, cols, p.cols); s != MXB200_OK)
+    return s;
+  static std::atomic<int> configured_for{-1};
+  if (int s = configure_once(mxb200_quantize_softcap_grad, kSoftcapSmemBytes, configured_for); s != MXB200_OK)
+    return s;
+  const StreamParams sp{p, static_cast<int>(tiles), next_stream_slot()};
+  mxb200_quantize_softcap_grad<<<static_cast<unsigned>(std::min<int64_t>(tiles, sms)), kThreads * kSoftcapGroups,
+                                 kSoftcapSmemBytes, stream>>>(map, sp);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return launch_status();
+}
+
+using Item = mxb200_quantize_item;
+
+bool asked(const Item& i) {
+  return i.job.out.data != nullptr || i.job.out_t.data != nullptr;
+}
+
+int64_t tiles_of(const Item& i) {
+  return (i.job.rows / kTile) * (i.job.cols / kTile);
+}
+
+bool wide_out_t(const mxb200_mx_out& o) {
+  return (reinterpret_cast<uintptr_t>(o.data) & 31u) == 0 && o.ld % 32 == 0;
+}
+
+template <int kMaxJobs>
+constexpr auto stream_kernel() {
+  if constexpr (kMaxJobs == kFewJobs)
+    return mxb200_quantize_stream;
+  else
+    return mxb200_quantize_stream_many;
+}
+
+// Streams up to kMaxJobs of the items, from the front; `taken`: how many it went over.
+template <int kMaxJobs>
+int launch_stream(const Item* items, int n, int* taken, bool floor_rule, int sms, cudaStream_t stream) {
+  constexpr auto kernel = stream_kernel<kMaxJobs>();
+  static std::atomic<int> configured_for{-1};
+  if (int s = configure_once(kernel, kStreamGroupBytes, configured_for); s != MXB200_OK)
+    return s;
+  StreamBatch<kMaxJobs> b;
+  b.n = 0;
+  int64_t units = 0;
+  int i = 0;
+  for (; i < n && b.n < kMaxJobs; ++i) {
+    const Item& it = items[i];
+    if (!asked(it))
+      continue;
+    const bool f32 = it.x_bf16 == 0;
+    const int64_t mine = tiles_of(it) * (f32 ? 2 : 1);
+    if (units + mine > 0x7fffffffLL)
+      break;
+    if (int s = make_input_map(&b.maps[b.n], it.job.x, f32, it.job.rows, it.job.cols, it.job.cols); s != MXB200_OK)
+      return s;
+    b.jobs[b.n++] = StreamJob{it.job.out, it.job.out_t, static_cast<int>(it.job.cols / kTile), static_cast<int>(units), f32,
+                              wide_out_t(it.job.out_t)};
+    units += mine;
+  }
+  *taken = i;
+  if (b.n == 0)
+    return MXB200_OK;
+  b.units = static_cast<int>(units);
+  b.slot = next_stream_slot();
+  b.floor_rule = floor_rule;
+  const int64_t most = kStreamCtasPerSm * static_cast<int64_t>(sms);
+  kernel<<<static_cast<unsigned>(std::min<int64_t>(units, most)), kThreads, kStreamGroupBytes, stream>>>(b);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return launch_status();
+}
+
+template <int kKinds>
+int launch_batch(const BatchParams& bp, int tiles, cudaStream_t stream) {
+  constexpr auto kernel = kKinds == kAllBf16 ? mxb200_quantize_batch_bf16
+                          : kKinds == kAllF32 ? mxb200_quantize_batch_f32 : mxb200_quantize_batch_mixed;
+  constexpr size_t smem = (kKinds == kAllBf16 ? 2 : 4) * kTile * kTile + 2 * kScaleTileBytes;
+  static std::atomic<int> configured_for{-1};
+  if (int s = configure_once(kernel, smem, configured_for); s != MXB200_OK)
+    return s;
+  kernel<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(bp);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return launch_status();
+}
+
+// No prologue: any mix of bf16 and fp32 tensors, all checked.
+// More input than the CTA-per-tile form holds at once (four CTAs per SM of bf16 tiles, two of fp32) streams through
+// persistent CTAs: those forms would run in several waves, each reading, computing and writing in turn. Below that the
+// CTA-per-tile form starts sooner: it needs no tensor map, no draw and no barrier before its first load.
+int quantize_items(const Item* items, int n, bool floor_rule, const DeviceInfo& dev, cudaStream_t stream) {
+  int64_t stages = 0;
+  bool bf16 = false, f32 = false;
+  for (int i = 0; i < n; ++i) {
+    if (!asked(items[i]))
+      continue;
+    stages += tiles_of(items[i]) * (items[i].x_bf16 != 0 ? 1 : 2);
+    (items[i].x_bf16 != 0 ? bf16 : f32) = true;
+  }
+  int i = 0;
+  if (stages > 4 * static_cast<int64_t>(dev.sms)) {
+    while (i < n) {
+      int taken = 0;
+      const int st = n - i <= kFewJobs ? launch_stream<kFewJobs>(items + i, n - i, &taken, floor_rule, dev.sms, stream)
+                                       : launch_stream<kManyJobs>(items + i, n - i, &taken, floor_rule, dev.sms, stream);
+      if (st != MXB200_OK)
+        return st;
+      i += taken;
+    }
+    return MXB200_OK;
+  }
+  while (i < n) {
+    BatchParams bp{};
+    bp.floor_rule = floor_rule;
+    int tiles = 0;
+    for (; i < n && bp.n < kMaxBatch; ++i) {
+      const Item& it = items[i];
+      if (!asked(it))
+        continue;
+      bp.jobs[bp.n++] = BatchJob{it.job.x, it.job.cols, it.job.out, it.job.out_t, static_cast<int>(it.job.cols / kTile), tiles,
+                                 it.x_bf16 == 0, (reinterpret_cast<uintptr_t>(it.job.x) & 31u) == 0, wide_out_t(it.job.out_t)};
+      tiles += static_cast<int>(tiles_of(it));
+    }
+    if (bp.n == 0)
+      break;
+    const int st = !f32 ? launch_batch<kAllBf16>(bp, tiles, stream)
+                   : !bf16 ? launch_batch<kAllF32>(bp, tiles, stream) : launch_batch<kMixed>(bp, tiles, stream);
+    if (st != MXB200_OK)
+      return st;
+  }
+  return MXB200_OK;
 }
 
 int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t cols, mxb200_mx_out out,
@@ -833,53 +1138,33 @@ int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t co
     p.ce = *ce;
   const int64_t tiles = (rows / kTile) * (cols / kTile);
   auto* s = static_cast<cudaStream_t>(stream);
-  if (!x_bf16)
-    return launch<true, kNone>(p, tiles, s);
+  if (pro == kNone) {
+    const Item item{{x, rows, cols, out, out_t}, x_bf16 ? 1 : 0};
+    return quantize_items(&item, 1, p.floor_rule, dev, s);
+  }
   switch (pro) {
-    case kNone:
-      // more tiles than the one-shot kernel holds at once (4 CTAs per SM): stream them through persistent CTAs
-      if (tiles > 4 * static_cast<int64_t>(dev.sms))
-        return launch_stream<kNone>(p, rows, cols, tiles, dev.sms, s);
-      return launch<false, kNone>(p, tiles, s);
     case kReluSquare:
-      return launch<false, kReluSquare>(p, tiles, s);
+      return launch<kReluSquare>(p, tiles, s);
     case kReluSquareBwd:
-      return launch<false, kReluSquareBwd>(p, tiles, s);
+      return launch<kReluSquareBwd>(p, tiles, s);
     case kSoftcapGrad:
-      return ce != nullptr ? launch_stream<kSoftcapGrad>(p, rows, cols, tiles, dev.sms, s) : MXB200_ERR_NULL;
+      return ce != nullptr ? launch_softcap(p, rows, cols, tiles, dev.sms, s) : MXB200_ERR_NULL;
     default:
       return MXB200_ERR_ARGUMENT;
   }
 }
 
-template <bool kIn32>
-int launch_batch(const BatchParams& bp, int tiles, cudaStream_t stream) {
-  constexpr size_t smem = (kIn32 ? 4 : 2) * kTile * kTile + 2 * kScaleTileBytes;
-  static std::atomic<int> configured_for{-1};
-  int device = 0;
-  cudaGetDevice(&device);
-  if (smem > 48 * 1024 && configured_for.load() != device) {
-    if (cudaFuncSetAttribute(quantize_batch_kernel<kIn32>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return MXB200_ERR_LAUNCH;
-    configured_for.store(device);
-  }
-  quantize_batch_kernel<kIn32>()<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(bp);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
-}
-
-int quantize_batch(const mxb200_quantize_job* jobs, int n_jobs, bool x_bf16, int scale_rule, void* stream) {
+int quantize_list(const Item* items, int n, int scale_rule, void* stream) {
   DeviceInfo dev;
   if (int s = current_device(&dev); s != MXB200_OK)
     return s;
-  if (n_jobs < 0 || (n_jobs > 0 && jobs == nullptr))
+  if (n < 0 || (n > 0 && items == nullptr))
     return MXB200_ERR_NULL;
   if (scale_rule != MXB200_SCALE_REFERENCE && scale_rule != MXB200_SCALE_OCP_FLOOR)
     return MXB200_ERR_ARGUMENT;
-  // every job is checked before anything is launched
-  for (int i = 0; i < n_jobs; ++i) {
-    const mxb200_quantize_job& j = jobs[i];
+  // every one is checked before anything is launched
+  for (int i = 0; i < n; ++i) {
+    const mxb200_quantize_job& j = items[i].job;
     if (j.x == nullptr)
       return MXB200_ERR_NULL;
     if (j.rows <= 0 || j.cols <= 0 || j.rows % kTile != 0 || j.cols % kTile != 0 ||
@@ -892,34 +1177,7 @@ int quantize_batch(const mxb200_quantize_job* jobs, int n_jobs, bool x_bf16, int
     if (int s = check_out(j.out_t, j.rows); s != MXB200_OK)
       return s;
   }
-  auto* s = static_cast<cudaStream_t>(stream);
-  int i = 0;
-  while (i < n_jobs) {
-    BatchParams bp{};
-    bp.floor_rule = scale_rule == MXB200_SCALE_OCP_FLOOR;
-    int64_t tiles = 0;
-    while (i < n_jobs && bp.n < kMaxBatch) {
-      const mxb200_quantize_job& j = jobs[i];
-      const int64_t mine = (j.rows / kTile) * (j.cols / kTile);
-      if (j.out.data == nullptr && j.out_t.data == nullptr) {  // nothing asked of this one
-        ++i;
-        continue;
-      }
-      if (tiles + mine > 0x7fffffffLL)
-        break;
-      bp.jobs[bp.n++] = BatchJob{j.x, j.cols, j.out, j.out_t, static_cast<int>(j.cols / kTile), static_cast<int>(tiles),
-                                 (reinterpret_cast<uintptr_t>(j.x) & 31u) == 0,
-                                 (reinterpret_cast<uintptr_t>(j.out_t.data) & 31u) == 0 && j.out_t.ld % 32 == 0};
-      tiles += mine;
-      ++i;
-    }
-    if (bp.n == 0)
-      continue;
-    const int st = x_bf16 ? launch_batch<false>(bp, static_cast<int>(tiles), s) : launch_batch<true>(bp, static_cast<int>(tiles), s);
-    if (st != MXB200_OK)
-      return st;
-  }
-  return MXB200_OK;
+  return quantize_items(items, n, scale_rule == MXB200_SCALE_OCP_FLOOR, dev, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace
@@ -942,9 +1200,47 @@ uint32_t take_quantize_watchdog_word() {
 }  // namespace mxb200
 
 
+namespace mxb200 {
+namespace {
+int columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t rows, int64_t cols, bool add, void* stream) {
+  DeviceInfo dev;
+  if (int s = current_device(&dev); s != MXB200_OK)
+    return s;
+  if (dst == nullptr || src == nullptr)
+    return MXB200_ERR_NULL;
+  if (rows <= 0 || cols <= 0 || dst_ld < cols || src_ld < cols || (rows * cols + 255) / 256 > 0x7fffffffLL)
+    return MXB200_ERR_SHAPE;
+  mxb200_columns_bf16<<<static_cast<unsigned>((rows * cols + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<__nv_bfloat16*>(dst), dst_ld, static_cast<const __nv_bfloat16*>(src), src_ld, rows * cols,
+        static_cast<int>(cols), add);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return launch_status();
+}
+}  // namespace
+}  // namespace mxb200
+
+extern "C" int mxb200_copy_columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t rows, int64_t cols,
+                                   void* stream) {
+  return mxb200::columns(dst, dst_ld, src, src_ld, rows, cols, false, stream);
+}
+
+extern "C" int mxb200_add_columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t rows, int64_t cols,
+                                  void* stream) {
+  return mxb200::columns(dst, dst_ld, src, src_ld, rows, cols, true, stream);
+}
+
+extern "C" int mxb200_quantize_mx_items(const mxb200_quantize_item* items, int n, int scale_rule, void* stream) {
+  return mxb200::quantize_list(items, n, scale_rule, stream);
+}
+
 extern "C" int mxb200_quantize_mx_batch(const mxb200_quantize_job* jobs, int n_jobs, int x_bf16, int scale_rule,
                                         void* stream) {
-  return mxb200::quantize_batch(jobs, n_jobs, x_bf16 != 0, scale_rule, stream);
+  if (n_jobs > 0 && jobs == nullptr)
+    return mxb200::quantize_list(nullptr, n_jobs, scale_rule, stream);
+  std::vector<mxb200_quantize_item> items(static_cast<size_t>(std::max(n_jobs, 0)));
+  for (int i = 0; i < n_jobs; ++i)
+    items[i] = {jobs[i], x_bf16 != 0};
+  return mxb200::quantize_list(items.data(), n_jobs, scale_rule, stream);
 }
 
 extern "C" int mxb200_quantize_mx(const void* x, int x_bf16, int64_t rows, int64_t cols, mxb200_mx_out out,

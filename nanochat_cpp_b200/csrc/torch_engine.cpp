@@ -17,6 +17,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 #include <torch/extension.h>
 
 #include "mxb200.h"
@@ -151,26 +152,30 @@ Tensor workspace(at::Device device, size_t bytes) {
   return t;
 }
 
-// d (M, N) = a (M, K) . b (N, K)^T, bf16 or fp32 (alpha, +=), split along K where the library says so.
-void gemm(void* d, bool f32, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device,
-          const float* alpha = nullptr, bool accumulate = false) {
-  const int splits = mxb200_gemm_splits(M, N, K);
-  if (splits > 1) {
-    const Tensor ws = workspace(device, mxb200_gemm_workspace_bytes(M, N, K, splits));
-    check(mxb200_gemm_splitk(a.data, a.scale, b.data, b.scale, d, f32 ? MXB200_OUT_F32 : MXB200_OUT_BF16, nullptr, M, N,
-                             K, alpha, accumulate, splits, ws.data_ptr(), ws.numel(), stream()),
-          f32 ? "mx_gemm_f32" : "mx_gemm");
-  } else if (f32) {
-    check(mxb200_gemm_f32(a.data, a.scale, b.data, b.scale, static_cast<float*>(d), M, N, K, alpha, accumulate, stream()),
-          "mx_gemm_f32");
-  } else {
-    check(mxb200_gemm_bf16(a.data, a.scale, b.data, b.scale, d, nullptr, M, N, K, stream()), "mx_gemm");
-  }
+// d (M, N) = a (M, K) . b (N, K)^T, bf16 or fp32 (alpha, +=).
+mxb200_gemm_desc gemm_desc(void* d, at::ScalarType dtype, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K,
+                           const float* alpha = nullptr, bool accumulate = false) {
+  return {a.data, a.scale, b.data, b.scale, d, nullptr, alpha, M, N, K,
+          dtype == at::kFloat ? MXB200_OUT_F32 : MXB200_OUT_BF16, accumulate};
+}
+
+// Independent GEMMs, in one launch where the library can, split along K where it says so.
+void run_gemms(const mxb200_gemm_desc* g, int n, at::Device device) {
+  const size_t bytes = mxb200_gemm_group_workspace_bytes(g, n);
+  Tensor ws;
+  if (bytes > 0)
+    ws = workspace(device, bytes);
+  check(mxb200_gemm_group(g, n, bytes > 0 ? ws.data_ptr() : nullptr, bytes > 0 ? ws.numel() : 0, stream()), "mx_gemm");
+}
+
+void gemm(void* d, at::ScalarType dtype, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device) {
+  const mxb200_gemm_desc g = gemm_desc(d, dtype, a, b, M, N, K);
+  run_gemms(&g, 1, device);
 }
 
 Tensor gemm_bf16(const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device) {
   Tensor d = empty({M, N}, at::kBFloat16, device);
-  gemm(d.data_ptr(), false, a, b, M, N, K, device);
+  gemm(d.data_ptr(), at::kBFloat16, a, b, M, N, K, device);
   return d;
 }
 
@@ -178,43 +183,71 @@ bool grad_direct(const Tensor& w) {  // fp8.h:114-116
   return w.is_leaf() && w.requires_grad() && w.scalar_type() == at::kFloat && w.is_contiguous();
 }
 
-// dW = alpha * go_t (n, K) . in_t (C, K)^T into the .grad of ws, whose rows concatenate to n: allocated (=) when
-// undefined, else accumulated (+=); several ws whose gradients share one buffer take one GEMM (fp8.cpp:470-514).
-void grad_weights(const Layout& go_t, const Layout& in_t, int64_t n, int64_t C, int64_t K, const std::vector<Tensor>& ws,
-                  const float* alpha, at::Device device) {
-  int64_t total = 0;
-  bool shapes = true, all = true;
-  for (const Tensor& w : ws)
-    total += w.size(0), shapes &= w.size(1) == C, all &= w.grad().defined();
-  require(shapes && total == n, "mx_grad_weights: weight rows must concatenate to the gradient's");
-  if (all) {
-    const Tensor& g0 = ws[0].grad();
-    const char* base = static_cast<const char*>(g0.data_ptr());
-    bool contiguous = true;
+// A weight gradient dW = alpha * go_t (n, K) . in_t (C, K)^T of weights whose rows concatenate to n, as the GEMM that makes
+// it and what follows. Direct (fp32 leaves): into their .grad, allocated (=) when undefined, else accumulated (+=); several
+// whose gradients share one buffer take one += (fp8.cpp:470-514). Else: returned to autograd in the weights' type.
+class WeightGrad {
+ public:
+  WeightGrad(const Layout& go_t, const Layout& in_t, int64_t n, int64_t C, int64_t K, std::vector<Tensor> weights,
+             bool direct, const float* alpha, at::Device device)
+      : ws_(std::move(weights)), direct_(direct) {
+    int64_t total = 0;
+    bool shapes = true, all = direct, bf16 = !direct && alpha == nullptr;
+    for (const Tensor& w : ws_) {
+      total += w.size(0), shapes &= w.size(1) == C;
+      all = all && w.grad().defined();
+      bf16 &= w.scalar_type() == at::kBFloat16;
+    }
+    require(shapes && total == n, "mx_grad_weights: weight rows must concatenate to the gradient's");
+    if (all) {
+      const Tensor& g0 = ws_[0].grad();
+      const char* base = static_cast<const char*>(g0.data_ptr());
+      bool contiguous = true;
+      int64_t row = 0;
+      for (const Tensor& w : ws_) {
+        const Tensor& g = w.grad();
+        contiguous &= g.is_contiguous() && g.scalar_type() == at::kFloat && g.data_ptr() == base + row * C * 4;
+        row += w.size(0);
+      }
+      if (contiguous && (ws_.size() == 1 || (g0.is_view() && g0._base().numel() == n * C))) {
+        done_ = true;
+        desc_ = gemm_desc(const_cast<char*>(base), at::kFloat, go_t, in_t, n, C, K, alpha, true);
+        return;
+      }
+    }
+    // bf16 weights: rounded once in the epilogue, as the cast of an fp32 result would round it
+    const auto dtype = bf16 ? at::kBFloat16 : at::kFloat;
+    buf_ = empty({n, C}, dtype, device);
+    desc_ = gemm_desc(buf_.data_ptr(), dtype, go_t, in_t, n, C, K, alpha, false);
+  }
+
+  const mxb200_gemm_desc& desc() const { return desc_; }
+
+  // After the GEMM has been launched: the gradients autograd gets, undefined where .grad already has them.
+  variable_list finish() {
+    variable_list out(ws_.size());
     int64_t row = 0;
-    for (const Tensor& w : ws) {
-      const Tensor& g = w.grad();
-      contiguous &= g.is_contiguous() && g.scalar_type() == at::kFloat && g.data_ptr() == base + row * C * 4;
+    for (size_t i = 0; i < ws_.size() && !done_; ++i) {
+      const Tensor& w = ws_[i];
+      // row blocks of one buffer, as the reference's merged q/k/v
+      Tensor part = ws_.size() == 1 ? buf_ : buf_.narrow(0, row, w.size(0));
       row += w.size(0);
+      if (!direct_)
+        out[i] = part.scalar_type() == w.scalar_type() ? part : part.to(w.scalar_type());
+      else if (w.grad().defined())
+        w.mutable_grad().add_(part);
+      else
+        w.mutable_grad() = part;
     }
-    if (contiguous && (ws.size() == 1 || (g0.is_view() && g0._base().numel() == n * C))) {
-      gemm(const_cast<char*>(base), true, go_t, in_t, n, C, K, device, alpha, true);
-      return;
-    }
+    return out;
   }
-  Tensor buf = empty({n, C}, at::kFloat, device);
-  gemm(buf.data_ptr(), true, go_t, in_t, n, C, K, device, alpha, false);
-  int64_t row = 0;
-  for (const Tensor& w : ws) {
-    // row blocks of one buffer, as the reference's merged q/k/v
-    Tensor part = ws.size() == 1 ? buf : buf.narrow(0, row, w.size(0));
-    if (w.grad().defined())
-      w.mutable_grad().add_(part);
-    else
-      w.mutable_grad() = part;
-    row += w.size(0);
-  }
-}
+
+ private:
+  std::vector<Tensor> ws_;
+  bool direct_, done_ = false;
+  Tensor buf_;
+  mxb200_gemm_desc desc_{};
+};
 
 // ---------------------------------------------------------------------------------------------------- weight cache
 
@@ -345,7 +378,7 @@ class QuantizeJobs {
  public:
   void add(const Tensor& x, const mxb200_mx_out& out, const mxb200_mx_out& out_t) {
     check_quantizable(x);
-    jobs_[x.scalar_type() == at::kBFloat16].push_back({x.data_ptr(), x.size(0), x.size(1), out, out_t});
+    items_.push_back({{x.data_ptr(), x.size(0), x.size(1), out, out_t}, x.scalar_type() == at::kBFloat16});
     hold_.push_back(x);
   }
   void add(const Tensor& x, const Layout& rows, const Layout& cols, bool need_cols = true) {
@@ -366,21 +399,14 @@ class QuantizeJobs {
     }
   }
   void run() {
-    for (int bf16 = 0; bf16 < 2; ++bf16) {
-      auto& j = jobs_[bf16];
-      if (j.size() == 1)
-        check(mxb200_quantize_mx(j[0].x, bf16, j[0].rows, j[0].cols, j[0].out, j[0].out_t, MXB200_PROLOGUE_NONE,
-                                 MXB200_SCALE_REFERENCE, stream()),
-              "quantize_mx");
-      else if (!j.empty())
-        check(mxb200_quantize_mx_batch(j.data(), static_cast<int>(j.size()), bf16, MXB200_SCALE_REFERENCE, stream()),
-              "quantize_mx");
-    }
+    if (!items_.empty())
+      check(mxb200_quantize_mx_items(items_.data(), static_cast<int>(items_.size()), MXB200_SCALE_REFERENCE, stream()),
+            "quantize_mx");
   }
 
  private:
-  std::vector<mxb200_quantize_job> jobs_[2];
-  std::vector<Tensor> hold_;
+  c10::SmallVector<mxb200_quantize_item, 8> items_;
+  c10::SmallVector<Tensor, 8> hold_;
 };
 
 // ---------------------------------------------------------------------------------------------------- Linear
@@ -430,17 +456,23 @@ struct Float8Matmul : torch::autograd::Function<Float8Matmul> {
     QuantizeJobs jobs;
     jobs.add(go, layout_of(g_rows, N, O), layout_of(g_cols, O, N));
     jobs.run();
-    Tensor dx, dw;
-    if (ctx->needs_input_grad(0))
-      dx = gemm_bf16(layout_of(g_rows, N, O), saved_layout(saved[1], saved[2], C, O), N, C, O, device);
-    const Layout g_t = layout_of(g_cols, O, N), x_t = layout_of(saved[0], C, N);
-    if (grad_direct(w)) {
-      grad_weights(g_t, x_t, O, C, N, {w}, nullptr, device);
-    } else if (ctx->needs_input_grad(1)) {
-      dw = empty({O, C}, at::kFloat, device);
-      gemm(dw.data_ptr(), true, g_t, x_t, O, C, N, device);
-      dw = dw.to(w.scalar_type());
+    // the weight gradient first: with K = tokens its tiles are the longer ones of the launch
+    mxb200_gemm_desc gemms[2];
+    int n = 0;
+    const bool direct = grad_direct(w);
+    std::optional<WeightGrad> wgrad;
+    if (direct || ctx->needs_input_grad(1)) {
+      wgrad.emplace(layout_of(g_cols, O, N), layout_of(saved[0], C, N), O, C, N, std::vector<Tensor>{w}, direct, nullptr, device);
+      gemms[n++] = wgrad->desc();
     }
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0)) {
+      dx = empty({N, C}, at::kBFloat16, device);
+      gemms[n++] = gemm_desc(dx.data_ptr(), at::kBFloat16, layout_of(g_rows, N, O), saved_layout(saved[1], saved[2], C, O), N, C, O);
+    }
+    run_gemms(gemms, n, device);
+    if (wgrad.has_value())
+      dw = wgrad->finish()[0];
     return {dx, dw, Tensor()};
   }
 };
@@ -482,8 +514,14 @@ variable_list qkv_forward(const Tensor& x, WeightUse& w, int64_t gate_cols, cons
     out.push_back(qkv.narrow(1, row, part.size(0)));
     row += part.size(0);
   }
-  if (gate_cols > 0)
-    out.push_back(x.narrow(1, 0, gate_cols).contiguous());
+  if (gate_cols > 0) {
+    if (x.scalar_type() == at::kBFloat16) {
+      out.push_back(empty({N, gate_cols}, at::kBFloat16, device));
+      check(mxb200_copy_columns(out.back().data_ptr(), gate_cols, x.data_ptr(), C, N, gate_cols, stream()), "fp8_qkv");
+    } else {
+      out.push_back(x.narrow(1, 0, gate_cols).contiguous());
+    }
+  }
   if (saved != nullptr) {
     if (x_mx != nullptr)
       *saved = {x_mx->data_t, x_mx->scale_t};
@@ -526,25 +564,23 @@ struct MxQkv : torch::autograd::Function<MxQkv> {
       row += ws[i].size(0);
     }
     jobs.run();
+    mxb200_gemm_desc gemms[2];
+    int count = 0;
+    WeightGrad wgrad(g_t, saved_layout(saved[0], saved[1], C, N), n, C, N, ws, direct, nullptr, device);
+    gemms[count++] = wgrad.desc();
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
-      dx = gemm_bf16(g, saved_layout(saved[2], saved[3], C, n), N, C, n, device);
-      if (gate_cols > 0 && grads[3].defined())
-        dx.narrow(1, 0, gate_cols).add_(grads[3]);
+      dx = empty({N, C}, at::kBFloat16, device);
+      gemms[count++] = gemm_desc(dx.data_ptr(), at::kBFloat16, g, saved_layout(saved[2], saved[3], C, n), N, C, n);
     }
-    const Layout x_t = saved_layout(saved[0], saved[1], C, N);
-    if (direct) {
-      grad_weights(g_t, x_t, n, C, N, ws, nullptr, device);
-      return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    run_gemms(gemms, count, device);
+    if (dx.defined() && gate_cols > 0 && grads[3].defined()) {
+      const Tensor gate = grads[3].to(at::kBFloat16).contiguous();
+      check(mxb200_add_columns(dx.data_ptr(), C, gate.data_ptr(), gate_cols, N, gate_cols, stream()), "fp8_qkv");
     }
-    Tensor dw = empty({n, C}, at::kFloat, device);
-    gemm(dw.data_ptr(), true, g_t, x_t, n, C, N, device);
     variable_list out{dx};
-    row = 0;
-    for (const Tensor& w : ws) {
-      out.push_back(dw.narrow(0, row, w.size(0)).to(w.scalar_type()));
-      row += w.size(0);
-    }
+    for (Tensor& dw : wgrad.finish())
+      out.push_back(std::move(dw));
     out.resize(7);
     return out;
   }
@@ -626,18 +662,6 @@ struct Fp8ReluSquareMlp : torch::autograd::Function<Fp8ReluSquareMlp> {
     ctx->saved_data["w_proj"] = w_proj;
     return y;
   }
-  static Tensor weight_grad(const Layout& g_t, const Layout& in_t, int64_t n, int64_t C, int64_t K, const Tensor& w,
-                            bool needed) {
-    if (grad_direct(w)) {
-      grad_weights(g_t, in_t, n, C, K, {w}, nullptr, w.device());
-      return Tensor();
-    }
-    if (!needed)
-      return Tensor();
-    Tensor dw = empty({n, C}, at::kFloat, w.device());
-    gemm(dw.data_ptr(), true, g_t, in_t, n, C, K, w.device());
-    return dw.to(w.scalar_type());
-  }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor w_fc = ctx->saved_data["w_fc"].toTensor(), w_proj = ctx->saved_data["w_proj"].toTensor();
@@ -650,20 +674,33 @@ struct Fp8ReluSquareMlp : torch::autograd::Function<Fp8ReluSquareMlp> {
     QuantizeJobs jobs;
     jobs.add(grad, go, go_t);
     jobs.run();
-    // the reference's order (fp8.cpp:299-337): fc's two GEMMs read dh while it is still in L2
-    const Tensor grad_proj =
-          weight_grad(go_t, layout_of(saved[7], H, N), O, H, N, w_proj, ctx->needs_input_grad(2));
     const Tensor dh_rows = layout_buffer(N, H, device), dh_cols = layout_buffer(H, N, device);
     const Layout dh = layout_of(dh_rows, N, H), dh_t = layout_of(dh_cols, H, N);
     const Layout proj_t = saved_layout(saved[4], saved[5], H, O);
     check(mxb200_gemm_relu_square_bwd(go.data, go.scale, proj_t.data, proj_t.scale, h.data_ptr(), dh.data, dh.scale,
                                       dh_t.data, dh_t.scale, N, H, O, stream()),
           "mx_gemm_relu_square_bwd");
+    // the three remaining GEMMs share a launch; fc's weight gradient and the input gradient read dh while it is in L2
+    mxb200_gemm_desc gemms[3];
+    int n = 0;
+    std::optional<WeightGrad> fc, proj;
+    const bool fc_direct = grad_direct(w_fc), proj_direct = grad_direct(w_proj);
+    if (fc_direct || ctx->needs_input_grad(1)) {
+      fc.emplace(dh_t, saved_layout(saved[0], saved[1], C, N), H, C, N, std::vector<Tensor>{w_fc}, fc_direct, nullptr, device);
+      gemms[n++] = fc->desc();
+    }
+    if (proj_direct || ctx->needs_input_grad(2)) {
+      proj.emplace(go_t, layout_of(saved[7], H, N), O, H, N, std::vector<Tensor>{w_proj}, proj_direct, nullptr, device);
+      gemms[n++] = proj->desc();
+    }
     Tensor dx;
-    if (ctx->needs_input_grad(0))
-      dx = gemm_bf16(dh, saved_layout(saved[2], saved[3], C, H), N, C, H, device);
-    const Tensor grad_fc = weight_grad(dh_t, saved_layout(saved[0], saved[1], C, N), H, C, N, w_fc, ctx->needs_input_grad(1));
-    return {dx, grad_fc, grad_proj, Tensor(), Tensor(), Tensor()};
+    if (ctx->needs_input_grad(0)) {
+      dx = empty({N, C}, at::kBFloat16, device);
+      gemms[n++] = gemm_desc(dx.data_ptr(), at::kBFloat16, dh, saved_layout(saved[2], saved[3], C, H), N, C, H);
+    }
+    run_gemms(gemms, n, device);
+    return {dx, fc.has_value() ? fc->finish()[0] : Tensor(), proj.has_value() ? proj->finish()[0] : Tensor(), Tensor(),
+            Tensor(), Tensor()};
   }
 };
 
@@ -739,7 +776,7 @@ void run_chunks(const Tensor& x, WeightUse& w, const Tensor& targets, const Loss
   for (int64_t begin = 0; begin < N; begin += args.chunk_rows) {
     const int64_t rows = std::min(N - begin, args.chunk_rows);
     const mxb200_mx_out x_chunk = view(xq, C, begin);
-    gemm(logits.data_ptr(), false, {x_chunk.data, x_chunk.scale}, wq, rows, V, C, device);
+    gemm(logits.data_ptr(), at::kBFloat16, {x_chunk.data, x_chunk.scale}, wq, rows, V, C, device);
     check(mxb200_softcap_ce_loss(logits.data_ptr(), rows, V, t + begin, static_cast<int>(args.vocab), static_cast<int>(V),
                                  static_cast<float>(args.softcap), out.losses != nullptr ? out.losses + begin : lse + rows_max,
                                  lse, s),
@@ -752,7 +789,7 @@ void run_chunks(const Tensor& x, WeightUse& w, const Tensor& targets, const Loss
                                     static_cast<int>(V), static_cast<float>(args.softcap), scale, out.grad_scale_stride,
                                     out.num_valid, view(g, V), view(g_t, N, 0, begin), MXB200_SCALE_REFERENCE, s),
           "softcap_ce_grad_mx");
-    gemm(static_cast<char*>(out.grad_x) + begin * C * 2, false, g, w.cols(), rows, C, V, device);
+    gemm(static_cast<char*>(out.grad_x) + begin * C * 2, at::kBFloat16, g, w.cols(), rows, C, V, device);
   }
 }
 
@@ -802,12 +839,11 @@ struct SoftcapReduced : torch::autograd::Function<SoftcapReduced> {
     const auto* alpha = static_cast<const float*>(g.data_ptr());
     const Layout g_t = layout_of(saved[1], V, N), x_t = layout_of(saved[2], C, N);
     Tensor dw;
-    if (grad_direct(weight)) {
-      grad_weights(g_t, x_t, V, C, N, {weight}, alpha, device);
-    } else if (ctx->needs_input_grad(1)) {
-      dw = empty({V, C}, at::kFloat, device);
-      gemm(dw.data_ptr(), true, g_t, x_t, V, C, N, device, alpha, false);
-      dw = dw.to(weight.scalar_type());
+    const bool direct = grad_direct(weight);
+    if (direct || ctx->needs_input_grad(1)) {
+      WeightGrad wgrad(g_t, x_t, V, C, N, {weight}, direct, alpha, device);
+      run_gemms(&wgrad.desc(), 1, device);
+      dw = wgrad.finish()[0];
     }
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
@@ -868,9 +904,9 @@ struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
       WeightUse use(nullptr, {weight});
       run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
     }
-    Tensor dw = empty({V, C}, at::kFloat, device);
-    gemm(dw.data_ptr(), true, layout_of(g_cols, V, N), layout_of(x_cols, C, N), V, C, N, device);
-    return {grad_x, dw.to(weight.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor()};
+    WeightGrad wgrad(layout_of(g_cols, V, N), layout_of(x_cols, C, N), V, C, N, {weight}, false, nullptr, device);
+    run_gemms(&wgrad.desc(), 1, device);
+    return {grad_x, wgrad.finish()[0], Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
