@@ -414,6 +414,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
   tcgen05_fence_before_sync();
   __syncthreads();
   tcgen05_fence_after_sync();
+  grid_dependency_wait();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
   if (warp == 0) {
@@ -912,6 +913,7 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
   cluster_arrive();  // the peer's barriers exist before anything is credited to them
   cluster_wait();
   tcgen05_fence_after_sync();
+  grid_dependency_wait();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
   if (warp == 0) {
@@ -1252,6 +1254,7 @@ __global__ void __launch_bounds__(mxb200::kReduceThreads) mxb200_gemm_sum_slices
   while (j + 1 < r.n && static_cast<int>(blockIdx.x) >= r.jobs[j + 1].first_block)
     ++j;
   const ReduceJob& job = r.jobs[j];
+  grid_dependency_wait();
   const int64_t at = (static_cast<int64_t>(static_cast<int>(blockIdx.x) - job.first_block) * kReduceThreads + threadIdx.x) * 8;
   if (at >= job.elements)
     return;
@@ -1526,9 +1529,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, in
   static bool configured[64] = {};
   if (int st = set_smem_once(one_cta_kernel<BN>(), Config<BN>::kSmemBytes, configured); st != MXB200_OK)
     return st;
-  one_cta_kernel<BN>()<<<grid, kThreads, Config<BN>::kSmemBytes, stream>>>(ma, mb, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(one_cta_kernel<BN>(), grid, kThreads, Config<BN>::kSmemBytes, stream, ma, mb, p);
 }
 
 template <int TN, int kProblems>
@@ -1537,9 +1538,7 @@ int launch_pair(const PairArgs<kProblems>& args, int pairs, cudaStream_t stream)
   static bool configured[64] = {};
   if (int st = set_smem_once(pair_kernel<TN, kProblems>(), C::kSmemBytes, configured); st != MXB200_OK)
     return st;
-  pair_kernel<TN, kProblems>()<<<2 * pairs, C::kThreads, C::kSmemBytes, stream>>>(args);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(pair_kernel<TN, kProblems>(), 2 * pairs, C::kThreads, C::kSmemBytes, stream, args);
 }
 
 template <int kProblems>
@@ -1555,9 +1554,7 @@ int launch_fused(const PairArgs<1>& args, const FuseMaps& fuse, int pairs, cudaS
   static bool configured[64] = {};
   if (int st = set_smem_once(fused_kernel<TN, kFuse>(), C::kSmemBytes, configured); st != MXB200_OK)
     return st;
-  fused_kernel<TN, kFuse>()<<<2 * pairs, C::kThreads, C::kSmemBytes, stream>>>(args, fuse);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(fused_kernel<TN, kFuse>(), 2 * pairs, C::kThreads, C::kSmemBytes, stream, args, fuse);
 }
 
 // (rows, cols) row-major bytes, box = 32 rows x 32 bytes: what one epilogue warp stores of a quantized layout
@@ -1705,9 +1702,7 @@ int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInf
   const auto sum_slices = [&](int status) {
     if (status != MXB200_OK || sums.n == 0)
       return status;
-    mxb200_gemm_sum_slices<<<static_cast<unsigned>(sum_blocks), kReduceThreads, 0, s>>>(sums);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return launch_status();
+    return launch_kernel(mxb200_gemm_sum_slices, static_cast<unsigned>(sum_blocks), kReduceThreads, 0, s, sums);
   };
   const int cap = g_max_ctas.load() > 0 ? g_max_ctas.load() : dev.sms;
   if (!plan.pair) {

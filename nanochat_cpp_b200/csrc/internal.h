@@ -42,4 +42,29 @@ inline int launch_status() {
   return cudaGetLastError() == cudaSuccess ? MXB200_OK : MXB200_ERR_LAUNCH;
 }
 
+// Launches a kernel of this library, all of which begin with grid_dependency_wait() (ptx_sm100.cuh): its blocks may be
+// placed while the stream's previous kernel still runs, as that one's leave their SMs, and wait there for its end with
+// their set-up done. That takes 1 to 2 us of launch latency and ramp-up out of every step of a chain of small kernels.
+template <typename... Params>
+int launch_kernel(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                  const Params&... params) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(block);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  void* arguments[] = {const_cast<void*>(static_cast<const void*>(&params))...};
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (cudaLaunchKernelExC(&config, reinterpret_cast<const void*>(kernel), arguments) != cudaSuccess) {
+    cudaGetLastError();
+    return MXB200_ERR_LAUNCH;
+  }
+  return MXB200_OK;
+}
+
 }  // namespace mxb200

@@ -34,6 +34,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Everything the stream did before this kernel is complete and visible after this; nothing may touch global memory before
+// it. Kernels launched by launch_kernel (internal.h) start with it, every thread. The next kernel's blocks may then be
+// placed as this one's leave their SMs.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -210,6 +210,7 @@ __device__ __forceinline__ void quantize_tile(const QuantParams& p, int tile_ind
   const int tile_r = tile_index / p.tiles_c, tile_c = tile_index % p.tiles_c;
   const int64_t row0 = static_cast<int64_t>(tile_r) * kTile, col0 = static_cast<int64_t>(tile_c) * kTile;
   const bool want_rows = p.out.data != nullptr, want_cols = p.out_t.data != nullptr;
+  grid_dependency_wait();
 
   // ---- row pass: 128 rows x 8 vectors of 16 values = 1024 vectors, 4 per thread
   constexpr int kIters = kTile * (kTile / 16) / kThreads;
@@ -580,6 +581,7 @@ __device__ __forceinline__ void quantize_stream_softcap(const CUtensorMap* map_x
     table[i] = softcap_tanh(logit_of_entry(i), p.ce.softcap);
   const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 8 * kLogitLow;
   __syncthreads();
+  grid_dependency_wait();
 
   // Thread 0 posts this CTA's i-th tile and starts its load into buffer i % stages. A number past the last tile is the
   // stop sign: posted once (a bare arrival completes the phase), after which nothing more is drawn or posted.
@@ -752,6 +754,7 @@ __device__ __forceinline__ void quantize_stream_batch(const StreamBatch<kMaxJobs
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_wait();
 
   // as in the softcap form: the first unit is the CTA's own number, later ones are drawn a whole unit ahead
   bool drawing = true;
@@ -894,6 +897,7 @@ MXB200_QUANTIZE_STREAM_KERNEL(mxb200_quantize_stream_many, mxb200::kManyJobs)
 __global__ void __launch_bounds__(256) mxb200_columns_bf16(__nv_bfloat16* dst, int64_t dst_ld, const __nv_bfloat16* src,
                                                            int64_t src_ld, int64_t n, int cols, bool add) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  mxb200::grid_dependency_wait();
   if (i >= n)
     return;
   const int64_t r = i / cols, c = i % cols;
@@ -935,9 +939,7 @@ int check_out(const mxb200_mx_out& o, int64_t ld_min) {
 template <int kPro>
 int launch(const QuantParams& p, int64_t tiles, cudaStream_t stream) {
   constexpr size_t smem = 2 * kTile * kTile + 2 * kScaleTileBytes;
-  quantize_kernel<kPro>()<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(quantize_kernel<kPro>(), static_cast<unsigned>(tiles), kThreads, smem, stream, p);
 }
 
 // (rows, ld) row-major, a box of one stage: 128 x 128 of bf16 or 64 x 128 of fp32.
@@ -980,10 +982,8 @@ int launch_softcap(const QuantParams& p, int64_t rows, int64_t cols, int64_t til
   if (int s = configure_once(mxb200_quantize_softcap_grad, kSoftcapSmemBytes, configured_for); s != MXB200_OK)
     return s;
   const StreamParams sp{p, static_cast<int>(tiles), next_stream_slot()};
-  mxb200_quantize_softcap_grad<<<static_cast<unsigned>(std::min<int64_t>(tiles, sms)), kThreads * kSoftcapGroups,
-                                 kSoftcapSmemBytes, stream>>>(map, sp);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_quantize_softcap_grad, static_cast<unsigned>(std::min<int64_t>(tiles, sms)),
+                       kThreads * kSoftcapGroups, kSoftcapSmemBytes, stream, map, sp);
 }
 
 using Item = mxb200_quantize_item;
@@ -1040,9 +1040,7 @@ int launch_stream(const Item* items, int n, int* taken, bool floor_rule, int sms
   b.slot = next_stream_slot();
   b.floor_rule = floor_rule;
   const int64_t most = kStreamCtasPerSm * static_cast<int64_t>(sms);
-  kernel<<<static_cast<unsigned>(std::min<int64_t>(units, most)), kThreads, kStreamGroupBytes, stream>>>(b);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(kernel, static_cast<unsigned>(std::min<int64_t>(units, most)), kThreads, kStreamGroupBytes, stream, b);
 }
 
 template <int kKinds>
@@ -1053,9 +1051,7 @@ int launch_batch(const BatchParams& bp, int tiles, cudaStream_t stream) {
   static std::atomic<int> configured_for{-1};
   if (int s = configure_once(kernel, smem, configured_for); s != MXB200_OK)
     return s;
-  kernel<<<static_cast<unsigned>(tiles), kThreads, smem, stream>>>(bp);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(kernel, static_cast<unsigned>(tiles), kThreads, smem, stream, bp);
 }
 
 // No prologue: any mix of bf16 and fp32 tensors, all checked.
@@ -1210,11 +1206,9 @@ int columns(void* dst, int64_t dst_ld, const void* src, int64_t src_ld, int64_t 
     return MXB200_ERR_NULL;
   if (rows <= 0 || cols <= 0 || dst_ld < cols || src_ld < cols || (rows * cols + 255) / 256 > 0x7fffffffLL)
     return MXB200_ERR_SHAPE;
-  mxb200_columns_bf16<<<static_cast<unsigned>((rows * cols + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(dst), dst_ld, static_cast<const __nv_bfloat16*>(src), src_ld, rows * cols,
-        static_cast<int>(cols), add);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_columns_bf16, static_cast<unsigned>((rows * cols + 255) / 256), 256, 0,
+                       static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(dst), dst_ld,
+                       static_cast<const __nv_bfloat16*>(src), src_ld, rows * cols, static_cast<int>(cols), add);
 }
 }  // namespace
 }  // namespace mxb200

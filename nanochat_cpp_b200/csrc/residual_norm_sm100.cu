@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1) mxb200_residual_norm_mx_kernel(co
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_wait();
 
   const int64_t tiles = a.rows / kRows;
 
@@ -344,9 +345,7 @@ int launch(NormParams& p, const DeviceInfo& dev, cudaStream_t stream) {
   }
   const int64_t tiles = p.a.rows / kRows;
   const int grid = static_cast<int>(std::min<int64_t>(tiles, static_cast<int64_t>(dev.sms)));
-  mxb200_residual_norm_mx_kernel<kIters><<<grid, kThreads, smem, stream>>>(p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_residual_norm_mx_kernel<kIters>, grid, kThreads, smem, stream, p);
 }
 
 }  // namespace

@@ -13,6 +13,7 @@
 
 #include "bf16x2_sm100.cuh"
 #include "internal.h"
+#include "ptx_sm100.cuh"
 #include "softcap_table_sm100.cuh"
 
 namespace mxb200 {
@@ -89,16 +90,13 @@ __global__ void __launch_bounds__(kThreads * kGroups, kCtas) mxb200_softcap_ce_l
   const int64_t row_step = static_cast<int64_t>(gridDim.x) * kGroups;
   constexpr int kStep = kThreads * kVec;
   // vectors in flight ahead of the one being added up (the additions are a serial chain per thread); those of a row's
-  // start are asked for before the table is made or the row before is summed up
+  // start are asked for before the row ahead of it is summed up. The table is made while the kernel before ends.
   constexpr int kAhead = kTable ? 4 : 2;
   uint4 next[kAhead];
   const auto load = [&](int64_t row, int j) {
     return row < p.rows && j < p.padded ? *reinterpret_cast<const uint4*>(p.logits + row * p.ld + j)
                                         : make_uint4(0u, 0u, 0u, 0u);
   };
-#pragma unroll
-  for (int k = 0; k < kAhead; ++k)
-    next[k] = load(first_row, t * kVec + k * kStep);
   if constexpr (kTable) {
     for (uint32_t i = threadIdx.x; i < kTermMagnitudes; i += kThreads * kGroups) {
       const float th = softcap_tanh(__uint_as_float((kTermLow + i) << 16), p.softcap);  // of -z: -th
@@ -107,6 +105,10 @@ __global__ void __launch_bounds__(kThreads * kGroups, kCtas) mxb200_softcap_ce_l
     }
     __syncthreads();
   }
+  grid_dependency_wait();
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k)
+    next[k] = load(first_row, t * kVec + k * kStep);
   const float at_zero = softcap_loss_term(0.f, p.softcap);
   const uint32_t table_base = static_cast<uint32_t>(__cvta_generic_to_shared(table)) - 4 * kTermLow;
   for (int64_t row = first_row; row < p.rows; row += row_step) {
@@ -172,9 +174,7 @@ int launch_loss(const LossParams& p, const DeviceInfo& dev, cudaStream_t stream)
     configured_for.store(dev.device);
   }
   const int64_t ctas = std::min<int64_t>(p.rows, static_cast<int64_t>(dev.sms) * kCtas);
-  kernel<<<static_cast<unsigned>(ctas), kThreads * kGroups, smem, stream>>>(p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(kernel, static_cast<unsigned>(ctas), kThreads * kGroups, smem, stream, p);
 }
 
 // ---- the small reductions around the chunks: one block each, a few microseconds for any batch of tokens
@@ -200,6 +200,7 @@ __device__ __forceinline__ T block_sum(T v, T* smem) {
 __global__ void __launch_bounds__(kReduceThreads) mxb200_count_valid_kernel(const int64_t* targets, int64_t n,
                                                                             int64_t* out) {
   __shared__ unsigned long long smem[kReduceThreads / 32];
+  grid_dependency_wait();
   unsigned long long count = 0;
   for (int64_t i = threadIdx.x; i < n; i += kReduceThreads)
     count += targets[i] >= 0 ? 1u : 0u;
@@ -212,6 +213,7 @@ __global__ void __launch_bounds__(kReduceThreads) mxb200_count_valid_kernel(cons
 __global__ void __launch_bounds__(kReduceThreads) mxb200_reduce_losses_kernel(const float* losses, int64_t n,
                                                                               const int64_t* num_valid, float* out) {
   __shared__ float smem[kReduceThreads / 32];
+  grid_dependency_wait();
   float sum = 0.f;
   for (int64_t i = threadIdx.x; i < n; i += kReduceThreads)
     sum += losses[i];
@@ -223,6 +225,7 @@ __global__ void __launch_bounds__(kReduceThreads) mxb200_reduce_losses_kernel(co
 // y = bf16(x * bf16(scale)), 16 bytes per thread and step; HBM-bound (4 bytes per value). torch's multiply by a 0-dim
 // fp32 tensor converts that operand per element and took 95 us where this takes 17 on 16384 x 1536.
 __global__ void __launch_bounds__(256) mxb200_scale_bf16_kernel(const uint4* x, const float* scale, uint4* y, int64_t n16) {
+  grid_dependency_wait();
   const float f = __bfloat162float(__float2bfloat16(*scale));
   const uint32_t s2 = pack_bf16x2_rn(f, f);
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < n16; i += static_cast<int64_t>(gridDim.x) * 256) {
@@ -266,9 +269,7 @@ extern "C" int mxb200_count_valid(const int64_t* targets, int64_t n, int64_t* ou
     return MXB200_ERR_NULL;
   if (n < 0)
     return MXB200_ERR_SHAPE;
-  mxb200_count_valid_kernel<<<1, kReduceThreads, 0, static_cast<cudaStream_t>(stream)>>>(targets, n, out);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_count_valid_kernel, 1, kReduceThreads, 0, static_cast<cudaStream_t>(stream), targets, n, out);
 }
 
 extern "C" int mxb200_reduce_losses(const float* losses, int64_t n, const int64_t* num_valid, float* out, void* stream) {
@@ -280,9 +281,8 @@ extern "C" int mxb200_reduce_losses(const float* losses, int64_t n, const int64_
     return MXB200_ERR_NULL;
   if (n < 0)
     return MXB200_ERR_SHAPE;
-  mxb200_reduce_losses_kernel<<<1, kReduceThreads, 0, static_cast<cudaStream_t>(stream)>>>(losses, n, num_valid, out);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_reduce_losses_kernel, 1, kReduceThreads, 0, static_cast<cudaStream_t>(stream), losses, n,
+                       num_valid, out);
 }
 
 extern "C" int mxb200_scale_bf16(const void* x, const float* scale, void* y, int64_t n, void* stream) {
@@ -298,8 +298,6 @@ extern "C" int mxb200_scale_bf16(const void* x, const float* scale, void* y, int
     return MXB200_ERR_ALIGNMENT;
   const int64_t n16 = n / kVec;
   const int64_t blocks = std::min<int64_t>((n16 + 255) / 256, static_cast<int64_t>(dev.sms) * 8);
-  mxb200_scale_bf16_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(x), scale, static_cast<uint4*>(y), n16);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return launch_status();
+  return launch_kernel(mxb200_scale_bf16_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                       static_cast<const uint4*>(x), scale, static_cast<uint4*>(y), n16);
 }
