@@ -627,9 +627,9 @@ __device__ __forceinline__ void park_block(const uint32_t* w, unsigned char* st,
 template <int kFuse>
 __device__ __forceinline__ void fused_quantize_chunk(const GemmParams& p, const CUtensorMap* map_d,
                                                      const CUtensorMap* map_q, const CUtensorMap* map_qt,
-                                                     unsigned char* stage, int lane, const float* acc, int64_t row,
-                                                     int col, int warp_row0, bool valid, uint4* h_pieces, int next_col,
-                                                     unsigned char* scale_stage, int chunk) {
+                                                     unsigned char* stage, int lane, uint32_t (&acc)[32],
+                                                     uint32_t next_acc, int64_t row, int col, int warp_row0, bool valid,
+                                                     uint4* h_pieces, int next_col, unsigned char* scale_stage, int chunk) {
   unsigned char* st_out = stage;         // TMA source (forward form); h hand-over buffer (backward form, never a source)
   unsigned char* st_tr = stage + 2048;   // transpose tile, only ever touched by this warp's threads
   unsigned char* st_q = stage + 4096;    // TMA source
@@ -643,7 +643,7 @@ __device__ __forceinline__ void fused_quantize_chunk(const GemmParams& p, const 
   if constexpr (kFuse == kFuseReluSquare) {
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-      o[k] = pack_bf16x2_rn(acc[2 * k], acc[2 * k + 1]);
+      o[k] = pack_bf16x2_rn(__uint_as_float(acc[2 * k]), __uint_as_float(acc[2 * k + 1]));
       const uint32_t r = relu_keep_nan_bf16x2(o[k]);
       v[k] = mul_bf16x2(r, r);
     }
@@ -674,10 +674,14 @@ __device__ __forceinline__ void fused_quantize_chunk(const GemmParams& p, const 
       load_h_pieces(p, lane, warp_row0, next_col, h_pieces);
 #pragma unroll
     for (int k = 0; k < 16; ++k) {  // dh = bf16(h <= 0 ? 0 : bf16(ga) * 2h)
-      const uint32_t g = pack_bf16x2_rn(acc[2 * k], acc[2 * k + 1]);
+      const uint32_t g = pack_bf16x2_rn(__uint_as_float(acc[2 * k]), __uint_as_float(acc[2 * k + 1]));
       v[k] = mul_bf16x2(g, add_bf16x2(hw[k], hw[k])) & positive_or_nan_mask_bf16x2(hw[k]);
     }
   }
+
+  // the accumulator's registers are free: the next chunk's columns have the rest of this one to arrive
+  if (next_col >= 0)
+    tmem_ld_32x32b_x32(next_acc, acc);
 
   // ---- columns, first half: into the transpose tile, 64 bytes per column (its 32 rows as bf16). A store instruction
   // puts one column's 32 rows there (32 lanes x 2 bytes, conflict-free); the 16-byte pieces of column c sit at piece
@@ -753,6 +757,8 @@ __device__ __forceinline__ void fused_quantize_chunk(const GemmParams& p, const 
     tma_store_2d(map_qt, st_qt, warp_row0, col);
     tma_store_commit();
   }
+  if (next_col >= 0)
+    tmem_ld_wait(acc);
 }
 
 // ------------------------------------------------------------------------------------------------ CTA-pair kernel
@@ -1132,30 +1138,42 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
           return i == 0 ? kChunks - 1 : first + i - 1;
         return first + i;
       };
-      uint32_t r[2][32];
-      tmem_ld_32x32b_x32(acc_t + chunk_of(0) * 32, r[0]);
-#pragma unroll
-      for (int i = 0; i < kMine; ++i) {
-        if (i >= n_mine)
-          break;
-        const int c = chunk_of(i);
-        tmem_ld_wait();
-        if (i + 1 < n_mine) {
-          tmem_ld_32x32b_x32(acc_t + chunk_of(i + 1) * 32, r[(i + 1) & 1]);
-        }
-        if (i == 0 && owns_shared) {
-          tcgen05_fence_before_sync();
-          __syncwarp();
-          if (lane == 0)
-            mbar_arrive_cluster(overlap_leader);
-        }
-        const int col = col0 + c * 32;
-        if constexpr (kFuse != kFuseNone) {
-          fused_quantize_chunk<kFuse>(p, &maps.d, map_q, map_qt, stage, lane, reinterpret_cast<const float*>(r[i & 1]),
-                                      row, col, warp_row0, row_ok && col < p.N, h_pieces,
-                                      i + 1 < n_mine ? col0 + chunk_of(i + 1) * 32 : -1,
+      const auto hand_over_shared = [&] {  // this warp has read its part of the columns both buffers use
+        tcgen05_fence_before_sync();
+        __syncwarp();
+        if (lane == 0)
+          mbar_arrive_cluster(overlap_leader);
+      };
+      if constexpr (kFuse != kFuseNone) {
+        // One set of accumulator registers, refilled as soon as a chunk's values are packed, and a rolled loop: with two
+        // sets and the chunks unrolled the compiler mixes their instructions and runs out of the 128 registers (350
+        // bytes of spills; 16384 x 6144 x 1536: forward 257 us, now 210, backward 312, now 207).
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(acc_t + chunk_of(0) * 32, r);
+        tmem_ld_wait(r);
+        if (owns_shared)
+          hand_over_shared();
+#pragma unroll 1
+        for (int i = 0; i < n_mine; ++i) {
+          const int c = chunk_of(i), col = col0 + c * 32, next = i + 1 < n_mine ? chunk_of(i + 1) : -1;
+          fused_quantize_chunk<kFuse>(p, &maps.d, map_q, map_qt, stage, lane, r, acc_t + next * 32, row, col, warp_row0,
+                                      row_ok && col < p.N, h_pieces, next >= 0 ? col0 + next * 32 : -1,
                                       C::kStageScales ? s_scales + buf * (4 * kScaleTileBytes) : nullptr, c);
-        } else {
+        }
+      } else {
+        uint32_t r[2][32];
+        tmem_ld_32x32b_x32(acc_t + chunk_of(0) * 32, r[0]);
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          if (i >= n_mine)
+            break;
+          const int c = chunk_of(i);
+          tmem_ld_wait(r[i & 1]);
+          if (i + 1 < n_mine)
+            tmem_ld_32x32b_x32(acc_t + chunk_of(i + 1) * 32, r[(i + 1) & 1]);
+          if (i == 0 && owns_shared)
+            hand_over_shared();
+          const int col = col0 + c * 32;
           const bool valid = row_ok && col < p.N;
           const bool issue = warp_row0 < p.M && col < p.N;
           uint32_t o[32];
@@ -1449,8 +1467,8 @@ double launch_cycles(const GemmDesc* g, int n, int tn, const int* splits, double
 // Tile width and slices with the least expected time. `fixed`: slices of a single GEMM given by the caller.
 TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed) {
   int forced = g_tile_n.load();
-  if (need_pair && (forced == 128 || forced == 256))
-    forced = 0;  // the fused-quantize epilogues exist in the CTA-pair kernel only
+  if (need_pair && forced != 384 && forced != 512)
+    forced = 0;  // the fused-quantize epilogues exist for these two only
   TilePlan t{};
   bool wide = true;
   for (int i = 0; i < n; ++i)

@@ -251,6 +251,14 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The same, tied to the registers a load fills: nothing that reads them moves ahead of it.
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
+  tmem_ld_wait();
+#pragma unroll
+  for (int k = 0; k < 32; ++k)
+    asm volatile("" : "+r"(r[k]));
+}
+
 // ---------------------------------------------------------------------------------------------- descriptors
 
 // Shared-memory matrix descriptor (tcgen05): start address, leading and stride byte offsets in 16-byte units,
