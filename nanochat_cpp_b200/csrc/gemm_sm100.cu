@@ -126,13 +126,13 @@ struct GemmParams {
 // than the machine has CTA pairs, or a round and a bit; together they fill it, and one launch is saved.
 constexpr int kMaxGroup = 3;
 
-struct PairMaps {
+struct ProblemMaps {
   CUtensorMap a, b, sfa, sfb, d;
 };
 
 template <int kProblems>
-struct PairArgs {
-  PairMaps maps[kProblems];
+struct LaunchArgs {
+  ProblemMaps maps[kProblems];
   GemmParams p[kProblems];
   int end[kProblems];  // one past the last unit of each
   int sched_slot;      // this launch's pair of words in g_sched_words
@@ -376,9 +376,20 @@ __device__ __forceinline__ void store_rows_tma(const CUtensorMap* map_d, unsigne
   }
 }
 
-template <int BN>
-__device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, const CUtensorMap* map_b,
-                                                    const GemmParams& p) {
+// which GEMM of a launch a unit belongs to; `unit` becomes its number within that one
+template <int kProblems>
+__device__ __forceinline__ int problem_of(const LaunchArgs<kProblems>& args, int* unit) {
+  int g = 0;
+#pragma unroll
+  for (int k = 0; k + 1 < kProblems; ++k)
+    g += *unit >= args.end[k] ? 1 : 0;
+  if (g > 0)
+    *unit -= args.end[g - 1];
+  return g;
+}
+
+template <int BN, int kProblems>
+__device__ __forceinline__ void one_cta_kernel_body(const LaunchArgs<kProblems>& args) {
   using C = Config<BN>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -388,7 +399,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
   Barriers* bars = reinterpret_cast<Barriers*>(s_sf + C::kStages * C::kSfBytes);
 
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-  const int total_units = p.tiles_m * p.tiles_n * p.splits;
+  const int total_units = args.end[kProblems - 1];
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
@@ -404,8 +415,11 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
     fence_mbar_init();
   }
   if (warp == 0 && lane == 0) {
-    prefetch_tensormap(map_a);
-    prefetch_tensormap(map_b);
+#pragma unroll
+    for (int g = 0; g < kProblems; ++g) {
+      prefetch_tensormap(&args.maps[g].a);
+      prefetch_tensormap(&args.maps[g].b);
+    }
   }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
@@ -424,7 +438,11 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x) {
+      for (int u = blockIdx.x; ok && u < total_units; u += gridDim.x) {
+        int unit = u;
+        const int g = problem_of(args, &unit);
+        const GemmParams& p = args.p[g];
+        const ProblemMaps& maps = args.maps[g];
         const TileCoord tc = decode_unit(p, unit);
         const int n_rows_left = p.N - tc.n * BN;
         const int sfb_tiles = n_rows_left >= BN ? C::kSfbTiles : n_rows_left / 128;
@@ -440,8 +458,8 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
           }
           uint64_t* full = &bars->full[stage];
           mbar_arrive_expect_tx(el, full, tx);
-          tma_load_2d(el, s_a + stage * C::kABytes, map_a, full, kt * kBK, tc.m * kBM);
-          tma_load_2d(el, s_b + stage * C::kBBytes, map_b, full, kt * kBK, tc.n * BN);
+          tma_load_2d(el, s_a + stage * C::kABytes, &maps.a, full, kt * kBK, tc.m * kBM);
+          tma_load_2d(el, s_b + stage * C::kBBytes, &maps.b, full, kt * kBK, tc.n * BN);
           unsigned char* sf = s_sf + stage * C::kSfBytes;
           bulk_load(el, sf, sfa_src + static_cast<int64_t>(kt) * kScaleTileBytes, kScaleTileBytes, full);
           for (int j = 0; j < sfb_tiles; ++j)
@@ -464,7 +482,9 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
       uint32_t local = 0;  // tiles this CTA has started
       bool ok = true;
       const uint32_t sfa_t = tmem_base + C::kSfaCol, sfb_t = tmem_base + C::kSfbCol;
-      for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x, ++local) {
+      for (int u = blockIdx.x; ok && u < total_units; u += gridDim.x, ++local) {
+        int unit = u;
+        const GemmParams& p = args.p[problem_of(args, &unit)];
         const TileCoord tc = decode_unit(p, unit);
         const int n_rows_left = p.N - tc.n * BN;
         const int n_valid = n_rows_left >= BN ? BN : n_rows_left;
@@ -521,11 +541,13 @@ __device__ __forceinline__ void one_cta_kernel_body(const CUtensorMap* map_a, co
     // ------------------------------------------------------------------ epilogue (warps 2..5)
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: 32 * (warp id % 4) ...
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? *p.alpha : 1.f;
     uint32_t local = 0;
     bool ok = true;
     constexpr int kChunks = BN / 32;
-    for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x, ++local) {
+    for (int u = blockIdx.x; ok && u < total_units; u += gridDim.x, ++local) {
+      int unit = u;
+      const GemmParams& p = args.p[problem_of(args, &unit)];
+      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
       if (!wait_bounded(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
@@ -849,7 +871,7 @@ struct PairConfig {
 // The kernel body; the kernels themselves are the non-template functions at the end of this file (plain global
 // names read the same in every profiler). The tensor maps stay in the kernels' parameter space and come by address.
 template <int TN, int kFuse, int kProblems>
-__device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args, const CUtensorMap* map_q,
+__device__ __forceinline__ void pair_kernel_body(const LaunchArgs<kProblems>& args, const CUtensorMap* map_q,
                                                  const CUtensorMap* map_qt) {
   using C = PairConfig<TN, kFuse>;
   extern __shared__ unsigned char smem_raw[];
@@ -866,16 +888,6 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
   const bool leader = rank == 0;
   const int num_pairs = static_cast<int>(gridDim.x) >> 1;
   const int total_units = args.end[kProblems - 1];
-  // which GEMM a unit belongs to; `unit` becomes its number within that one
-  const auto problem_of = [&](int* unit) {
-    int g = 0;
-#pragma unroll
-    for (int k = 0; k + 1 < kProblems; ++k)
-      g += *unit >= args.end[k] ? 1 : 0;
-    if (g > 0)
-      *unit -= args.end[g - 1];
-    return g;
-  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
@@ -968,9 +980,9 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
         }
         if (unit >= total_units)
           break;
-        const int g = problem_of(&unit);
+        const int g = problem_of(args, &unit);
         const GemmParams& p = args.p[g];
-        const PairMaps& maps = args.maps[g];
+        const ProblemMaps& maps = args.maps[g];
         const TileCoord tc = decode_unit(p, unit);
         const int k_begin = tc.split * p.k_tiles_split;
         const int k_end = min(k_begin + p.k_tiles_split, p.k_tiles_total);
@@ -1029,7 +1041,7 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
         }
         if (unit >= total_units)
           break;
-        const GemmParams& p = args.p[problem_of(&unit)];
+        const GemmParams& p = args.p[problem_of(args, &unit)];
         const TileCoord tc = decode_unit(p, unit);
         const uint32_t buf = local & 1u, use = local >> 1;
         if (!wait_bounded_warp(&bars->tmem_empty[buf], (use & 1u) ^ 1u, bars, kSiteMmaTmemEmpty)) {
@@ -1106,9 +1118,9 @@ __device__ __forceinline__ void pair_kernel_body(const PairArgs<kProblems>& args
       }
       if (unit >= total_units)
         break;
-      const int g = problem_of(&unit);
+      const int g = problem_of(args, &unit);
       const GemmParams& p = args.p[g];
-      const PairMaps& maps = args.maps[g];
+      const ProblemMaps& maps = args.maps[g];
       const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
@@ -1295,27 +1307,26 @@ __global__ void __launch_bounds__(mxb200::kReduceThreads) mxb200_gemm_sum_slices
 // (src/nanochat/model/fp8/fp8_kernel.cu:174-175): a launch list or a timeline shows which tile shape and which
 // epilogue ran without decoding template arguments. <rows>x<columns> is the output tile; the CTA-pair kernels share
 // it between the two SMs of a TPC.
-#define MXB200_GEMM_KERNEL(name, BN)                                                                                   \
-  __global__ void __launch_bounds__(mxb200::kThreads, 1) name(const __grid_constant__ CUtensorMap map_a,               \
-                                                              const __grid_constant__ CUtensorMap map_b,               \
-                                                              const mxb200::GemmParams p) {                            \
-    mxb200::one_cta_kernel_body<BN>(&map_a, &map_b, p);                                                                \
+#define MXB200_GEMM_KERNEL(name, BN, PROBLEMS)                                                                         \
+  __global__ void __launch_bounds__(mxb200::kThreads, 1) name(const __grid_constant__ mxb200::LaunchArgs<PROBLEMS> args) { \
+    mxb200::one_cta_kernel_body<BN, PROBLEMS>(args);                                                                   \
   }
 
 #define MXB200_GEMM_PAIR_KERNEL(name, TN, PROBLEMS)                                                                    \
   __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(mxb200::PairConfig<TN>::kThreads, 1)                     \
-        name(const __grid_constant__ mxb200::PairArgs<PROBLEMS> args) {                                                \
+        name(const __grid_constant__ mxb200::LaunchArgs<PROBLEMS> args) {                                                \
     mxb200::pair_kernel_body<TN, mxb200::kFuseNone, PROBLEMS>(args, nullptr, nullptr);                                 \
   }
 
 #define MXB200_GEMM_FUSED_KERNEL(name, TN, FUSE)                                                                       \
   __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(mxb200::PairConfig<TN, FUSE>::kThreads, 1)               \
-        name(const __grid_constant__ mxb200::PairArgs<1> args, const __grid_constant__ mxb200::FuseMaps fuse) {        \
+        name(const __grid_constant__ mxb200::LaunchArgs<1> args, const __grid_constant__ mxb200::FuseMaps fuse) {        \
     mxb200::pair_kernel_body<TN, FUSE, 1>(args, &fuse.q, &fuse.qt);                                                    \
   }
 
-MXB200_GEMM_KERNEL(mxb200_gemm_128x128, 128)
-MXB200_GEMM_KERNEL(mxb200_gemm_128x256, 256)
+MXB200_GEMM_KERNEL(mxb200_gemm_128x128, 128, 1)
+MXB200_GEMM_KERNEL(mxb200_gemm_128x256, 256, 1)
+MXB200_GEMM_KERNEL(mxb200_gemm_group_128x128, 128, mxb200::kMaxGroup)
 MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x128, 128, 1)
 MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x192, 192, 1)
 MXB200_GEMM_PAIR_KERNEL(mxb200_gemm_pair_256x256, 256, 1)
@@ -1330,11 +1341,12 @@ MXB200_GEMM_FUSED_KERNEL(mxb200_gemm_pair_256x256_relu_square_bwd, 256, mxb200::
 namespace mxb200 {
 namespace {
 
-using GemmKernel = void (*)(CUtensorMap, CUtensorMap, GemmParams);
-
-template <int BN>
-constexpr GemmKernel one_cta_kernel() {
-  return BN == 256 ? mxb200_gemm_128x256 : mxb200_gemm_128x128;
+template <int BN, int kProblems>
+constexpr auto one_cta_kernel() {
+  if constexpr (kProblems == 1)
+    return BN == 256 ? mxb200_gemm_128x256 : mxb200_gemm_128x128;
+  else
+    return mxb200_gemm_group_128x128;
 }
 
 template <int TN, int kProblems>
@@ -1419,78 +1431,96 @@ struct TilePlan {
   int64_t tiles(int64_t M, int64_t N) const { return (M + tile_m - 1) / tile_m * ((N + tile_n - 1) / tile_n); }
 };
 
-// What the planner expects of the CTA-pair kernel, in SM cycles.
-//   A K step of 128 costs a CTA its share of the operands over the path from L2, about 50 bytes per cycle when all SMs pull
-//   (16384 + 64 TN + scales; the MMA's own 2 TN cycles stay below that at every width), an output tile its bytes over the
-//   same path; 256-wide tiles pay a hand-over bubble between tiles. Fitted to singles and groups from 256 x 768 x 768 to
-//   16384 x 6144 x 1536 at the clocks those run at.
+// What the planner expects of a kernel, in SM cycles.
+//   A K step of 128 costs a CTA what its tensor core and its chain of loads need when it has the path from L2 to itself
+//   (`alone`, from the slope over K of shapes of a few tiles), or its share of that path, about 50 bytes per cycle and CTA
+//   when all SMs pull. An output tile costs its bytes over the same path; the 256-wide pair tile pays a hand-over bubble
+//   between tiles. `start`: what a launch takes besides, over the 128 x 128 form (a cluster's launch and its handshakes,
+//   the last tile's longer epilogue).
 //   A K slice writes an fp32 tile, and the launch that sums the slices comes on top.
-double step_cycles(int tn) {
-  return (16384.0 + tn * 64.0 + (tn == 128 ? 1024.0 : 1536.0)) / 50.0;
+//   The constants are fitted to the measured times of 31 single shapes and 32 groups in every tile, from 128 x 768 x 768 to
+//   32768 x 1536 x 16384: what they choose is on average 2% behind the best tile (22% at worst).
+struct TileKind {
+  bool pair;
+  int tile_n;
+  double alone, start, tile;
+};
+constexpr TileKind kTileKinds[] = {
+    {true, 256, 580.0, 3000.0, 1200.0}, {true, 192, 475.0, 2750.0, 430.0}, {true, 128, 355.0, 2500.0, 730.0},
+    {false, 256, 600.0, 1500.0, 0.0},   {false, 128, 520.0, 0.0, 350.0},
+};
+constexpr double kShareBytes = 50.0, kStoreCost = 1.2;
+
+double step_cycles(const TileKind& t, double busy) {
+  const double bytes = t.pair ? 16384.0 + t.tile_n * 64.0 + (t.tile_n == 128 ? 1024.0 : 1536.0)
+                              : 0.92 * (16384.0 + t.tile_n * 128.0 + 512.0 * (1 + t.tile_n / 128));
+  return std::max(t.alone, bytes / kShareBytes * busy);
 }
-double out_cycles(int tn, const GemmDesc& g) {
-  const double bytes = g.out_kind == kOutF32 ? (g.accumulate ? 8.0 : 4.0) : (g.resid != nullptr ? 4.0 : 2.0);
-  return 128.0 * tn * bytes / 50.0;
+double out_bytes(const GemmDesc& g) {
+  return g.out_kind == kOutF32 ? (g.accumulate ? 8.0 : 4.0) : (g.resid != nullptr ? 4.0 : 2.0);
 }
-constexpr double kBubbleCycles = 1200.0, kTileCycles = 300.0;
+double out_cycles(const TileKind& t, double bytes) {
+  return kStoreCost * 128.0 * t.tile_n * bytes / kShareBytes;
+}
 double sum_cycles(const GemmDesc& g, int splits) {
-  return 4500.0 + static_cast<double>(g.M) * g.N * 4.0 * splits / 3500.0;
+  return 4900.0 + static_cast<double>(g.M) * g.N * 4.0 * splits / 2350.0;
 }
 
-// Expected cycles of n GEMMs in one launch with TN-wide tiles and the given slices, taken up in the order given. Pairs draw
-// their units from a counter: with many short units per pair a launch ends within a fraction of one of the average share,
-// with few long ones on a whole round.
-double launch_cycles(const GemmDesc* g, int n, int tn, const int* splits, double slots) {
-  double work = 0.0, least = 0.0, last = 0.0, units = 0.0, tail = 0.0;
+// Expected cycles of n GEMMs in one launch with these tiles and slices, taken up in the order given. Pairs draw their units
+// from a counter: with many short units per pair a launch ends within a fraction of one of the average share, with few long
+// ones on a whole round.
+double launch_cycles(const GemmDesc* g, int n, const TileKind& t, const int* splits, int sms) {
+  const double slots = std::max(t.pair ? sms / 2 : sms, 1);
+  const int64_t tile_m = t.pair ? 256 : 128;
+  double units[kMaxGroup], slice[kMaxGroup], total = 0.0;
   for (int i = 0; i < n; ++i) {
-    const int64_t k = g[i].K / 128, slice = (k + splits[i] - 1) / splits[i];
-    const double u = static_cast<double>((g[i].M + 255) / 256 * ((g[i].N + tn - 1) / tn)) * static_cast<double>((k + slice - 1) / slice);
-    double c = static_cast<double>(slice) * step_cycles(tn) + kTileCycles;
-    c += splits[i] > 1 ? 128.0 * tn * 4.0 / 50.0 : out_cycles(tn, g[i]);
-    if (tn == 256)
-      c += kBubbleCycles;
-    work += u * c;
-    units += u;
-    // units of this GEMM alone, behind what came before it
-    const double before = (work - u * c) / slots;
-    const double rounds = u / slots < 4.0 ? std::ceil(u / slots) : u / slots + 0.25;
+    const int64_t k = g[i].K / 128, per = (k + splits[i] - 1) / splits[i];
+    slice[i] = static_cast<double>(per);
+    units[i] = static_cast<double>((g[i].M + tile_m - 1) / tile_m * ((g[i].N + t.tile_n - 1) / t.tile_n)) *
+               static_cast<double>((k + per - 1) / per);
+    total += units[i];
+  }
+  const double step = step_cycles(t, std::min(total / slots, 1.0));
+  double work = 0.0, least = 0.0, last = 0.0, tail = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double c = slice[i] * step + t.tile + (splits[i] > 1 ? out_cycles(t, 4.0) : out_cycles(t, out_bytes(g[i])));
+    const double before = work / slots;
+    work += units[i] * c;
+    const double share = units[i] / slots, rounds = share < 4.0 ? std::ceil(share) : share + 0.25;
     least = std::max(least, i == 0 ? rounds * c : before + c);
     last = c;
     if (splits[i] > 1)
       tail += sum_cycles(g[i], splits[i]);
   }
-  if (n == 1)
-    return least + tail;
-  return std::max(least, work / slots + (units > slots ? 0.5 * last : 0.0)) + tail;
+  if (n > 1)
+    least = std::max(least, work / slots + (total > slots ? 0.5 * last : 0.0));
+  return t.start + least + tail;
 }
 
-// Tile width and slices with the least expected time. `fixed`: slices of a single GEMM given by the caller.
+// Tile and slices with the least expected time. `fixed`: slices of a single GEMM given by the caller. The 128 x 256 tile is
+// for single GEMMs, the pair tiles for matrices of at least 256 rows (any, when set by mxb200_set_gemm_config).
 TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed) {
   int forced = g_tile_n.load();
   if (need_pair && forced != 384 && forced != 512)
     forced = 0;  // the fused-quantize epilogues exist for these two only
-  TilePlan t{};
   bool wide = true;
   for (int i = 0; i < n; ++i)
     wide &= g[i].M >= 256 && g[i].N >= 256;
-  if (!(forced >= 384 || need_pair || (forced == 0 && wide))) {
-    t.pair = false, t.tile_m = 128;
-    t.tile_n = (forced == 128 || forced == 256) ? forced : (g[0].N >= 256 ? 256 : 128);
-    t.splits[0] = std::max(fixed, 1);
-    return t;
-  }
-  t.pair = true, t.tile_m = 256;
-  const double slots = std::max(sms / 2, 1);
+  TilePlan plan{};
   double best = 0.0;
-  for (int tn : {256, 192, 128}) {
-    if ((need_pair && tn == 128) || (forced >= 384 && tn != (forced == 512 ? 256 : forced == 384 ? 192 : 128)))
+  for (const TileKind& t : kTileKinds) {
+    const int name = t.pair ? (t.tile_n == 256 ? 512 : t.tile_n == 192 ? 384 : 640) : t.tile_n;  // in mxb200_set_gemm_config
+    if (forced != 0 ? name != forced : (t.pair && !wide && !need_pair))
+      continue;
+    if ((need_pair && (!t.pair || t.tile_n == 128)) || (n > 1 && !t.pair && t.tile_n == 256))
       continue;
     int splits[kMaxGroup] = {1, 1, 1};
     const auto consider = [&] {
-      const double cost = launch_cycles(g, n, tn, splits, slots);
+      const double cost = launch_cycles(g, n, t, splits, sms);
       if (best == 0.0 || cost < best * 0.99) {
-        best = cost, t.tile_n = tn;
-        std::copy(splits, splits + kMaxGroup, t.splits);
+        best = cost;
+        plan.pair = t.pair, plan.tile_m = t.pair ? 256 : 128, plan.tile_n = t.tile_n;
+        std::copy(splits, splits + kMaxGroup, plan.splits);
       }
     };
     if (fixed > 0 || need_pair) {
@@ -1502,19 +1532,19 @@ TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed
     // K slices, one GEMM at a time: each takes the count that helps most given the others
     for (int i = 0; i < n; ++i) {
       int kept = 1;
-      double least = launch_cycles(g, n, tn, splits, slots);
+      double least = launch_cycles(g, n, t, splits, sms);
       for (int s = 2; s <= 8; s *= 2) {
         if (g[i].K / 128 / s < 8)
           break;
         splits[i] = s;
-        if (const double c = launch_cycles(g, n, tn, splits, slots); c < least * 0.97)
+        if (const double c = launch_cycles(g, n, t, splits, sms); c < least * 0.97)
           least = c, kept = s;
       }
       splits[i] = kept;
     }
     consider();
   }
-  return t;
+  return plan;
 }
 
 TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, int fixed) {
@@ -1542,16 +1572,16 @@ int set_smem_once(Kernel kernel, size_t bytes, bool* configured) {
   return MXB200_OK;
 }
 
-template <int BN>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int grid, cudaStream_t stream) {
+template <int BN, int kProblems>
+int launch_one_cta(const LaunchArgs<kProblems>& args, int grid, cudaStream_t stream) {
   static bool configured[64] = {};
-  if (int st = set_smem_once(one_cta_kernel<BN>(), Config<BN>::kSmemBytes, configured); st != MXB200_OK)
+  if (int st = set_smem_once(one_cta_kernel<BN, kProblems>(), Config<BN>::kSmemBytes, configured); st != MXB200_OK)
     return st;
-  return launch_kernel(one_cta_kernel<BN>(), grid, kThreads, Config<BN>::kSmemBytes, stream, ma, mb, p);
+  return launch_kernel(one_cta_kernel<BN, kProblems>(), grid, kThreads, Config<BN>::kSmemBytes, stream, args);
 }
 
 template <int TN, int kProblems>
-int launch_pair(const PairArgs<kProblems>& args, int pairs, cudaStream_t stream) {
+int launch_pair(const LaunchArgs<kProblems>& args, int pairs, cudaStream_t stream) {
   using C = PairConfig<TN>;
   static bool configured[64] = {};
   if (int st = set_smem_once(pair_kernel<TN, kProblems>(), C::kSmemBytes, configured); st != MXB200_OK)
@@ -1560,14 +1590,14 @@ int launch_pair(const PairArgs<kProblems>& args, int pairs, cudaStream_t stream)
 }
 
 template <int kProblems>
-int launch_pair_width(int tile_n, const PairArgs<kProblems>& args, int pairs, cudaStream_t stream) {
+int launch_pair_width(int tile_n, const LaunchArgs<kProblems>& args, int pairs, cudaStream_t stream) {
   return tile_n == 256   ? launch_pair<256, kProblems>(args, pairs, stream)
          : tile_n == 192 ? launch_pair<192, kProblems>(args, pairs, stream)
                          : launch_pair<128, kProblems>(args, pairs, stream);
 }
 
 template <int TN, int kFuse>
-int launch_fused(const PairArgs<1>& args, const FuseMaps& fuse, int pairs, cudaStream_t stream) {
+int launch_fused(const LaunchArgs<1>& args, const FuseMaps& fuse, int pairs, cudaStream_t stream) {
   using C = PairConfig<TN, kFuse>;
   static bool configured[64] = {};
   if (int st = set_smem_once(fused_kernel<TN, kFuse>(), C::kSmemBytes, configured); st != MXB200_OK)
@@ -1657,7 +1687,7 @@ GemmParams gemm_params(const GemmDesc& g, const TilePlan& plan, int splits, cons
   return p;
 }
 
-int pair_maps(PairMaps* m, const GemmDesc& g, const TilePlan& plan, const GemmParams& p) {
+int pair_maps(ProblemMaps* m, const GemmDesc& g, const TilePlan& plan, const GemmParams& p) {
   if (int st = make_operand_map(&m->a, g.a, g.M, g.K, 128); st != MXB200_OK)
     return st;
   if (int st = make_operand_map(&m->b, g.b, g.N, g.K, plan.tile_n / 2); st != MXB200_OK)
@@ -1684,7 +1714,7 @@ int next_sched_slot() {
 template <int kProblems>
 int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInfo& dev, void* workspace,
                  size_t workspace_bytes, cudaStream_t s, const FusedOut& fused) {
-  PairArgs<kProblems> args{};
+  LaunchArgs<kProblems> args{};
   int64_t units = 0;
   ReduceParams sums{};
   int sum_blocks = 0;
@@ -1724,13 +1754,19 @@ int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInf
   };
   const int cap = g_max_ctas.load() > 0 ? g_max_ctas.load() : dev.sms;
   if (!plan.pair) {
-    CUtensorMap ma, mb;
-    if (int st = make_operand_map(&ma, g[0].a, g[0].M, g[0].K, kBM); st != MXB200_OK)
-      return st;
-    if (int st = make_operand_map(&mb, g[0].b, g[0].N, g[0].K, plan.tile_n); st != MXB200_OK)
-      return st;
+    for (int i = 0; i < n; ++i) {
+      if (int st = make_operand_map(&args.maps[i].a, g[i].a, g[i].M, g[i].K, kBM); st != MXB200_OK)
+        return st;
+      if (int st = make_operand_map(&args.maps[i].b, g[i].b, g[i].N, g[i].K, plan.tile_n); st != MXB200_OK)
+        return st;
+    }
+    for (int i = n; i < kProblems; ++i)
+      args.maps[i] = args.maps[n - 1];
     const int grid = static_cast<int>(std::min<int64_t>(units, cap));
-    return sum_slices(plan.tile_n == 256 ? launch<256>(ma, mb, args.p[0], grid, s) : launch<128>(ma, mb, args.p[0], grid, s));
+    if constexpr (kProblems == 1)
+      if (plan.tile_n == 256)
+        return sum_slices(launch_one_cta<256, 1>(args, grid, s));
+    return sum_slices(launch_one_cta<128, kProblems>(args, grid, s));
   }
   for (int i = 0; i < n; ++i)
     if (int st = pair_maps(&args.maps[i], g[i], plan, args.p[i]); st != MXB200_OK)
@@ -1770,13 +1806,9 @@ int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale,
   return launch_gemms<1>(&g, 1, plan, dev, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), fused);
 }
 
-// Whether GEMMs i.. of a list go together, and how many: the CTA-pair kernel takes up to kMaxGroup of them.
-int group_size(const GemmDesc* g, int n) {
-  const int forced = g_tile_n.load();
-  int k = 0;
-  while (k < n && k < kMaxGroup && (forced >= 384 || (forced == 0 && g[k].M >= 256 && g[k].N >= 256)))
-    ++k;
-  return std::max(k, 1);
+// How many GEMMs from the front of a list share a launch: all that fit one, except with the 128 x 256 tile set by hand.
+int group_size(int n) {
+  return g_tile_n.load() == 256 ? 1 : std::min(n, kMaxGroup);
 }
 
 size_t plan_workspace_bytes(const GemmDesc* g, int n, const TilePlan& plan) {
@@ -1789,7 +1821,7 @@ size_t plan_workspace_bytes(const GemmDesc* g, int n, const TilePlan& plan) {
 size_t group_workspace_bytes(const GemmDesc* g, int n, int sms) {
   size_t most = 0;
   for (int i = 0; i < n;) {
-    const int k = group_size(g + i, n - i);
+    const int k = group_size(n - i);
     most = std::max(most, plan_workspace_bytes(g + i, k, plan_tiles(g + i, k, sms, false, 0)));
     i += k;
   }
@@ -1807,7 +1839,7 @@ int gemm_group(const GemmDesc* g, int n, void* workspace, size_t workspace_bytes
     if (int s = check_gemm(g[i], none, 1); s != MXB200_OK)
       return s;
   for (int i = 0; i < n;) {
-    const int k = group_size(g + i, n - i);
+    const int k = group_size(n - i);
     const TilePlan plan = plan_tiles(g + i, k, dev.sms, false, 0);
     auto* s = static_cast<cudaStream_t>(stream);
     const int st = k == 1 ? launch_gemms<1>(g + i, 1, plan, dev, workspace, workspace_bytes, s, none)
@@ -1838,7 +1870,11 @@ extern "C" int mxb200_gemm_splits(int64_t M, int64_t N, int64_t K) {
   mxb200::DeviceInfo dev;
   if (mxb200::current_device(&dev) != MXB200_OK || M <= 0 || N <= 0 || K <= 0)
     return 1;
-  return mxb200::plan_tiles(M, N, K, dev.sms, 0).splits[0];
+  // what the slices of a count chosen here take always fits mxb200_gemm_splitk_static's scratch
+  int splits = mxb200::plan_tiles(M, N, K, dev.sms, 0).splits[0];
+  while (splits > 1 && mxb200_gemm_workspace_bytes(M, N, K, splits) > MXB200_STATIC_SCRATCH_BYTES)
+    splits /= 2;
+  return splits;
 }
 
 extern "C" size_t mxb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int splits) {

@@ -7,10 +7,8 @@
 // thousand tokens was bound by the host (fp8_matmul of 2048 x 768 -> 3072, forward and backward: 59 us of kernels in a
 // 250 us pass). Here a call costs a few allocations from torch's caching allocator and the launches. Tensors that
 // nobody outside sees (quantized operands) are one byte buffer per lifetime, data then scales.
-#include <mutex>
 #include <optional>
 #include <stdexcept>
-#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -136,22 +134,6 @@ void quantize(const Tensor& x, const mxb200_mx_out& out, const mxb200_mx_out& ou
         "quantize_mx");
 }
 
-// Split-K scratch, grown on demand and kept per (device, stream): GEMMs on different streams may overlap and must not
-// share partial tiles; launches on one stream are ordered and reuse theirs (the reference borrows torch's per-stream
-// cuBLAS workspace, mx_gemm.cpp:236-237). A replaced buffer goes back to the caching allocator, which keeps it for the
-// stream it was allocated on until that stream's queued work has run.
-Tensor workspace(at::Device device, size_t bytes) {
-  static std::mutex mu;
-  static auto* buffers = new std::unordered_map<uint64_t, Tensor>();  // never destroyed: outlives the CUDA context
-  const auto s = c10::cuda::getCurrentCUDAStream(device.index());
-  const uint64_t key = (static_cast<uint64_t>(device.index()) << 48) ^ reinterpret_cast<uint64_t>(s.stream());
-  std::lock_guard<std::mutex> lock(mu);
-  Tensor& t = (*buffers)[key];
-  if (!t.defined() || static_cast<size_t>(t.numel()) < bytes)
-    t = empty({static_cast<int64_t>(std::max<size_t>(bytes, size_t(1) << 20))}, at::kByte, device);
-  return t;
-}
-
 // d (M, N) = a (M, K) . b (N, K)^T, bf16 or fp32 (alpha, +=).
 mxb200_gemm_desc gemm_desc(void* d, at::ScalarType dtype, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K,
                            const float* alpha = nullptr, bool accumulate = false) {
@@ -162,10 +144,10 @@ mxb200_gemm_desc gemm_desc(void* d, at::ScalarType dtype, const Layout& a, const
 // Independent GEMMs, in one launch where the library can, split along K where it says so.
 void run_gemms(const mxb200_gemm_desc* g, int n, at::Device device) {
   const size_t bytes = mxb200_gemm_group_workspace_bytes(g, n);
-  Tensor ws;
+  Tensor ws;  // K slices: the caching allocator hands it on along this stream only, behind the launches that use it
   if (bytes > 0)
-    ws = workspace(device, bytes);
-  check(mxb200_gemm_group(g, n, bytes > 0 ? ws.data_ptr() : nullptr, bytes > 0 ? ws.numel() : 0, stream()), "mx_gemm");
+    ws = empty({static_cast<int64_t>(bytes)}, at::kByte, device);
+  check(mxb200_gemm_group(g, n, bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream()), "mx_gemm");
 }
 
 void gemm(void* d, at::ScalarType dtype, const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t K, at::Device device) {
