@@ -826,7 +826,8 @@ __device__ __forceinline__ bool sched_read(Barriers* bars, uint32_t seq, bool ar
 // TN = 256: the widest tile (least L2 traffic per flop); its two accumulator buffers overlap by 32 columns, so
 // the next tile's first MMA waits until the previous tile's epilogue has read those columns: a bubble of about
 // 1500 cycles per tile, negligible for long K. TN = 192: two disjoint buffers, no bubble, for shapes with a
-// short main loop. Scale tiles of B are loaded as the two 128-row tiles covering the tile's columns; the tile's
+// short main loop. TN = 128: twice the tiles for launches that would leave pairs idle (the (C, C) weight gradient beside its
+// input gradient), at 1.5 times the L2 traffic per flop of TN = 256. Scale tiles of B are loaded as the two 128-row tiles covering the tile's columns; the tile's
 // first column is ((n * TN) % 128) / 32 TMEM columns into the first of them. That offset must be even: a scale
 // address at an odd column (a tile starting 32 or 96 rows into a scale tile, as a 224-wide tiling would) is a
 // misaligned-address fault, so tile widths are multiples of 64.

@@ -13,8 +13,9 @@
 //                (a warp reads 128 contiguous bytes per row, conflict-free), needs no shuffle, and writes
 //                32 contiguous bytes of each transposed row with one 256-bit store (a full DRAM sector).
 //   scales:      staged in shared memory in swizzled order and written as 16-byte vectors, 512 bytes per tile.
-// Two schedules: one CTA per tile (every input type and prologue; tensors of up to one wave), and for plain bf16
-// tensors of more than one wave persistent CTAs that draw tiles from a counter and bring them in by TMA a tile ahead.
+// Three schedules: one CTA per tile (every input type and prologue; lists of up to one wave), for plain input of more than
+// one wave, bf16 and fp32 tensors in one list, persistent CTAs that draw tiles from a counter and bring them in by TMA a
+// tile ahead, and the same in three groups around a shared table for the softcap gradient.
 // HBM traffic is the algorithmic minimum: every input byte read once, every output byte written once.
 #include <algorithm>
 #include <vector>
@@ -364,7 +365,7 @@ __device__ __forceinline__ void quantize_tile(const QuantParams& p, int tile_ind
   write_scale_tiles(p, tile_r, tile_c, sc_rows, sc_cols, t);
 }
 
-// ---- streaming form for plain bf16 input: persistent CTAs, tiles drawn from a counter and brought in by TMA
+// ---- streaming forms: persistent CTAs, tiles drawn from a counter and brought in by TMA
 //
 // The one-shot kernel above holds a tile's loads in registers, so a CTA reads, computes and writes in turn and only
 // the other CTAs of its SM overlap with it. Here three CTAs per SM each keep two 32 KB tile buffers: while all threads
