@@ -165,6 +165,23 @@ def test_weight_grad_accumulates_and_ignores_chunk_size():
     assert torch.allclose(grads[0], single[0] + single[1], rtol=1e-5, atol=1e-8)
 
 
+@pytest.mark.parametrize("tokens,chunk,embd", [(256, 256, 128), (640, 256, 128), (384, 128, 384), (1152, 512, 768)])
+def test_chunks_share_launches_and_keep_their_bits(tokens, chunk, embd):
+    """A chunk's input gradient shares its launch with the next chunk's logits, which overwrite the buffer its gradient came
+    from; the last chunk may be short. Rows do not depend on one another and 1024 columns are too few for K slices, so every
+    chunk's input gradient has the bits of a call of its own."""
+    vocab, padded = 1000, 1024
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, embd, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(padded, embd, device="cuda", generator=g) * 0.5).requires_grad_()
+    targets = torch.randint(-1, vocab, (tokens,), device="cuda", generator=g)
+    nc.softcap_cross_entropy(x, w, targets, vocab, 15, chunk, "sum").backward()
+    for begin in range(0, tokens, chunk):
+        part = x.detach()[begin:begin + chunk].clone().requires_grad_()
+        nc.softcap_cross_entropy(part, w, targets[begin:begin + chunk], vocab, 15, chunk, "sum").backward()
+        assert torch.equal(x.grad[begin:begin + chunk], part.grad)
+
+
 def test_argument_errors():
     x = torch.zeros(128, 128, dtype=torch.bfloat16, device="cuda")
     w = torch.zeros(256, 128, device="cuda")
