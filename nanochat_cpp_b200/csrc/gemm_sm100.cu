@@ -1498,9 +1498,28 @@ double launch_cycles(const GemmDesc* g, int n, const TileKind& t, const int* spl
   return t.start + least + tail;
 }
 
-// Tile and slices with the least expected time. `fixed`: slices of a single GEMM given by the caller. The 128 x 256 tile is
-// for single GEMMs, the pair tiles for matrices of at least 256 rows (any, when set by mxb200_set_gemm_config).
-TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed) {
+// K slices of a GEMM, from its shape and the machine alone: neither the GEMMs that share its launch, nor its output's type, nor
+// whether it accumulates have a say, so that the order of its fp32 sum, and with it every bit, is that of the same GEMM by
+// itself. Slices cost a round trip of fp32 matrices and a launch, so they are for what fills at most a quarter of the machine
+// and leaves each slice 32 K steps: 768 x 768 x 16384 takes 28.0 us in one, 17.4 in four, 768 x 768 x 8192 16.4 in one, 13.8 in
+// two. Just past the line they gain less (768 x 1536 x 16384 28.6 and 23.1 in four, 768 x 768 x 4096 10.5 and 9.7, 2048 x 768 x
+// 32768 60.0 and 49.6 in two), too little to give these shapes another order of summation.
+int plan_splits(int64_t M, int64_t N, int64_t K, int sms) {
+  const bool pair = M >= 256 && N >= 256;
+  const int64_t tile_m = pair ? 256 : 128, tile_n = pair ? 192 : N >= 256 ? 256 : 128;
+  const int64_t slots = pair ? sms / 2 : sms;
+  if (M <= 0 || N <= 0 || K <= 0)
+    return 1;
+  const int64_t tiles = ((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n);
+  int splits = 1;
+  for (int s = 2; s <= 4 && tiles * 4 <= slots && K / 128 / s >= 32; s *= 2)
+    splits = s;
+  return splits;
+}
+
+// Tile with the least expected time for GEMMs cut into the given slices. The 128 x 256 tile is for single GEMMs, the pair tiles
+// for matrices of at least 256 rows (any, when set by mxb200_set_gemm_config).
+TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, const int* splits) {
   int forced = g_tile_n.load();
   if (need_pair && forced != 384 && forced != 512)
     forced = 0;  // the fused-quantize epilogues exist for these two only
@@ -1508,6 +1527,7 @@ TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed
   for (int i = 0; i < n; ++i)
     wide &= g[i].M >= 256 && g[i].N >= 256;
   TilePlan plan{};
+  std::copy(splits, splits + n, plan.splits);
   double best = 0.0;
   for (const TileKind& t : kTileKinds) {
     const int name = t.pair ? (t.tile_n == 256 ? 512 : t.tile_n == 192 ? 384 : 640) : t.tile_n;  // in mxb200_set_gemm_config
@@ -1515,43 +1535,20 @@ TilePlan plan_tiles(const GemmDesc* g, int n, int sms, bool need_pair, int fixed
       continue;
     if ((need_pair && (!t.pair || t.tile_n == 128)) || (n > 1 && !t.pair && t.tile_n == 256))
       continue;
-    int splits[kMaxGroup] = {1, 1, 1};
-    const auto consider = [&] {
-      const double cost = launch_cycles(g, n, t, splits, sms);
-      if (best == 0.0 || cost < best * 0.99) {
-        best = cost;
-        plan.pair = t.pair, plan.tile_m = t.pair ? 256 : 128, plan.tile_n = t.tile_n;
-        std::copy(splits, splits + kMaxGroup, plan.splits);
-      }
-    };
-    if (fixed > 0 || need_pair) {
-      splits[0] = std::max(fixed, 1);
-      consider();
-      continue;
+    const double cost = launch_cycles(g, n, t, plan.splits, sms);
+    if (best == 0.0 || cost < best * 0.99) {
+      best = cost;
+      plan.pair = t.pair, plan.tile_m = t.pair ? 256 : 128, plan.tile_n = t.tile_n;
     }
-    consider();
-    // K slices, one GEMM at a time: each takes the count that helps most given the others
-    for (int i = 0; i < n; ++i) {
-      int kept = 1;
-      double least = launch_cycles(g, n, t, splits, sms);
-      for (int s = 2; s <= 8; s *= 2) {
-        if (g[i].K / 128 / s < 8)
-          break;
-        splits[i] = s;
-        if (const double c = launch_cycles(g, n, t, splits, sms); c < least * 0.97)
-          least = c, kept = s;
-      }
-      splits[i] = kept;
-    }
-    consider();
   }
   return plan;
 }
 
-TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, int fixed) {
+// The tile of a single GEMM depends on its shape and slices only.
+TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, int splits) {
   GemmDesc g{};
   g.M = M, g.N = N, g.K = K, g.out_kind = kOutF32;
-  return plan_tiles(&g, 1, sms, false, fixed);
+  return plan_tiles(&g, 1, sms, false, &splits);
 }
 
 // Bytes of a GEMM's K slices; 0 when K is not split.
@@ -1802,8 +1799,8 @@ int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale,
   const GemmDesc g{a, a_scale, b, b_scale, d, resid, alpha, M, N, K, out_kind, accumulate};
   if (int s = check_gemm(g, fused, splits); s != MXB200_OK)
     return s;
-  // the plan of a single GEMM depends on its shape and slices only, as the workspace query's does
-  const TilePlan plan = fused.fuse != kFuseNone ? plan_tiles(&g, 1, dev.sms, true, 1) : plan_tiles(M, N, K, dev.sms, splits);
+  const int one = 1;
+  const TilePlan plan = fused.fuse != kFuseNone ? plan_tiles(&g, 1, dev.sms, true, &one) : plan_tiles(M, N, K, dev.sms, splits);
   return launch_gemms<1>(&g, 1, plan, dev, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), fused);
 }
 
@@ -1812,19 +1809,13 @@ int group_size(int n) {
   return g_tile_n.load() == 256 ? 1 : std::min(n, kMaxGroup);
 }
 
-size_t plan_workspace_bytes(const GemmDesc* g, int n, const TilePlan& plan) {
-  size_t bytes = 0;
-  for (int i = 0; i < n; ++i)
-    bytes += slice_bytes(g[i], plan.splits[i]);
-  return bytes;
-}
-
 size_t group_workspace_bytes(const GemmDesc* g, int n, int sms) {
   size_t most = 0;
   for (int i = 0; i < n;) {
-    const int k = group_size(n - i);
-    most = std::max(most, plan_workspace_bytes(g + i, k, plan_tiles(g + i, k, sms, false, 0)));
-    i += k;
+    size_t bytes = 0;
+    for (const int end = i + group_size(n - i); i < end; ++i)
+      bytes += slice_bytes(g[i], plan_splits(g[i].M, g[i].N, g[i].K, sms));
+    most = std::max(most, bytes);
   }
   return most;
 }
@@ -1841,7 +1832,10 @@ int gemm_group(const GemmDesc* g, int n, void* workspace, size_t workspace_bytes
       return s;
   for (int i = 0; i < n;) {
     const int k = group_size(n - i);
-    const TilePlan plan = plan_tiles(g + i, k, dev.sms, false, 0);
+    int splits[kMaxGroup];
+    for (int j = 0; j < k; ++j)
+      splits[j] = plan_splits(g[i + j].M, g[i + j].N, g[i + j].K, dev.sms);
+    const TilePlan plan = plan_tiles(g + i, k, dev.sms, false, splits);
     auto* s = static_cast<cudaStream_t>(stream);
     const int st = k == 1 ? launch_gemms<1>(g + i, 1, plan, dev, workspace, workspace_bytes, s, none)
                           : launch_gemms<kMaxGroup>(g + i, k, plan, dev, workspace, workspace_bytes, s, none);
@@ -1869,13 +1863,8 @@ extern "C" int mxb200_gemm_f32(const void* a, const void* a_scale, const void* b
 
 extern "C" int mxb200_gemm_splits(int64_t M, int64_t N, int64_t K) {
   mxb200::DeviceInfo dev;
-  if (mxb200::current_device(&dev) != MXB200_OK || M <= 0 || N <= 0 || K <= 0)
-    return 1;
-  // what the slices of a count chosen here take always fits mxb200_gemm_splitk_static's scratch
-  int splits = mxb200::plan_tiles(M, N, K, dev.sms, 0).splits[0];
-  while (splits > 1 && mxb200_gemm_workspace_bytes(M, N, K, splits) > MXB200_STATIC_SCRATCH_BYTES)
-    splits /= 2;
-  return splits;
+  // at most a quarter of the machine's tiles in four slices: 19 MB, which always fits mxb200_gemm_splitk_static's scratch
+  return mxb200::current_device(&dev) == MXB200_OK ? mxb200::plan_splits(M, N, K, dev.sms) : 1;
 }
 
 extern "C" size_t mxb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int splits) {

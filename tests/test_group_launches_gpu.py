@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 lib, capi = nc.capi.lib, nc.capi
 
 TOL_BF16 = 2e-3  # one bf16 rounding per value: 2^-9 at most, relative to the value
-TOL_F32 = 1e-5   # fp32 sums of up to 4096 products in another order
+TOL_F32 = 1e-5   # fp32 sums of up to 16384 products in another order
 
 
 @pytest.fixture(autouse=True)
@@ -54,14 +54,15 @@ def gemm_group(problems):
     return need
 
 
-# tiles of 128 and 256 rows that are half empty, one 128-row matrix in a group, K of one tile beside a K that is cut into
-# slices, lists of one to four (a fourth takes a launch of its own)
+# tiles of 128 and 256 rows that are half empty, one 128-row matrix in a group, K of one tile beside a deep one and beside one
+# that is cut into slices (from 8192 on), lists of one to four (a fourth takes a launch of its own)
 GROUPS = [
     [(128, 128, 128)],
     [(256, 384, 512), (640, 256, 128)],
     [(128, 768, 4096), (384, 256, 256)],
     [(256, 256, 4096), (256, 384, 2048), (896, 640, 384)],
     [(384, 128, 256), (256, 256, 128), (128, 512, 384), (640, 384, 256)],
+    [(256, 384, 8192), (384, 256, 128), (128, 256, 16384)],
 ]
 
 
