@@ -402,6 +402,27 @@ inline bool grad_mode(std::initializer_list<const Tensor*> inputs) {
   return false;
 }
 
+// x (N, C) quantized by the caller. The transposed layout is read by the backward only. The scales' type is the caller's: any
+// of one byte.
+Mx given_mx(const std::vector<Tensor>& t, const Tensor& x, bool grad, const char* what) {
+  const Mx q{t.at(0), t.at(1), t.at(2), t.at(3)};
+  const auto layout = [&](const Tensor& data, const Tensor& scale, int64_t rows, int64_t cols) {
+    for (const Tensor* p : {&data, &scale}) {
+      require_cuda(*p, what);
+      if (p->device() != x.device() || !p->is_contiguous())
+        throw std::runtime_error(std::string(what) + ": expected contiguous operands on the input's device");
+    }
+    if (data.sizes() != at::IntArrayRef{rows, cols} || data.scalar_type() != kE4M3)
+      throw std::runtime_error(std::string(what) + ": shape mismatch");
+    if (scale.numel() != rows * cols / 32 || scale.element_size() != 1)
+      throw std::runtime_error(std::string(what) + ": expected e4m3 operands with their MX scales");
+  };
+  layout(q.data, q.scale, x.size(0), x.size(1));
+  if (grad)
+    layout(q.data_t, q.scale_t, x.size(1), x.size(0));
+  return q;
+}
+
 // One Linear under MX: y = x . w^T, dX = dY . w, dW = dY^T . x, every operand E4M3 with per-32 scales along the
 // contraction (fp8.cpp:240-260).
 Tensor linear_forward(const Tensor& x, WeightUse& w, bool grad, Tensor* x_cols) {
@@ -578,18 +599,11 @@ variable_list fp8_qkv(const Tensor& x_2d, const Tensor& wq, const Tensor& wk, co
   require(wq.size(1) == x_2d.size(1), "mx_gemm: shape mismatch");
   require_cuda(x_2d, "quantize_mx");
   const Tensor x = x_2d.contiguous();
-  Mx given;
-  if (x_mx.has_value()) {
-    const auto& t = *x_mx;
-    given = {t.at(0), t.at(1), t.at(2), t.at(3)};
-    require(given.data.sizes() == x.sizes() && given.data.scalar_type() == kE4M3 && given.data.is_contiguous() &&
-                  given.scale.numel() == x.numel() / 32 && given.data_t.numel() == x.numel() &&
-                  given.data_t.is_contiguous() && given.scale_t.numel() == x.numel() / 32,
-            "mx_gemm: shape mismatch");
-  }
+  const bool grad = grad_mode({&x, &wq, &wk, &wv});
+  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x, grad, "mx_gemm") : Mx{};
   WeightUse use(cache, {wq, wk, wv});
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
-  if (!grad_mode({&x, &wq, &wk, &wv}))
+  if (!grad)
     return qkv_forward(x, use, gate_cols, mx, false, nullptr);
   return MxQkv::apply(x, wq, wk, wv, gate_cols, &use, mx);
 }
@@ -694,18 +708,11 @@ Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor&
           "fp8_relu_square_mlp: MX needs N, in, hidden, out % 128");
   require_cuda(x_2d, "quantize_mx");
   const Tensor x = x_2d.contiguous();
-  Mx given;
-  if (x_mx.has_value()) {
-    const auto& t = *x_mx;
-    given = {t.at(0), t.at(1), t.at(2), t.at(3)};
-    require(given.data.sizes() == x.sizes() && given.data.scalar_type() == kE4M3 && given.data.is_contiguous() &&
-                  given.scale.numel() == x.numel() / 32 && given.data_t.numel() == x.numel() &&
-                  given.data_t.is_contiguous() && given.scale_t.numel() == x.numel() / 32,
-            "mx_gemm_relu_square: shape mismatch");
-  }
+  const bool grad = grad_mode({&x, &w_fc, &w_proj});
+  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x, grad, "mx_gemm_relu_square") : Mx{};
   WeightUse fc(fc_cache, {w_fc}), proj(proj_cache, {w_proj});
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
-  if (!grad_mode({&x, &w_fc, &w_proj}))
+  if (!grad)
     return mlp_forward(x, fc, proj, mx, false, nullptr);
   return Fp8ReluSquareMlp::apply(x, w_fc, w_proj, &fc, &proj, mx);
 }

@@ -105,3 +105,51 @@ def test_first_call_of_a_fresh_thread_may_be_a_gemm():
     t.join()
     torch.cuda.synchronize()
     assert status == [0] and torch.equal(got, want)
+
+
+def _x_mx_users(x, x_mx):
+    w = [torch.randn(n, x.size(1), device="cuda").requires_grad_() for n in (256, 128, 128)]
+    proj = torch.randn(128, 256, device="cuda").requires_grad_()
+    return [lambda: nc.fp8_qkv(x, *w, x_mx=x_mx), lambda: nc.fp8_relu_square_mlp(x, w[0], proj, x_mx=x_mx)]
+
+
+BAD_X_MX = {
+    "host data": lambda q: setattr(q, "data", q.data.cpu()),
+    "host scale": lambda q: setattr(q, "inv_scale", q.inv_scale.cpu()),
+    "host data_t": lambda q: setattr(q, "data_t", q.data_t.cpu()),
+    "host scale_t": lambda q: setattr(q, "inv_scale_t", q.inv_scale_t.cpu()),
+    "data_t of data's shape": lambda q: setattr(q, "data_t", q.data_t.view(q.data.shape)),
+    "data_t of another type": lambda q: setattr(q, "data_t", q.data_t.view(torch.uint8)),
+    "data_t transposed view": lambda q: setattr(q, "data_t", q.data.t()),
+    "short scale": lambda q: setattr(q, "inv_scale", q.inv_scale[:-1]),
+    "short scale_t": lambda q: setattr(q, "inv_scale_t", q.inv_scale_t[:-1]),
+    "wide scale_t": lambda q: setattr(q, "inv_scale_t", q.inv_scale_t.to(torch.float32)),
+}
+
+
+@pytest.mark.parametrize("bad", BAD_X_MX)
+def test_x_mx_is_checked_before_anything_is_launched(bad):
+    """Host checks only: nothing is launched on the operands that are refused."""
+    x = torch.randn(256, 384, device="cuda").to(torch.bfloat16).requires_grad_()
+    q = nc.quantize_mx(x.detach())
+    BAD_X_MX[bad](q)
+    launches = nc.capi.launch_count()
+    for call in _x_mx_users(x, q):
+        with pytest.raises(RuntimeError):
+            call()
+    assert nc.capi.launch_count() == launches
+
+
+def test_x_mx_scales_may_be_bytes_and_no_grad_reads_rows_only():
+    x = torch.randn(256, 384, device="cuda").to(torch.bfloat16).requires_grad_()
+    q = nc.quantize_mx(x.detach())
+    raw = nc.Fp8Tensor(q.data, q.data_t, q.inv_scale.view(torch.uint8), q.inv_scale_t.view(torch.uint8))
+    rows = nc.Fp8Tensor(q.data, q.data.t(), q.inv_scale, q.inv_scale[:1])
+    for call in _x_mx_users(x, raw):
+        out = call()
+        out = out if isinstance(out, tuple) else (out,)
+        torch.autograd.backward(out, [torch.ones_like(t) for t in out])
+    assert x.grad is not None
+    with torch.no_grad():
+        for call in _x_mx_users(x, rows):
+            call()
