@@ -247,11 +247,12 @@ typedef struct mxb200_gemm_desc {
   int32_t accumulate;
 } mxb200_gemm_desc;
 
-/* n independent GEMMs in as few launches as possible, bit for bit what n calls of mxb200_gemm_bf16 / mxb200_gemm_f32 (or
+/* n GEMMs in as few launches as possible, bit for bit what n calls of mxb200_gemm_bf16 / mxb200_gemm_f32 (or
  * mxb200_gemm_splitk, where the library splits K) give. For the GEMMs a backward runs on the same operands (the
  * reference launches them one after another, fp8.cpp:299-337, 456-460): the tiles of up to three share one launch, so
  * that shapes with fewer tiles than the machine has CTA pairs fill it together. They run in the order given as far as
- * their tiles are taken up in order. workspace: mxb200_gemm_group_workspace_bytes (0: none needed), 256-byte aligned,
+ * their tiles are taken up in order; one that writes what an earlier one reads or writes (two weight gradients accumulating into
+ * one matrix) starts a launch of its own behind it. workspace: mxb200_gemm_group_workspace_bytes (0: none needed), 256-byte aligned,
  * uninitialised, reusable by later calls on the same stream. */
 MXB200_API size_t mxb200_gemm_group_workspace_bytes(const mxb200_gemm_desc* g, int n);
 MXB200_API int mxb200_gemm_group(const mxb200_gemm_desc* g, int n, void* workspace, size_t workspace_bytes, void* stream);

@@ -1804,16 +1804,45 @@ int gemm(const void* a, const void* a_scale, const void* b, const void* b_scale,
   return launch_gemms<1>(&g, 1, plan, dev, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), fused);
 }
 
-// How many GEMMs from the front of a list share a launch: all that fit one, except with the 128 x 256 tile set by hand.
-int group_size(int n) {
-  return g_tile_n.load() == 256 ? 1 : std::min(n, kMaxGroup);
+// Bytes of memory that a GEMM reads or writes.
+struct Span {
+  uintptr_t begin, end;
+  Span(const void* p, int64_t bytes)
+      : begin(reinterpret_cast<uintptr_t>(p)), end(begin + (p != nullptr && bytes > 0 ? static_cast<uintptr_t>(bytes) : 0)) {}
+  bool meets(const Span& o) const { return begin < o.end && o.begin < end; }
+};
+
+Span output_span(const GemmDesc& g) {
+  return {g.d, g.M * g.N * (g.out_kind == kOutF32 ? 4 : 2)};
+}
+
+// Whether what w writes is also written or read by g.
+bool writes_into(const GemmDesc& w, const GemmDesc& g) {
+  const Span out = output_span(w);
+  const int64_t a = g.M * g.K, b = g.N * g.K;
+  for (const Span& s : {output_span(g), Span{g.a, a}, Span{g.b, b}, Span{g.a_scale, a / 32}, Span{g.b_scale, b / 32},
+                        Span{g.resid, g.M * g.N * 2}, Span{g.alpha, 4}})
+    if (out.meets(s))
+      return true;
+  return false;
+}
+
+// How many GEMMs from the front of a list share a launch: all that fit one, up to the first that has to follow an earlier one
+// (weight gradients accumulating into one matrix, say), except with the 128 x 256 tile set by hand.
+int group_size(const GemmDesc* g, int n) {
+  const int most = g_tile_n.load() == 256 ? 1 : std::min(n, kMaxGroup);
+  for (int i = 1; i < most; ++i)
+    for (int j = 0; j < i; ++j)
+      if (writes_into(g[i], g[j]) || writes_into(g[j], g[i]))
+        return i;
+  return most;
 }
 
 size_t group_workspace_bytes(const GemmDesc* g, int n, int sms) {
   size_t most = 0;
   for (int i = 0; i < n;) {
     size_t bytes = 0;
-    for (const int end = i + group_size(n - i); i < end; ++i)
+    for (const int end = i + group_size(g + i, n - i); i < end; ++i)
       bytes += slice_bytes(g[i], plan_splits(g[i].M, g[i].N, g[i].K, sms));
     most = std::max(most, bytes);
   }
@@ -1831,7 +1860,7 @@ int gemm_group(const GemmDesc* g, int n, void* workspace, size_t workspace_bytes
     if (int s = check_gemm(g[i], none, 1); s != MXB200_OK)
       return s;
   for (int i = 0; i < n;) {
-    const int k = group_size(n - i);
+    const int k = group_size(g + i, n - i);
     int splits[kMaxGroup];
     for (int j = 0; j < k; ++j)
       splits[j] = plan_splits(g[i + j].M, g[i + j].N, g[i + j].K, dev.sms);

@@ -141,7 +141,7 @@ mxb200_gemm_desc gemm_desc(void* d, at::ScalarType dtype, const Layout& a, const
           dtype == at::kFloat ? MXB200_OUT_F32 : MXB200_OUT_BF16, accumulate};
 }
 
-// Independent GEMMs, in one launch where the library can, split along K where it says so.
+// GEMMs in one launch where the library can, split along K where it says so.
 void run_gemms(const mxb200_gemm_desc* g, int n, at::Device device) {
   const size_t bytes = mxb200_gemm_group_workspace_bytes(g, n);
   Tensor ws;  // K slices: the caching allocator hands it on along this stream only, behind the launches that use it
@@ -681,14 +681,21 @@ struct Fp8ReluSquareMlp : torch::autograd::Function<Fp8ReluSquareMlp> {
     int n = 0;
     std::optional<WeightGrad> fc, proj;
     const bool fc_direct = grad_direct(w_fc), proj_direct = grad_direct(w_proj);
-    if (fc_direct || ctx->needs_input_grad(1)) {
-      fc.emplace(dh_t, saved_layout(saved[0], saved[1], C, N), H, C, N, std::vector<Tensor>{w_fc}, fc_direct, nullptr, device);
-      gemms[n++] = fc->desc();
-    }
+    const auto fc_grad = [&] {
+      if (fc_direct || ctx->needs_input_grad(1)) {
+        fc.emplace(dh_t, saved_layout(saved[0], saved[1], C, N), H, C, N, std::vector<Tensor>{w_fc}, fc_direct, nullptr, device);
+        gemms[n++] = fc->desc();
+      }
+    };
+    const bool tied = w_fc.is_same(w_proj);  // both into one .grad, in the order of the Linears' backwards
+    if (!tied)
+      fc_grad();
     if (proj_direct || ctx->needs_input_grad(2)) {
       proj.emplace(go_t, layout_of(saved[7], H, N), O, H, N, std::vector<Tensor>{w_proj}, proj_direct, nullptr, device);
       gemms[n++] = proj->desc();
     }
+    if (tied)
+      fc_grad();
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
       dx = empty({N, C}, at::kBFloat16, device);

@@ -36,6 +36,27 @@ def test_queries_take_any_shape(M, N, K):
     assert lib.mxb200_gemm_splits(M, N, K) == 1
 
 
+def test_gemms_that_touch_one_output_do_not_share_a_launch():
+    """By the workspace that the launches need together (256 x 256 x 8192 is cut into two slices): nothing is launched."""
+    M = N = 256
+    K, slices = 8192, 2 * 256 * 256 * 4
+
+    def need(**second):
+        arr = (capi.GemmDesc * 2)()
+        for d, base in zip(arr, (1 << 32, 1 << 33)):
+            d.a, d.b, d.a_scale, d.b_scale, d.d = (base + (i << 24) for i in range(5))
+            d.M, d.N, d.K, d.out_kind, d.accumulate = M, N, K, capi.OUT_F32, 1
+        for name, value in second.items():
+            setattr(arr[1], name, value)
+        return lib.mxb200_gemm_group_workspace_bytes(arr, 2)
+
+    first = (1 << 32) + (4 << 24)  # the first one's output, M * N * 4 bytes
+    assert need() == 2 * slices and need(d=first + M * N * 4) == 2 * slices and need(d=first - M * N * 4) == 2 * slices
+    for name in ("d", "a", "b", "a_scale", "b_scale", "resid", "alpha"):
+        assert need(**{name: first + M * N * 4 - 4}) == slices, name
+    assert need(d=(1 << 32) + 16) == slices  # writes into the first one's operand
+
+
 def operand(rows, k, seed):
     x = torch.randn(rows, k, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
     return nc.quantize_mx(x.to(torch.bfloat16), True, False)
@@ -91,3 +112,17 @@ def test_mlp_equals_two_linears_over_micro_batches(tokens, embd, input_grad):
         assert torch.equal(y, y2)
         assert not input_grad or torch.equal(x.grad, x2.grad)
     assert torch.equal(fc.grad, fc2.grad) and torch.equal(proj.grad, proj2.grad)
+
+
+@pytest.mark.gpu
+def test_mlp_with_one_weight_for_both_projections():
+    """Two weight gradients into one .grad, over micro-batches: as two Linears on that weight."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = torch.randn(768, 768, generator=g, device="cuda") * 768 ** -0.5
+    w, w2 = w.clone().requires_grad_(), w.clone().requires_grad_()
+    for _ in range(3):
+        x = torch.randn(512, 768, generator=g, device="cuda").to(torch.bfloat16)
+        dy = torch.randn(512, 768, generator=g, device="cuda").to(torch.bfloat16)
+        nc.fp8_relu_square_mlp(x, w, w).backward(dy)
+        nc.fp8_matmul(torch.relu(nc.fp8_matmul(x, w2)).square(), w2).backward(dy)
+        assert torch.equal(w.grad, w2.grad)
