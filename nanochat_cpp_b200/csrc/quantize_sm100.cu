@@ -839,8 +839,9 @@ __device__ __forceinline__ void quantize_stream_batch(const StreamBatch<kMaxJobs
     int drawn = 0;
     if (t == 0 && drawing)
       drawn = static_cast<int>(gridDim.x + atomicAdd(&sched[0], 1u));
-    const bool landed = stream_wait(&bars->full[s], static_cast<uint32_t>(i / kStreamStages) & 1u, bars,
-                                    kStreamWaitLimitNs, static_cast<uint32_t>(i));
+    // the passes shuffle within a warp: its lanes take them together or not at all, also when some gave up waiting
+    const bool landed = __all_sync(0xffffffffu, stream_wait(&bars->full[s], static_cast<uint32_t>(i / kStreamStages) & 1u,
+                                                            bars, kStreamWaitLimitNs, static_cast<uint32_t>(i))) != 0;
     const int u = landed ? *reinterpret_cast<volatile int*>(&bars->tile_of[s]) : -1;
     const StreamJob& job = b.jobs[u >= 0 ? *reinterpret_cast<volatile int*>(&bars->job_of[s]) : 0];
     const bool f32 = job.f32;
