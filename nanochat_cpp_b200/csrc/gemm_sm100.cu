@@ -550,7 +550,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const LaunchArgs<kProblems>&
       const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
-      if (!wait_bounded(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
+      if (!wait_bounded_warp(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
         ok = false;
         break;
       }
@@ -1132,7 +1132,7 @@ __device__ __forceinline__ void pair_kernel_body(const LaunchArgs<kProblems>& ar
         load_h_pieces(p, lane, tc.m * C::kTileM + static_cast<int>(rank) * 128 + quarter * 32, tc.n * C::kTileN + c0 * 32,
                       h_pieces);
       }
-      if (!wait_bounded(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
+      if (!wait_bounded_warp(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
         ok = false;
         break;
       }
