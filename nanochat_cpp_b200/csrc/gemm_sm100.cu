@@ -547,7 +547,7 @@ __device__ __forceinline__ void one_cta_kernel_body(const LaunchArgs<kProblems>&
     for (int u = blockIdx.x; ok && u < total_units; u += gridDim.x, ++local) {
       int unit = u;
       const GemmParams& p = args.p[problem_of(args, &unit)];
-      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
+      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? *p.alpha : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
       if (!wait_bounded_warp(&bars->tmem_full[buf], use & 1u, bars, kSiteEpilogueFull)) {
@@ -614,8 +614,8 @@ __device__ __forceinline__ void load_h_pieces(const GemmParams& p, int lane, int
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int r = j * 8 + (lane >> 2), piece = lane & 3;
-    pieces[j] = inside ? __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.h_in) +
-                                                              (static_cast<int64_t>(warp_row0) + r) * p.N + col + piece * 8))
+    pieces[j] = inside ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.h_in) +
+                                                         (static_cast<int64_t>(warp_row0) + r) * p.N + col + piece * 8)
                        : make_uint4(0, 0, 0, 0);
   }
 }
@@ -1122,7 +1122,7 @@ __device__ __forceinline__ void pair_kernel_body(const LaunchArgs<kProblems>& ar
       const int g = problem_of(args, &unit);
       const GemmParams& p = args.p[g];
       const ProblemMaps& maps = args.maps[g];
-      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? __ldg(p.alpha) : 1.f;
+      const float alpha = (p.out_kind == kOutF32 && p.alpha != nullptr) ? *p.alpha : 1.f;
       const TileCoord tc = decode_unit(p, unit);
       const uint32_t buf = local & 1u, use = local >> 1;
       // the relu^2 backward form reads h: the first chunk's block is requested before the accumulator is waited for
@@ -1289,7 +1289,7 @@ __global__ void __launch_bounds__(mxb200::kReduceThreads) mxb200_gemm_sum_slices
   const int64_t at = (static_cast<int64_t>(static_cast<int>(blockIdx.x) - job.first_block) * kReduceThreads + threadIdx.x) * 8;
   if (at >= job.elements)
     return;
-  const float alpha = job.p.out_kind == kOutF32 && job.p.alpha != nullptr ? __ldg(job.p.alpha) : 1.f;
+  const float alpha = job.p.out_kind == kOutF32 && job.p.alpha != nullptr ? *job.p.alpha : 1.f;
   float acc[8] = {};
 #pragma unroll 4
   for (int s = 0; s < job.splits; ++s) {

@@ -36,7 +36,8 @@ __device__ __forceinline__ bool elect_one() {
 
 // Everything the stream did before this kernel is complete and visible after this; nothing may touch global memory before
 // it. Kernels launched by launch_kernel (internal.h) start with it, every thread. The next kernel's blocks may then be
-// placed as this one's leave their SMs.
+// placed as this one's leave their SMs. What they read is therefore not read-only for a kernel's whole life: no ld.global.nc
+// or __ldg.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
