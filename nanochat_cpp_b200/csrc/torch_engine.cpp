@@ -12,6 +12,7 @@
 #include <utility>
 #include <vector>
 
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
@@ -393,7 +394,13 @@ class QuantizeJobs {
 
 // ---------------------------------------------------------------------------------------------------- Linear
 
+// Whether a call of these inputs gets an autograd node. What a node refuses, forward-mode tangents and function transforms
+// (vmap, jvp), is refused without one too: the outputs would come back as constants.
 inline bool grad_mode(std::initializer_list<const Tensor*> inputs) {
+  for (const Tensor* t : inputs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(0).defined(), "MX: forward-mode differentiation is not implemented");
+  if (const auto& transforms = at::functorch::functorchTLSAccessor())
+    transforms->checkSupportsCppAutogradFunction();
   if (!at::GradMode::is_enabled())
     return false;
   for (const Tensor* t : inputs)

@@ -153,3 +153,32 @@ def test_x_mx_scales_may_be_bytes_and_no_grad_reads_rows_only():
     with torch.no_grad():
         for call in _x_mx_users(x, rows):
             call()
+
+
+@pytest.mark.parametrize("which", ["x", "w"])
+@pytest.mark.parametrize("no_grad", [False, True])
+def test_forward_mode_is_refused(which, no_grad):
+    """Without a node a tangent would be dropped, which reads as a derivative of zero."""
+    import torch.autograd.forward_ad as fwd
+    x, w = torch.randn(128, 256, device="cuda").to(torch.bfloat16), torch.randn(256, 256, device="cuda")
+    t = torch.zeros(128, dtype=torch.int64, device="cuda")
+    with fwd.dual_level(), torch.set_grad_enabled(not no_grad):
+        if which == "x":
+            x = fwd.make_dual(x, torch.ones_like(x))
+        else:
+            w = fwd.make_dual(w, torch.ones_like(w))
+        for call in (lambda: nc.fp8_matmul(x, w), lambda: nc.fp8_qkv(x, w, w, w), lambda: nc.fp8_relu_square_mlp(x, w, w),
+                     lambda: nc.softcap_cross_entropy(x, w, t, 256, 15.0, 128)):
+            with pytest.raises(NotImplementedError):
+                call()
+
+
+def test_function_transforms_are_refused():
+    x, w = torch.randn(2, 128, 256, device="cuda").to(torch.bfloat16), torch.randn(256, 256, device="cuda")
+    q = nc.quantize_mx(x[0])
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda a: nc.fp8_matmul(a, w))(x)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda a: nc.fp8_relu_square_mlp(a, w, w, x_mx=q))(x)
+    with pytest.raises(RuntimeError):
+        torch.func.jvp(lambda a: nc.fp8_relu_square_mlp(a, w, w, x_mx=q), (x[0],), (x[0],))
