@@ -585,8 +585,11 @@ struct MxQkv : torch::autograd::Function<MxQkv> {
     }
     run_gemms(gemms, count, device);
     if (dx.defined() && gate_cols > 0 && grads[3].defined()) {
-      const Tensor gate = grads[3].to(at::kBFloat16).contiguous();
-      check(mxb200_add_columns(dx.data_ptr(), C, gate.data_ptr(), gate_cols, N, gate_cols, stream()), "fp8_qkv");
+      const Tensor gate = grads[3].contiguous();
+      if (gate.scalar_type() == at::kBFloat16)
+        check(mxb200_add_columns(dx.data_ptr(), C, gate.data_ptr(), gate_cols, N, gate_cols, stream()), "fp8_qkv");
+      else  // of an fp32 input: added in fp32, rounded once
+        dx.narrow(1, 0, gate_cols).add_(gate);
     }
     variable_list out{dx};
     for (Tensor& dw : wgrad.finish())

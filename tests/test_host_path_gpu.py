@@ -182,3 +182,19 @@ def test_function_transforms_are_refused():
         torch.func.vmap(lambda a: nc.fp8_relu_square_mlp(a, w, w, x_mx=q))(x)
     with pytest.raises(RuntimeError):
         torch.func.jvp(lambda a: nc.fp8_relu_square_mlp(a, w, w, x_mx=q), (x[0],), (x[0],))
+
+
+def test_gate_gradient_of_an_fp32_input_is_rounded_once():
+    """The gate's columns of an fp32 x carry an fp32 gradient: dx = bf16(dx of the projections + that gradient)."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(256, 256, generator=g, device="cuda").requires_grad_()
+    w = [(torch.randn(128, 256, generator=g, device="cuda") * 0.06).requires_grad_() for _ in range(3)]
+    dy = [torch.randn(256, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    gate = torch.randn(256, 12, generator=g, device="cuda")
+    grads = []
+    for gate_grad in (torch.zeros_like(gate), gate):
+        x.grad = None
+        torch.autograd.backward(nc.fp8_qkv(x, *w, gate_cols=12), [*dy, gate_grad])
+        grads.append(x.grad)
+    assert torch.equal(grads[1][:, :12], (grads[0][:, :12] + gate).to(torch.bfloat16).float())
+    assert torch.equal(grads[1][:, 12:], grads[0][:, 12:])
