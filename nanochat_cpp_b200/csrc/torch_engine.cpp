@@ -162,7 +162,8 @@ Tensor gemm_bf16(const Layout& a, const Layout& b, int64_t M, int64_t N, int64_t
   return d;
 }
 
-bool grad_direct(const Tensor& w) {  // fp8.h:114-116
+// fp8.h:114-116. The Linears ask in forward: a weight frozen there gets no gradient from that pass, whatever it is in backward.
+bool grad_direct(const Tensor& w) {
   return w.is_leaf() && w.requires_grad() && w.scalar_type() == at::kFloat && w.is_contiguous();
 }
 
@@ -454,6 +455,7 @@ struct Float8Matmul : torch::autograd::Function<Float8Matmul> {
     use->save(saved);
     ctx->save_for_backward(std::move(saved));
     ctx->saved_data["w"] = w;
+    ctx->saved_data["direct"] = grad_direct(w);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -469,7 +471,7 @@ struct Float8Matmul : torch::autograd::Function<Float8Matmul> {
     // the weight gradient first: with K = tokens its tiles are the longer ones of the launch
     mxb200_gemm_desc gemms[2];
     int n = 0;
-    const bool direct = grad_direct(w);
+    const bool direct = ctx->saved_data["direct"].toBool();
     std::optional<WeightGrad> wgrad;
     if (direct || ctx->needs_input_grad(1)) {
       wgrad.emplace(layout_of(g_cols, O, N), layout_of(saved[0], C, N), O, C, N, std::vector<Tensor>{w}, direct, nullptr, device);
@@ -551,6 +553,7 @@ struct MxQkv : torch::autograd::Function<MxQkv> {
     ctx->saved_data["w"] = std::vector<Tensor>{wq, wk, wv};
     ctx->saved_data["gate_cols"] = gate_cols;
     ctx->saved_data["tokens"] = x.size(0);
+    ctx->saved_data["direct"] = grad_direct(wq) && grad_direct(wk) && grad_direct(wv);
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -559,10 +562,10 @@ struct MxQkv : torch::autograd::Function<MxQkv> {
     const int64_t gate_cols = ctx->saved_data["gate_cols"].toInt(), N = ctx->saved_data["tokens"].toInt();
     const auto device = ws[0].device();
     const int64_t C = ws[0].size(1);
+    const bool direct = ctx->saved_data["direct"].toBool();
     int64_t n = 0;
-    bool direct = true;
     for (const Tensor& w : ws)
-      n += w.size(0), direct &= grad_direct(w);
+      n += w.size(0);
     const Tensor g_rows = layout_buffer(N, n, device), g_cols = layout_buffer(n, N, device);
     const Layout g = layout_of(g_rows, N, n), g_t = layout_of(g_cols, n, N);
     QuantizeJobs jobs;

@@ -198,3 +198,19 @@ def test_gate_gradient_of_an_fp32_input_is_rounded_once():
         grads.append(x.grad)
     assert torch.equal(grads[1][:, :12], (grads[0][:, :12] + gate).to(torch.bfloat16).float())
     assert torch.equal(grads[1][:, 12:], grads[0][:, 12:])
+
+
+def test_whether_a_weight_gets_a_gradient_is_decided_in_forward():
+    """Frozen for the forward and thawed before the backward, as the discriminator of a generator's step: no gradient."""
+    x = torch.randn(128, 128, device="cuda").to(torch.bfloat16).requires_grad_()
+    w = [torch.randn(128, 128, device="cuda") for _ in range(3)]
+    for call, used in ((lambda: (nc.fp8_matmul(x, w[0]),), w[:1]), (lambda: nc.fp8_qkv(x, *w), w)):
+        for frozen in (True, False):
+            for t in used:
+                t.requires_grad_(not frozen)
+                t.grad = None
+            out = call()
+            for t in used:
+                t.requires_grad_(frozen)
+            torch.autograd.backward(out, [torch.ones_like(t) for t in out])
+            assert all((t.grad is None) == frozen for t in used)
