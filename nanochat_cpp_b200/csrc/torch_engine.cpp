@@ -256,7 +256,7 @@ class WeightCache {
     if (kind != kind_ || weights.size() != keys_.size())
       return false;
     for (size_t i = 0; i < weights.size(); ++i)
-      if (!(keys_[i] == Key(weights[i])))
+      if (!keys_[i].is(weights[i]))
         return false;
     return true;
   }
@@ -275,13 +275,17 @@ class WeightCache {
   }
 
  private:
+  // The weak reference keeps a dead weight's address from being another tensor's while the key stands.
   struct Key {
-    const void* impl;
+    c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> impl;
     const void* data;
     int64_t version;
     explicit Key(const Tensor& w)
-        : impl(w.unsafeGetTensorImpl()), data(w.data_ptr()), version(static_cast<int64_t>(w._version())) {}
-    bool operator==(const Key& o) const { return impl == o.impl && data == o.data && version == o.version; }
+        : impl(w.getIntrusivePtr()), data(w.data_ptr()), version(static_cast<int64_t>(w._version())) {}
+    bool is(const Tensor& w) const {
+      return impl._unsafe_get_target() == w.unsafeGetTensorImpl() && data == w.data_ptr() &&
+             version == static_cast<int64_t>(w._version());
+    }
   };
   int kind_ = -1;
   std::vector<Key> keys_;
