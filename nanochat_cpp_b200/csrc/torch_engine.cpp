@@ -292,17 +292,44 @@ class WeightCache {
   py::object value_;
 };
 
+// An (R, C) tensor quantized by the caller. The transposed layout is read by the backward only. The scales' type is the
+// caller's: any of one byte.
+Mx given_mx(const std::vector<Tensor>& t, int64_t R, int64_t C, at::Device device, bool grad, const char* what) {
+  const Mx q{t.at(0), t.at(1), t.at(2), t.at(3)};
+  const auto layout = [&](const Tensor& data, const Tensor& scale, int64_t rows, int64_t cols) {
+    for (const Tensor* p : {&data, &scale}) {
+      require_cuda(*p, what);
+      if (p->device() != device || !p->is_contiguous())
+        throw std::runtime_error(std::string(what) + ": expected contiguous operands on the input's device");
+    }
+    if (data.sizes() != at::IntArrayRef{rows, cols} || data.scalar_type() != kE4M3)
+      throw std::runtime_error(std::string(what) + ": shape mismatch");
+    if (scale.numel() != rows * cols / 32 || scale.element_size() != 1)
+      throw std::runtime_error(std::string(what) + ": expected e4m3 operands with their MX scales");
+  };
+  layout(q.data, q.scale, R, C);
+  if (grad)
+    layout(q.data_t, q.scale_t, C, R);
+  return q;
+}
+
 // The quantized copy of a (merged) weight: from the cache when it holds it, else to be quantized by the caller, into
 // `keep` when a cache wants it afterwards and into unnamed buffers otherwise.
 struct WeightUse {
   WeightCache* cache = nullptr;  // null: no caching
   std::vector<Tensor> weights;
-  Mx mx;        // cached, or freshly made for the cache
+  Mx mx;        // cached or given, or freshly made for the cache
   bool ready = false;
   Tensor rows_buffer, cols_buffer;  // without a cache
 
-  WeightUse(WeightCache* c, std::vector<Tensor> ws) : weights(std::move(ws)) {
-    if (c != nullptr && c->enabled) {
+  // `from`: a cache or a list of the four tensors that a cache of another class gave (with the GIL held), or None or null.
+  WeightUse(const py::object* from, std::vector<Tensor> ws, bool grad) : weights(std::move(ws)) {
+    if (from == nullptr || from->is_none())
+      return;
+    if (!py::isinstance<WeightCache>(*from)) {
+      mx = given_mx(from->cast<std::vector<Tensor>>(), out_features(), in_features(), weights[0].device(), grad, "mx_gemm");
+      ready = true;
+    } else if (auto* c = from->cast<WeightCache*>(); c->enabled) {
       cache = c;
       if (c->hit(1, weights))
         mx = c->mx(), ready = true;
@@ -414,27 +441,6 @@ inline bool grad_mode(std::initializer_list<const Tensor*> inputs) {
   return false;
 }
 
-// x (N, C) quantized by the caller. The transposed layout is read by the backward only. The scales' type is the caller's: any
-// of one byte.
-Mx given_mx(const std::vector<Tensor>& t, const Tensor& x, bool grad, const char* what) {
-  const Mx q{t.at(0), t.at(1), t.at(2), t.at(3)};
-  const auto layout = [&](const Tensor& data, const Tensor& scale, int64_t rows, int64_t cols) {
-    for (const Tensor* p : {&data, &scale}) {
-      require_cuda(*p, what);
-      if (p->device() != x.device() || !p->is_contiguous())
-        throw std::runtime_error(std::string(what) + ": expected contiguous operands on the input's device");
-    }
-    if (data.sizes() != at::IntArrayRef{rows, cols} || data.scalar_type() != kE4M3)
-      throw std::runtime_error(std::string(what) + ": shape mismatch");
-    if (scale.numel() != rows * cols / 32 || scale.element_size() != 1)
-      throw std::runtime_error(std::string(what) + ": expected e4m3 operands with their MX scales");
-  };
-  layout(q.data, q.scale, x.size(0), x.size(1));
-  if (grad)
-    layout(q.data_t, q.scale_t, x.size(1), x.size(0));
-  return q;
-}
-
 // One Linear under MX: y = x . w^T, dX = dY . w, dW = dY^T . x, every operand E4M3 with per-32 scales along the
 // contraction (fp8.cpp:240-260).
 Tensor linear_forward(const Tensor& x, WeightUse& w, bool grad, Tensor* x_cols) {
@@ -493,14 +499,15 @@ struct Float8Matmul : torch::autograd::Function<Float8Matmul> {
   }
 };
 
-Tensor fp8_matmul(const Tensor& input, const Tensor& w, WeightCache* cache) {
+Tensor fp8_matmul(const Tensor& input, const Tensor& w, const py::object& cache) {
   require(input.dim() == 2 && w.dim() == 2 && fits(input.size(0), input.size(1)) && fits(w.size(0), w.size(1)),
           "fp8_matmul: MX needs N, in, out % 128");
   require(input.size(1) == w.size(1), "mx_gemm: shape mismatch");
   require_cuda(input, "quantize_mx");
   const Tensor x = input.contiguous();
-  WeightUse use(cache, {w});
-  if (!grad_mode({&x, &w}))
+  const bool grad = grad_mode({&x, &w});
+  WeightUse use(&cache, {w}, grad);
+  if (!grad)
     return linear_forward(x, use, false, nullptr);
   return Float8Matmul::apply(x, w, &use);
 }
@@ -607,7 +614,7 @@ struct MxQkv : torch::autograd::Function<MxQkv> {
 };
 
 variable_list fp8_qkv(const Tensor& x_2d, const Tensor& wq, const Tensor& wk, const Tensor& wv, int64_t gate_cols,
-                      WeightCache* cache, const std::optional<std::vector<Tensor>>& x_mx) {
+                      const py::object& cache, const std::optional<std::vector<Tensor>>& x_mx) {
   bool ok = x_2d.dim() == 2 && fits(x_2d.size(0), x_2d.size(1)) && gate_cols >= 0 && gate_cols <= x_2d.size(1);
   for (const Tensor* w : {&wq, &wk, &wv})
     ok &= w->dim() == 2 && w->size(0) % 128 == 0;
@@ -617,8 +624,8 @@ variable_list fp8_qkv(const Tensor& x_2d, const Tensor& wq, const Tensor& wk, co
   require_cuda(x_2d, "quantize_mx");
   const Tensor x = x_2d.contiguous();
   const bool grad = grad_mode({&x, &wq, &wk, &wv});
-  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x, grad, "mx_gemm") : Mx{};
-  WeightUse use(cache, {wq, wk, wv});
+  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x.size(0), x.size(1), x.device(), grad, "mx_gemm") : Mx{};
+  WeightUse use(&cache, {wq, wk, wv}, grad);
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
   if (!grad)
     return qkv_forward(x, use, gate_cols, mx, false, nullptr);
@@ -724,8 +731,8 @@ struct Fp8ReluSquareMlp : torch::autograd::Function<Fp8ReluSquareMlp> {
   }
 };
 
-Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor& w_proj, WeightCache* fc_cache,
-                           WeightCache* proj_cache, const std::optional<std::vector<Tensor>>& x_mx) {
+Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor& w_proj, const py::object& fc_cache,
+                           const py::object& proj_cache, const std::optional<std::vector<Tensor>>& x_mx) {
   require(x_2d.dim() == 2 && w_fc.dim() == 2 && w_proj.dim() == 2 && fits(x_2d.size(0), x_2d.size(1)) &&
                 fits(w_fc.size(0), w_fc.size(1)) && fits(w_proj.size(0), w_proj.size(1)) &&
                 w_fc.size(1) == x_2d.size(1) && w_proj.size(1) == w_fc.size(0),
@@ -733,8 +740,8 @@ Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor&
   require_cuda(x_2d, "quantize_mx");
   const Tensor x = x_2d.contiguous();
   const bool grad = grad_mode({&x, &w_fc, &w_proj});
-  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x, grad, "mx_gemm_relu_square") : Mx{};
-  WeightUse fc(fc_cache, {w_fc}), proj(proj_cache, {w_proj});
+  const Mx given = x_mx.has_value() ? given_mx(*x_mx, x.size(0), x.size(1), x.device(), grad, "mx_gemm_relu_square") : Mx{};
+  WeightUse fc(&fc_cache, {w_fc}, grad), proj(&proj_cache, {w_proj}, grad);
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
   if (!grad)
     return mlp_forward(x, fc, proj, mx, false, nullptr);
@@ -926,10 +933,11 @@ struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
     if (cache != ctx->saved_data.end()) {
       py::gil_scoped_acquire gil;
       auto* holder = static_cast<CacheHolder*>(cache->second.toCapsule().get());
-      WeightUse use(py::handle(holder->object).cast<WeightCache*>(), {weight});
+      const auto object = py::reinterpret_borrow<py::object>(holder->object);
+      WeightUse use(&object, {weight}, true);
       run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
     } else {
-      WeightUse use(nullptr, {weight});
+      WeightUse use(nullptr, {weight}, true);
       run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
     }
     WeightGrad wgrad(layout_of(g_cols, V, N), layout_of(x_cols, C, N), V, C, N, {weight}, false, nullptr, device);
@@ -942,11 +950,10 @@ Tensor softcap_cross_entropy(const Tensor& x_in, const Tensor& weight, const Ten
                              double softcap, int64_t chunk_rows, int reduction, py::object cache_object) {
   const Tensor x = x_in.contiguous(), targets = targets_in.to(at::kLong).contiguous();
   require_cuda(targets, "softcap_cross_entropy");
-  auto* cache = cache_object.is_none() ? nullptr : cache_object.cast<WeightCache*>();
   const LossArgs args{vocab, chunk_rows, softcap};
-  WeightUse use(cache, {weight});
-  const bool mean = reduction == 0, none = reduction == 2;
-  if (grad_mode({&x, &weight}))
+  const bool mean = reduction == 0, none = reduction == 2, grad = grad_mode({&x, &weight});
+  WeightUse use(&cache_object, {weight}, grad);
+  if (grad)
     return none ? SoftcapPerToken::apply(x, weight, targets, &args, &use, &cache_object)
                 : SoftcapReduced::apply(x, weight, targets, &args, mean, &use);
   const Tensor losses = empty({x.size(0)}, at::kFloat, x.device());

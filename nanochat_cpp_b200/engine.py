@@ -216,7 +216,17 @@ class Fp8WeightCache(native.WeightCache):
         super().__init__(enabled)
 
     def __reduce__(self):  # a copy starts empty
-        return Fp8WeightCache, (self.enabled,)
+        return type(self), (self.enabled,), vars(self) or None
+
+
+def _weight_source(cache, *weights):
+    """What the native functions take for the quantized copy of (merged) weights: None or the native cache itself, or the
+    four tensors that the get() of any other cache, or of a subclass, returns."""
+    if cache is None or type(cache) is Fp8WeightCache or getattr(type(cache), "get", None) is native.WeightCache.get:
+        return cache
+    if len(weights) == 3:
+        return list(mx_qkv_weights(*weights, cache))
+    return _mx_list(quantize_fp8_weight(*weights, cache))
 
 
 def quantize_fp8_weight(w: torch.Tensor, cache: Optional[Fp8WeightCache] = None) -> Fp8Tensor:
@@ -442,7 +452,7 @@ def fp8_qkv(x_2d: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, wv: torch.Te
     gate's columns only."""
     if x_mx is not None and (x_mx.data is None or x_mx.data_t is None):
         raise RuntimeError("fp8_qkv: x_mx needs both layouts")
-    return tuple(native.fp8_qkv(x_2d, wq, wk, wv, gate_cols, cache, _mx_list(x_mx)))
+    return tuple(native.fp8_qkv(x_2d, wq, wk, wv, gate_cols, _weight_source(cache, wq, wk, wv), _mx_list(x_mx)))
 
 
 def relu_square_mlp_mx(N: int, cin: int, w_fc: torch.Tensor, w_proj: torch.Tensor) -> bool:
@@ -460,14 +470,15 @@ def fp8_relu_square_mlp(x_2d: torch.Tensor, w_fc: torch.Tensor, w_proj: torch.Te
     x_mx: x_2d already quantized in both layouts (residual_norm_mx); x_2d then only carries autograd."""
     if x_mx is not None and (x_mx.data is None or x_mx.data_t is None):
         raise RuntimeError("fp8_relu_square_mlp: x_mx needs both layouts")
-    return native.fp8_relu_square_mlp(x_2d, w_fc, w_proj, fc_cache, proj_cache, _mx_list(x_mx))
+    return native.fp8_relu_square_mlp(x_2d, w_fc, w_proj, _weight_source(fc_cache, w_fc),
+                                      _weight_source(proj_cache, w_proj), _mx_list(x_mx))
 
 
 def fp8_matmul(input_2d: torch.Tensor, weight: torch.Tensor, cache: Optional[Fp8WeightCache] = None) -> torch.Tensor:
     """input_2d (N, in) bf16, weight (out, in) -> (N, out) bf16 under the MX recipe
     (src/nanochat/model/fp8/fp8.h:40-44, fp8.cpp:566-571). Dims must be % 128: the reference falls back to its
     tensorwise recipe otherwise, which is outside this library."""
-    return native.fp8_matmul(input_2d, weight, cache)
+    return native.fp8_matmul(input_2d, weight, _weight_source(cache, weight))
 
 
 # ------------------------------------------------------------------------------------------------ chunked lm_head loss
@@ -532,4 +543,4 @@ def softcap_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.
             and weight.size(0) >= vocab_size and weight.size(1) == x.size(1)):
         raise RuntimeError("softcap_cross_entropy: MX needs N, C, chunk_rows and the padded vocab % 128")
     return native.softcap_cross_entropy(x, weight, targets, int(vocab_size), float(softcap), int(chunk_rows),
-                                        ("mean", "sum", "none").index(reduction), cache)
+                                        ("mean", "sum", "none").index(reduction), _weight_source(cache, weight))

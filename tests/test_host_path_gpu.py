@@ -214,3 +214,56 @@ def test_whether_a_weight_gets_a_gradient_is_decided_in_forward():
                 t.requires_grad_(frozen)
             torch.autograd.backward(out, [torch.ones_like(t) for t in out])
             assert all((t.grad is None) == frozen for t in used)
+
+
+class _Counting(nc.Fp8WeightCache):
+    def __init__(self, enabled=False):
+        super().__init__(enabled)
+        self.asked = []
+
+    def get(self, kind, weights, make):
+        self.asked.append((kind, len(weights)))
+        return super().get(kind, weights, make)
+
+
+class _Plain:
+    """A cache that is none of the library's classes."""
+
+    def __init__(self):
+        self.value, self.asked = None, []
+
+    def get(self, kind, weights, make):
+        self.asked.append((kind, len(weights)))
+        self.value = make() if self.value is None else self.value
+        return self.value
+
+
+@pytest.mark.parametrize("cls", [lambda: _Counting(True), _Plain])
+def test_any_cache_is_asked_through_its_get(cls):
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.randn(128, 256, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(256, 256, generator=g, device="cuda")
+    t = torch.randint(0, 256, (128,), generator=g, device="cuda")
+    calls = {
+        "matmul": (lambda x, w, c: nc.fp8_matmul(x, w, c), [(1, 1)]),
+        "qkv": (lambda x, w, c: torch.cat(nc.fp8_qkv(x, w, w[:128], w[128:], cache=c), 1), [(1, 3)]),
+        "mlp": (lambda x, w, c: nc.fp8_relu_square_mlp(x, w, w, c, None), [(1, 1)]),
+        "loss": (lambda x, w, c: nc.softcap_cross_entropy(x, w, t, 256, 15.0, 128, "none", c), [(1, 1)]),
+    }
+    for name, (call, asked) in calls.items():
+        got = []
+        for cache in (None, cls()):
+            a, b = x.clone().requires_grad_(), w.clone().requires_grad_()
+            out = call(a, b, cache)
+            out.backward(torch.ones_like(out))
+            got.append((out, a.grad, b.grad))
+        assert cache.asked[:1] == asked, name
+        assert all(torch.equal(u, v) for u, v in zip(*got)), name
+
+
+def test_a_copied_cache_is_empty_and_of_its_class():
+    import copy
+    cache = _Counting(True)
+    cache.get(1, [torch.zeros(1)], lambda: [1])
+    other = copy.deepcopy(cache)
+    assert type(other) is _Counting and other.enabled and other.asked == [(1, 1)]
