@@ -6,7 +6,8 @@
 // ctypes call and a handful of tensor objects per launch cost the host 30 to 50 us each, so every shape up to a few
 // thousand tokens was bound by the host (fp8_matmul of 2048 x 768 -> 3072, forward and backward: 59 us of kernels in a
 // 250 us pass). Here a call costs a few allocations from torch's caching allocator and the launches. Tensors that
-// nobody outside sees (quantized operands) are one byte buffer per lifetime, data then scales.
+// nobody outside sees (quantized operands) are one byte buffer per lifetime, data then scales. The launches run without the
+// GIL: a full launch queue blocks its own thread only, and threads that drive several GPUs do not wait for one another.
 #include <optional>
 #include <stdexcept>
 #include <utility>
@@ -373,6 +374,7 @@ struct WeightUse {
   }
   void publish() {
     if (cache != nullptr && !ready) {
+      py::gil_scoped_acquire gil;
       py::list l;
       for (const Tensor& t : {mx.data, mx.data_t, mx.scale, mx.scale_t})
         l.append(py::cast(t));
@@ -507,6 +509,7 @@ Tensor fp8_matmul(const Tensor& input, const Tensor& w, const py::object& cache)
   const Tensor x = input.contiguous();
   const bool grad = grad_mode({&x, &w});
   WeightUse use(&cache, {w}, grad);
+  const py::gil_scoped_release nogil;
   if (!grad)
     return linear_forward(x, use, false, nullptr);
   return Float8Matmul::apply(x, w, &use);
@@ -627,6 +630,7 @@ variable_list fp8_qkv(const Tensor& x_2d, const Tensor& wq, const Tensor& wk, co
   const Mx given = x_mx.has_value() ? given_mx(*x_mx, x.size(0), x.size(1), x.device(), grad, "mx_gemm") : Mx{};
   WeightUse use(&cache, {wq, wk, wv}, grad);
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
+  const py::gil_scoped_release nogil;
   if (!grad)
     return qkv_forward(x, use, gate_cols, mx, false, nullptr);
   return MxQkv::apply(x, wq, wk, wv, gate_cols, &use, mx);
@@ -743,6 +747,7 @@ Tensor fp8_relu_square_mlp(const Tensor& x_2d, const Tensor& w_fc, const Tensor&
   const Mx given = x_mx.has_value() ? given_mx(*x_mx, x.size(0), x.size(1), x.device(), grad, "mx_gemm_relu_square") : Mx{};
   WeightUse fc(&fc_cache, {w_fc}, grad), proj(&proj_cache, {w_proj}, grad);
   const Mx* mx = x_mx.has_value() ? &given : nullptr;
+  const py::gil_scoped_release nogil;
   if (!grad)
     return mlp_forward(x, fc, proj, mx, false, nullptr);
   return Fp8ReluSquareMlp::apply(x, w_fc, w_proj, &fc, &proj, mx);
@@ -902,7 +907,7 @@ struct CacheHolder : torch::CustomClassHolder {
 // Reduction none: the backward re-runs the chunks with the per-row gradient.
 struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& targets,
-                        const LossArgs* args, WeightUse* use, py::object* cache) {
+                        const LossArgs* args, WeightUse* use, const py::object* cache) {
     const Tensor losses = empty({x.size(0)}, at::kFloat, x.device());
     ChunkOutputs out;
     out.losses = static_cast<float*>(losses.data_ptr());
@@ -911,8 +916,10 @@ struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
     ctx->saved_data["vocab"] = args->vocab;
     ctx->saved_data["chunk_rows"] = args->chunk_rows;
     ctx->saved_data["softcap"] = args->softcap;
-    if (!cache->is_none())
+    if (!cache->is_none()) {
+      py::gil_scoped_acquire gil;
       ctx->saved_data["cache"] = c10::IValue::make_capsule(c10::make_intrusive<CacheHolder>(*cache));
+    }
     return losses;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -929,17 +936,15 @@ struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
     out.grad_scale = static_cast<const float*>(g.data_ptr());
     out.grad_scale_stride = 1;
     Tensor x_cols, g_cols;
-    const auto cache = ctx->saved_data.find("cache");
-    if (cache != ctx->saved_data.end()) {
+    std::optional<WeightUse> use;
+    if (const auto cache = ctx->saved_data.find("cache"); cache != ctx->saved_data.end()) {
       py::gil_scoped_acquire gil;
-      auto* holder = static_cast<CacheHolder*>(cache->second.toCapsule().get());
-      const auto object = py::reinterpret_borrow<py::object>(holder->object);
-      WeightUse use(&object, {weight}, true);
-      run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
+      const auto object = py::reinterpret_borrow<py::object>(static_cast<CacheHolder*>(cache->second.toCapsule().get())->object);
+      use.emplace(&object, std::vector<Tensor>{weight}, true);
     } else {
-      WeightUse use(nullptr, {weight}, true);
-      run_chunks(x, use, targets, args, out, &x_cols, &g_cols);
+      use.emplace(nullptr, std::vector<Tensor>{weight}, true);
     }
+    run_chunks(x, *use, targets, args, out, &x_cols, &g_cols);
     WeightGrad wgrad(layout_of(g_cols, V, N), layout_of(x_cols, C, N), V, C, N, {weight}, false, nullptr, device);
     run_gemms(&wgrad.desc(), 1, device);
     return {grad_x, wgrad.finish()[0], Tensor(), Tensor(), Tensor(), Tensor()};
@@ -947,12 +952,13 @@ struct SoftcapPerToken : torch::autograd::Function<SoftcapPerToken> {
 };
 
 Tensor softcap_cross_entropy(const Tensor& x_in, const Tensor& weight, const Tensor& targets_in, int64_t vocab,
-                             double softcap, int64_t chunk_rows, int reduction, py::object cache_object) {
+                             double softcap, int64_t chunk_rows, int reduction, const py::object& cache_object) {
   const Tensor x = x_in.contiguous(), targets = targets_in.to(at::kLong).contiguous();
   require_cuda(targets, "softcap_cross_entropy");
   const LossArgs args{vocab, chunk_rows, softcap};
   const bool mean = reduction == 0, none = reduction == 2, grad = grad_mode({&x, &weight});
   WeightUse use(&cache_object, {weight}, grad);
+  const py::gil_scoped_release nogil;
   if (grad)
     return none ? SoftcapPerToken::apply(x, weight, targets, &args, &use, &cache_object)
                 : SoftcapReduced::apply(x, weight, targets, &args, mean, &use);
@@ -1032,6 +1038,7 @@ void quantize_mx_batch_into(const py::sequence& jobs, int scale_rule) {
             "MX: expected aligned, contiguous 2D tensors of one dtype with dims % 128");
     list.push_back({x.data_ptr(), x.size(0), x.size(1), mx_out_of(po.ptr()), mx_out_of(pt.ptr())});
   }
+  const py::gil_scoped_release nogil;
   check(mxb200_quantize_mx_batch(list.data(), static_cast<int>(count), *dtype == at::kBFloat16, scale_rule, stream()),
         "quantize_mx_batch");
 }
@@ -1058,6 +1065,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("fp8_qkv", &fp8_qkv);
   m.def("fp8_relu_square_mlp", &fp8_relu_square_mlp);
   m.def("softcap_cross_entropy", &softcap_cross_entropy);
-  m.def("residual_norm_mx", &residual_norm_mx);
+  m.def("residual_norm_mx", &residual_norm_mx, py::call_guard<py::gil_scoped_release>());
   m.def("quantize_mx_batch_into", &quantize_mx_batch_into);
 }

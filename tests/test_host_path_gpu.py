@@ -267,3 +267,36 @@ def test_a_copied_cache_is_empty_and_of_its_class():
     cache.get(1, [torch.zeros(1)], lambda: [1])
     other = copy.deepcopy(cache)
     assert type(other) is _Counting and other.enabled and other.asked == [(1, 1)]
+
+
+def test_calls_let_other_python_threads_run():
+    """Nothing else hands the interpreter over for 100 seconds: the other thread runs when a call gives it up."""
+    import sys
+    import threading
+    x = torch.randn(128, 128, device="cuda").to(torch.bfloat16)
+    w = torch.randn(128, 128, device="cuda")
+    t = torch.zeros(128, dtype=torch.int64, device="cuda")
+    q = nc.quantize_mx(w)
+    outs = nc.mx_outs(q)
+    calls = [lambda: nc.fp8_matmul(x, w), lambda: nc.fp8_qkv(x, w, w, w), lambda: nc.fp8_relu_square_mlp(x, w, w),
+             lambda: nc.softcap_cross_entropy(x, w, t, 128, 15.0, 128), lambda: nc.residual_norm_mx(x),
+             lambda: nc.quantize_mx_batch_into([(w, *outs)])]
+    interval = sys.getswitchinterval()
+    for call in calls:
+        call()
+        torch.cuda.synchronize()
+        ran, start = [], threading.Event()
+        thread = threading.Thread(target=lambda: (start.wait(), ran.append(True)))
+        thread.start()
+        sys.setswitchinterval(100.0)
+        try:
+            start.set()
+            for _ in range(500):
+                call()
+                if ran:
+                    break
+        finally:
+            sys.setswitchinterval(interval)
+        seen = bool(ran)
+        thread.join()
+        assert seen
