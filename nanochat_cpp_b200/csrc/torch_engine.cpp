@@ -18,6 +18,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/util/SmallVector.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
 
 #include "mxb200.h"
@@ -33,18 +34,20 @@ constexpr auto kE8M0 = at::kFloat8_e8m0fnu;
 
 // ---------------------------------------------------------------------------------------------------- plumbing
 
-struct StatusError : std::runtime_error {
-  int status;
-  std::string what_failed;
-  StatusError(int s, const char* w)
-      : std::runtime_error(std::string(w) + ": " + mxb200_strerror(s) + " (status " + std::to_string(s) + ")"),
-        status(s),
-        what_failed(w) {}
-};
+// The library's status as the Python error it is everywhere (capi.Mxb200Error), from an autograd worker's thread too.
+[[noreturn]] void raise_status(int status, const char* what) {
+  py::gil_scoped_acquire gil;
+  const py::object type = py::module_::import("nanochat_cpp_b200.capi").attr("Mxb200Error");
+  const py::object error = type(status, what);
+  PyErr_SetObject(type.ptr(), error.ptr());
+  python_error e;
+  e.persist();
+  throw e;
+}
 
 inline void check(int status, const char* what) {
   if (status != MXB200_OK)
-    throw StatusError(status, what);
+    raise_status(status, what);
 }
 
 [[noreturn]] void fail(const char* message) {
@@ -1051,10 +1054,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     try {
       if (p)
         std::rethrow_exception(p);
-    } catch (const StatusError& e) {
-      const py::object type = py::module_::import("nanochat_cpp_b200.capi").attr("Mxb200Error");
-      const py::object error = type(e.status, e.what_failed);
-      PyErr_SetObject(type.ptr(), error.ptr());
+    } catch (python_error& e) {
+      e.restore();
     }
   });
   py::class_<WeightCache>(m, "WeightCache")

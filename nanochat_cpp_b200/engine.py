@@ -222,7 +222,7 @@ class Fp8WeightCache(native.WeightCache):
 def _weight_source(cache, *weights):
     """What the native functions take for the quantized copy of (merged) weights: None or the native cache itself, or the
     four tensors that the get() of any other cache, or of a subclass, returns."""
-    if cache is None or type(cache) is Fp8WeightCache or getattr(type(cache), "get", None) is native.WeightCache.get:
+    if cache is None or getattr(type(cache), "get", None) is native.WeightCache.get:
         return cache
     if len(weights) == 3:
         return list(mx_qkv_weights(*weights, cache))
@@ -478,7 +478,9 @@ def fp8_matmul(input_2d: torch.Tensor, weight: torch.Tensor, cache: Optional[Fp8
     """input_2d (N, in) bf16, weight (out, in) -> (N, out) bf16 under the MX recipe
     (src/nanochat/model/fp8/fp8.h:40-44, fp8.cpp:566-571). Dims must be % 128: the reference falls back to its
     tensorwise recipe otherwise, which is outside this library."""
-    return native.fp8_matmul(input_2d, weight, _weight_source(cache, weight))
+    if cache is not None and type(cache) is not Fp8WeightCache:
+        cache = _weight_source(cache, weight)
+    return native.fp8_matmul(input_2d, weight, cache)
 
 
 # ------------------------------------------------------------------------------------------------ chunked lm_head loss

@@ -300,3 +300,19 @@ def test_calls_let_other_python_threads_run():
         seen = bool(ran)
         thread.join()
         assert seen
+
+
+def test_a_refusal_is_the_librarys_error_in_forward_and_backward():
+    """An operand off its 16 bytes is refused on the host; its status is the error's, also from autograd's worker."""
+    def off(t):  # contiguous, two bytes past an aligned address
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+    x = torch.randn(128, 128, device="cuda").to(torch.bfloat16)
+    w = torch.randn(128, 128, device="cuda").requires_grad_()
+    for call in (lambda a: nc.fp8_matmul(a, w), lambda a: nc.fp8_relu_square_mlp(a, w, w), lambda a: nc.fp8_qkv(a, w, w, w)[0]):
+        with pytest.raises(nc.capi.Mxb200Error) as forward:
+            call(off(x))
+        y = call(x)
+        with pytest.raises(nc.capi.Mxb200Error) as backward:
+            y.backward(off(torch.ones_like(y)))
+        assert forward.value.status == backward.value.status == nc.capi.ERR_ALIGNMENT
+        assert "quantize_mx" in str(backward.value)
