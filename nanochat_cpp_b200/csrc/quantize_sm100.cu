@@ -18,7 +18,6 @@
 // tile ahead, and the same in three groups around a shared table for the softcap gradient.
 // HBM traffic is the algorithmic minimum: every input byte read once, every output byte written once.
 #include <algorithm>
-#include <vector>
 
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -1035,6 +1034,17 @@ int launch_softcap(const QuantParams& p, int64_t rows, int64_t cols, int64_t til
 
 using Item = mxb200_quantize_item;
 
+// A caller's list from some member on: of items, or of jobs of one input type.
+struct ItemList {
+  const Item* items;
+  const mxb200_quantize_job* jobs;
+  int32_t x_bf16;
+  Item operator[](int i) const { return items != nullptr ? items[i] : Item{jobs[i], x_bf16}; }
+  ItemList from(int i) const {
+    return {items != nullptr ? items + i : nullptr, jobs != nullptr ? jobs + i : nullptr, x_bf16};
+  }
+};
+
 bool asked(const Item& i) {
   return i.job.out.data != nullptr || i.job.out_t.data != nullptr;
 }
@@ -1057,7 +1067,7 @@ constexpr auto stream_kernel() {
 
 // Streams up to kMaxJobs of the items, from the front; `taken`: how many it went over.
 template <int kMaxJobs>
-int launch_stream(const Item* items, int n, int* taken, bool floor_rule, int sms, cudaStream_t stream) {
+int launch_stream(const ItemList& items, int n, int* taken, bool floor_rule, int sms, cudaStream_t stream) {
   constexpr auto kernel = stream_kernel<kMaxJobs>();
   static std::atomic<int> configured_for{-1};
   if (int s = configure_once(kernel, kStreamGroupBytes, configured_for); s != MXB200_OK)
@@ -1067,7 +1077,7 @@ int launch_stream(const Item* items, int n, int* taken, bool floor_rule, int sms
   int64_t units = 0;
   int i = 0;
   for (; i < n && b.n < kMaxJobs; ++i) {
-    const Item& it = items[i];
+    const Item it = items[i];
     if (!asked(it))
       continue;
     const bool f32 = it.x_bf16 == 0;
@@ -1105,21 +1115,22 @@ int launch_batch(const BatchParams& bp, int tiles, cudaStream_t stream) {
 // More input than the CTA-per-tile form holds at once (four CTAs per SM of bf16 tiles, two of fp32) streams through
 // persistent CTAs: those forms would run in several waves, each reading, computing and writing in turn. Below that the
 // CTA-per-tile form starts sooner: it needs no tensor map, no draw and no barrier before its first load.
-int quantize_items(const Item* items, int n, bool floor_rule, const DeviceInfo& dev, cudaStream_t stream) {
+int quantize_items(const ItemList& items, int n, bool floor_rule, const DeviceInfo& dev, cudaStream_t stream) {
   int64_t stages = 0;
   bool bf16 = false, f32 = false;
   for (int i = 0; i < n; ++i) {
-    if (!asked(items[i]))
+    const Item it = items[i];
+    if (!asked(it))
       continue;
-    stages += tiles_of(items[i]) * (items[i].x_bf16 != 0 ? 1 : 2);
-    (items[i].x_bf16 != 0 ? bf16 : f32) = true;
+    stages += tiles_of(it) * (it.x_bf16 != 0 ? 1 : 2);
+    (it.x_bf16 != 0 ? bf16 : f32) = true;
   }
   int i = 0;
   if (stages > 4 * static_cast<int64_t>(dev.sms)) {
     while (i < n) {
       int taken = 0;
-      const int st = n - i <= kFewJobs ? launch_stream<kFewJobs>(items + i, n - i, &taken, floor_rule, dev.sms, stream)
-                                       : launch_stream<kManyJobs>(items + i, n - i, &taken, floor_rule, dev.sms, stream);
+      const int st = n - i <= kFewJobs ? launch_stream<kFewJobs>(items.from(i), n - i, &taken, floor_rule, dev.sms, stream)
+                                       : launch_stream<kManyJobs>(items.from(i), n - i, &taken, floor_rule, dev.sms, stream);
       if (st != MXB200_OK)
         return st;
       i += taken;
@@ -1131,7 +1142,7 @@ int quantize_items(const Item* items, int n, bool floor_rule, const DeviceInfo& 
     bp.floor_rule = floor_rule;
     int tiles = 0;
     for (; i < n && bp.n < kMaxBatch; ++i) {
-      const Item& it = items[i];
+      const Item it = items[i];
       if (!asked(it))
         continue;
       bp.jobs[bp.n++] = BatchJob{it.job.x, it.job.cols, it.job.out, it.job.out_t, static_cast<int>(it.job.cols / kTile), tiles,
@@ -1183,7 +1194,7 @@ int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t co
   auto* s = static_cast<cudaStream_t>(stream);
   if (pro == kNone) {
     const Item item{{x, rows, cols, out, out_t}, x_bf16 ? 1 : 0};
-    return quantize_items(&item, 1, p.floor_rule, dev, s);
+    return quantize_items({&item, nullptr, 0}, 1, p.floor_rule, dev, s);
   }
   switch (pro) {
     case kReluSquare:
@@ -1197,17 +1208,17 @@ int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t co
   }
 }
 
-int quantize_list(const Item* items, int n, int scale_rule, void* stream) {
+int quantize_list(const ItemList& items, int n, int scale_rule, void* stream) {
   DeviceInfo dev;
   if (int s = current_device(&dev); s != MXB200_OK)
     return s;
-  if (n < 0 || (n > 0 && items == nullptr))
+  if (n < 0 || (n > 0 && items.items == nullptr && items.jobs == nullptr))
     return MXB200_ERR_NULL;
   if (scale_rule != MXB200_SCALE_REFERENCE && scale_rule != MXB200_SCALE_OCP_FLOOR)
     return MXB200_ERR_ARGUMENT;
   // every one is checked before anything is launched
   for (int i = 0; i < n; ++i) {
-    const mxb200_quantize_job& j = items[i].job;
+    const mxb200_quantize_job j = items[i].job;
     if (j.x == nullptr)
       return MXB200_ERR_NULL;
     if (j.rows <= 0 || j.cols <= 0 || j.rows % kTile != 0 || j.cols % kTile != 0 ||
@@ -1271,17 +1282,12 @@ extern "C" int mxb200_add_columns(void* dst, int64_t dst_ld, const void* src, in
 }
 
 extern "C" int mxb200_quantize_mx_items(const mxb200_quantize_item* items, int n, int scale_rule, void* stream) {
-  return mxb200::quantize_list(items, n, scale_rule, stream);
+  return mxb200::quantize_list({items, nullptr, 0}, n, scale_rule, stream);
 }
 
 extern "C" int mxb200_quantize_mx_batch(const mxb200_quantize_job* jobs, int n_jobs, int x_bf16, int scale_rule,
                                         void* stream) {
-  if (n_jobs > 0 && jobs == nullptr)
-    return mxb200::quantize_list(nullptr, n_jobs, scale_rule, stream);
-  std::vector<mxb200_quantize_item> items(static_cast<size_t>(std::max(n_jobs, 0)));
-  for (int i = 0; i < n_jobs; ++i)
-    items[i] = {jobs[i], x_bf16 != 0};
-  return mxb200::quantize_list(items.data(), n_jobs, scale_rule, stream);
+  return mxb200::quantize_list({nullptr, jobs, x_bf16 != 0}, n_jobs, scale_rule, stream);
 }
 
 extern "C" int mxb200_quantize_mx(const void* x, int x_bf16, int64_t rows, int64_t cols, mxb200_mx_out out,
