@@ -1167,7 +1167,8 @@ int quantize(const void* x, const void* h, bool x_bf16, int64_t rows, int64_t co
     return s;
   if (x == nullptr || (pro == kReluSquareBwd && h == nullptr))
     return MXB200_ERR_NULL;
-  if (rows <= 0 || cols <= 0 || rows % kTile != 0 || cols % kTile != 0 || rows * cols / (kTile * kTile) > 0x7fffffffLL)
+  const int64_t most_tiles = x_bf16 ? 0x7fffffffLL : 0x3fffffffLL;  // an fp32 tile is two units of a launch
+  if (rows <= 0 || cols <= 0 || rows % kTile != 0 || cols % kTile != 0 || rows * cols / (kTile * kTile) > most_tiles)
     return MXB200_ERR_SHAPE;
   if (scale_rule != MXB200_SCALE_REFERENCE && scale_rule != MXB200_SCALE_OCP_FLOOR)
     return MXB200_ERR_ARGUMENT;
