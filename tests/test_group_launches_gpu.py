@@ -68,8 +68,9 @@ GROUPS = [
 
 @pytest.mark.parametrize("shapes", GROUPS, ids=len)
 @pytest.mark.parametrize("tile_n", [0, 128, 256, 384, 512, 640])
-def test_gemm_group(shapes, tile_n):
-    lib.mxb200_set_gemm_config(tile_n, 0)
+@pytest.mark.parametrize("max_ctas", [0, 4])  # 4: a CTA (or pair) goes from one member to the next, several times
+def test_gemm_group(shapes, tile_n, max_ctas):
+    lib.mxb200_set_gemm_config(tile_n, max_ctas)
     problems, wants = [], []
     for i, (M, N, K) in enumerate(shapes):
         qa, qb = operand(M, K, 2 * i), operand(N, K, 2 * i + 1)
