@@ -56,9 +56,22 @@ def _run(cmd: list, what: str, verbose: bool) -> None:
         raise RuntimeError(f"{what} failed")
 
 
+def _built_for() -> str:
+    """What _torch_engine.so depends on beside its sources, as it is compiled into it: torch's and Python's C++ interfaces."""
+    import torch
+    return f"mxb200-engine-for torch {torch.__version__} {sysconfig.get_config_var('SOABI')};"
+
+
+def _engine_stale() -> bool:
+    if _stale(ENGINE, [ENGINE_SOURCE]):
+        return True
+    with open(ENGINE, "rb") as f:
+        return _built_for().encode() not in f.read()
+
+
 def build_engine(force: bool = False, verbose: bool = False) -> str:
     """The torch extension; needs libmxb200.so beside it (found again at run time through $ORIGIN)."""
-    if not force and not _stale(ENGINE, [ENGINE_SOURCE]):
+    if not force and not _engine_stale():
         return ENGINE
     import torch
     tdir = os.path.dirname(torch.__file__)
@@ -68,7 +81,8 @@ def build_engine(force: bool = False, verbose: bool = False) -> str:
            sysconfig.get_paths()["include"]]
     tmp = f"{ENGINE}.{os.getpid()}"
     _run(["g++", "-std=c++20", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_torch_engine",
-          "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          "-DTORCH_API_INCLUDE_EXTENSION_H", f'-DMXB200_BUILT_FOR="{_built_for()}"',
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
           *(x for d in inc for x in ("-isystem" if d.startswith(tdir) else "-I", d)), ENGINE_SOURCE, "-o", tmp,
           "-L", HERE, "-l:libmxb200.so", "-L", os.path.join(tdir, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu",
           "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], "build of _torch_engine.so", verbose)

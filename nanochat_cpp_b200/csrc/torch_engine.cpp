@@ -1050,6 +1050,7 @@ void quantize_mx_batch_into(const py::sequence& jobs, int scale_rule) {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "Native host path of nanochat_cpp_b200.engine.";
+  m.attr("built_for") = MXB200_BUILT_FOR;  // build.py looks for it in the file
   py::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p)
