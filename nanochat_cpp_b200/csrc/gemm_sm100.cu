@@ -1500,19 +1500,22 @@ double launch_cycles(const GemmDesc* g, int n, const TileKind& t, const int* spl
 
 // K slices of a GEMM, from its shape and the machine alone: neither the GEMMs that share its launch, nor its output's type, nor
 // whether it accumulates have a say, so that the order of its fp32 sum, and with it every bit, is that of the same GEMM by
-// itself. Slices cost a round trip of fp32 matrices and a launch, so they are for what fills at most a quarter of the machine
-// and leaves each slice 32 K steps: 768 x 768 x 16384 takes 28.0 us in one, 17.4 in four, 768 x 768 x 8192 16.4 in one, 13.8 in
-// two. Just past the line they gain less (768 x 1536 x 16384 28.6 and 23.1 in four, 768 x 768 x 4096 10.5 and 9.7, 2048 x 768 x
-// 32768 60.0 and 49.6 in two), too little to give these shapes another order of summation.
+// itself. Slices cost a round trip of fp32 matrices and a launch.
+//   K from 8192 on: for what fills at most a quarter of the machine, as long as a slice keeps 32 K steps. 768 x 768 x 16384 takes
+//   28.0 us in one, 17.4 in four, 768 x 768 x 8192 16.4 in one, 13.8 in two. Just past the line they gain less (768 x 1536 x
+//   16384 28.6 and 23.1 in four, 2048 x 768 x 32768 60.0 and 49.6 in two): too little to give these another order of summation.
+//   K from 4096: for as many slices as fit the machine in one 128 x 128 tile per SM (few tokens through a wide layer). 128 x 1536
+//   x 6144 takes 16.3 us in one, 9.9 in four, 512 x 1536 x 6144 13.4 in one, 12.5 in two, 14.3 in four.
+//   Below, a slice is too short: 256 x 768 x 3072 takes 8.8 us in one, 9.1 in two, 128 x 512 x 2048 7.5 and 7.9.
 int plan_splits(int64_t M, int64_t N, int64_t K, int sms) {
-  const bool pair = M >= 256 && N >= 256;
-  const int64_t tile_m = pair ? 256 : 128, tile_n = pair ? 192 : N >= 256 ? 256 : 128;
-  const int64_t slots = pair ? sms / 2 : sms;
-  if (M <= 0 || N <= 0 || K <= 0)
+  if (M <= 0 || N <= 0 || K < 4096)
     return 1;
+  const bool deep = K >= 8192, pair = deep && M >= 256 && N >= 256;
+  const int64_t tile_m = pair ? 256 : 128, tile_n = pair ? 192 : deep && N >= 256 ? 256 : 128;
+  const int64_t slots = pair ? sms / 2 : sms;
   const int64_t tiles = ((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n);
   int splits = 1;
-  for (int s = 2; s <= 4 && tiles * 4 <= slots && K / 128 / s >= 32; s *= 2)
+  for (int s = 2; s <= 4 && tiles * (deep ? 4 : s) <= slots && (!deep || K / 128 / s >= 32); s *= 2)
     splits = s;
   return splits;
 }

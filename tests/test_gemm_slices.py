@@ -29,6 +29,15 @@ def test_slices_follow_from_the_shape(tokens, embd):
         assert workspace((*fc, *form), (*proj, *form), (*dx, capi.OUT_BF16, 0)) == sum(s for sizes in alone for s in sizes)
 
 
+@pytest.mark.parametrize("M,N,K,slices", [
+    (128, 1536, 6144, 4), (384, 1536, 6144, 4), (512, 1536, 6144, 2), (1024, 1536, 6144, 1), (128, 768, 3968, 1), (128, 768, 4096, 4),
+    (256, 256, 8064, 4), (256, 256, 8192, 2), (256, 256, 16384, 4), (768, 1152, 16384, 4), (768, 1280, 16384, 1), (128, 9472, 16384, 4),
+    (128, 9600, 16384, 1)])
+def test_slices_at_the_rules_lines(M, N, K, slices):
+    """On 148 SMs, by the workspace asked for."""
+    assert workspace((M, N, K, capi.OUT_BF16, 0)) == (M * N * 4 * slices if slices > 1 else 0)
+
+
 @pytest.mark.parametrize("M,N,K", [(256, 256, 64), (128, 128, 0), (0, 256, 8192), (-128, 256, 8192), (256, 256, -128)])
 def test_queries_take_any_shape(M, N, K):
     """A shape that no GEMM accepts needs no workspace; the refusal is the call's."""

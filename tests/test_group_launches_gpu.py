@@ -54,8 +54,8 @@ def gemm_group(problems):
     return need
 
 
-# tiles of 128 and 256 rows that are half empty, one 128-row matrix in a group, K of one tile beside a deep one and beside one
-# that is cut into slices (from 8192 on), lists of one to four (a fourth takes a launch of its own)
+# tiles of 128 and 256 rows that are half empty, one 128-row matrix in a group, K of one tile beside a K that is cut into
+# slices (from 4096 on), lists of one to four (a fourth takes a launch of its own)
 GROUPS = [
     [(128, 128, 128)],
     [(256, 384, 512), (640, 256, 128)],
