@@ -121,8 +121,8 @@ struct GemmParams {
   bool floor_rule;
 };
 
-// Up to kMaxGroup independent GEMMs share one launch of the CTA-pair kernel: their output tiles form one list of units,
-// the first GEMM's first. The backward of a Linear is two GEMMs (input and weight gradient) that often have fewer tiles
+// Up to kMaxGroup independent GEMMs share one launch of either kernel (the one-CTA kernel in its 128 x 128 form): their output
+// tiles form one list of units, the first GEMM's first. The backward of a Linear is two GEMMs (input and weight gradient) that often have fewer tiles
 // than the machine has CTA pairs, or a round and a bit; together they fill it, and one launch is saved.
 constexpr int kMaxGroup = 3;
 
@@ -1159,8 +1159,9 @@ __device__ __forceinline__ void pair_kernel_body(const LaunchArgs<kProblems>& ar
       };
       if constexpr (kFuse != kFuseNone) {
         // One set of accumulator registers, refilled as soon as a chunk's values are packed, and a rolled loop: with two
-        // sets and the chunks unrolled the compiler mixes their instructions and runs out of the 128 registers (350
-        // bytes of spills; 16384 x 6144 x 1536: forward 257 us, now 210, backward 312, now 207).
+        // sets and the chunks unrolled the compiler mixes their instructions and, at the 128 registers there are, spills
+        // (350 bytes per thread once the branch for K slices was gone). 16384 x 6144 x 1536 against the unrolled form with
+        // that branch: forward 173 -> 170 us, backward 221 -> 194 (the plain GEMM takes 130).
         uint32_t r[32];
         tmem_ld_32x32b_x32(acc_t + chunk_of(0) * 32, r);
         tmem_ld_wait(r);
@@ -1711,7 +1712,7 @@ int next_sched_slot() {
   return static_cast<int>(launch_seq.fetch_add(1, std::memory_order_relaxed) % kSchedLaunchSlots);
 }
 
-// n independent GEMMs, each with its slices; one launch of the CTA-pair kernel where the plan is for it (always with n > 1).
+// n independent GEMMs, each with its slices, in one launch of the kernel that the plan is for.
 template <int kProblems>
 int launch_gemms(const GemmDesc* g, int n, const TilePlan& plan, const DeviceInfo& dev, void* workspace,
                  size_t workspace_bytes, cudaStream_t s, const FusedOut& fused) {

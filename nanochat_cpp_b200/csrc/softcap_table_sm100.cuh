@@ -2,10 +2,10 @@
 //
 // tanh(z / softcap), and for the loss pass exp(softcap * tanh(z / softcap) - softcap), are functions of one bf16 value:
 // 65536 inputs at most, of which a chunk of logits meets a few thousand some 67 million times. A CTA therefore evaluates
-// them once per |z| in [2^-16, 2^7) into shared memory and then looks them up, with the bits of the direct evaluation
-// because the entries are made by it. A division, a tanhf and an expf are about 60 instructions; a lookup is 3 plus a
-// shared-memory read whose 32 random addresses take about 3.5 bank cycles. Values outside the range are evaluated
-// directly.
+// them once per |z| below 2^7, from 2^-16 on for the gradient's tanh and from 2^-25 on for the loss's terms, into shared memory
+// and then looks them up, with the bits of the direct evaluation because the entries are made by it. A division, a tanhf and
+// an expf are about 60 instructions; a lookup is 3 plus a shared-memory read whose 32 random addresses take about 3.5 bank
+// cycles. Values outside the range are evaluated directly.
 #pragma once
 
 #include <cstdint>

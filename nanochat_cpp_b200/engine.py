@@ -270,7 +270,7 @@ _workspaces: dict = {}
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
     """Split-K scratch, grown on demand and kept per (device, stream): split-K GEMMs on different streams may
-    overlap on the GPU and must not share partial tiles and counters, while launches on one stream are ordered
+    overlap on the GPU and must not share their K slices, while launches on one stream are ordered
     and reuse theirs (the reference's cuBLASLt path likewise borrows torch's per-stream workspace,
     src/nanochat/model/fp8/mx_gemm.cpp:236-237). A replaced tensor is handed back to the caching allocator, which
     keeps it for the stream it was allocated on until that stream's queued work has run."""
@@ -465,8 +465,8 @@ def relu_square_mlp_mx(N: int, cin: int, w_fc: torch.Tensor, w_proj: torch.Tenso
 def fp8_relu_square_mlp(x_2d: torch.Tensor, w_fc: torch.Tensor, w_proj: torch.Tensor,
                         fc_cache: Optional[Fp8WeightCache] = None, proj_cache: Optional[Fp8WeightCache] = None,
                         x_mx: Optional[Fp8Tensor] = None) -> torch.Tensor:
-    """The MLP's c_proj(relu(c_fc(x)).square()) with both matmuls as fp8_matmul, bit for bit
-    (src/nanochat/model/fp8/fp8.h:46-54). x_2d (N, in) bf16, w_fc (hidden, in), w_proj (out, hidden) -> (N, out).
+    """The MLP's c_proj(relu(c_fc(x)).square()) with both matmuls as fp8_matmul, bit for bit as long as in and out are below
+    4096, from where a GEMM may be cut into K slices but the fused ones are not (src/nanochat/model/fp8/fp8.h:46-54). x_2d (N, in) bf16, w_fc (hidden, in), w_proj (out, hidden) -> (N, out).
     x_mx: x_2d already quantized in both layouts (residual_norm_mx); x_2d then only carries autograd."""
     if x_mx is not None and (x_mx.data is None or x_mx.data_t is None):
         raise RuntimeError("fp8_relu_square_mlp: x_mx needs both layouts")
